@@ -978,7 +978,10 @@ class Model:
 
     def head(self, x: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
         """fp32 logits ``[R, vocab]`` (this rank's vocab shard gathered over TP)."""
-        h = self.final_hidden(x, rows)
+        return self.logits_of(self.final_hidden(x, rows))
+
+    def logits_of(self, h: torch.Tensor) -> torch.Tensor:
+        """fp32 logits of final-normed rows."""
         logits = self.ops.linear(self.lm_head, h, out_dtype=torch.float32)
         if self.tp.world > 1 and self.tp.group is not None:
             logits = self.tp.group.all_gather_cols(logits)
