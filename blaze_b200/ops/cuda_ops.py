@@ -757,11 +757,14 @@ class CudaOps:
         for lo, hi, count in tiers:
             nmax = 16
             rb = (hi + nmax - 1) // nmax
-            work = max(count, 1) * Hkv * rb
-            sp = splits if splits > 0 else (1 if work >= 3 * self._sm else max(1, min(8, tiles, (3 * self._sm) // max(work, 1))))
+            # Items for every CTA that fits at once (two per SM, one beyond 8 rows): whole items.  Fewer: their tiles shared out
+            # evenly, and the pieces merged by a second kernel.  Measured, whole / shared: 512 items 36 / 56 us (64 sequences, 8 rows),
+            # 392 items 39 / 38 us (49 sequences, 4 rows), 48 items 158 / 42 us (6 long ones).
+            items, most = B * Hkv * rb, (2 if hi <= 8 else 1) * self._sm
+            sp = splits if splits > 0 else 1 if max(count, 1) * Hkv * rb >= most else 1 + (most + items - 1) // items
             po = pm = None
             if sp > 1:
-                n = B * Hkv * rb * sp * nmax
+                n = (items + min(items * (sp - 1), 2 * self._sm)) * nmax
                 po = self._buf("attn_part_o", n * D * 4).view(torch.float32)
                 pm = self._buf("attn_part_ml", n * 2 * 4).view(torch.float32)
             self._check(self.lib.blz_attn_decode_tree(_ptr(q), _ptr(out), _ptr(kv.kv[layer_idx]), _ptr(kv.block_table),

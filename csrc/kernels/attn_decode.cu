@@ -5,13 +5,29 @@
 // problem is transposed:
 //     S^T = K Q^T   : A = K tile [128 tokens x D] (smem, straight from the page pool), B = Q [NMAX rows x D]
 //     O^T_t = V^T P^T : A = V^T tile [D x 128 tokens] (smem, from the pool), B = P [NMAX rows x 128 tokens]
-// so every softmax thread owns one key position and touches only NMAX (16 or 32) columns of tensor memory, and
-// every accumulate thread owns one output dimension with NMAX running sums in registers.  Row maxima are
+// so every softmax thread owns one key position and touches only RMAX (4, 8 or 16) columns of tensor memory, and
+// every accumulate thread owns one output dimension with RMAX running sums in registers.  Row maxima are
 // exchanged across the four softmax warps once per tile; row sums are reduced once per work item.
 //
-// Work item = (sequence, kv head, block of NMAX rows, kv split); persistent CTAs; 320 threads (page loader warp,
-// MMA warp, two sets of four softmax warps that take alternate tiles and are merged per work item like kv splits);
-// 2 CTAs per SM when at most 8 rows are live.  Every wait is a bounded mbarrier wait.
+// Work item = (sequence, kv head, block of NMAX rows); persistent CTAs; 320 threads (page loader warp, MMA warp, two sets
+// of four softmax warps that take alternate tiles and are merged per work item); 2 CTAs per SM when at most 8 rows are
+// live.  Every wait is a bounded mbarrier wait.
+//
+// Sharing out the work: with work for every CTA the items are taken whole, in turn.  With less (splits > 1) their 128-key tiles are
+// laid end to end and every CTA takes an equal run of them, found from the lengths on the device (a captured step sees other
+// lengths on every replay).  An item that a run's end cuts leaves partial sums (at most two pieces per CTA) that
+// attn_decode_combine_kernel merges.  Equal splits of every sequence, which this replaces, left the longest one's as the
+// tail: six sequences of 6 K to 16 K tokens took 57 us, now 42.
+//
+// What bounds it: the pages' bytes at 4 rows (85 % of copy bandwidth at 256 x 1.2 K tokens), the softmax warps at 8.  Their loops
+// run over all RMAX rows without a test of how many are live (a branch per row kept the rows' chains of maximum, exponential
+// and conversion from overlapping), tiles that no mask touches skip the masks, and what is done once per item is short: code
+// that runs once per item comes from beyond the instruction caches.  256 sequences of 1.2 K tokens, 8 kv heads of 4 rows:
+// 120 -> 113 us; 4 kv heads of 8 rows: 99 -> 77 us; 64 sequences, 8 kv heads of 8 rows: 52 -> 36 us; 16 sequences of 1.0 K to
+// 2.1 K tokens with 20 rows: 86 -> 59 us.
+// (Warp MMAs with the rows as M and probabilities in half precision need no word between warps until an item ends and took
+// 43 us there, but 189 instead of 113 us for 4 rows; and a token verified in one kernel and decoded in the other would see its
+// probabilities rounded differently.)
 //
 // Reference counterparts: kernels/src/cuda/mha_nvfp4.cu mha_decode_kernel :259 and mha_combine_kernel :572,
 // kernels/src/cuda/mha_verify.cu verify_kernel :50.
@@ -20,7 +36,7 @@
 
 namespace blz {
 
-// NMAX = MMA N (rows per work item, 16 or 32); RMAX = rows kept in registers by the softmax threads (>= live rows).
+// NMAX = MMA N (rows per work item); RMAX = rows kept in registers by the softmax threads (4, 8 or 16, >= live rows).
 template <int NMAX, int RMAX>
 struct DecCfg {
   static constexpr int D = 128;
@@ -32,22 +48,92 @@ struct DecCfg {
   static constexpr int Q_BYTES = NMAX * D;
   static constexpr int P_BYTES = NMAX * 128;
   static constexpr int NB = 3;                       // S^T / P / O^T buffers (softmax runs up to two tiles ahead of the fold)
-  static constexpr int TMEM_COLS = NMAX <= 16 ? 128 : 256;
+  static constexpr int TMEM_COLS = 128;
   static constexpr int SMEM = 2 * Q_BYTES + STAGES * 2 * TILE_BYTES + NB * P_BYTES + 128 + 640;
 };
 
-__device__ __forceinline__ bool timed_wait(long long& acc, bool on, uint64_t* bar, uint32_t par, volatile int* abort_flag,
+// The wait counters live in shared memory: thirteen 64-bit registers for a run that is not profiled would spill the others.
+__device__ __forceinline__ bool timed_wait(long long* acc, bool on, uint64_t* bar, uint32_t par, volatile int* abort_flag,
                                            int* status) {
   if (!on) return mbar_wait(bar, par, abort_flag, status);
   const long long t = clock64();
   const bool r = mbar_wait(bar, par, abort_flag, status);
-  acc += clock64() - t;
+  if ((threadIdx.x & 31) == 0) *acc += clock64() - t;
   return r;
+}
+
+// Tiles of 128 keys and row blocks of sequence b (no rows, or rows of another tier: none).
+template <int NMAX>
+__device__ __forceinline__ int seq_units(const AttnParams& p, int group, int b, int& tiles) {
+  const int rows = (p.q_start[b + 1] - p.q_start[b]) * group;
+  if (rows < p.min_rows || rows > p.max_rows || rows <= 0) { tiles = 0; return 0; }
+  tiles = (p.ctx_len[b] + 127) >> 7;
+  return min((rows + NMAX - 1) / NMAX, p.row_blocks) * p.Hkv;
+}
+
+constexpr int kMaxRuns = 1024;        // CTAs of one launch
+
+// Runs 0 .. i hold the first run_end(total, i, runs) tiles.
+__device__ __forceinline__ long long run_end(long long total, int i, int runs) { return total * (i + 1) / runs; }
+
+// The run of tiles of CTA `cta`, when the tiles of all items (sequence-major, then row block, then kv head) are laid end to end:
+// its length, and where it starts (sequence, item of the sequence, tile of the item) in `at`, for every thread.  `runs`: in, the
+// CTAs of the launch; out, the runs there are (one tile at least in each).  Called by all threads of a block.
+template <int NMAX>
+__device__ __forceinline__ int find_run(const AttnParams& p, int group, int cta, int& runs, int* at, long long& all) {
+  __shared__ int s_sum[33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int per = (p.num_items + blockDim.x - 1) / blockDim.x;
+  const int b0 = min((int)threadIdx.x * per, p.num_items), b1 = min(b0 + per, p.num_items);
+  int mine = 0, tiles;
+  for (int b = b0; b < b1; ++b) { const int u = seq_units<NMAX>(p, group, b, tiles); mine += u * tiles; }
+  int incl = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  int before = 0, total = 0;
+  for (int w = 0; w < nw; ++w) { if (w < warp) before += s_sum[w]; total += s_sum[w]; }
+  all = total;
+  runs = min(runs, max(total, 1));
+  if (cta >= runs) return 0;                             // the same for every thread
+  const int start = (int)run_end(total, cta - 1, runs), end = (int)run_end(total, cta, runs);
+  int left = start - (before + incl - mine);
+  if (left >= 0 && left < mine) {
+    for (int b = b0; b < b1; ++b) {
+      const int n = seq_units<NMAX>(p, group, b, tiles) * tiles;
+      if (left < n) { at[0] = b; at[1] = left / tiles; at[2] = left % tiles; break; }
+      left -= n;
+    }
+  }
+  __syncthreads();
+  return end - start;
+}
+
+// Sums of every row over the warp's lanes, R rows per lane: lane r gets row r's (r < R; a power of two, at most 32).  Each step
+// halves the rows a lane carries, so it takes R - 1 + log2(32 / R) exchanges instead of 5 R.
+template <int R>
+__device__ __forceinline__ float sum_rows(float (&v)[R], int lane) {
+#pragma unroll
+  for (int n = R / 2, bit = 1; n > 0; n >>= 1, bit <<= 1) {
+    const bool hi = lane & bit;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float give = hi ? v[2 * i] : v[2 * i + 1], keep = hi ? v[2 * i + 1] : v[2 * i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+    }
+  }
+#pragma unroll
+  for (int bit = R; bit < 32; bit <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+  return v[0];
 }
 
 template <int N>
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&r)[N]) {
-  if constexpr (N == 16) tmem_ld16(taddr, r); else tmem_ld32(taddr, r);
+  if constexpr (N == 4) tmem_ld4(taddr, r);
+  else if constexpr (N == 8) tmem_ld8(taddr, r);
+  else if constexpr (N == 16) tmem_ld16(taddr, r);
+  else tmem_ld32(taddr, r);
 }
 
 template <int NMAX, int RMAX>
@@ -78,12 +164,16 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
   uint64_t* acc_free = fin_bar + 1;        // [1] set 0 has consumed set 1's partial results
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  __shared__ float s_c[2][NMAX];
+  __shared__ __align__(16) float s_c[2][NMAX];
   __shared__ int s_pos[2][NMAX];
+  __shared__ int s_at[3];
+  __shared__ long long s_prof[3][13];
   __shared__ uint32_t s_mask[2][NMAX];   // tree verify: which of the sequence's new tokens a row may see (bit per token)
-  __shared__ float s_wmax[Cfg::NB][4][NMAX];
+  __shared__ __align__(16) float s_wmax[Cfg::NB][4][RMAX];
   __shared__ float s_l[2][4][RMAX];                  // [set][warp][row] partial row sums
-  __shared__ float s_m[RMAX];                        // set 1's row maxima
+  __shared__ float s_m[2][RMAX];                     // row maxima of the two sets
+  __shared__ float2 s_f[4][RMAX];                    // [warp of set 0][row]: what the two sets' sums are multiplied by
+  __shared__ int s_off[4][RMAX];                     // ... and the row (of the output, or of the piece) they go to
   __shared__ float s_acc[RMAX][128];                 // set 1's output sums
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -108,38 +198,56 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
   pdl_wait();          // the queries and this step's K/V rows come from the kernel before this one
 
   const int group = p.Hq / p.Hkv;
-  const int total = p.num_items * p.Hkv * p.row_blocks * p.splits;
   int g = 0, item_it = 0;
-  long long pc[13];
-#pragma unroll
-  for (int i = 0; i < 13; ++i) pc[i] = 0;
-  const long long t_start = clock64();
-#define TW(cat, bar, par) timed_wait(pc[cat], p.prof != nullptr, bar, par, abort_flag, p.status)
+  const bool prof = p.prof != nullptr && blockIdx.x < 8 && warp < 3;
+  long long* pc = s_prof[prof ? warp : 0];
+  if (prof && lane == 0) {
+    for (int i = 0; i < 12; ++i) pc[i] = 0;
+    pc[12] = -clock64();
+  }
+#define TW(cat, bar, par) timed_wait(&pc[cat], prof, bar, par, abort_flag, p.status)
 
-  for (int w = blockIdx.x; w < total; w += gridDim.x) {
-    const int split = w % p.splits;
-    const int rb = (w / p.splits) % p.row_blocks;
-    const int kh = (w / (p.splits * p.row_blocks)) % p.Hkv;
-    const int b = w / (p.splits * p.row_blocks * p.Hkv);
+  // whole items in turn (splits = 1), or this CTA's run of tiles
+  const int items_all = p.num_items * p.Hkv * p.row_blocks;
+  int left = 0, w = blockIdx.x, at_b = 0, at_u = 0, at_t = 0;
+  if (p.splits > 1) {
+    long long total;
+    int runs = gridDim.x;
+    left = find_run<NMAX>(p, group, blockIdx.x, runs, s_at, total);
+    at_b = s_at[0]; at_u = s_at[1]; at_t = s_at[2];
+  }
+  while (true) {
+    int b, u, t0 = 0, n, tiles_all, units;
+    if (p.splits > 1) {
+      if (left <= 0) break;
+      units = seq_units<NMAX>(p, group, at_b, tiles_all);
+      if (at_u >= units) { ++at_b; at_u = 0; continue; }
+      b = at_b; u = at_u; t0 = at_t;
+      n = min(tiles_all - t0, left);
+      left -= n; at_t = 0; ++at_u;
+    } else {
+      if (w >= items_all) break;
+      b = w / (p.row_blocks * p.Hkv); u = w % (p.row_blocks * p.Hkv);
+      w += gridDim.x;
+      units = seq_units<NMAX>(p, group, b, tiles_all);
+      if (u >= units) continue;
+      n = tiles_all;
+    }
+    const int kh = u % p.Hkv, rb = u / p.Hkv;
+    // where a cut item's partial sums go: what a run's end cuts off, then the items' last pieces
+    const int piece = n == tiles_all ? -1 : t0 + n < tiles_all ? (int)blockIdx.x : (int)gridDim.x + b * p.Hkv * p.row_blocks + u;
     const int r0 = p.q_start[b], qlen = p.q_start[b + 1] - r0;
     const int rows_total = qlen * group;
-    if (rows_total < p.min_rows || rows_total > p.max_rows) continue;
     const int row0 = rb * NMAX;
     const int nrows = min(NMAX, rows_total - row0);
-    if (nrows <= 0) continue;
     const int ctx = p.ctx_len[b];
-    const int kv_end = ctx - qlen + (row0 + nrows - 1) / group + 1;       // keys visible to the block's last row
-    const int tiles_all = (kv_end + 127) >> 7;
-    const int per = (tiles_all + p.splits - 1) / p.splits;
-    const int t0 = split * per;
-    const int n = max(min(tiles_all, t0 + per) - t0, 0);
     const int slot = p.slots[b];
 
     if (warp == 0) {
       // -------------------------------------------------------------- page loader
       const int* bt = p.block_table + (size_t)slot * p.bt_stride;
-      const int npages = (kv_end + 15) >> 4;
-      if (n > 0) {
+      const int npages = (ctx + 15) >> 4;
+      {
         // ---- this item's Q rows → e4m3 in the K-major core-matrix layout, plus the per-row constants
         // Items of at most 8 live rows (plain decode at group 4 or 8, two verify rows) are prepared by the K half of the
         // warp alone, 4 or 2 lanes per row: the two halves then never meet, and this half moves on to the next item's Q
@@ -203,7 +311,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
       // (the page number of the next tile is fetched before the wait for its ring slot, off the critical path)
       if (lane < 16) {
         int page = 0;
-        if (lane < 8 && n > 0) { const int pidx = t0 * 8 + lane; page = pidx < npages ? bt[pidx] : 0; }
+        if (lane < 8) { const int pidx = t0 * 8 + lane; page = pidx < npages ? bt[pidx] : 0; }
         for (int i = 0; i < n; ++i) {
           const int gi = g + i, s = gi % ST;
           int next = 0;
@@ -220,7 +328,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
         }
       } else {
         int page = 0;
-        if (lane < 24 && n > 0) { const int pidx = t0 * 8 + lane - 16; page = pidx < npages ? bt[pidx] : 0; }
+        if (lane < 24) { const int pidx = t0 * 8 + lane - 16; page = pidx < npages ? bt[pidx] : 0; }
         for (int i = 0; i < n; ++i) {
           const int gi = g + i, s = gi % ST;
           int next = 0;
@@ -240,7 +348,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
       if constexpr (RMAX > 8) __syncwarp();
     } else if (warp == 1) {
       // -------------------------------------------------------------- MMA issuer
-      if (lane == 0 && n > 0) {
+      if (lane == 0) {
         bool ok = TW(6, &q_full[item_it & 1], (item_it >> 1) & 1);
         tc_fence_after();
         const uint32_t q_addr = smem_u32(sQ + (item_it & 1) * Cfg::Q_BYTES);
@@ -290,74 +398,102 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
       for (int i = 0; i < RMAX; ++i) { m_run[i] = -INFINITY; l_part[i] = 0.f; acc[i] = 0.f; }
       bool ok = true;
       const int qb = item_it & 1;
-      if (n > 0 && !TW(6, &q_full[qb], (item_it >> 1) & 1)) break;     // per-row constants are published with Q
+      if (!TW(6, &q_full[qb], (item_it >> 1) & 1)) break;     // per-row constants are published with Q
       // add tile gj's O^T (relative to this set's row maxima at tile gj) to the running sums
       auto fold = [&](int gj) -> bool {
         const int ob = gj % NB;
         if (!TW(9, &o_full[ob], (gj / NB) & 1)) return false;
         tc_fence_after();
         // only the first RMAX columns hold live rows: a plain decode step reads 4 of the 16
-        constexpr int LDN = RMAX <= 4 ? 4 : NMAX;
-        uint32_t o[LDN];
-        if constexpr (RMAX <= 4) tmem_ld4(tmem + NB * NMAX + ob * NMAX + lane_bits, o);
-        else tmem_ldn<NMAX>(tmem + NB * NMAX + ob * NMAX + lane_bits, o);
+        uint32_t o[RMAX];
+        tmem_ldn<RMAX>(tmem + NB * NMAX + ob * NMAX + lane_bits, o);
         tmem_ld_wait();
-#pragma unroll
-        for (int r = 0; r < RMAX; ++r) {
-          if (r >= nrows) break;
-          acc[r] += __uint_as_float(o[r]);
-        }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&o_empty[ob]);
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) acc[r] += __uint_as_float(o[r]);
         return true;
       };
+      // All rows are computed, dead ones (beyond nrows: their Q rows are zero) too: nothing of them is written.
+      const int first_new = ctx - qlen;                  // keys before it are visible to every row
       int last = -1;
       for (int i = set; i < n && ok; i += 2) {
         const int gi = g + i, sb = gi % NB;
         if (!TW(7, &s_full[sb], (gi / NB) & 1)) { ok = false; break; }
         tc_fence_after();
-        constexpr int LDN = RMAX <= 4 ? 4 : NMAX;
-        uint32_t v[LDN];
-        if constexpr (RMAX <= 4) tmem_ld4(tmem + sb * NMAX + lane_bits, v);
-        else tmem_ldn<NMAX>(tmem + sb * NMAX + lane_bits, v);
+        uint32_t v[RMAX];
+        tmem_ldn<RMAX>(tmem + sb * NMAX + lane_bits, v);
         tmem_ld_wait();
-        const int key = (t0 + i) * 128 + t;
+        const int key0 = (t0 + i) * 128, key = key0 + t;
         float x[RMAX];
 #pragma unroll
-        for (int r = 0; r < RMAX; ++r) {
-          if (r >= nrows) break;
-          bool vis = key <= s_pos[qb][r];
-          if constexpr (RMAX > 4) {
-            // tree verify: among the sequence's own new tokens (keys from ctx - qlen on) a row sees its ancestors only
-            // (a word covers the first 32 new tokens; plain causal rows - no tree mask - may be longer and are not masked)
-            const int j = key - (ctx - qlen);
-            if (vis && p.tree_mask != nullptr && j >= 0 && j < 32) vis = (s_mask[qb][r] >> j) & 1u;
+        for (int r = 0; r < RMAX; r += 4) {
+          const float4 c = *reinterpret_cast<const float4*>(&s_c[qb][r]);
+          x[r] = __uint_as_float(v[r]) * c.x; x[r + 1] = __uint_as_float(v[r + 1]) * c.y;
+          x[r + 2] = __uint_as_float(v[r + 2]) * c.z; x[r + 3] = __uint_as_float(v[r + 3]) * c.w;
+        }
+        if (key0 + 127 >= first_new) {
+#pragma unroll
+          for (int r = 0; r < RMAX; ++r) {
+            bool vis = key <= s_pos[qb][r];
+            if constexpr (RMAX > 4) {
+              // tree verify: among the sequence's own new tokens (keys from ctx - qlen on) a row sees its ancestors only
+              // (a word covers the first 32 new tokens; plain causal rows - no tree mask - may be longer and are not masked)
+              const int j = key - first_new;
+              if (p.tree_mask != nullptr && j >= 0 && j < 32) vis = vis && ((s_mask[qb][r] >> j) & 1u);
+            }
+            if (!vis) x[r] = -INFINITY;
           }
-          x[r] = vis ? __uint_as_float(v[r]) * s_c[qb][r] : -INFINITY;
-          const float wm = warp_max_redux(x[r]);
-          if (lane == 0) s_wmax[sb][qd][r] = wm;
+        }
+        float wm[RMAX];
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) wm[r] = warp_max_redux(x[r]);
+        if (lane == 0) {
+#pragma unroll
+          for (int r = 0; r < RMAX; r += 4)
+            *reinterpret_cast<float4*>(&s_wmax[sb][qd][r]) = make_float4(wm[r], wm[r + 1], wm[r + 2], wm[r + 3]);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&wm_bar[sb]);
         // fold this set's previous tile while the other warps of the set catch up
         if (last >= 0 && !fold(last)) { ok = false; break; }
         if (!TW(8, &wm_bar[sb], (gi / NB) & 1)) { ok = false; break; }
+        // A row may see no key so far (an earlier chain row when the new tokens straddle a tile boundary): its maximum stays
+        // -inf, and 0 stands for it in the differences.
+        bool grew = false;
+#pragma unroll
+        for (int r = 0; r < RMAX; r += 4) {
+          float4 m4 = *reinterpret_cast<const float4*>(&s_wmax[sb][0][r]);
+#pragma unroll
+          for (int k = 1; k < 4; ++k) {
+            const float4 o4 = *reinterpret_cast<const float4*>(&s_wmax[sb][k][r]);
+            m4.x = fmaxf(m4.x, o4.x); m4.y = fmaxf(m4.y, o4.y); m4.z = fmaxf(m4.z, o4.z); m4.w = fmaxf(m4.w, o4.w);
+          }
+          wm[r] = m4.x; wm[r + 1] = m4.y; wm[r + 2] = m4.z; wm[r + 3] = m4.w;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) grew |= wm[r + k] > m_run[r + k];
+        }
+        if (grew) {                                      // the same in every warp of the set
+#pragma unroll
+          for (int r = 0; r < RMAX; ++r) {
+            const float m_new = fmaxf(m_run[r], wm[r]);
+            const float alpha = ex2(m_run[r] - (m_new == -INFINITY ? 0.f : m_new));     // ex2(-inf) = 0 on the first visible keys
+            l_part[r] *= alpha;
+            acc[r] *= alpha;
+            m_run[r] = m_new;
+          }
+        }
         uint8_t* pdst = sP + sb * Cfg::P_BYTES + (t >> 4) * 128 + (t & 15);
 #pragma unroll
-        for (int r = 0; r < RMAX; ++r) {
-          if (r >= nrows) break;
-          const float mt = fmaxf(fmaxf(s_wmax[sb][0][r], s_wmax[sb][1][r]), fmaxf(s_wmax[sb][2][r], s_wmax[sb][3][r]));
-          const float m_new = fmaxf(m_run[r], mt);
-          // A row may see no key of this tile (an earlier chain row when the new tokens straddle a tile boundary); if that
-          // is the first tile this warp set handles for the row, both maxima are -inf and their difference is not a number.
-          const bool none = m_new == -INFINITY;
-          const float alpha = none ? 1.f : ex2(m_run[r] - m_new);     // ex2(-inf) = 0 on the first tile with visible keys
-          const float pr = none ? 0.f : ex2(x[r] - m_new + 8.f);      // masked keys: ex2(-inf) = 0; P scaled by 2^8
-          l_part[r] = l_part[r] * alpha + pr;
-          acc[r] *= alpha;
-          m_run[r] = m_new;
-          pdst[(r >> 3) * 1024 + (r & 7) * 16] = (uint8_t)__nv_cvt_float_to_fp8(pr, __NV_SATFINITE, __NV_E4M3);
+        for (int r = 0; r < RMAX; r += 2) {
+          const float ma = m_run[r] == -INFINITY ? 0.f : m_run[r], mb = m_run[r + 1] == -INFINITY ? 0.f : m_run[r + 1];
+          const float pa = ex2(x[r] - ma + 8.f), pb = ex2(x[r + 1] - mb + 8.f);      // masked keys: ex2(-inf) = 0; P scaled by 2^8
+          l_part[r] += pa;
+          l_part[r + 1] += pb;
+          const uint32_t two = __nv_cvt_float2_to_fp8x2(make_float2(pa, pb), __NV_SATFINITE, __NV_E4M3);
+          pdst[(r >> 3) * 1024 + (r & 7) * 16] = (uint8_t)two;
+          pdst[(r >> 3) * 1024 + (r & 7) * 16 + 16] = (uint8_t)(two >> 8);
         }
         fence_async_smem();
         tc_fence_before();
@@ -368,63 +504,66 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
       if (ok && last >= 0) ok = fold(last);
       if (!ok) break;
       // ---- merge the two sets and the four warps of each: row sums, maxima, output sums
-      if (n > 0) {
-        // the exchange buffers are single: set 1 writes them only after set 0 has read the previous item's
-        if (set == 1 && !TW(11, acc_free, (item_it & 1) ^ 1)) break;
+      // the exchange buffers are single: set 1 writes them only after set 0 has read the previous item's
+      if (set == 1 && !TW(11, acc_free, (item_it & 1) ^ 1)) break;
+      const float ls = sum_rows<RMAX>(l_part, lane);
+      if (lane < RMAX) s_l[set][qd][lane] = ls;
+      if (t == 0) {
 #pragma unroll
-        for (int r = 0; r < RMAX; ++r) {
-          if (r >= nrows) break;
-          const float ws = warp_sum(l_part[r]);
-          if (lane == 0) s_l[set][qd][r] = ws;
-          if (set == 1) s_acc[r][t] = acc[r];
-          if (set == 1 && t == 0) s_m[r] = m_run[r];
+        for (int r = 0; r < RMAX; ++r) s_m[set][r] = m_run[r];
+      }
+      if (set == 1) {
+#pragma unroll
+        for (int r = 0; r < RMAX; ++r) s_acc[r][t] = acc[r];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(fin_bar);
+      if (!TW(11, fin_bar, item_it & 1)) break;
+      if (set == 0) {
+        // Lane r works out what row r needs, once per warp: the code per row and thread stays short.  (It runs once per item and
+        // does not stay in the instruction caches: divisions and exponentials unrolled per row took longer than the tiles.)
+        if (lane < RMAX) {
+          const int r = lane;
+          const float ma = s_m[0][r], mb = s_m[1][r];
+          const float m = fmaxf(ma, mb);
+          // (a set that saw no visible key of the row has maximum -inf and contributes nothing)
+          float fa = ma == -INFINITY ? 0.f : ex2(ma - m), fb = mb == -INFINITY ? 0.f : ex2(mb - m);
+          const float l = (s_l[0][0][r] + s_l[0][1][r] + s_l[0][2][r] + s_l[0][3][r]) * fa +
+                          (s_l[1][0][r] + s_l[1][1][r] + s_l[1][2][r] + s_l[1][3][r]) * fb;
+          if (piece < 0) {
+            const float inv = l > 0.f ? p.v_scale / l : 0.f;
+            fa *= inv;
+            fb *= inv;
+            const int tq = (row0 + r) / group;
+            s_off[qd][r] = (r0 + tq) * p.Hq + kh * group + (row0 + r - tq * group);
+          } else {
+            s_off[qd][r] = piece * NMAX + r;
+            if (qd == 0 && r < nrows) *reinterpret_cast<float2*>(&p.part_ml[((size_t)piece * NMAX + r) * 2]) = make_float2(m, l);
+          }
+          s_f[qd][r] = make_float2(fa, fb);
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(fin_bar);
-        if (!TW(11, fin_bar, item_it & 1)) break;
-        if (set == 0) {
 #pragma unroll
-          for (int r = 0; r < RMAX; ++r) {
-            if (r >= nrows) break;
-            const float mb = s_m[r];
-            const float m = fmaxf(m_run[r], mb);
-            // (a set that saw no visible key of the row has maximum -inf and contributes nothing)
-            const float fa = m_run[r] == -INFINITY ? 0.f : ex2(m_run[r] - m), fb = mb == -INFINITY ? 0.f : ex2(mb - m);
-            const float l = (s_l[0][0][r] + s_l[0][1][r] + s_l[0][2][r] + s_l[0][3][r]) * fa +
-                            (s_l[1][0][r] + s_l[1][1][r] + s_l[1][2][r] + s_l[1][3][r]) * fb;
-            const float o = acc[r] * fa + s_acc[r][t] * fb;
-            const int R = row0 + r;
-            const int tq = R / group, hq = kh * group + R % group;
-            if (p.splits == 1) {
-              p.out[((size_t)(r0 + tq) * p.Hq + hq) * D + t] = __float2bfloat16(l > 0.f ? o * p.v_scale / l : 0.f);
-            } else {
-              p.part_o[((size_t)w * NMAX + r) * D + t] = o;
-              if (t == 0) {
-                p.part_ml[((size_t)w * NMAX + r) * 2] = m;
-                p.part_ml[((size_t)w * NMAX + r) * 2 + 1] = l;
-              }
-            }
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acc_free);
-        }
-      } else if (set == 0 && p.splits > 1) {
-        for (int r = 0; r < nrows; ++r) {
-          p.part_o[((size_t)w * NMAX + r) * D + t] = 0.f;
-          if (t == 0) {
-            p.part_ml[((size_t)w * NMAX + r) * 2] = -INFINITY;
-            p.part_ml[((size_t)w * NMAX + r) * 2 + 1] = 0.f;
+        for (int r = 0; r < RMAX; ++r) {
+          const float2 f = s_f[qd][r];
+          const float o = acc[r] * f.x + s_acc[r][t] * f.y;
+          const size_t at = (size_t)s_off[qd][r] * D + t;
+          if (r < nrows) {
+            if (piece < 0) p.out[at] = __float2bfloat16(o);
+            else p.part_o[at] = o;
           }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_free);
       }
     }
     g += n;
-    if (n > 0) ++item_it;
+    ++item_it;
     if (*abort_flag) break;
   }
 #undef TW
-  if (p.prof && blockIdx.x < 8 && lane == 0 && warp < 3) {
-    pc[12] = clock64() - t_start;
+  if (prof && lane == 0) {
+    pc[12] += clock64();
     for (int i = 0; i < 13; ++i) p.prof[((size_t)blockIdx.x * 3 + warp) * 16 + i] = pc[i];
   }
   tc_fence_before();
@@ -435,65 +574,104 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
   }
 }
 
-// Merge kv-split partials of the decode kernel.  One CTA per (sequence, kv head, row block); thread = dimension.
+// Merge the pieces of the items that the runs' ends cut: one block per run, for the item that begins in this run and goes on
+// after it.  A warp per row; its lanes weigh the pieces side by side, then sum them up with loads that do not wait for one
+// another.
 template <int NMAX>
-__global__ void attn_decode_combine_kernel(AttnParams p) {
+__global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) {
   pdl_trigger();
   pdl_wait();
   constexpr int D = 128;
-  const int rb = blockIdx.x % p.row_blocks;
-  const int kh = (blockIdx.x / p.row_blocks) % p.Hkv;
-  const int b = blockIdx.x / (p.row_blocks * p.Hkv);
-  const int group = p.Hq / p.Hkv;
-  const int r0 = p.q_start[b], qlen = p.q_start[b + 1] - r0;
-  const int rows_total = qlen * group;
-  if (rows_total < p.min_rows || rows_total > p.max_rows) return;
-  const int row0 = rb * NMAX;
-  const int nrows = min(NMAX, rows_total - row0);
-  const int t = threadIdx.x;
-  for (int r = 0; r < nrows; ++r) {
-    float m = -INFINITY;
-    for (int s = 0; s < p.splits; ++s) {
-      const size_t w = (size_t)blockIdx.x * p.splits + s;
-      if (p.part_ml[(w * NMAX + r) * 2 + 1] > 0.f) m = fmaxf(m, p.part_ml[(w * NMAX + r) * 2]);
+  __shared__ int s_at[3];
+  const int group = p.Hq / p.Hkv, cta = blockIdx.x;
+  long long total;
+  int runs = gridDim.x;
+  const int left = find_run<NMAX>(p, group, cta, runs, s_at, total);
+  if (left <= 0) return;
+  // the item of the run's last tile, and where it begins, in tiles from the run's start
+  int b = s_at[0], u = s_at[1], begin = -s_at[2], tiles;
+  while (true) {
+    const int units = seq_units<NMAX>(p, group, b, tiles);
+    if (u >= units) { ++b; u = 0; continue; }
+    if (begin + tiles >= left) break;
+    begin += tiles;
+    ++u;
+  }
+  if (begin < 0 || begin + tiles == left) return;        // it began in an earlier run (whose block merges it), or ends here
+  // its pieces: the ends of this run and of the next ones up to the run in which it ends, and the beginning of that run
+  const long long item_end = run_end(total, cta - 1, runs) + begin + tiles;
+  int n = 2;
+  while (run_end(total, cta + n - 1, runs) < item_end) ++n;
+  const int r0 = p.q_start[b], kh = u % p.Hkv, row0 = u / p.Hkv * NMAX;
+  const int nrows = min(NMAX, (p.q_start[b + 1] - r0) * group - row0);
+  const int last = (int)gridDim.x + b * p.Hkv * p.row_blocks + u;
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < nrows; r += blockDim.x >> 5) {
+    auto at = [&](int i) { return (size_t)(i < n - 1 ? cta + i : last) * NMAX + r; };
+    auto max_sum = [&](int i) {
+      return i < n ? *reinterpret_cast<const float2*>(&p.part_ml[at(i) * 2]) : make_float2(-INFINITY, 0.f);
+    };
+    float m = -INFINITY, l = 0.f;
+    for (int i = lane; i < n; i += 32) { const float2 ml = max_sum(i); if (ml.y > 0.f) m = fmaxf(m, ml.x); }
+    m = warp_max(m);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const float2 ml = max_sum(i0 + lane);
+      const float mine = ml.y > 0.f ? exp2f(ml.x - m) : 0.f;
+      l += ml.y * mine;
+      const int here = min(32, n - i0);
+#pragma unroll 4
+      for (int i = 0; i < here; ++i) {
+        const float f = __shfl_sync(0xffffffffu, mine, i);
+        const float4 x = *reinterpret_cast<const float4*>(&p.part_o[at(i0 + i) * D + lane * 4]);
+        o.x += x.x * f; o.y += x.y * f; o.z += x.z * f; o.w += x.w * f;
+      }
     }
-    float l = 0.f, o = 0.f;
-    for (int s = 0; s < p.splits; ++s) {
-      const size_t w = (size_t)blockIdx.x * p.splits + s;
-      const float ls = p.part_ml[(w * NMAX + r) * 2 + 1];
-      if (!(ls > 0.f)) continue;
-      const float f = exp2f(p.part_ml[(w * NMAX + r) * 2] - m);
-      l += ls * f;
-      o += p.part_o[(w * NMAX + r) * D + t] * f;
-    }
-    const int R = row0 + r;
-    const int tq = R / group, hq = kh * group + R % group;
-    p.out[((size_t)(r0 + tq) * p.Hq + hq) * D + t] = __float2bfloat16(l > 0.f ? o * p.v_scale / l : 0.f);
+    l = warp_sum(l);
+    const float inv = l > 0.f ? p.v_scale / l : 0.f;
+    const int R = row0 + r, tq = R / group, hq = kh * group + R % group;
+    *reinterpret_cast<uint2*>(&p.out[((size_t)(r0 + tq) * p.Hq + hq) * D + lane * 4]) =
+        make_uint2(pack_bf16x2(o.x * inv, o.y * inv), pack_bf16x2(o.z * inv, o.w * inv));
   }
 }
 
-template <int NMAX, int RMAX>
-static cudaError_t launch_decode(const AttnParams& p, int max_ctas, cudaStream_t stream) {
-  using Cfg = DecCfg<NMAX, RMAX>;
-  static PerDeviceOnce configured;
-  {
-    cudaError_t e = configured.smem_limit(attn_decode_kernel<NMAX, RMAX>, Cfg::SMEM);
-    if (e != cudaSuccess) return e;
-  }
-  const int total = p.num_items * p.Hkv * p.row_blocks * p.splits;
-  const int cap = Cfg::CTAS_PER_SM * sm_count();
-  int grid = total < cap ? total : cap;
+// CTAs of a launch: what fits at once; with splits, a piece for every run and every item at most: (splits - 1) * items runs fit
+// scratch for splits * items pieces.
+static int decode_grid(const AttnParams& p, int ctas_per_sm, int max_ctas) {
+  const int items = p.num_items * p.Hkv * p.row_blocks;
+  const long long most = p.splits == 1 ? items : (long long)items * (p.splits - 1);
+  int grid = ctas_per_sm * sm_count();
+  if (grid > most) grid = (int)most;
+  if (grid > kMaxRuns) grid = kMaxRuns;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  cudaError_t e = launch_pdl(attn_decode_kernel<NMAX, RMAX>, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
+  return grid;
+}
+
+template <typename Cfg, typename K>
+static cudaError_t launch_form(K kernel, PerDeviceOnce& configured, const AttnParams& p, int max_ctas, cudaStream_t stream) {
+  cudaError_t e = configured.smem_limit(kernel, Cfg::SMEM);
+  if (e != cudaSuccess) return e;
+  const int grid = decode_grid(p, Cfg::CTAS_PER_SM, max_ctas);
+  e = launch_pdl(kernel, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
   if (e != cudaSuccess || p.splits == 1) return e;
-  return launch_pdl(attn_decode_combine_kernel<NMAX>, dim3(p.num_items * p.Hkv * p.row_blocks), dim3(128), 0, stream, p);
+  return launch_pdl(attn_decode_combine_kernel<16>, dim3(grid), dim3(512), 0, stream, p);
+}
+
+// The most rows of any work item choose the kernel (16 rows an item).  Draft trees need the mask that the 4-row one leaves out.
+static cudaError_t launch_decode(const AttnParams& p, int max_ctas, cudaStream_t stream) {
+  static PerDeviceOnce four, eight, sixteen;
+  if (p.max_rows <= 4 && !p.tree_mask) return launch_form<DecCfg<16, 4>>(attn_decode_kernel<16, 4>, four, p, max_ctas, stream);
+  if (p.max_rows <= 8) return launch_form<DecCfg<16, 8>>(attn_decode_kernel<16, 8>, eight, p, max_ctas, stream);
+  return launch_form<DecCfg<16, 16>>(attn_decode_kernel<16, 16>, sixteen, p, max_ctas, stream);
 }
 
 }  // namespace blz
 
 // Decode / verify attention for every sequence with min_rows <= q_len * (Hq / Hkv) <= max_rows.
-// nmax: 16 or 32 rows per work item; row_blocks = ceil(max rows of any processed sequence / nmax).
-// Scratch for splits > 1: part_o = B*Hkv*row_blocks*splits*nmax*128 floats, part_ml = ...*nmax*2 floats.
+// nmax: 16 or 32; row_blocks = ceil(max rows of any processed sequence / nmax).  (Work items have 16 rows either way.)
+// splits = 1: every item whole; more: the items' tiles shared out evenly over up to B*Hkv*row_blocks*(splits - 1) CTAs (no
+// more than are resident at once).  Scratch then: nmax*128 (part_o) and nmax*2 (part_ml) floats for each of B*Hkv*row_blocks
+// items and each of those CTAs; B*Hkv*row_blocks*splits of each are enough.
 // tree_mask (optional, [T] int32, indexed like q's rows): bit j of row i's word = row i may attend to the j-th new token
 // of its sequence (itself and its ancestors in a draft tree; at most 32 new tokens per sequence).  Null = causal rows.
 // Plain decode work items (at most 4 live rows per KV head) ignore it: a single new token sees only itself.
@@ -517,15 +695,11 @@ BLZ_API int blz_attn_decode_tree(const void* q, void* out, const void* pool, con
   p.item_seq = nullptr; p.item_q0 = nullptr; p.part_o = part_o; p.part_ml = part_ml;
   p.num_items = num_seqs; p.Hq = Hq; p.Hkv = Hkv; p.bt_stride = bt_stride; p.splits = splits;
   p.scale_log2 = scale * 1.4426950408889634f * k_scale; p.v_scale = v_scale;
-  p.tokens_per_block = 0; p.min_rows = min_rows; p.max_rows = max_rows; p.row_blocks = row_blocks;
+  p.tokens_per_block = 0; p.min_rows = min_rows; p.max_rows = max_rows; p.row_blocks = row_blocks * (nmax / 16);
   p.status = status_word();
   p.prof = prof;
   p.tree_mask = tree_mask;
-  if (nmax == 32) return (int)launch_decode<32, 32>(p, max_ctas, stream);
-  const int live = max_rows < 16 ? max_rows : 16;     // most live rows of any work item
-  if (live <= 4 && !tree_mask) return (int)launch_decode<16, 4>(p, max_ctas, stream);
-  if (live <= 8) return (int)launch_decode<16, 8>(p, max_ctas, stream);
-  return (int)launch_decode<16, 16>(p, max_ctas, stream);
+  return (int)launch_decode(p, max_ctas, stream);
 }
 
 BLZ_API int blz_attn_decode(const void* q, void* out, const void* pool, const int* block_table, const int* slots,
@@ -650,10 +824,7 @@ extern "C" __attribute__((visibility("default"))) int blz_attn_decode_noalloc(
   p.tokens_per_block = 0; p.min_rows = min_rows; p.max_rows = max_rows; p.row_blocks = row_blocks;
   p.status = d.status;
   p.prof = nullptr;
-  const int live = max_rows < 16 ? max_rows : 16;
-  if (live <= 4) e = launch_decode<16, 4>(p, max_ctas, stream);
-  else if (live <= 8) e = launch_decode<16, 8>(p, max_ctas, stream);
-  else e = launch_decode<16, 16>(p, max_ctas, stream);
+  e = launch_decode(p, max_ctas, stream);
   if (e != cudaSuccess) snprintf(g_noalloc_err, sizeof(g_noalloc_err), "launch failed: %s", cudaGetErrorString(e));
   return (int)e;
 }
