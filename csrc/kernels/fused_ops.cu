@@ -255,25 +255,32 @@ __device__ __forceinline__ uint32_t pack_e4m3x4_f(float a, float b, float c, flo
   return lo | (hi << 16);
 }
 
-// Quantise this thread's 8 elements [e0, e0+8) of row t.  Every lane of the warp must call it (shuffles); `valid` gates the stores.
+// Quantise this thread's 8 elements [e0, e0+8) of row t, neighbouring lanes holding neighbouring elements (a warp starts at a
+// multiple of 256).  Every lane of the warp must call it (shuffles); `valid` gates the stores.
+// These kernels move two bytes in for half a byte out, and what bounded them were a scale byte stored per 16 elements (a memory
+// sector each, as for a full one) and three divisions per 8 elements: four scales make one store (they are neighbours in the
+// 128x4 tiles; those of a row's padded columns are written as 0), the row's factor comes as a reciprocal.  8192 rows of 12288
+// activations: 101 -> 72 us.
 template <int QUANT>
 __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, int t, int e0, int W, float g, uint8_t* q_out,
                                              uint8_t* sf_out, int ct) {
   const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&packed);
+  const int lane = threadIdx.x & 31;
   float v[8];
   float bm = 0.f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) { v[j] = valid ? bf2f(e[j]) : 0.f; bm = fmaxf(bm, fabsf(v[j])); }
   bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
   if (QUANT == 1) {
-    const uint8_t sf = f2e4m3(bm / 6.f / g);
+    const uint8_t sf = f2e4m3(bm * __frcp_rn(6.f * g));
     const float denom = e4m32f(sf) * g;
-    const float inv = denom > 0.f ? 1.f / denom : 0.f;
+    const float inv = denom > 0.f ? __frcp_rn(denom) : 0.f;
     const uint32_t codes = pack_e2m1x8(v, inv);
-    if (valid) {
-      *reinterpret_cast<uint32_t*>(q_out + (size_t)t * (W / 2) + e0 / 2) = codes;
-      if ((e0 & 15) == 0) sf_out[sf_offset(t, e0 >> 4, ct)] = sf;
-    }
+    if (valid) *reinterpret_cast<uint32_t*>(q_out + (size_t)t * (W / 2) + e0 / 2) = codes;
+    uint32_t four = valid ? (uint32_t)sf << (8 * ((lane >> 1) & 3)) : 0u;
+    four |= __shfl_xor_sync(0xffffffffu, four, 2);
+    four |= __shfl_xor_sync(0xffffffffu, four, 4);
+    if (valid && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 4, ct)) = four;
   } else {
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
     bm = fmaxf(bm, 1.17549435e-38f);
@@ -284,8 +291,11 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
       *reinterpret_cast<uint2*>(q_out + (size_t)t * W + e0) =
           make_uint2(pack_e4m3x4_f(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv),
                      pack_e4m3x4_f(v[4] * inv, v[5] * inv, v[6] * inv, v[7] * inv));
-      if ((e0 & 31) == 0) sf_out[sf_offset(t, e0 >> 5, ct)] = (uint8_t)(ex + 127);
     }
+    uint32_t four = valid ? (uint32_t)(ex + 127) << (8 * ((lane >> 2) & 3)) : 0u;
+    four |= __shfl_xor_sync(0xffffffffu, four, 4);
+    four |= __shfl_xor_sync(0xffffffffu, four, 8);
+    if (valid && (lane & 15) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 5, ct)) = four;
   }
 }
 
@@ -359,10 +369,11 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
   }
 }
 
-template <int MODE, int CH>
+// ACT: the source rows are activations already (no up half): without its registers twice the rows are in flight per SM.
+template <int MODE, int CH, bool ACT>
 __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                                            uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
-                                                           float* __restrict__ row_scale, int I, int src_is_act, int sf_col_tiles,
+                                                           float* __restrict__ row_scale, int I, int sf_col_tiles,
                                                            const int* __restrict__ row_list) {
   pdl_trigger();
   pdl_wait();
@@ -370,16 +381,17 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
   // row_list (optional): the rows to process, one per CTA, -1 = none (routed expert rows in their padded row space)
   const int t = row_list ? row_list[blockIdx.x] : (int)blockIdx.x;
   if (t < 0) return;
-  const __nv_bfloat16* g = gu + (size_t)t * (src_is_act ? I : 2 * I);
+  const __nv_bfloat16* g = gu + (size_t)t * (ACT ? I : 2 * I);
   const __nv_bfloat16* up = g + I;
-  uint4 a[CH], b[CH];
+  uint4 a[CH], b[ACT ? 1 : CH];
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
-    a[c] = b[c] = make_uint4(0, 0, 0, 0);
+    a[c] = make_uint4(0, 0, 0, 0);
+    if constexpr (!ACT) b[c] = a[c];
     if (i < I) {
       a[c] = *reinterpret_cast<const uint4*>(g + i);
-      if (!src_is_act) b[c] = *reinterpret_cast<const uint4*>(up + i);
+      if constexpr (!ACT) b[c] = *reinterpret_cast<const uint4*>(up + i);
     }
   }
   float amax = 0.f;
@@ -387,8 +399,8 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
     __nv_bfloat16* eg = reinterpret_cast<__nv_bfloat16*>(&a[c]);
-    const __nv_bfloat16* eu = reinterpret_cast<const __nv_bfloat16*>(&b[c]);
-    if (!src_is_act) {
+    const __nv_bfloat16* eu = reinterpret_cast<const __nv_bfloat16*>(&b[ACT ? 0 : c]);
+    if constexpr (!ACT) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float x = bf2f(eg[j]);
@@ -613,21 +625,185 @@ __global__ void __launch_bounds__(512) attn_prep_kernel(const __nv_bfloat16* __r
   }
 }
 
-__global__ void mul_sigmoid_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    x[i] = __float2bfloat16(bf2f(x[i]) / (1.f + __expf(-bf2f(gate[i]))));
+// The same for head_dim 128 and 256 without the Hadamard rotation, 8 dims per lane: D / 8 lanes per head, so the rotary pairs and
+// norm weights of a lane's dims stay in registers for all heads, and a warp does two heads of 128 at once.
+// Values: one token's value is a byte in each of D 16-byte rows of its page (V is kept transposed), and a byte costs the memory
+// system what a sector does.  With `v_blocks`, a page that 16 consecutive tokens fill is written as whole rows by a block of its own
+// (one per 16 tokens behind the T token blocks, for the page that begins among them); the token blocks write the other values.
+// Measured on a B200, 8192 tokens, 32 + 2 x 8 heads of 128 (184 MB, 28 us at copy bandwidth): 117 us by head and token
+// (220 instructions per head and warp, byte stores of the values), now 64 us.
+template <int D>
+__global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
+                                 __nv_bfloat16* __restrict__ gate_out, uint8_t* __restrict__ kv_pool,
+                                 const int* __restrict__ positions, const int* __restrict__ slot_mapping,
+                                 const float* __restrict__ inv_freq, const __nv_bfloat16* __restrict__ q_norm_w,
+                                 const __nv_bfloat16* __restrict__ k_norm_w, int T, int Hq, int Hkv, int rot_dim,
+                                 float eps, float rope_scale, int gated, int zero_centered, float k_scale_inv,
+                                 float v_scale_inv, long long page_stride, long long head_stride, int v_blocks,
+                                 long long pos_stride, int mrope0, int mrope1) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int LPH = D / 8, HPW = 32 / LPH;          // lanes per head, heads per warp
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int qw = Hq * D * (gated ? 2 : 1);
+  const size_t row_w = (size_t)qw + 2 * (size_t)Hkv * D;
+  if ((int)blockIdx.x >= T) {
+    // ---- values of the page that tokens fill from one of t0 .. t0 + 15 on (there is one such page at most)
+    __shared__ int s_slot[31];
+    const int t0 = ((int)blockIdx.x - T) * 16;
+    if (threadIdx.x < 31) s_slot[threadIdx.x] = t0 + (int)threadIdx.x < T ? slot_mapping[t0 + threadIdx.x] : -1;
+    __syncthreads();
+    constexpr int VPL = D / 32;
+    for (int i = 0; i < 16; ++i) {
+      const int slot = s_slot[i];
+      if (slot < 0 || (slot & 15) != 0 || !__all_sync(0xffffffffu, s_slot[i + (lane & 15)] == slot + (lane & 15))) continue;
+      for (int h = warp; h < Hkv; h += nwarps) {
+        const __nv_bfloat16* src = qkv + (size_t)(t0 + i) * row_w + qw + (size_t)(Hkv + h) * D + lane * VPL;
+        uint8_t* dst = kv_pool + (size_t)(slot >> 4) * page_stride + (size_t)h * head_stride + 16 * D + lane * VPL * 16;
+        uint32_t word[VPL][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          __align__(16) __nv_bfloat16 raw[4][VPL];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if constexpr (VPL == 4) *reinterpret_cast<uint2*>(raw[j]) = *reinterpret_cast<const uint2*>(src + (size_t)(4 * k + j) * row_w);
+            else *reinterpret_cast<uint4*>(raw[j]) = *reinterpret_cast<const uint4*>(src + (size_t)(4 * k + j) * row_w);
+          }
+#pragma unroll
+          for (int d = 0; d < VPL; ++d)
+            word[d][k] = pack_e4m3x4_f(bf2f(raw[0][d]) * v_scale_inv, bf2f(raw[1][d]) * v_scale_inv, bf2f(raw[2][d]) * v_scale_inv,
+                                       bf2f(raw[3][d]) * v_scale_inv);
+        }
+#pragma unroll
+        for (int d = 0; d < VPL; ++d) *reinterpret_cast<uint4*>(dst + d * 16) = make_uint4(word[d][0], word[d][1], word[d][2], word[d][3]);
+      }
+      return;
+    }
+    return;
+  }
+  __shared__ float2 cs[D / 2];
+  const int t = blockIdx.x;
+  const int half = rot_dim / 2;
+  {
+    // M-RoPE as above
+    const float p0 = (float)positions[t];
+    const float p1 = pos_stride > 0 ? (float)positions[pos_stride + t] : p0;
+    const float p2 = pos_stride > 0 ? (float)positions[2 * pos_stride + t] : p0;
+    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+      const float pos = pos_stride > 0 ? (i < mrope0 ? p0 : (i < mrope1 ? p1 : p2)) : p0;
+      float s, c;
+      sincosf(pos * inv_freq[i], &s, &c);
+      cs[i] = make_float2(c * rope_scale, s * rope_scale);
+    }
+  }
+  const int sub = lane / LPH, i0 = (lane % LPH) * 8;  // the lane's head of the warp's, and its first dim
+  const int lanes_half = half / 8;                    // partner lane distance (power of two)
+  const bool turned = i0 < rot_dim;
+  const int slot = slot_mapping[t];
+  bool paged = false;                                 // a block of its own writes this token's values (same in all warps)
+  if (v_blocks && slot >= 0) {
+    const int first = t - (slot & 15), at = lane & 15;
+    if (first >= 0 && first + 15 < T) paged = __all_sync(0xffffffffu, slot_mapping[first + at] == (slot & ~15) + at);
+  }
+  const __nv_bfloat16* row = qkv + t * row_w;
+  uint4 wq = make_uint4(0, 0, 0, 0), wk = wq;
+  if (q_norm_w) wq = *reinterpret_cast<const uint4*>(q_norm_w + i0);
+  if (k_norm_w) wk = *reinterpret_cast<const uint4*>(k_norm_w + i0);
+  __syncthreads();
+  // a lane's dims all lie in the first half of the pairs, in the second, or beyond: x cos - y sin, or x cos + y sin
+  float2 rot[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    rot[j] = make_float2(1.f, 0.f);
+    if (turned) { rot[j] = cs[i0 < half ? i0 + j : i0 + j - half]; if (i0 < half) rot[j].y = -rot[j].y; }
+  }
+  const int heads = Hq + (paged ? Hkv : 2 * Hkv);
+  for (int h0 = warp * HPW; h0 < heads; h0 += nwarps * HPW) {
+    const int h = h0 + sub;
+    const bool is_q = h < Hq, is_v = h >= Hq + Hkv, live = h < heads && (is_q || slot >= 0);
+    const __nv_bfloat16* src = row + (is_q ? (size_t)h * D * (gated ? 2 : 1) : (size_t)qw + (size_t)(h - Hq) * D) + i0;
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    if (live) raw = *reinterpret_cast<const uint4*>(src);
+    const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    float v[8], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { v[j] = bf2f(e[j]); ss += v[j] * v[j]; }
+    if (live && is_q && gated)
+      *reinterpret_cast<uint4*>(gate_out + ((size_t)t * Hq + h) * D + i0) = *reinterpret_cast<const uint4*>(src + D);
+#pragma unroll
+    for (int o = 1; o < LPH; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (!is_v && (is_q ? q_norm_w != nullptr : k_norm_w != nullptr)) {
+      const float rstd = rsqrtf(ss / D + eps);
+      const uint4 w8 = is_q ? wq : wk;
+      const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(&w8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = bf2f(__float2bfloat16(v[j] * rstd * (bf2f(w[j]) + (zero_centered ? 1.f : 0.f))));
+    }
+    float o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float other = __shfl_xor_sync(0xffffffffu, v[j], lanes_half);
+      o[j] = is_v || !turned ? v[j] : v[j] * rot[j].x + other * rot[j].y;
+    }
+    if (!live) continue;                                // (no shuffle follows in this iteration)
+    if (is_q) {
+      *reinterpret_cast<uint4*>(q_out + ((size_t)t * Hq + h) * D + i0) =
+          make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+      continue;
+    }
+    uint8_t* blk = kv_pool + (size_t)(slot >> 4) * page_stride + (size_t)(is_v ? h - Hq - Hkv : h - Hq) * head_stride;
+    const int tp = slot & 15;
+    if (is_v) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) blk[16 * D + (i0 + j) * 16 + tp] = f2e4m3(o[j] * v_scale_inv);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = bf2f(__float2bfloat16(o[j])) * k_scale_inv;
+      // the lane's dims are half of a 16-byte core-matrix row
+      *reinterpret_cast<uint2*>(blk + (tp >> 3) * 8 * D + (i0 >> 4) * 128 + (tp & 7) * 16 + (i0 & 15)) =
+          make_uint2(pack_e4m3x4_f(o[0], o[1], o[2], o[3]), pack_e4m3x4_f(o[4], o[5], o[6], o[7]));
+    }
+  }
+}
+
+// Elementwise kernels on bf16, eight elements per thread and step where pointers and sizes allow 16-byte accesses (one element
+// per thread took 80 us for a sum of 8192 x 4096, now 40; the bytes take 31 at copy bandwidth).
+template <typename F>
+__device__ __forceinline__ uint4 each8(const uint4& a, const uint4& b, F f) {
+  uint4 o;
+  const __nv_bfloat16 *x = reinterpret_cast<const __nv_bfloat16*>(&a), *y = reinterpret_cast<const __nv_bfloat16*>(&b);
+  __nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(&o);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) z[j] = __float2bfloat16(f(bf2f(x[j]), bf2f(y[j])));
+  return o;
+}
+__device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+// out[i] = f(a[i], b[i]) for i < n (out may be a)
+template <typename F>
+__device__ __forceinline__ void each(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, size_t n, size_t first, size_t step, F f) {
+  size_t done = 0;
+  if (aligned16(a, b, out)) {
+    for (size_t i = first; i < n / 8; i += step)
+      reinterpret_cast<uint4*>(out)[i] = each8(reinterpret_cast<const uint4*>(a)[i], reinterpret_cast<const uint4*>(b)[i], f);
+    done = n / 8 * 8;
+  }
+  for (size_t i = done + first; i < n; i += step) out[i] = __float2bfloat16(f(bf2f(a[i]), bf2f(b[i])));
+}
+__global__ void mul_sigmoid_kernel(__nv_bfloat16* x, const __nv_bfloat16* gate, size_t n) {
+  each(x, gate, x, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x,
+       [](float v, float g) { return v / (1.f + __expf(-g)); });
 }
 __global__ void add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16(bf2f(a[i]) + bf2f(b[i]));
+  each(a, b, out, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, [](float x, float y) { return x + y; });
 }
 // out[t, :] = a[t, :] + b[t, :] * bf16(sigmoid(gate_logit[t]))
 __global__ void add_sigmoid_scaled_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, const __nv_bfloat16* gl,
                                           __nv_bfloat16* out, int H) {
-  const int t = blockIdx.x;
-  const float s = bf2f(__float2bfloat16(1.f / (1.f + __expf(-bf2f(gl[t])))));
-  for (int i = threadIdx.x; i < H; i += blockDim.x)
-    out[(size_t)t * H + i] = __float2bfloat16(bf2f(a[(size_t)t * H + i]) + bf2f(b[(size_t)t * H + i]) * s);
+  const size_t row = (size_t)blockIdx.x * H;
+  const float s = bf2f(__float2bfloat16(1.f / (1.f + __expf(-bf2f(gl[blockIdx.x])))));
+  each(a + row, b + row, out + row, H, threadIdx.x, blockDim.x, [s](float x, float y) { return x + y * s; });
 }
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ rows,
                                    __nv_bfloat16* __restrict__ out, int H) {
@@ -811,12 +987,14 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   int rt, ch;
   reg_shape(I, T, &rt, &ch);
   if (ch) {
-#define BLZ_SW(C)                                                                                                              \
-  if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, src_is_act, 0, row_list); \
-  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list); \
-  else launch_pdl(swiglu_reg_kernel<2, C>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list)
+#define BLZ_SW2(C, ACT)                                                                                                        \
+  if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
+  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list); \
+  else launch_pdl(swiglu_reg_kernel<2, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
+#define BLZ_SW(C) if (src_is_act) { BLZ_SW2(C, true); } else { BLZ_SW2(C, false); }
     BLZ_CH_SWITCH(ch, BLZ_SW)
 #undef BLZ_SW
+#undef BLZ_SW2
     return (int)cudaGetLastError();
   }
   if (mode == 0) swiglu_kernel<0><<<T, thr, 0, s>>>((const bf16*)gu, (bf16*)out, nullptr, nullptr, nullptr, I, src_is_act, 0, row_list);
@@ -838,6 +1016,25 @@ BLZ_API int blz_attn_prep(const void* qkv, void* q_out, void* gate_out, void* kv
   int wpb = (Hq + 2 * Hkv) >= 8 ? 8 : (Hq + 2 * Hkv);
   { static int wide = -1; if (wide < 0) { const char* e = getenv("BLAZE_ROW_THREADS"); wide = (e && atoi(e) == 256) ? 0 : 1; }
     if (wide && T <= 1024 && (Hq + 2 * Hkv) >= 16) wpb = 16; }
+  // 8 dims per lane: head_dim 128 and 256, no rotation, the rotated pairs a whole number of lanes apart, rows on 16 bytes
+  const bool on16 = !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(gate_out) |
+                       reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w) | reinterpret_cast<uintptr_t>(kv_pool)) & 15);
+  if (D != 64 && !rotate && half % 8 == 0 && half > 0 && on16 && page_stride % 16 == 0 && head_stride % 16 == 0) {
+    // Values in blocks of their own from 64 tokens on (fewer: hardly a page is filled).  Few tokens take a warp for every pass over
+    // the heads, so that nothing waits in turn; many keep blocks of four warps.
+    const int v_blocks = T >= 64 ? (T + 15) / 16 : 0, hpw = 256 / D;
+    const int passes = (Hq + 2 * Hkv + hpw - 1) / hpw;
+    const int warps = T > 1024 ? 4 : passes < 4 ? 4 : passes > 16 ? 16 : passes;
+#define BLZ_PREP(DD)                                                                                                 \
+  launch_pdl(attn_prep_heads_kernel<DD>, dim3(T + v_blocks), dim3(warps * 32), 0, s, (const bf16*)qkv, (bf16*)q_out,     \
+             (bf16*)gate_out, (uint8_t*)kv_pool, positions, slot_mapping, inv_freq, (const bf16*)q_norm_w,              \
+             (const bf16*)k_norm_w, T, Hq, Hkv, rot_dim, eps, rope_scale, gated, zero_centered, 1.f / k_scale,          \
+             1.f / v_scale, page_stride > 0 ? page_stride : (long long)Hkv * 2 * 16 * D,                                \
+             head_stride > 0 ? head_stride : (long long)2 * 16 * D, v_blocks, pos_stride, mrope0, mrope1)
+    if (D == 128) BLZ_PREP(128); else BLZ_PREP(256);
+#undef BLZ_PREP
+    return (int)cudaGetLastError();
+  }
   const int grid = T;
 #define BLZ_PREP(DD)                                                                                                 \
   launch_pdl(attn_prep_kernel<DD>, dim3(grid), dim3(wpb * 32), 0, s, (const bf16*)qkv, (bf16*)q_out, (bf16*)gate_out,  \
