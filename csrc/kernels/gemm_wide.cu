@@ -364,30 +364,37 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
             }
           } else if (p.act) {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)tok * p.ldc + c0 / 2;
+            // The gated activation's exponentials and divisions keep the eight warps busy about as long as the tensor pipe has work
+            // for the next tile: the division is the approximate one (2 ulp of 32 bits, before the rounding to bf16), and the
+            // activation is told apart outside of the loop.  8192 x 24576 x 4096, NVFP4: 525 -> 427 us.
+            auto gated = [&](auto act) {
 #pragma unroll
-            for (int gq = 0; gq < CPT; gq += 32) {
-              uint32_t pk[8];
+              for (int gq = 0; gq < CPT; gq += 32) {
+                uint32_t pk[8];
 #pragma unroll
-              for (int i = 0; i < 16; i += 2) {
-                float a[2];
+                for (int i = 0; i < 16; i += 2) {
+                  float a[2];
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                  const int cg = half * CPT + gq + i + j, cu = cg + 16;
-                  const float gf = fmaf(__uint_as_float(r[gq + i + j]) * ls, s_cs[cg], s_cb[cg]);
-                  const float uf = fmaf(__uint_as_float(r[gq + 16 + i + j]) * ls, s_cs[cu], s_cb[cu]);
-                  if (p.act == 2) {
-                    a[j] = clamped_glu_fast(gf, uf, p.act_limit);
-                  } else {
-                    const float g = bf2f(__float2bfloat16(gf)), u = bf2f(__float2bfloat16(uf));
-                    a[j] = g / (1.f + __expf(-g)) * u;
+                  for (int j = 0; j < 2; ++j) {
+                    const int cg = half * CPT + gq + i + j, cu = cg + 16;
+                    a[j] = act(fmaf(__uint_as_float(r[gq + i + j]) * ls, s_cs[cg], s_cb[cg]),
+                               fmaf(__uint_as_float(r[gq + 16 + i + j]) * ls, s_cs[cu], s_cb[cu]));
                   }
+                  pk[i / 2] = pack_bf16x2(a[0], a[1]);
                 }
-                pk[i / 2] = pack_bf16x2(a[0], a[1]);
+                if (c0 + gq + 32 <= p.cols_total) {
+                  *reinterpret_cast<uint4*>(dst + gq / 2) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                  *reinterpret_cast<uint4*>(dst + gq / 2 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+                }
               }
-              if (c0 + gq + 32 <= p.cols_total) {
-                *reinterpret_cast<uint4*>(dst + gq / 2) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-                *reinterpret_cast<uint4*>(dst + gq / 2 + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-              }
+            };
+            if (p.act == 2) {
+              gated([&](float gf, float uf) { return clamped_glu_fast(gf, uf, p.act_limit); });
+            } else {
+              gated([](float gf, float uf) {
+                const float g = bf2f(__float2bfloat16(gf)), u = bf2f(__float2bfloat16(uf));
+                return __fdividef(g, 1.f + __expf(-g)) * u;
+              });
             }
           } else {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)tok * p.ldc + c0;
