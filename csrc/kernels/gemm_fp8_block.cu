@@ -205,6 +205,255 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
+// The same product for at most 64 rows (decoding): features on the MMA's 128 lanes, the rows, rounded up to 32, on its columns, so
+// that a k block costs 16 KB of weights and 8 of activations, and half the tensor and promotion time.  A small layer has few
+// feature tiles (40 of the 148 SMs worked on 5120 x 8192): the K range is split over a cluster of `ks` CTAs, whose fp32 sums meet
+// in distributed shared memory; CTA r owns row-column groups [r * ng / ks, (r + 1) * ng / ks) and adds the parts in rank order.
+// 192 threads (producer, MMA issuer, four promotion warps: lane = feature, column = row of X), two CTAs per SM.  A k block's 64
+// activation scales ride behind the operands in a ring of eight: they outlive the operand stage (the promotion is at most four
+// blocks behind the MMA, the producer at most four ahead of it).  Weight bytes bound it.
+// Measured, us, this kernel / the one above: 16 rows 10240 x 5120 18.8 / 18.5, 5120 x 8192 17.5 / 24.4, 51200 x 5120 57 / 64, 5120 x
+// 25600 34 / 76; 64 rows 25.1 / 18.5, 22.4 / 24.4, 71 / 64, 45 / 76: beyond 32 rows it is taken for layers of few tiles only.
+struct FrCfg {
+  static constexpr int W_BYTES = 128 * 128, X_BYTES = 64 * 128, STAGES = 4;
+  static constexpr int NBUF = 4, TMEM_COLS = NBUF * 64;
+  static constexpr int SA_SLOTS = 8, SA_BYTES = 64 * 4;
+  static constexpr int RING = STAGES * (W_BYTES + X_BYTES);
+  static constexpr int SMEM = RING + SA_SLOTS * SA_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int GROUP = 8;                      // row columns that change hands together in the reduction
+  static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
+  static_assert(STAGES + NBUF <= SA_SLOTS, "a scale slot is read before it is filled again");
+};
+
+__global__ void __launch_bounds__(192, 2)
+gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, FbParams p, int ks) {
+  using Cfg = FrCfg;
+  constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, GW = Cfg::GROUP;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sW = smem;
+  uint8_t* sX = sW + STAGES * Cfg::W_BYTES;
+  float* sSA = reinterpret_cast<float*>(smem + Cfg::RING);            // [SA_SLOTS][64]
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::RING + Cfg::SA_SLOTS * Cfg::SA_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* part_full = empty + STAGES;    // [NBUF] a k block's products are complete in TMEM buffer b
+  uint64_t* part_empty = part_full + NBUF; // [NBUF] the promotion warps have read it (4 arrivals)
+  uint64_t* sa_full = part_empty + NBUF;   // [SA_SLOTS]
+  uint64_t* ring_free = sa_full + Cfg::SA_SLOTS;       // every CTA of the cluster has finished its main loop (ks remote arrivals)
+  uint64_t* part_ready = ring_free + 1;    // every CTA of the cluster has parked its sums here
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part_ready + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kr = ks > 1 ? (int)cluster_ctarank() : 0;
+  const int nt = blockIdx.x / ks;
+  const int nkb_all = p.K / 128;
+  const int kb0 = (int)((long long)kr * nkb_all / ks), nkb = (int)((long long)(kr + 1) * nkb_all / ks) - kb0;      // >= 1: ks <= nkb_all
+  const int ncols = (p.M + 31) & ~31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < NBUF; ++i) { mbar_init(&part_full[i], 1); mbar_init(&part_empty[i], 4); }
+    for (int i = 0; i < Cfg::SA_SLOTS; ++i) mbar_init(&sa_full[i], 1);
+    mbar_init(ring_free, ks);
+    mbar_init(part_ready, ks);
+    *abort_flag = 0;
+    mbar_fence_init();
+    prefetch_tmap(&tmW);
+    prefetch_tmap(&tmX);
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  pdl_trigger();
+  if (ks > 1) cluster_arrive();            // the peers' barriers are initialised before anyone arrives on them remotely
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int pre = min(STAGES, nkb);
+      const uint32_t sa_bytes = (uint32_t)((p.M + 3) & ~3) * 4u;
+      auto weights = [&](int s, int i) {
+        mbar_expect_tx(&full[s], Cfg::W_BYTES + (uint32_t)ncols * 128u);
+        tma_load_2d(sW + s * Cfg::W_BYTES, &tmW, (kb0 + i) * 128, nt * 128, &full[s]);
+      };
+      for (int i = 0; i < pre; ++i) weights(i, i);     // they do not depend on the kernel before this one
+      pdl_wait();
+      int s = 0; uint32_t ph = 0;
+      for (int i = 0; i < nkb; ++i) {
+        if (i >= pre) {
+          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) break;
+          weights(s, i);
+        }
+        for (int c = 0; c < ncols; c += 32) tma_load_2d(sX + s * Cfg::X_BYTES + c * 128, &tmX, (kb0 + i) * 128, c, &full[s]);
+        const int slot = i % Cfg::SA_SLOTS;
+        mbar_expect_tx(&sa_full[slot], sa_bytes);
+        bulk_load(sSA + slot * 64, p.sa + (size_t)(kb0 + i) * p.ld_sa, sa_bytes, &sa_full[slot]);
+        if (++s == STAGES) { s = 0; ph ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      int s = 0; uint32_t ph = 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int b = i % NBUF;
+        if (i >= NBUF && !mbar_wait(&part_empty[b], (uint32_t)((i / NBUF - 1) & 1), abort_flag, p.status)) break;
+        if (!mbar_wait(&full[s], ph, abort_flag, p.status)) break;
+        tc_fence_after();
+        const uint32_t w_addr = smem_u32(sW + s * Cfg::W_BYTES), x_addr = smem_u32(sX + s * Cfg::X_BYTES);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          mma_f8(tmem + b * 64, desc_sw128(w_addr + j * 32), desc_sw128(x_addr + j * 32), make_idesc(0, 0, 128, ncols), j > 0 ? 1u : 0u);
+        mma_commit(&empty[s]);
+        mma_commit(&part_full[b]);
+        if (++s == STAGES) { s = 0; ph ^= 1; }
+      }
+    }
+  }
+  __syncwarp();
+  if (ks > 1) cluster_wait();              // all threads, unconditionally (pairs with cluster_arrive above)
+  if (warp >= 2) {
+    const int q = warp & 3, fl = q * 32 + lane, f = nt * 128 + fl;
+    float acc[64];
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+    const float* sb = p.sb + (size_t)nt * nkb_all + kb0;
+    bool ok = true;
+    float sb_next = __ldg(sb);
+#pragma unroll 1
+    for (int i = 0; i < nkb; ++i) {
+      const int b = i % NBUF, slot = i % Cfg::SA_SLOTS;
+      const float sbv = sb_next;
+      if (i + 1 < nkb) sb_next = __ldg(sb + i + 1);
+      // tcgen05.ld is warp-collective: the outcome of the waits is made warp-uniform before any lane loads
+      ok = __all_sync(0xffffffffu, mbar_wait(&sa_full[slot], (uint32_t)((i / Cfg::SA_SLOTS) & 1), abort_flag, p.status) &&
+                                       mbar_wait(&part_full[b], (uint32_t)((i / NBUF) & 1), abort_flag, p.status));
+      if (!ok) break;
+      tc_fence_after();
+      const float4* sa = reinterpret_cast<const float4*>(sSA + slot * 64);
+      const uint32_t t0 = tmem + b * 64 + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h * 32 >= ncols) break;
+        uint32_t r[32];
+        tmem_ld32(t0 + h * 32, r);
+        tmem_ld_wait();
+        if ((h + 1) * 32 >= ncols) {       // the products are in registers: hand the buffer back
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&part_empty[b]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 s4 = sa[h * 8 + j];
+          float* a = acc + h * 32 + j * 4;
+          a[0] = fmaf(__uint_as_float(r[4 * j]), s4.x * sbv, a[0]);
+          a[1] = fmaf(__uint_as_float(r[4 * j + 1]), s4.y * sbv, a[1]);
+          a[2] = fmaf(__uint_as_float(r[4 * j + 2]), s4.z * sbv, a[2]);
+          a[3] = fmaf(__uint_as_float(r[4 * j + 3]), s4.w * sbv, a[3]);
+        }
+      }
+    }
+    const float bias = p.bias && f < p.N ? bf2f(p.bias[f]) : 0.f;
+    auto store = [&](int row, float v) {
+      if (row >= p.M || f >= p.N) return;
+      if (p.out_f32) reinterpret_cast<float*>(p.C)[(size_t)row * p.ldc + f] = v + bias;
+      else reinterpret_cast<__nv_bfloat16*>(p.C)[(size_t)row * p.ldc + f] = __float2bfloat16(v + bias);
+    };
+    if (ks == 1) {
+      if (ok) {
+#pragma unroll
+        for (int j = 0; j < 64; ++j) store(j, acc[j]);
+      }
+    } else {
+      const int ng = ncols / GW, GL = (ng + ks - 1) / ks;
+      const uint32_t recv = smem_u32(smem);            // slot [source CTA][group][column quad][feature], over the operand ring
+      if (threadIdx.x == 64) {
+        for (int r = 0; r < ks; ++r) mbar_arrive_remote(mapa_shared(smem_u32(ring_free), r));
+      }
+      // an aborted CTA still arrives and still waits, so that its peers are not left waiting for it
+      const bool free_all = __all_sync(0xffffffffu, mbar_wait_cluster(ring_free, 0, abort_flag, p.status));
+      if (ok && free_all) {
+#pragma unroll
+        for (int cq = 0; cq < 16; ++cq) {
+          if (cq * 4 >= ncols) break;
+          const int g = cq / 2, owner = (g * ks + ks - 1) / ng, gl = g - owner * ng / ks;       // owner * ng / ks <= g
+          st_dsmem_f4(mapa_shared(recv + (uint32_t)(((kr * GL + gl) * 2 + (cq & 1)) * 128 + fl) * 16u, owner), acc[4 * cq], acc[4 * cq + 1],
+                      acc[4 * cq + 2], acc[4 * cq + 3]);
+        }
+      }
+      fence_acq_rel_cluster();
+      bar_sync(1, 128);
+      if (threadIdx.x == 64) {
+        for (int r = 0; r < ks; ++r) mbar_arrive_remote(mapa_shared(smem_u32(part_ready), r));
+      }
+      const bool all = __all_sync(0xffffffffu, mbar_wait_cluster(part_ready, 0, abort_flag, p.status));
+      if (all && ok && free_all && !*abort_flag) {
+        const float4* got = reinterpret_cast<const float4*>(smem);
+        const int g0 = kr * ng / ks, g1 = (kr + 1) * ng / ks;
+        for (int cq = g0 * 2; cq < g1 * 2; ++cq) {
+          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int r = 0; r < ks; ++r) {               // rank order: the sum does not depend on timing
+            const float4 x = got[((r * GL + (cq / 2 - g0)) * 2 + (cq & 1)) * 128 + fl];
+            v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+          }
+          store(cq * 4, v.x); store(cq * 4 + 1, v.y); store(cq * 4 + 2, v.z); store(cq * 4 + 3, v.w);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, Cfg::TMEM_COLS);
+  }
+}
+
+// CTAs that share a feature tile: powers of two (odd clusters pack badly), both slots of every SM at most, a group of columns each.
+static int fp8_rows_ks(const FbParams& p) {
+  const int tiles = (p.N + 127) / 128, nkb = p.K / 128, ng = ((p.M + 31) & ~31) / FrCfg::GROUP;
+  int ks = 1;
+  while (ks * 2 <= ng && ks * 2 <= nkb && tiles * ks * 2 <= 2 * sm_count()) ks *= 2;
+  return ks;
+}
+
+static cudaError_t launch_fp8_rows(const FbParams& p, const void* A, long long lda, const void* B, long long ldb, cudaStream_t stream) {
+  const int tiles = (p.N + 127) / 128, ks = fp8_rows_ks(p);
+  CUtensorMap tmW, tmX;
+  cudaError_t e = encode_tmap(&tmW, B, 1, (uint64_t)p.K, p.N, ldb, 128, 128, 3);
+  if (e != cudaSuccess) return e;
+  e = encode_tmap(&tmX, A, 1, (uint64_t)p.K, p.M, lda, 128, 32, 3);
+  if (e != cudaSuccess) return e;
+  static PerDeviceOnce configured;
+  e = configured.smem_limit(gemm_fp8_rows_kernel, FrCfg::SMEM);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles * ks));
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = FrCfg::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (ks > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = ks;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, gemm_fp8_rows_kernel, tmW, tmX, p, ks);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
 // Activation quantiser: bf16 [T, K] -> e4m3 [T, K] with one fp32 scale per (row, 128-column group), scale = amax / 448,
 // written k-block-major ([K / 128, ld_s]) so that the GEMM's promotion warps read them coalesced.  One warp per group.
 __global__ void __launch_bounds__(256)
@@ -246,6 +495,9 @@ BLZ_API int blz_gemm_fp8_block(const void* A, long long lda, const void* B, long
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_f32 = out_f32;
   p.sa = sa; p.ld_sa = ld_sa; p.sb = sb; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.status = status_word();
+  // the scales' rows are copied by 16 bytes: they start and step on them (blz_quant_fp8_block's do)
+  if (M <= 64 && ld_sa % 4 == 0 && (reinterpret_cast<uintptr_t>(sa) & 15) == 0 && (M <= 32 || fp8_rows_ks(p) >= 4))
+    return (int)launch_fp8_rows(p, A, lda, B, ldb, stream);
   CUtensorMap tmA, tmB;
   cudaError_t e = encode_tmap(&tmA, A, 1, (uint64_t)K, M, lda, 128, 128, 3);
   if (e != cudaSuccess) return (int)e;
