@@ -34,3 +34,47 @@ def test_fp8_block_product_of_few_rows(ops, M, N, K):      # noqa: F811
     xd = (q.view(torch.float8_e4m3fn).double().view(M, K // 128, 128) * sc[:, :M].t().double().unsqueeze(-1)).view(M, K)
     assert _rel(got, xd @ lin.dequant().double().t() + lin.bias.double()) < 1e-5
     assert torch.equal(ops.linear(lin, x), got.bfloat16())      # and the same sums when they are rounded
+
+
+@pytest.mark.parametrize("fmt,T,E,k,H,I", [(Format.NVFP4, 300, 5, 2, 512, 256), (Format.MXFP8, 250, 8, 4, 256, 128), (Format.NVFP4, 128, 3, 3, 256, 384)])
+def test_expert_product_of_up_to_a_tile_of_rows(ops, fmt, T, E, k, H, I):      # noqa: F811
+    """Experts with no row, a few and more than a tile of 128, around the most rows per expert that the narrow kernel takes: it gives
+    what the tiles of the grouped product do."""
+    ex = _experts(E, H, I, fmt, 5)
+    g = torch.Generator(device=DEV).manual_seed(6)
+    x = torch.randn(T, H, generator=g, device=DEV).bfloat16()
+    logits = torch.randn(T, E, generator=g, device=DEV) + torch.linspace(3, -3, E, device=DEV)
+    if E > k:
+        logits[:, -1] = -50                        # nothing for the last one
+    outs, old = [], ops.MOE_NARROW_ROWS
+    try:
+        for ops.MOE_NARROW_ROWS in (1 << 20, 0):
+            w, ids = ops.router_topk(logits, k, True, 0, E)
+            outs.append(ops.moe(x, w, ids, ex))
+    finally:
+        ops.MOE_NARROW_ROWS = old
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
+    assert _rel(outs[0], outs[1]) < 2e-3           # one may round a sum to the neighbouring bf16
+    assert _rel(outs[0], ref.moe_forward(x, w, ids, ex.forward_one, E)) < 0.08
+
+
+@pytest.mark.parametrize("E,T,k", [(1, 5, 1), (33, 300, 4), (512, 700, 10)])
+def test_expert_plan(ops, E, T, k):      # noqa: F811
+    """Offsets of the experts' rows in tiles of 128 and each tile's expert and live rows."""
+    from blaze_b200.ops.cuda_ops import VP, _ptr
+    counts = torch.bincount(torch.randint(0, E, (T * k,), generator=torch.Generator().manual_seed(1)), minlength=E).to(torch.int32)
+    tiles = (T * k + 127) // 128 + E
+    dev = counts.to(DEV)
+    off, fill, te, tr = [torch.full((n,), -7, dtype=torch.int32, device=DEV) for n in (E, E, tiles, tiles)]
+    assert ops.lib.blz_moe_plan(_ptr(dev), _ptr(off), _ptr(fill), _ptr(te), _ptr(tr), E, tiles, VP(0)) == 0
+    torch.cuda.synchronize()
+    want_te, want_tr, at = [], [], []
+    for e, n in enumerate(counts.tolist()):
+        at.append(len(want_te) * 128)
+        for r in range(0, n, 128):
+            want_te.append(e)
+            want_tr.append(min(128, n - r))
+    pad = tiles - len(want_te)
+    assert te.tolist() == want_te + [-1] * pad and tr.tolist() == want_tr + [0] * pad
+    assert off.tolist() == at and fill.tolist() == [0] * E
