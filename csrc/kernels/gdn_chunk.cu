@@ -60,12 +60,12 @@ __device__ __forceinline__ uint32_t op_off(int row, int k) {      // byte offset
 __device__ __forceinline__ int f_idx(int row, int col) { return row * GC + (col ^ ((row & 7) << 2)); }
 
 // Z[rows o_z.., cols c_z..] (S x S) = sign * X (S x S at rx, cx) * Y (S x S at ry, cy), all inside the scratch matrix.
-// 128 threads cover 128 / (2 S) independent products at once (pair index p shifts every origin by p * 2 S on both axes).
+// NT threads cover 128 / (2 S) independent products at once (pair index p shifts every origin by p * 2 S on both axes).
 // CLEAR_Y: afterwards the Y block is set to zero (it was scratch above the diagonal, which later steps read as part of T).
-template <int S, bool CLEAR_Y>
+template <int S, bool CLEAR_Y, int NT = 128>
 __device__ __forceinline__ void tri_product(float* M, int tid, int zr, int zc, int xr, int xc, int yr, int yc, float sign) {
-  constexpr int W = S / 2;
-  const int pair = tid / (2 * S), i = (tid % (2 * S)) >> 1, c0 = (tid & 1) * W;
+  constexpr int PER_ROW = NT / 64, W = S / PER_ROW;         // threads of a row, columns of a thread
+  const int pair = tid / (PER_ROW * S), i = (tid % (PER_ROW * S)) / PER_ROW, c0 = (tid % PER_ROW) * W;
   const int o = pair * 2 * S;
   float acc[W];
 #pragma unroll
@@ -476,12 +476,12 @@ struct GdnSplitParams {
 // chunk id of the first chunk of sequence b (sequences with fewer than min_rows new tokens own no chunk)
 __device__ __forceinline__ int first_chunk_of(const GdnChunkParams& p, int b, int tid, float* scratch) {
   int mine = 0;
-  for (int i = tid; i < b; i += 128) {
+  for (int i = tid; i < b && tid < 128; i += 128) {
     const int n = p.q_start[i + 1] - p.q_start[i];
     if (n >= p.min_rows && n > 0) mine += (n + GC - 1) / GC;
   }
   int* si = reinterpret_cast<int*>(scratch);
-  si[tid] = mine;
+  if (tid < 128) si[tid] = mine;
   __syncthreads();
   for (int o = 64; o > 0; o >>= 1) {
     if (tid < o) si[tid] += si[tid + o];
@@ -492,13 +492,17 @@ __device__ __forceinline__ int first_chunk_of(const GdnChunkParams& p, int b, in
   return r;
 }
 
-__global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
+// 256 threads: two per row (token) of the chunk, each with half of the row's columns in every register pass, or one with K and the
+// other with Q and V.  The chunk's buffers fill an SM's shared memory, so its warps are all that hide each other's waits: with one
+// thread per row (a warp per scheduler) a chunk took 65 us.  4096 tokens, 32 value heads: 457 -> 357 us.
+__global__ void __launch_bounds__(256, 1) gdn_prep_kernel(GdnSplitParams sp) {
   const GdnChunkParams& p = sp.c;
   const int b = blockIdx.x, hv = blockIdx.y, ch = blockIdx.z;
   const int r0 = p.q_start[b], n = p.q_start[b + 1] - r0;
   const int c0 = ch * GC;
   if (n < p.min_rows || n <= 0 || c0 >= n) return;
   const int tid = threadIdx.x, warp = tid >> 5;
+  const int rt = tid & (GC - 1), half = tid >> 7;      // row of the chunk, half of its columns
   const int hk = hv / (p.Hv / p.Hk);
   const int Cch = 2 * p.Hk * GC + p.Hv * GC;
 
@@ -528,7 +532,7 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t T_1 = tmem + 128 + lane_base, T_2 = tmem + 256 + lane_base, T_3 = tmem + 384 + lane_base;
   uint32_t phase = 0;
   bool ok = true;
@@ -555,8 +559,8 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
   const float Aexp = __expf(p.A_log[hv]);
   const float dtb = p.dt_bias[hv];
   const int L = min(GC, n - c0);
-  const bool live = tid < L;
-  const size_t row = (size_t)(r0 + c0 + tid);
+  const bool live = rt < L;
+  const size_t row = (size_t)(r0 + c0 + rt);
   float g = 0.f, beta = 0.f;
   if (live) {
     const float av = bf2f(p.a_in[row * p.ld_ab + hv]) + dtb;
@@ -572,12 +576,11 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
   }
   if ((tid & 31) == 31) s_w[warp] = G;
   __syncthreads();
-  for (int w = 0; w < warp; ++w) G += s_w[w];
-  s_G[tid] = G;
-  s_beta[tid] = beta;
+  for (int w = warp & 4; w < warp; ++w) G += s_w[w];     // (both halves have the sums)
+  if (half == 0) { s_G[rt] = G; s_beta[rt] = beta; }
   __syncthreads();
   const float G_C = s_G[GC - 1];
-  {
+  if (half == 0) {
     const __nv_bfloat16* src = p.conv + row * Cch + (size_t)p.Hk * GC + (size_t)hk * GC;
     uint4 u[16];
     float ss = 0.f;
@@ -596,12 +599,12 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         o8[q] = __float2bfloat16(bf2f(e[q]) * kn);
-        *reinterpret_cast<__nv_bfloat16*>(bKT + op_off(j * 8 + q, tid)) = o8[q];
+        *reinterpret_cast<__nv_bfloat16*>(bKT + op_off(j * 8 + q, rt)) = o8[q];
       }
-      *reinterpret_cast<uint4*>(bK + op_off(tid, j * 8)) = *reinterpret_cast<const uint4*>(o8);
+      *reinterpret_cast<uint4*>(bK + op_off(rt, j * 8)) = *reinterpret_cast<const uint4*>(o8);
     }
   }
-  {
+  if (half == 1) {
     const __nv_bfloat16* src = p.conv + row * Cch + (size_t)hk * GC;
     uint4 u[16];
     float ss = 0.f;
@@ -619,67 +622,73 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
       __nv_bfloat16 o8[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) o8[q] = __float2bfloat16(bf2f(e[q]) * qn);
-      *reinterpret_cast<uint4*>(bQ + op_off(tid, j * 8)) = *reinterpret_cast<const uint4*>(o8);
+      *reinterpret_cast<uint4*>(bQ + op_off(rt, j * 8)) = *reinterpret_cast<const uint4*>(o8);
     }
   }
-  {
+  if (half == 1) {
     const __nv_bfloat16* src = p.conv + row * Cch + 2 * (size_t)p.Hk * GC + (size_t)hv * GC;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const uint4 u = live ? *reinterpret_cast<const uint4*>(src + j * 8) : make_uint4(0, 0, 0, 0);
       const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&u);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) *reinterpret_cast<__nv_bfloat16*>(bVT + op_off(j * 8 + q, tid)) = e[q];
+      for (int q = 0; q < 8; ++q) *reinterpret_cast<__nv_bfloat16*>(bVT + op_off(j * 8 + q, rt)) = e[q];
     }
   }
   run([&] { mma(128, bK, bK, false); mma(256, bQ, bK, false); });
   if (ok) {
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = half * 2; c < half * 2 + 2; ++c) {
       uint32_t r[32];
       tmem_ld32(T_1 + c * 32, r);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int col = c * 32 + j;
-        Mf[f_idx(tid, col)] = col < tid ? beta * __uint_as_float(r[j]) * __expf(G - s_G[col]) : 0.f;
+        Mf[f_idx(rt, col)] = col < rt ? beta * __uint_as_float(r[j]) * __expf(G - s_G[col]) : 0.f;
       }
     }
     __syncthreads();
     {
-      const int bb = tid >> 4, cc = tid & 15, o = bb * 16;
+      const int bb = rt >> 4, cc = rt & 15, o = bb * 16;
       float x[16];
+      if (half == 0) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float acc = (i == cc) ? 1.f : 0.f;
+        for (int i = 0; i < 16; ++i) {
+          float acc = (i == cc) ? 1.f : 0.f;
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < i) acc -= Mf[f_idx(o + i, o + j)] * x[j];
-        x[i] = i >= cc ? acc : 0.f;
+          for (int j = 0; j < 16; ++j)
+            if (j < i) acc -= Mf[f_idx(o + i, o + j)] * x[j];
+          x[i] = i >= cc ? acc : 0.f;
+        }
       }
       __syncthreads();
+      if (half == 0) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) Mf[f_idx(o + i, o + cc)] = x[i];
+        for (int i = 0; i < 16; ++i) Mf[f_idx(o + i, o + cc)] = x[i];
+      }
       __syncthreads();
     }
-    tri_product<16, false>(Mf, tid, 0, 16, 16, 0, 0, 0, 1.f);
-    tri_product<16, true>(Mf, tid, 16, 0, 16, 16, 0, 16, -1.f);
-    tri_product<32, false>(Mf, tid, 0, 32, 32, 0, 0, 0, 1.f);
-    tri_product<32, true>(Mf, tid, 32, 0, 32, 32, 0, 32, -1.f);
-    tri_product<64, false>(Mf, tid, 0, 64, 64, 0, 0, 0, 1.f);
-    tri_product<64, true>(Mf, tid, 64, 0, 64, 64, 0, 64, -1.f);
+    tri_product<16, false, 256>(Mf, tid, 0, 16, 16, 0, 0, 0, 1.f);
+    tri_product<16, true, 256>(Mf, tid, 16, 0, 16, 16, 0, 16, -1.f);
+    tri_product<32, false, 256>(Mf, tid, 0, 32, 32, 0, 0, 0, 1.f);
+    tri_product<32, true, 256>(Mf, tid, 32, 0, 32, 32, 0, 32, -1.f);
+    tri_product<64, false, 256>(Mf, tid, 0, 64, 64, 0, 0, 0, 1.f);
+    tri_product<64, true, 256>(Mf, tid, 64, 0, 64, 64, 0, 64, -1.f);
   }
-  float trow[GC];
+  constexpr int HC = GC / 2;
+  const int j0 = half * HC;
+  float trow[HC];
 #pragma unroll
-  for (int j = 0; j < GC; ++j) trow[j] = (ok && j <= tid) ? Mf[f_idx(tid, j)] : 0.f;
+  for (int j = 0; j < HC; ++j) trow[j] = (ok && j0 + j <= rt) ? Mf[f_idx(rt, j0 + j)] : 0.f;
   __syncthreads();
   auto write_T = [&](bool with_gamma) {
 #pragma unroll
-    for (int j = 0; j < GC; j += 8) {
+    for (int j = 0; j < HC; j += 8) {
       float s[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) s[q] = trow[j + q] * s_beta[j + q] * (with_gamma ? __expf(s_G[j + q]) : 1.f);
-      *reinterpret_cast<uint4*>(bT + op_off(tid, j)) =
+      for (int q = 0; q < 8; ++q) s[q] = trow[j + q] * s_beta[j0 + j + q] * (with_gamma ? __expf(s_G[j0 + j + q]) : 1.f);
+      *reinterpret_cast<uint4*>(bT + op_off(rt, j0 + j)) =
           make_uint4(pack_bf16x2(s[0], s[1]), pack_bf16x2(s[2], s[3]), pack_bf16x2(s[4], s[5]), pack_bf16x2(s[6], s[7]));
     }
   };
@@ -694,20 +703,20 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
   if (ok) {
     // W rows -> bK, U rows -> bT, P rows -> bVT (V^T is no longer needed), Q rows scaled by gamma, K^T columns by e^{G_C - G_j}
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
+    for (int c = half * 2; c < half * 2 + 2; ++c) {
       uint32_t r[32];
       tmem_ld32(T_3 + c * 32, r);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 8)
-        *reinterpret_cast<uint4*>(bK + op_off(tid, c * 32 + j)) =
+        *reinterpret_cast<uint4*>(bK + op_off(rt, c * 32 + j)) =
             make_uint4(pack_bf16x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), pack_bf16x2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
                        pack_bf16x2(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5])), pack_bf16x2(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7])));
       tmem_ld32(T_1 + c * 32, r);
       tmem_ld_wait();
 #pragma unroll
       for (int j = 0; j < 32; j += 8)
-        *reinterpret_cast<uint4*>(bT + op_off(tid, c * 32 + j)) =
+        *reinterpret_cast<uint4*>(bT + op_off(rt, c * 32 + j)) =
             make_uint4(pack_bf16x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), pack_bf16x2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
                        pack_bf16x2(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5])), pack_bf16x2(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7])));
       tmem_ld32(T_2 + c * 32, r);
@@ -716,27 +725,27 @@ __global__ void __launch_bounds__(128, 1) gdn_prep_kernel(GdnSplitParams sp) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         const int col = c * 32 + j;
-        pv[j] = col <= tid ? __uint_as_float(r[j]) * __expf(G - s_G[col]) : 0.f;
+        pv[j] = col <= rt ? __uint_as_float(r[j]) * __expf(G - s_G[col]) : 0.f;
       }
 #pragma unroll
       for (int j = 0; j < 32; j += 8)
-        *reinterpret_cast<uint4*>(bVT + op_off(tid, c * 32 + j)) =
+        *reinterpret_cast<uint4*>(bVT + op_off(rt, c * 32 + j)) =
             make_uint4(pack_bf16x2(pv[j], pv[j + 1]), pack_bf16x2(pv[j + 2], pv[j + 3]), pack_bf16x2(pv[j + 4], pv[j + 5]),
                        pack_bf16x2(pv[j + 6], pv[j + 7]));
     }
     {
       const float gam = __expf(G), kap = __expf(G_C - G);
 #pragma unroll
-      for (int j = 0; j < GC; j += 8) {
-        uint4 u = *reinterpret_cast<uint4*>(bQ + op_off(tid, j));
+      for (int j = j0; j < j0 + HC; j += 8) {
+        uint4 u = *reinterpret_cast<uint4*>(bQ + op_off(rt, j));
         __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&u);
 #pragma unroll
         for (int q = 0; q < 8; ++q) e[q] = __float2bfloat16(bf2f(e[q]) * gam);
-        *reinterpret_cast<uint4*>(bQ + op_off(tid, j)) = u;
+        *reinterpret_cast<uint4*>(bQ + op_off(rt, j)) = u;
       }
 #pragma unroll 4
-      for (int d = 0; d < GC; ++d) {
-        __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(bKT + op_off(d, tid));
+      for (int d = j0; d < j0 + HC; ++d) {
+        __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(bKT + op_off(d, rt));
         *e = __float2bfloat16(bf2f(*e) * kap);
       }
     }
@@ -988,7 +997,7 @@ BLZ_API int blz_gdn_chunk_split(const void* conv, const void* a_in, const void* 
   if (e != cudaSuccess) return (int)e;
   e = c2.smem_limit(gdn_scan_kernel, SCAN_SMEM);
   if (e != cudaSuccess) return (int)e;
-  gdn_prep_kernel<<<dim3(B, Hv, (max_q + GC - 1) / GC), 128, PREP_SMEM, s>>>(sp);
+  gdn_prep_kernel<<<dim3(B, Hv, (max_q + GC - 1) / GC), 256, PREP_SMEM, s>>>(sp);
   e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   gdn_scan_kernel<<<dim3(B, Hv), 128, SCAN_SMEM, s>>>(sp);
