@@ -58,6 +58,7 @@ class StepBatch:
                                               # j-th new token of its sequence (causal rows: bits 0..own index)
     tiny_rows_max: int = 0        # largest q_len * group among sequences with at most TINY_ROWS rows (plain decode)
     num_tiny: int = 0
+    split_seqs: int = 0           # captured steps: the sequences whose number settles how keys are split (0: those the batch has rows for)
     small_rows_max: int = 0       # largest q_len * group among the other sequences handled by the decode attention kernel
     num_small: int = 0
     num_large: int = 0            # sequences handled by the row-block (prefill) attention kernel

@@ -726,6 +726,14 @@ class CudaOps:
         self._check(self.lib.blz_kv_move_rows(_ptr(pool), _ptr(src), _ptr(dst), _ptr(seg), seg.numel() - 1, pool.shape[1], D,
                                               pool.stride(0), pool.stride(1), self._stream()), "kv_move_rows")
 
+    def decode_splits(self, work: int, tiles: int) -> int:
+        """Runs that the keys of an item are cut into by the decode attention kernel (``work`` = items: three CTAs' worth per SM)."""
+        return 1 if work >= 3 * self._sm else max(1, min(8, tiles, (3 * self._sm) // max(work, 1)))
+
+    def row_block_splits(self, work: int, tiles: int) -> int:
+        """The same by the row-block kernel: one CTA's worth per SM."""
+        return 1 if work >= self._sm else max(1, min(8, tiles, self._sm // max(work, 1)))
+
     def attention(self, q, model, batch, kv, layer_idx, scale, splits: int = 0, max_ctas: int = 0, allowed=None):
         """Sequences with few query rows (decode, verify) go to the decode kernel, the rest to the row-block kernel."""
         if allowed is not None:
@@ -760,14 +768,10 @@ class CudaOps:
         for lo, hi, count in tiers:
             nmax = 16
             rb = (hi + nmax - 1) // nmax
-            # Items for every CTA that fits at once (two per SM, one beyond 8 rows): whole items.  Fewer: their tiles shared out
-            # evenly, and the pieces merged by a second kernel.  Measured, whole / shared: 512 items 36 / 56 us (64 sequences, 8 rows),
-            # 392 items 39 / 38 us (49 sequences, 4 rows), 48 items 158 / 42 us (6 long ones).
-            items, most = B * Hkv * rb, (2 if hi <= 8 else 1) * self._sm
-            sp = splits if splits > 0 else 1 if max(count, 1) * Hkv * rb >= most else 1 + (most + items - 1) // items
+            sp = splits if splits > 0 else self.decode_splits(max(batch.split_seqs or count, 1) * Hkv * rb, tiles)
             po = pm = None
             if sp > 1:
-                n = (items + min(items * (sp - 1), 2 * self._sm)) * nmax
+                n = B * Hkv * rb * sp * nmax
                 po = self._buf("attn_part_o", n * D * 4).view(torch.float32)
                 pm = self._buf("attn_part_ml", n * 2 * 4).view(torch.float32)
             self._check(self.lib.blz_attn_decode_tree(_ptr(q), _ptr(out), _ptr(kv.kv[layer_idx]), _ptr(kv.block_table),
@@ -781,7 +785,7 @@ class CudaOps:
         if batch.item_seq is not None:
             n_items = batch.item_seq.numel()
             work = n_items * Hkv
-            sp = splits if splits > 0 else (1 if work >= self._sm else max(1, min(8, tiles, self._sm // max(work, 1))))
+            sp = splits if splits > 0 else self.row_block_splits((batch.split_seqs or n_items) * Hkv, tiles)
             po = pm = None
             if sp > 1:
                 n = work * sp * 128

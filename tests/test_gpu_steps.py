@@ -19,6 +19,18 @@ def _rel(a, b):
     return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30)).item()
 
 
+@pytest.mark.parametrize("Hq,Hkv,ctxs,q", [
+    (32, 8, [1], 1), (32, 8, [129], 1), (32, 8, [5000, 3, 128, 1291], 1),          # fewer items than CTAs: runs of tiles
+    (16, 2, [2600, 40, 1025], 1), (32, 4, [700], 2), (32, 8, [900, 260], 5), (32, 4, [1500, 64], 8),      # 8, 16, 20 and 64 rows
+    (32, 8, [33 + 7 * i for i in range(40)], 1), (64, 8, [200 + i for i in range(19)], 3),                 # more items than CTAs
+])
+def test_decode_attention_runs_of_tiles(ops, Hq, Hkv, ctxs, q):      # noqa: F811
+    got, want = _attention_case(ops, Hq, Hkv, ctxs, [q] * len(ctxs))
+    assert torch.isfinite(got.float()).all() and _rel(got, want) < 0.06
+    err = (got.float() - want.float()).flatten(1).norm(dim=1) / want.float().flatten(1).norm(dim=1)
+    assert err.max().item() < 0.15                 # row by row: an item that got a wrong piece is off by its size
+
+
 @pytest.mark.parametrize("M", [1, 31, 32, 33, 64, 65])
 @pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (1024, 5120), (5120, 8192), (40000, 256)])
 def test_fp8_block_product_of_few_rows(ops, M, N, K):      # noqa: F811
