@@ -31,6 +31,18 @@ def test_decode_attention_runs_of_tiles(ops, Hq, Hkv, ctxs, q):      # noqa: F81
     assert err.max().item() < 0.15                 # row by row: an item that got a wrong piece is off by its size
 
 
+@pytest.mark.parametrize("Hq,Hkv,ctxs,qlens,splits", [
+    (8, 2, [17], [17], 0), (32, 8, [128, 129, 33], [128, 129, 33], 0), (8, 1, [1100, 40], [300, 40], 1),      # blocks of 128 rows and parts
+    (4, 4, [700], [513], 1), (16, 2, [2000, 90], [70, 60], 3), (32, 4, [300], [40], 8),                        # split key ranges, some empty
+])
+def test_prompt_attention(ops, Hq, Hkv, ctxs, qlens, splits):      # noqa: F811
+    """Blocks whose rows see no key of a tile, few keys of it, or all; runs of tiles whose maxima grow and do not."""
+    got, want = _attention_case(ops, Hq, Hkv, ctxs, qlens, splits=splits)
+    assert torch.isfinite(got.float()).all() and _rel(got, want) < 0.06
+    err = (got.float() - want.float()).flatten(1).norm(dim=1) / want.float().flatten(1).norm(dim=1)
+    assert err.max().item() < 0.15
+
+
 @pytest.mark.parametrize("M", [1, 31, 32, 33, 64, 65])
 @pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (1024, 5120), (5120, 8192), (40000, 256)])
 def test_fp8_block_product_of_few_rows(ops, M, N, K):      # noqa: F811
