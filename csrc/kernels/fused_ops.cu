@@ -7,6 +7,7 @@
 // mul_sigmoid :161, silu_mul :166, argmax_kernel :249, gather_rows :346), kernels/src/cuda/nvfp4_gemm.cu
 // quant_rows_kernel :33, kernels/src/cuda/nvfp4_kv.cu kv_store_dense_kernel :188 and embed.cu:6 — fused so
 // that each activation makes one trip through HBM between GEMMs.
+#include "blaze/glu.cuh"
 #include "blaze/host.h"
 #include "blaze/sm100.cuh"
 
@@ -257,10 +258,9 @@ __device__ __forceinline__ uint32_t pack_e4m3x4_f(float a, float b, float c, flo
 
 // Quantise this thread's 8 elements [e0, e0+8) of row t, neighbouring lanes holding neighbouring elements (a warp starts at a
 // multiple of 256).  Every lane of the warp must call it (shuffles); `valid` gates the stores.
-// These kernels move two bytes in for half a byte out, and what bounded them were a scale byte stored per 16 elements (a memory
-// sector each, as for a full one) and three divisions per 8 elements: four scales make one store (they are neighbours in the
-// 128x4 tiles; those of a row's padded columns are written as 0), the row's factor comes as a reciprocal.  8192 rows of 12288
-// activations: 101 -> 72 us.
+// A scale byte stored by itself costs the memory system a sector, as a full one does: four of them (neighbours in the 128x4 tiles)
+// make one store, and those of a row's padded columns are written as 0.  8192 rows of 12288 activations: 101 -> 82 us, together
+// with the registers that the plain form of the kernel below no longer carries.
 template <int QUANT>
 __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, int t, int e0, int W, float g, uint8_t* q_out,
                                              uint8_t* sf_out, int ct) {
@@ -272,7 +272,7 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
   for (int j = 0; j < 8; ++j) { v[j] = valid ? bf2f(e[j]) : 0.f; bm = fmaxf(bm, fabsf(v[j])); }
   bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
   if (QUANT == 1) {
-    const uint8_t sf = f2e4m3(bm * __frcp_rn(6.f * g));
+    const uint8_t sf = f2e4m3(bm / 6.f / g);           // (ties between two scales are common: the same roundings as ever)
     const float denom = e4m32f(sf) * g;
     const float inv = denom > 0.f ? __frcp_rn(denom) : 0.f;
     const uint32_t codes = pack_e2m1x8(v, inv);
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float x = bf2f(eg[j]);
-        eg[j] = __float2bfloat16(x / (1.f + __expf(-x)) * bf2f(eu[j]));
+        eg[j] = __float2bfloat16(silu(x) * bf2f(eu[j]));
       }
     }
 #pragma unroll
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const __nv_bfloat16* _
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float x = bf2f(eg[j]);
-      eg[j] = __float2bfloat16(x / (1.f + __expf(-x)) * bf2f(eu[j]));
+      eg[j] = __float2bfloat16(silu(x) * bf2f(eu[j]));
     }
   }
 #pragma unroll
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(512) attn_prep_kernel(const __nv_bfloat16* __r
 // system what a sector does.  With `v_blocks`, a page that 16 consecutive tokens fill is written as whole rows by a block of its own
 // (one per 16 tokens behind the T token blocks, for the page that begins among them); the token blocks write the other values.
 // Measured on a B200, 8192 tokens, 32 + 2 x 8 heads of 128 (184 MB, 28 us at copy bandwidth): 117 us by head and token
-// (220 instructions per head and warp, byte stores of the values), now 64 us.
+// (220 instructions per head and warp, byte stores of the values), now 63 us.
 template <int D>
 __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ q_out,
                                  __nv_bfloat16* __restrict__ gate_out, uint8_t* __restrict__ kv_pool,
@@ -644,6 +644,7 @@ __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat1
   pdl_trigger();
   pdl_wait();
   constexpr int LPH = D / 8, HPW = 32 / LPH;          // lanes per head, heads per warp
+  constexpr int PART = D / 32;                        // dims of a partial sum of squares
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int qw = Hq * D * (gated ? 2 : 1);
   const size_t row_w = (size_t)qw + 2 * (size_t)Hkv * D;
@@ -702,20 +703,25 @@ __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat1
   const int slot = slot_mapping[t];
   bool paged = false;                                 // a block of its own writes this token's values (same in all warps)
   if (v_blocks && slot >= 0) {
-    const int first = t - (slot & 15), at = lane & 15;
-    if (first >= 0 && first + 15 < T) paged = __all_sync(0xffffffffu, slot_mapping[first + at] == (slot & ~15) + at);
+    const int begin = t - (slot & 15), at = lane & 15;
+    if (begin >= 0 && begin + 15 < T) paged = __all_sync(0xffffffffu, slot_mapping[begin + at] == (slot & ~15) + at);
   }
   const __nv_bfloat16* row = qkv + t * row_w;
   uint4 wq = make_uint4(0, 0, 0, 0), wk = wq;
   if (q_norm_w) wq = *reinterpret_cast<const uint4*>(q_norm_w + i0);
   if (k_norm_w) wk = *reinterpret_cast<const uint4*>(k_norm_w + i0);
   __syncthreads();
-  // a lane's dims all lie in the first half of the pairs, in the second, or beyond: x cos - y sin, or x cos + y sin
+  // a lane's dims all lie in the first half of the pairs, in the second, or beyond: x cos - y sin, or y sin + x cos (the last product
+  // is the one that is rounded by itself)
+  const bool first = i0 < half;
   float2 rot[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     rot[j] = make_float2(1.f, 0.f);
-    if (turned) { rot[j] = cs[i0 < half ? i0 + j : i0 + j - half]; if (i0 < half) rot[j].y = -rot[j].y; }
+    if (turned) {
+      const float2 cj = cs[first ? i0 + j : i0 + j - half];
+      rot[j] = first ? make_float2(cj.x, -cj.y) : make_float2(cj.y, cj.x);
+    }
   }
   const int heads = Hq + (paged ? Hkv : 2 * Hkv);
   for (int h0 = warp * HPW; h0 < heads; h0 += nwarps * HPW) {
@@ -725,13 +731,21 @@ __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat1
     uint4 raw = make_uint4(0, 0, 0, 0);
     if (live) raw = *reinterpret_cast<const uint4*>(src);
     const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&raw);
-    float v[8], ss = 0.f;
+    // squares are summed as the kernel above does: 32 partial sums per head, added up by a butterfly from the farthest
+    float v[8], sq[8 / PART];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { v[j] = bf2f(e[j]); ss += v[j] * v[j]; }
+    for (int j = 0; j < 8; ++j) {
+      v[j] = bf2f(e[j]);
+      sq[j / PART] = j % PART == 0 ? v[j] * v[j] : fmaf(v[j], v[j], sq[j / PART]);
+    }
     if (live && is_q && gated)
       *reinterpret_cast<uint4*>(gate_out + ((size_t)t * Hq + h) * D + i0) = *reinterpret_cast<const uint4*>(src + D);
 #pragma unroll
-    for (int o = 1; o < LPH; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    for (int o = LPH / 2; o > 0; o >>= 1) {
+#pragma unroll
+      for (int j = 0; j < 8 / PART; ++j) sq[j] += __shfl_xor_sync(0xffffffffu, sq[j], o);
+    }
+    const float ss = PART == 8 ? sq[0] : sq[0] + sq[8 / PART - 1];
     if (!is_v && (is_q ? q_norm_w != nullptr : k_norm_w != nullptr)) {
       const float rstd = rsqrtf(ss / D + eps);
       const uint4 w8 = is_q ? wq : wk;
@@ -743,7 +757,8 @@ __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat1
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float other = __shfl_xor_sync(0xffffffffu, v[j], lanes_half);
-      o[j] = is_v || !turned ? v[j] : v[j] * rot[j].x + other * rot[j].y;
+      const float turn = fmaf(first ? v[j] : other, rot[j].x, (first ? other : v[j]) * rot[j].y);
+      o[j] = is_v || !turned ? v[j] : turn;
     }
     if (!live) continue;                                // (no shuffle follows in this iteration)
     if (is_q) {

@@ -385,7 +385,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                   a[j] = clamped_glu_fast(gf, uf, p.act_limit);
                 } else {
                   const float g = bf2f(__float2bfloat16(gf)), u = bf2f(__float2bfloat16(uf));
-                  a[j] = g / (1.f + __expf(-g)) * u;
+                  a[j] = silu(g) * u;
                 }
               }
               pk[i / 2] = pack_bf16x2(a[0], a[1]);

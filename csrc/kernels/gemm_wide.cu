@@ -365,8 +365,8 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
           } else if (p.act) {
             __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)tok * p.ldc + c0 / 2;
             // The gated activation's exponentials and divisions keep the eight warps busy about as long as the tensor pipe has work
-            // for the next tile: the division is the approximate one (2 ulp of 32 bits, before the rounding to bf16), and the
-            // activation is told apart outside of the loop.  8192 x 24576 x 4096, NVFP4: 525 -> 427 us.
+            // for the next tile: the division is glu.cuh's, without the checks of the general one, and the activation is told
+            // apart outside of the loop.  8192 x 24576 x 4096, NVFP4: 489 -> 387 us; 825 rows 66 -> 51.
             auto gated = [&](auto act) {
 #pragma unroll
               for (int gq = 0; gq < CPT; gq += 32) {
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
             } else {
               gated([](float gf, float uf) {
                 const float g = bf2f(__float2bfloat16(gf)), u = bf2f(__float2bfloat16(uf));
-                return __fdividef(g, 1.f + __expf(-g)) * u;
+                return silu(g) * u;
               });
             }
           } else {

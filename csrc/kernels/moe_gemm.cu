@@ -80,7 +80,7 @@ struct MgCfg {
 __device__ __forceinline__ float mg_silu_mul(float g, float u) {
   g = bf2f(__float2bfloat16(g));
   u = bf2f(__float2bfloat16(u));
-  return g / (1.f + __expf(-g)) * u;
+  return silu(g) * u;
 }
 
 template <int KIND>

@@ -43,6 +43,90 @@ def test_prompt_attention(ops, Hq, Hkv, ctxs, qlens, splits):      # noqa: F811
     assert err.max().item() < 0.15
 
 
+@pytest.mark.parametrize("D,Hq,Hkv,rot,gated", [(128, 8, 2, 128, False), (128, 6, 3, 64, True), (256, 4, 2, 64, True), (256, 2, 1, 256, False)])
+@pytest.mark.parametrize("chunks", [[(0, 64)], [(11, 90), (0, 17)], [(5, 1)] * 3 + [(16, 70), (15, 1), (0, 40)], [(3, 20)], [(0, 1100)]])
+def test_attention_preparation_writes_pages(ops, D, Hq, Hkv, rot, gated, chunks):      # noqa: F811
+    """Queries, keys and values of steps with whole pages, parts of pages and single tokens: every page byte as the reference has
+    it, nothing written for rows without a slot."""
+    cfg = ModelConfig(hidden_size=Hq * D, num_heads=Hq, num_kv_heads=Hkv, head_dim=D, num_layers=1, attn_output_gate=gated,
+                      rope=RopeConfig(theta=1e6, partial_rotary_factor=rot / D))
+    cfg.layer_types = ["full_attention"]
+    g = torch.Generator(device=DEV).manual_seed(7)
+    per = max((c + n + 15) // 16 for c, n in chunks)
+    kv = KVCache(cfg, 1 + per * len(chunks), len(chunks), per, "fp8", DEV, "umma")
+    order = torch.randperm(per * len(chunks), generator=torch.Generator().manual_seed(2)).tolist()
+    for b in range(len(chunks)):
+        kv.set_pages(b, [1 + p for p in order[b * per:(b + 1) * per]])
+    kv.kv[0].fill_(0x35)
+    batch = build_batch([SeqChunk(b, [0] * n, c) for b, (c, n) in enumerate(chunks)], kv.block_table_host, DEV, attn_group=Hq // Hkv)
+    T = batch.num_rows
+    if T > 20:
+        batch.slot_mapping[T - 3] = -1             # a padded row
+    model, attn = _A(), _A()
+    model.cfg, model.rope_scale, model.kv_rotate = cfg, 1.0, False
+    model.inv_freq = torch.tensor(inv_freq(cfg), dtype=torch.float32, device=DEV)
+    attn.heads, attn.kv_heads = Hq, Hkv
+    attn.q_norm, attn.k_norm = [(1 + 0.1 * torch.randn(D, generator=g, device=DEV)).bfloat16() for _ in range(2)]
+    qkv = torch.randn(T, (Hq * (2 if gated else 1) + 2 * Hkv) * D, generator=g, device=DEV).bfloat16()
+    q, gate = ops.attn_prep_store(qkv, attn, model, batch, kv, 0, None)
+    cos, sin = ref.rope_cos_sin(batch.positions, model.inv_freq)
+    qr, kr, vr, gr = ref.attn_prep(qkv, Hq, Hkv, D, attn.q_norm, attn.k_norm, 1e-6, cos, sin, gated=gated)
+    torch.cuda.synchronize()
+    assert _rel(q, qr) < 4e-3
+    if gated:
+        assert torch.equal(gate.view(T, Hq, D), gr.reshape(T, Hq, D))
+    kl, vl = kv.logical_kv(0)
+    slots = batch.slot_mapping.long()
+    live = slots >= 0
+    page, off = slots[live] // 16, slots[live] % 16
+    assert torch.equal(vl[page, :, off].float(), vr[live].to(torch.float8_e4m3fn).float())
+    # a key near the edge between two codes may fall on either side (sums of squares in another order)
+    assert _rel(kl[page, :, off].float(), kr[live].float()) < 0.04
+    touched = torch.zeros(kl.shape[0], 16, dtype=torch.bool, device=DEV)
+    touched[page, off] = True
+    old = torch.tensor(0x35, dtype=torch.uint8).view(torch.float8_e4m3fn).float().item()
+    for pool in (kl, vl):
+        assert (pool.float().permute(0, 2, 1, 3)[~touched] == old).all()
+
+
+@pytest.mark.parametrize("fmt", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("T,K", [(1, 32), (3, 96), (129, 1056), (5, 1024), (1030, 4128), (2, 12288)])
+def test_quantised_rows(ops, fmt, T, K):      # noqa: F811
+    """Row quantisers at widths that end inside a tile of scales, against the reference quantisers."""
+    if fmt == Format.NVFP4 and K % 64:
+        K = (K + 63) // 64 * 64                    # what a product in that format can have
+    g = torch.Generator(device=DEV).manual_seed(3)
+    x = (torch.randn(T, K, generator=g, device=DEV) * torch.rand(T, 1, generator=g, device=DEV) * 8).bfloat16()
+    x[T // 2] = 0
+    lin = Linear(fmt, 128, K)
+    lin.act_quant = True
+    qa = ops.quantize_rows(x, lin)
+    per = 16 if fmt == Format.NVFP4 else 32
+    sf = quant.unswizzle_sf_128x4(qa.sf, T, K // per)
+    if fmt == Format.NVFP4:
+        got = quant.nvfp4_dequantize(qa.data, sf.view(torch.float8_e4m3fn), qa.row_scale)
+        g_row = x.float().abs().amax(1) / torch.full((T,), 2688.0, device=DEV)      # (by a constant, torch multiplies with its reciprocal)
+        want = quant.nvfp4_dequantize(*quant.nvfp4_quantize(x, g_row.clamp_min(1e-30), per_row=True))
+    else:
+        got = quant.mxfp8_dequantize(qa.data.view(torch.float8_e4m3fn), sf)
+        want = quant.mxfp8_dequantize(*quant.mxfp8_quantize(x))
+    # The kernel multiplies by a block's reciprocal: a value on the edge between two codes may take the other one.  Quotients of
+    # numbers with 8-bit mantissas do lie there, about one in two thousand, and a code is up to a quarter of its value away.
+    assert (got != want).float().mean().item() < 1e-3 and _rel(got, want) < 1e-2
+
+
+@pytest.mark.parametrize("T,H,shift", [(1, 8, 0), (3, 20, 0), (7, 2048, 0), (5, 4096, 1), (1, 33, 3)])
+def test_elementwise(ops, T, H, shift):      # noqa: F811
+    g = torch.Generator(device=DEV).manual_seed(5)
+    a, b = [torch.randn(T * H + shift, generator=g, device=DEV).bfloat16()[shift:].view(T, H) for _ in range(2)]
+    gl = torch.randn(T, 1, generator=g, device=DEV).bfloat16()
+    assert torch.equal(ops.add(a, b), (a.float() + b.float()).bfloat16())
+    want = (a.float() + b.float() * torch.sigmoid(gl.float()).bfloat16().float()).bfloat16()
+    assert _rel(ops.add_sigmoid_scaled(a, b, gl), want) < 4e-3
+    want = (a.float() * torch.sigmoid(b.float())).bfloat16()
+    assert _rel(ops.mul_sigmoid(a.clone(), b), want) < 4e-3
+
+
 @pytest.mark.parametrize("M", [1, 31, 32, 33, 64, 65])
 @pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (1024, 5120), (5120, 8192), (40000, 256)])
 def test_fp8_block_product_of_few_rows(ops, M, N, K):      # noqa: F811
