@@ -461,11 +461,22 @@ class Engine:
         return (self.model.tp.world == 1 and not self.model.capture_layers
                 and all(c.want_logits == 1 and not c.defer_state and c.parents is None for c in chunks))
 
+    def _key_splits(self, n: int) -> int:
+        """Runs the attention kernels cut the keys of a decode step of ``n`` sequences into.  A captured step with logits keeps the
+        number that ``n`` sequences get, not the one of its padded batch: partial sums are rounded, so the logits of a step would
+        otherwise depend on whether it was replayed."""
+        heads = n * self.model.cfg.num_kv_heads
+        if self.attn_group == 0:
+            return 1
+        if self.attn_all_items:
+            return self.model.ops.row_block_splits(heads, 8)
+        return self.model.ops.decode_splits(heads * ((self.attn_group + 15) // 16), 8)
+
     def _forward_graph(self, chunks: Sequence[SeqChunk], feedback: bool = False, rows_per_seq: int = 1, mode: str = "greedy"):
         B = len(chunks)
         bucket = self._bucket(B)
         key = (("decode", bucket) if rows_per_seq == 1 and mode == "greedy" else
-               ("logits", bucket) if mode == "logits" else ("verify", bucket, rows_per_seq, mode))
+               ("logits", bucket, self._key_splits(B)) if mode == "logits" else ("verify", bucket, rows_per_seq, mode))
         g = self._graphs.get(key)
         if g is None:
             seen = self._seen.get(key, 0)
@@ -474,7 +485,7 @@ class Engine:
                 raise RuntimeError("token feedback needs a captured decode step")
             if seen == 0:   # first sight: run eagerly (also warms allocator and lazy inits)
                 return self._run(self._build(chunks), mode)
-            g = _Graph(self, bucket, rows_per_seq, mode)
+            g = _Graph(self, bucket, rows_per_seq, mode, B if mode == "logits" else 0)
             self._graphs[key] = g
         return g.replay(chunks, feedback)
 
@@ -555,7 +566,7 @@ class _Graph:
     """A captured step for a fixed sequence bucket with ``L`` rows per sequence (1 = decode, more = chain verify); inputs live
     in static buffers."""
 
-    def __init__(self, eng: Engine, bucket: int, rows_per_seq: int = 1, mode: str = "greedy"):
+    def __init__(self, eng: Engine, bucket: int, rows_per_seq: int = 1, mode: str = "greedy", split_seqs: int = 0):
         self.eng, self.bucket, self.L, self.mode = eng, bucket, rows_per_seq, mode
         dev = eng.device
         n, L = bucket, rows_per_seq
@@ -582,6 +593,7 @@ class _Graph:
         self.batch.h_ctx_len = [L] * n
         self.batch.h_logit_rows = list(range(T))
         self.batch.max_ctx = eng.ecfg.max_model_len
+        self.batch.split_seqs = split_seqs
         from .batch import TINY_ROWS
         g = max(eng.attn_group, 1) * L
         if eng.attn_all_items:

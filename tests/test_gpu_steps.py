@@ -19,6 +19,29 @@ def _rel(a, b):
     return ((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30)).item()
 
 
+def test_logits_steps_replay_a_captured_step():
+    """A decode step with logits: the first of a batch size runs launch by launch, the others replay it; the tensors handed out
+    stay as they were."""
+    from blaze_b200.llm import LLM
+    cfg = ModelConfig(vocab_size=2048, hidden_size=512, num_layers=2, num_heads=8, num_kv_heads=2, head_dim=128, intermediate_size=1024,
+                      rope=RopeConfig(theta=1e6))
+    cfg.layer_types = ["full_attention"] * 2
+    eng = LLM(cfg, weight_format="nvfp4", max_seqs=8, max_model_len=256, seed=4).engine
+    gen = torch.Generator().manual_seed(1)
+    seqs = [eng.open_from() for _ in range(3)]
+    eng.forward(eng.plan([(s, torch.randint(0, 2048, (n,), generator=gen).tolist(), 0) for s, n in zip(seqs, (40, 7, 100))]), "none")
+    base, outs = [s.length for s in seqs], []
+    for tok in (5, 5, 5, 900):
+        for s, n in zip(seqs, base):
+            s.length = n
+        outs.append(eng.forward(eng.plan([(s, [tok], 1) for s in seqs]), "logits"))
+    assert any(k[:2] == ("logits", 4) for k in eng._graphs) and outs[0].shape == (3, 2048) and outs[0].dtype == torch.float32
+    assert torch.equal(outs[1], outs[2]) and not torch.equal(outs[2], outs[3])
+    assert torch.equal(outs[1], outs[0])           # launch by launch and replayed: the keys are split alike
+    some = eng.forward(eng.plan([(seqs[0], [1], 1), (seqs[1], [1], 0)]), "logits")
+    assert some.shape[0] == 1                      # rows without logits: not a step of that kind
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [
     (32, 8, [1], 1), (32, 8, [129], 1), (32, 8, [5000, 3, 128, 1291], 1),          # fewer items than CTAs: runs of tiles
     (16, 2, [2600, 40, 1025], 1), (32, 4, [700], 2), (32, 8, [900, 260], 5), (32, 4, [1500, 64], 8),      # 8, 16, 20 and 64 rows
