@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(128) gdn_recurrent_kernel(
 
 // one warp per (token, head): y = rmsnorm(o) * w * gate(z), gate = silu, or sigmoid with flag bit 1 (a checkpoint's
 // output_gate_type); flag bit 0: w is stored as w - 1.  N consecutive elements per lane and access: 4 where heads and rows lie on 8
-// bytes (with single elements 4096 tokens of 32 heads of 128 took 62 us, now 36; their bytes take 15).
+// bytes.  4096 tokens of 32 heads of 128: 67 us with single elements, 50 with four; their bytes take 15.  (40 with the squares added up
+// by runs of four and the approximate quotient, which round differently.)
 template <int N>
 __global__ void gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ z, long long ldz,
                                      const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int rows, int Hv, int DV,
@@ -241,11 +242,9 @@ __global__ void gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ o, const 
   const __nv_bfloat16* src = o + ((size_t)t * Hv + h) * DV;
   const __nv_bfloat16* zz = z + (size_t)t * ldz + (size_t)h * DV;
   float x[N], g[N], wf[N], ss = 0.f;
-  for (int i = lane * N; i < DV; i += 32 * N) {
-    cv_ldv<__nv_bfloat16, N>(src + i, x);
-#pragma unroll
-    for (int j = 0; j < N; ++j) ss += x[j] * x[j];
-  }
+  // The squares are added up by lanes of single elements whatever N is (the row is read again below, from the cache): with runs of N
+  // the sum's roundings would depend on the pointers.
+  for (int i = lane; i < DV; i += 32) { const float f = bf2f(src[i]); ss += f * f; }
   ss = warp_sum(ss);
   const float rstd = rsqrtf(ss / DV + eps);
   for (int i = lane * N; i < DV; i += 32 * N) {
@@ -254,8 +253,8 @@ __global__ void gated_rmsnorm_kernel(const __nv_bfloat16* __restrict__ o, const 
     cv_ldv<__nv_bfloat16, N>(w + i, wf);
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      const float sg = __fdividef(1.f, 1.f + __expf(-g[j]));
-      x[j] *= rstd * (wf[j] + (zero_centered ? 1.f : 0.f)) * (sigmoid_gate ? sg : g[j] * sg);
+      const float sg = 1.f / (1.f + __expf(-g[j]));        // (rounded: the approximate quotient is 0 for gates below -87.3, too)
+      x[j] = x[j] * rstd * (wf[j] + (zero_centered ? 1.f : 0.f)) * (sigmoid_gate ? sg : g[j] * sg);
     }
     cv_stv<__nv_bfloat16, N>(y + ((size_t)t * Hv + h) * DV + i, x);
   }

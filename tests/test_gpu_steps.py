@@ -209,3 +209,28 @@ def test_expert_plan(ops, E, T, k):      # noqa: F811
     pad = tiles - len(want_te)
     assert te.tolist() == want_te + [-1] * pad and tr.tolist() == want_tr + [0] * pad
     assert off.tolist() == at and fill.tolist() == [0] * E
+
+
+@pytest.mark.parametrize("T,Hv,DV", [(1, 1, 4), (7, 3, 64), (33, 2, 132), (300, 32, 128), (5, 2, 129)])
+@pytest.mark.parametrize("flags", [0, 1, 2, 3])
+def test_gated_norm(ops, T, Hv, DV, flags):      # noqa: F811
+    """Single elements and runs of four give the same bits, and both what 64 bits give, rounded: also for gates whose sigmoid lies
+    near the end of the range (1 + e^-z beyond 2^126)."""
+    from blaze_b200.ops.cuda_ops import VP, _ptr
+    g = torch.Generator(device=DEV).manual_seed(9)
+    o, z = [torch.randn(T, Hv * DV, generator=g, device=DEV).mul(s).bfloat16() for s in (1.0, 3.0)]
+    z[:, ::7] = torch.tensor([-87.0, -87.5, -88.0, 88.0, -40.0, 0.0], device=DEV).repeat(-(-z[:, ::7].numel() // 6))[:z[:, ::7].numel()].view_as(z[:, ::7])
+    w = (0.3 * torch.randn(DV, generator=g, device=DEV)).bfloat16()
+    outs = []
+    for shift in (0, 1):                           # rows on 8 bytes, and one element off
+        a, b, c = [torch.empty(t.numel() + 1, dtype=torch.bfloat16, device=DEV)[shift:shift + t.numel()].view_as(t).copy_(t) for t in (o, z, w)]
+        y = torch.empty_like(o)
+        assert ops.lib.blz_gated_rmsnorm(_ptr(a), _ptr(b), b.stride(0), _ptr(c), _ptr(y), T, Hv, DV, 1e-6, flags, VP(0)) == 0
+        outs.append(y)
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1])
+    x, zd = o.double().view(T, Hv, DV), z.double().view(T, Hv, DV)
+    want = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * (w.double() + (flags & 1)) * zd.sigmoid() * (1 if flags & 2 else zd)
+    # half a step of bf16 (8 bits: up to 2^-8 of the value), and the fast exponential: 2 ulp and, of its argument, 88 * 2^-24
+    err = (outs[0].double().view_as(want) - want).abs()
+    assert (err <= want.abs() * (2.0 ** -8 + 2e-5) + 1e-40).all()
