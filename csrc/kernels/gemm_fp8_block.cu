@@ -210,19 +210,22 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 // feature tiles (40 of the 148 SMs worked on 5120 x 8192): the K range is split over a cluster of `ks` CTAs, whose fp32 sums meet
 // in distributed shared memory; CTA r owns row-column groups [r * ng / ks, (r + 1) * ng / ks) and adds the parts in rank order.
 // 192 threads (producer, MMA issuer, four promotion warps: lane = feature, column = row of X), two CTAs per SM.  A k block's 64
-// activation scales ride behind the operands in a ring of eight: they outlive the operand stage (the promotion is at most four
-// blocks behind the MMA, the producer at most four ahead of it).  Weight bytes bound it.
+// activation scales ride behind the operands in a ring of their own, since they outlive the operand stage.  A slot is free once all
+// promotion warps have read it.  The producer knows that of the blocks before i - STAGES - NBUF only, when it fills the slot of block
+// i: it has seen the MMA of block i - STAGES complete, which waited until the accumulator of block i - STAGES - NBUF was handed back,
+// and a warp hands that back before it reads the block's scales, but after those of the block before.  Weight bytes bound it.
 // Measured, us, this kernel / the one above: 16 rows 10240 x 5120 18.8 / 18.5, 5120 x 8192 17.5 / 24.4, 51200 x 5120 57 / 64, 5120 x
 // 25600 34 / 76; 64 rows 25.1 / 18.5, 22.4 / 24.4, 71 / 64, 45 / 76: beyond 32 rows it is taken for layers of few tiles only.
 struct FrCfg {
   static constexpr int W_BYTES = 128 * 128, X_BYTES = 64 * 128, STAGES = 4;
   static constexpr int NBUF = 4, TMEM_COLS = NBUF * 64;
-  static constexpr int SA_SLOTS = 8, SA_BYTES = 64 * 4;
+  static constexpr int SA_SLOTS = 16, SA_BYTES = 64 * 4;
   static constexpr int RING = STAGES * (W_BYTES + X_BYTES);
-  static constexpr int SMEM = RING + SA_SLOTS * SA_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SMEM = RING + SA_SLOTS * SA_BYTES + 1024 /*align*/ + 384 /*barriers*/;
   static constexpr int GROUP = 8;                      // row columns that change hands together in the reduction
   static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
-  static_assert(STAGES + NBUF <= SA_SLOTS, "a scale slot is read before it is filled again");
+  static_assert((2 * STAGES + 2 * NBUF + SA_SLOTS + 2) * 8 + 8 <= 384, "barriers");
+  static_assert(STAGES + NBUF < SA_SLOTS, "a scale slot is read before it is filled again");
 };
 
 __global__ void __launch_bounds__(192, 2)

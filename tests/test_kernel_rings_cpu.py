@@ -1,0 +1,33 @@
+"""Order of a kernel's ring buffers, from the waits in its source: a slot is read before it is filled again."""
+import os
+import re
+
+SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "kernels", "gemm_fp8_block.cu")
+
+
+def test_scales_of_few_rows_are_read_before_their_slot_is_filled_again():
+    """The events of a CTA of the FP8 product of few rows (copy of a block's scales, MMA, hand-back of its accumulator, reading of its
+    scales) and what each waits for.  A warp that is held up before it reads must not find the scales of a later block."""
+    text = open(SRC).read()
+    cfg = text[text.index("struct FrCfg"):]
+    stages, nbuf, slots = [int(re.search(rf"\b{n} = (\d+)", cfg).group(1)) for n in ("STAGES", "NBUF", "SA_SLOTS")]
+    body = text[text.index("gemm_fp8_rows_kernel("):]
+    back_first = body.index("mbar_arrive(&part_empty") < body.index("= sa[")      # the accumulator is handed back before the scales are read
+    n, before = 4 * slots, {}
+    for i in range(n):
+        before["copy", i] = [("copy", i - 1), ("mma", i - stages)]                # the operand stage is free
+        before["mma", i] = [("mma", i - 1), ("copy", i), ("back", i - nbuf)]
+        first, second = ("back", "read") if back_first else ("read", "back")
+        before[first, i] = [("mma", i), (second, i - 1)]
+        before[second, i] = [(first, i)]
+
+    def earlier(event):
+        seen, todo = set(), [event]
+        while todo:
+            for e in before.get(todo.pop(), []):
+                if e[1] >= 0 and e not in seen:
+                    seen.add(e)
+                    todo.append(e)
+        return seen
+    for i in range(slots, n):
+        assert ("read", i - slots) in earlier(("copy", i)), f"block {i} overwrites scales that may not have been read"
