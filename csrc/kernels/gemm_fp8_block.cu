@@ -214,8 +214,6 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 // promotion warps have read it.  The producer knows that of the blocks before i - STAGES - NBUF only, when it fills the slot of block
 // i: it has seen the MMA of block i - STAGES complete, which waited until the accumulator of block i - STAGES - NBUF was handed back,
 // and a warp hands that back before it reads the block's scales, but after those of the block before.  Weight bytes bound it.
-// Measured, us, this kernel / the one above: 16 rows 10240 x 5120 18.8 / 18.5, 5120 x 8192 17.5 / 24.4, 51200 x 5120 57 / 64, 5120 x
-// 25600 34 / 76; 64 rows 25.1 / 18.5, 22.4 / 24.4, 71 / 64, 45 / 76: beyond 32 rows it is taken for layers of few tiles only.
 struct FrCfg {
   static constexpr int W_BYTES = 128 * 128, X_BYTES = 64 * 128, STAGES = 4;
   static constexpr int NBUF = 4, TMEM_COLS = NBUF * 64;
@@ -414,16 +412,36 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   }
 }
 
-// CTAs that share a feature tile: powers of two (odd clusters pack badly), both slots of every SM at most, a group of columns each.
+// CTAs that share a feature tile (1, 2, 4 or 8; odd clusters pack badly), 0: the kernel above is the faster one.
+// The kernel above walks all k blocks in one CTA per 128 features (5 us + 0.3 us a block while they fit on the chip at once), this one
+// a part of them, for an exchange of 4 us that grows with the number of CTAs.  Clusters of four find room up to 8/5 CTAs per SM (beyond,
+// some wait for a second turn), and more than 32 rows double the exchange.  Time over the kernel above's at N x K, 16 - 32 rows:
+//   four CTAs    N <= 4096: K 1024 1.04 - 1.10, 2048 0.86 - 0.95, 4096 0.67 - 0.77, 7168 0.55 - 0.64; N 5120, 7168: K 3072 1.01 - 1.05,
+//                4096 0.89 - 0.97, 5120 0.79 - 0.89, 25600 0.47; N 9216: K 5120 1.04 - 1.34
+//   two          N 5120 - 9216: K 2048 0.94 - 1.04, 3072 0.84 - 0.98, 4096 0.77 - 0.95, 5120 0.72 - 0.90; N 12288 - 18432: K 4096
+//                0.88 - 0.94 (16 rows), 0.85 - 0.97 (24), 0.91 - 1.11 (28 - 32), 5120 1.00 - 1.06 (28 - 32), 7168 0.78 - 0.96
+//   one          N 24576, 36864 (more tiles than SMs): K 1024 - 7168 0.61 - 0.83
+// and at 36 - 64 rows:
+//   eight        N <= 1024: K 2048 1.06 - 1.09, 3072 0.90 - 0.93, 7168 0.60 - 0.62; N 2048: K 4096 1.01
+//   four         N 2048 - 4096: K 2048 1.04 - 1.11, 3072 0.92 - 0.99, 7168 0.69 - 0.75; N 5120, 7168: K 5120 1.03 - 1.07, 7168
+//                0.94 - 0.98, 8192 0.91, 25600 0.59; N 9216: K 7168 1.42
+// The fp32 sums of a row's parts differ from the sum block by block in their roundings: error against 64 bits 6e-8 - 1.4e-7 where that
+// has 8e-8 - 2.6e-7 (K 2048 - 25600).
 static int fp8_rows_ks(const FbParams& p) {
-  const int tiles = (p.N + 127) / 128, nkb = p.K / 128, ng = ((p.M + 31) & ~31) / FrCfg::GROUP;
-  int ks = 1;
-  while (ks * 2 <= ng && ks * 2 <= nkb && tiles * ks * 2 <= 2 * sm_count()) ks *= 2;
-  return ks;
+  const int tiles = (p.N + 127) / 128, nkb = p.K / 128, sms = sm_count();
+  const bool four = tiles * 4 <= sms, four_fit = tiles * 4 <= sms * 8 / 5;
+  if (p.M > 32) {
+    if (nkb >= 24 && four) return tiles * 16 <= sms ? 8 : 4;
+    return nkb >= 56 && four_fit ? 4 : 0;
+  }
+  if (tiles > sms) return 1;
+  if (four) return nkb >= 16 ? 4 : 0;
+  if (tiles * 2 <= sms) return nkb >= 40 && four_fit ? 4 : nkb >= 24 ? 2 : 0;
+  return nkb >= (p.M <= 24 ? 32 : 56) ? 2 : 0;
 }
 
-static cudaError_t launch_fp8_rows(const FbParams& p, const void* A, long long lda, const void* B, long long ldb, cudaStream_t stream) {
-  const int tiles = (p.N + 127) / 128, ks = fp8_rows_ks(p);
+static cudaError_t launch_fp8_rows(const FbParams& p, int ks, const void* A, long long lda, const void* B, long long ldb, cudaStream_t stream) {
+  const int tiles = (p.N + 127) / 128;
   CUtensorMap tmW, tmX;
   cudaError_t e = encode_tmap(&tmW, B, 1, (uint64_t)p.K, p.N, ldb, 128, 128, 3);
   if (e != cudaSuccess) return e;
@@ -499,8 +517,10 @@ BLZ_API int blz_gemm_fp8_block(const void* A, long long lda, const void* B, long
   p.sa = sa; p.ld_sa = ld_sa; p.sb = sb; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.status = status_word();
   // the scales' rows are copied by 16 bytes: they start and step on them (blz_quant_fp8_block's do)
-  if (M <= 64 && ld_sa % 4 == 0 && (reinterpret_cast<uintptr_t>(sa) & 15) == 0 && (M <= 32 || fp8_rows_ks(p) >= 4))
-    return (int)launch_fp8_rows(p, A, lda, B, ldb, stream);
+  if (M <= 64 && ld_sa % 4 == 0 && (reinterpret_cast<uintptr_t>(sa) & 15) == 0) {
+    const int ks = fp8_rows_ks(p);
+    if (ks > 0) return (int)launch_fp8_rows(p, ks, A, lda, B, ldb, stream);
+  }
   CUtensorMap tmA, tmB;
   cudaError_t e = encode_tmap(&tmA, A, 1, (uint64_t)K, M, lda, 128, 128, 3);
   if (e != cudaSuccess) return (int)e;

@@ -150,8 +150,8 @@ def test_elementwise(ops, T, H, shift):      # noqa: F811
     assert _rel(ops.mul_sigmoid(a.clone(), b), want) < 4e-3
 
 
-@pytest.mark.parametrize("M", [1, 31, 32, 33, 64, 65])
-@pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (512, 25600), (1024, 5120), (5120, 8192), (40000, 256)])
+@pytest.mark.parametrize("M", [1, 24, 25, 31, 32, 33, 64, 65])
+@pytest.mark.parametrize("N,K", [(128, 128), (200, 384), (512, 25600), (1024, 5120), (2200, 2176), (4100, 3328), (5120, 8192), (6144, 3072), (12288, 4096), (40000, 256)])
 def test_fp8_block_product_of_few_rows(ops, M, N, K):      # noqa: F811
     """Rows on the MMA's columns and K over a cluster, against the stored codes and scales in 64 bits."""
     g = torch.Generator(device=DEV).manual_seed(11)
