@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
     const int n = max(min(tiles_all, t0 + per) - t0, 0);
     const int slot = p.slots[b];
     if (n == 0) {
-      // a run without a tile: nothing to add
-      if (warp == 2)
+      // a run without a tile: nothing to add.  (Without splits there is nowhere to say so: rows that see no key are left alone.)
+      if (p.splits > 1 && warp == 2)
         for (int r = lane; r < nrows; r += 32)
           *reinterpret_cast<float2*>(&p.part_ml[((size_t)w * NMAX + r) * 2]) = make_float2(-INFINITY, 0.f);
       continue;

@@ -54,6 +54,41 @@ def test_decode_attention_runs_of_tiles(ops, Hq, Hkv, ctxs, q):      # noqa: F81
     assert err.max().item() < 0.15                 # row by row: an item that got a wrong piece is off by its size
 
 
+def _raw_decode(ops, kv, q, out, ctxs, Hq, Hkv, splits, po, pm):      # noqa: F811
+    """``blz_attn_decode_tree`` for one row per sequence, as another program calls it."""
+    from blaze_b200.ops.cuda_ops import VP, _ptr
+    B, D, pool = len(ctxs), 128, kv.kv[0]
+    slots, q_start, ctx = [torch.tensor(v, dtype=torch.int32, device=DEV) for v in (range(B), range(B + 1), ctxs)]
+    rc = ops.lib.blz_attn_decode_tree(_ptr(q), _ptr(out), _ptr(pool), _ptr(kv.block_table), _ptr(slots), _ptr(q_start), _ptr(ctx), B, Hq, Hkv, D,
+                                      kv.block_table.stride(0), pool.stride(0), pool.stride(1), D ** -0.5, 1.0, 1.0, 16, 1, 1, Hq // Hkv, splits,
+                                      _ptr(po), _ptr(pm), 0, VP(0), VP(0), VP(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    assert rc == 0 and ops.take_status() == 0
+
+
+def _decode_inputs(Hq, Hkv, ctxs):
+    """A cache with the sequences' keys and values (finite codes) and one query row each."""
+    cfg = ModelConfig(hidden_size=Hq * 128, num_heads=Hq, num_kv_heads=Hkv, head_dim=128, num_layers=1, rope=RopeConfig(theta=1e6))
+    cfg.layer_types = ["full_attention"]
+    g = torch.Generator(device=DEV).manual_seed(3)
+    pages = (max(ctxs) + 15) // 16 + 1
+    kv = KVCache(cfg, 1 + len(ctxs) * pages, len(ctxs), pages, "fp8", DEV, "umma")
+    for b in range(len(ctxs)):
+        kv.set_pages(b, list(range(1 + b * pages, 1 + (b + 1) * pages)))
+    kv.flush()
+    kv.kv[0][1:].copy_(torch.randn(kv.kv[0][1:].shape, generator=g, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8))
+    return kv, torch.randn(len(ctxs), Hq, 128, generator=g, device=DEV).bfloat16()
+
+
+def test_decode_attention_leaves_rows_without_a_key_alone(ops):      # noqa: F811
+    """A sequence whose row sees no key, without splits and without scratch: nothing is written for it, nor anywhere else."""
+    kv, q = _decode_inputs(8, 2, [300, 16, 1500])
+    out, want = [torch.full_like(q, 7.0) for _ in range(2)]
+    _raw_decode(ops, kv, q, out, [300, 0, 1500], 8, 2, 1, None, None)
+    _raw_decode(ops, kv, q, want, [300, 16, 1500], 8, 2, 1, None, None)
+    assert (out[1] == 7).all() and torch.equal(out[[0, 2]], want[[0, 2]]) and not (want == 7).all()
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,qlens,splits", [
     (8, 2, [17], [17], 0), (32, 8, [128, 129, 33], [128, 129, 33], 0), (8, 1, [1100, 40], [300, 40], 1),      # blocks of 128 rows and parts
     (4, 4, [700], [513], 1), (16, 2, [2000, 90], [70, 60], 3), (32, 4, [300], [40], 8),                        # split key ranges, some empty
