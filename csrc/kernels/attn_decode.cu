@@ -90,6 +90,8 @@ __device__ __forceinline__ int row_of_lane(int lane) {        // -1: another lan
   return (lane & ((32 >> BITS) - 1)) ? -1 : (int)(__brev((unsigned)lane) >> 27) & (R - 1);
 }
 
+__device__ __forceinline__ void put_pair(float* p, float a, float b) { p[0] = a; p[1] = b; }      // (the caller's array: on 4 bytes)
+
 template <int N>
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&r)[N]) {
   if constexpr (N == 4) tmem_ld4(taddr, r);
@@ -208,7 +210,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
       // a run without a tile: nothing to add.  (Without splits there is nowhere to say so: rows that see no key are left alone.)
       if (p.splits > 1 && warp == 2)
         for (int r = lane; r < nrows; r += 32)
-          *reinterpret_cast<float2*>(&p.part_ml[((size_t)w * NMAX + r) * 2]) = make_float2(-INFINITY, 0.f);
+          put_pair(&p.part_ml[((size_t)w * NMAX + r) * 2], -INFINITY, 0.f);
       continue;
     }
 
@@ -507,7 +509,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
             s_off[qd][r] = (r0 + tq) * p.Hq + kh * group + (row0 + r - tq * group);
           } else {
             s_off[qd][r] = w * NMAX + r;
-            if (qd == 0 && r < nrows) *reinterpret_cast<float2*>(&p.part_ml[((size_t)w * NMAX + r) * 2]) = make_float2(m, l);
+            if (qd == 0 && r < nrows) put_pair(&p.part_ml[((size_t)w * NMAX + r) * 2], m, l);
           }
           s_f[qd][r] = make_float2(fa, fb);
         }
@@ -547,7 +549,8 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
 // Merge an item's runs: one block per (sequence, kv head, row block), a warp per row, four dims per lane.  The lanes weigh the runs
 // side by side, and the runs' sums are added up (in their order) by loads that do not wait for one another; with a thread per
 // dim, a row after the other and a branch around every run it took 10.5 us for 48 items of 8 runs, now 5.3.
-template <int NMAX>
+// WIDE: the caller's arrays and output lie on 16 bytes (else they are read and written by elements).
+template <int NMAX, bool WIDE>
 __global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) {
   pdl_trigger();
   pdl_wait();
@@ -564,7 +567,9 @@ __global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) 
   for (int r = threadIdx.x >> 5; r < nrows; r += blockDim.x >> 5) {
     auto at = [&](int i) { return ((size_t)blockIdx.x * p.splits + i) * NMAX + r; };
     auto max_sum = [&](int i) {
-      return i < p.splits ? *reinterpret_cast<const float2*>(&p.part_ml[at(i) * 2]) : make_float2(-INFINITY, 0.f);
+      const float* ml = &p.part_ml[at(i < p.splits ? i : 0) * 2];
+      const float2 v = WIDE ? *reinterpret_cast<const float2*>(ml) : make_float2(ml[0], ml[1]);
+      return i < p.splits ? v : make_float2(-INFINITY, 0.f);
     };
     float m = -INFINITY, l = 0.f;
     for (int i = lane; i < p.splits; i += 32) { const float2 ml = max_sum(i); if (ml.y > 0.f) m = fmaxf(m, ml.x); }
@@ -578,15 +583,23 @@ __global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) 
       for (int i = 0; i < here; ++i) {
         const float f = __shfl_sync(0xffffffffu, mine, i), ls = __shfl_sync(0xffffffffu, ml.y, i);
         // (a run without a visible key has written no outputs)
-        const float4 x = ls > 0.f ? *reinterpret_cast<const float4*>(&p.part_o[at(i0 + i) * D + lane * 4]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* po = &p.part_o[at(i0 + i) * D + lane * 4];
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ls > 0.f) x = WIDE ? *reinterpret_cast<const float4*>(po) : make_float4(po[0], po[1], po[2], po[3]);
         l = fmaf(ls, f, l);
         o.x = fmaf(x.x, f, o.x); o.y = fmaf(x.y, f, o.y); o.z = fmaf(x.z, f, o.z); o.w = fmaf(x.w, f, o.w);
       }
     }
     const int R = row0 + r, tq = R / group, hq = kh * group + R % group;
     auto fin = [&](float v) { return l > 0.f ? v * p.v_scale / l : 0.f; };
-    *reinterpret_cast<uint2*>(&p.out[((size_t)(r0 + tq) * p.Hq + hq) * D + lane * 4]) =
-        make_uint2(pack_bf16x2(fin(o.x), fin(o.y)), pack_bf16x2(fin(o.z), fin(o.w)));
+    __nv_bfloat16* dst = &p.out[((size_t)(r0 + tq) * p.Hq + hq) * D + lane * 4];
+    if constexpr (WIDE) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(fin(o.x), fin(o.y)), pack_bf16x2(fin(o.z), fin(o.w)));
+    } else {
+      const float v[4] = {fin(o.x), fin(o.y), fin(o.z), fin(o.w)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dst[j] = __float2bfloat16(v[j]);
+    }
   }
 }
 
@@ -599,7 +612,8 @@ static cudaError_t launch_form(K kernel, PerDeviceOnce& configured, const AttnPa
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   e = launch_pdl(kernel, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
   if (e != cudaSuccess || p.splits == 1) return e;
-  return launch_pdl(attn_decode_combine_kernel<16>, dim3(items), dim3(512), 0, stream, p);
+  const bool wide = !((reinterpret_cast<uintptr_t>(p.part_o) | reinterpret_cast<uintptr_t>(p.part_ml) | reinterpret_cast<uintptr_t>(p.out)) & 15);
+  return launch_pdl(wide ? attn_decode_combine_kernel<16, true> : attn_decode_combine_kernel<16, false>, dim3(items), dim3(512), 0, stream, p);
 }
 
 // The most rows of any work item choose the kernel (16 rows an item).  Draft trees need the mask that the 4-row one leaves out.

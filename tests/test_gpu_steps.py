@@ -89,6 +89,20 @@ def test_decode_attention_leaves_rows_without_a_key_alone(ops):      # noqa: F81
     assert (out[1] == 7).all() and torch.equal(out[[0, 2]], want[[0, 2]]) and not (want == 7).all()
 
 
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_decode_attention_merges_runs_at_any_address(ops, shift):      # noqa: F811
+    """Scratch and output that lie on their elements' size only."""
+    ctxs, splits = [700, 16, 1500], 4
+    kv, q = _decode_inputs(8, 2, ctxs)
+    n, outs = len(ctxs) * 2 * splits * 16, []
+    for s in (0, shift):
+        po, pm = [torch.empty(m + s, dtype=torch.float32, device=DEV)[s:] for m in (n * 128, n * 2)]
+        out = torch.zeros(q.numel() + s, dtype=torch.bfloat16, device=DEV)[s:].view_as(q)
+        _raw_decode(ops, kv, q, out, ctxs, 8, 2, splits, po, pm)
+        outs.append(out)
+    assert torch.equal(*outs) and outs[0].float().abs().amax(-1).min().item() > 0
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,qlens,splits", [
     (8, 2, [17], [17], 0), (32, 8, [128, 129, 33], [128, 129, 33], 0), (8, 1, [1100, 40], [300, 40], 1),      # blocks of 128 rows and parts
     (4, 4, [700], [513], 1), (16, 2, [2000, 90], [70, 60], 3), (32, 4, [300], [40], 8),                        # split key ranges, some empty
