@@ -577,12 +577,12 @@ __global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) 
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int i0 = 0; i0 < p.splits; i0 += 32) {
       const float2 ml = max_sum(i0 + lane);
-      const float mine = ml.y > 0.f ? exp2f(ml.x - m) : 0.f;
+      const float mine = ml.y > 0.f ? exp2f(ml.x - m) : 0.f, sum = ml.y > 0.f ? ml.y : 0.f;
       const int here = min(32, p.splits - i0);
 #pragma unroll 8
       for (int i = 0; i < here; ++i) {
-        const float f = __shfl_sync(0xffffffffu, mine, i), ls = __shfl_sync(0xffffffffu, ml.y, i);
-        // (a run without a visible key has written no outputs)
+        const float f = __shfl_sync(0xffffffffu, mine, i), ls = __shfl_sync(0xffffffffu, sum, i);
+        // (a run without a visible key has written no outputs; one whose sum is not a number, for a key that is none, does not count)
         const float* po = &p.part_o[at(i0 + i) * D + lane * 4];
         float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
         if (ls > 0.f) x = WIDE ? *reinterpret_cast<const float4*>(po) : make_float4(po[0], po[1], po[2], po[3]);

@@ -103,6 +103,24 @@ def test_decode_attention_merges_runs_at_any_address(ops, shift):      # noqa: F
     assert torch.equal(*outs) and outs[0].float().abs().amax(-1).min().item() > 0
 
 
+def test_decode_attention_runs_that_are_not_a_number(ops):      # noqa: F811
+    """Keys that are not a number spoil the run that they lie in: the merged row is that of the other runs."""
+    ctxs, splits, Hkv = [512], 4, 2
+    kv, q = _decode_inputs(8, Hkv, ctxs)
+    n = Hkv * splits * 16
+    po, pm = [torch.empty(m, dtype=torch.float32, device=DEV) for m in (n * 128, n * 2)]
+    got = torch.zeros_like(q)
+    kv.kv[0][kv.block_table[0, 16:24].long(), :, 0] = 0x7F       # the third run's keys
+    _raw_decode(ops, kv, q, got, ctxs, 8, Hkv, splits, po, pm)
+    ml = pm.view(Hkv, splits, 16, 2)[:, :, :4]
+    sums = po.view(Hkv, splits, 16, 128)[:, :, :4].double()
+    assert ml[:, 2, :, 1].isnan().all() and (ml[:, [0, 1, 3], :, 1] > 0).all()
+    f = torch.exp2(ml[:, [0, 1, 3], :, 0].double() - ml[:, [0, 1, 3], :, 0].amax(1, keepdim=True).double())[..., None]
+    want = ((sums[:, [0, 1, 3]] * f).sum(1) / (ml[:, [0, 1, 3], :, 1, None].double() * f).sum(1)).view(1, 8, 128)
+    # half a step of bf16; a few roundings of 24 bits per run, of terms that may cancel
+    assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-5).all()
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,qlens,splits", [
     (8, 2, [17], [17], 0), (32, 8, [128, 129, 33], [128, 129, 33], 0), (8, 1, [1100, 40], [300, 40], 1),      # blocks of 128 rows and parts
     (4, 4, [700], [513], 1), (16, 2, [2000, 90], [70, 60], 3), (32, 4, [300], [40], 8),                        # split key ranges, some empty
