@@ -357,7 +357,7 @@ class Engine:
                 r += len(c.tokens)
         plain = not any(c.rope_delta or c.pos3 is not None or c.embeds or c.logit_at is not None for c in chunks)     # captured steps carry text rows only
         graphable = (plain and hidden_in is None and self.ecfg.use_graphs and self.device.type == "cuda" and decode_only
-                     and (mode == "greedy" or (mode == "logits" and self._logits_graphable(chunks)))
+                     and (mode == "greedy" or (mode == "logits" and not feedback and self._logits_graphable(chunks)))
                      and self.model.is_first_stage and self.model.is_last_stage and self.model.ops.is_cuda)
         # verify steps of equal-length chains (the scheduler pads drafts to one length) replay a captured graph as well
         L = len(chunks[0].tokens) if chunks else 0
@@ -457,8 +457,9 @@ class Engine:
         """A decode step whose logits the sampler takes replays a captured step up to the final norm; the head runs after it, into a
         tensor of its own (the logits of a large batch would otherwise stay allocated for every bucket, or be copied out).  Issuing
         a step's launches one by one takes 2.0 ms of host time for 12 layers of the 8B shape, against 1.2 ms on the GPU at one
-        sequence and 2.9 ms at 256; 48 layers with experts take 25 ms.  On one rank only, and for rows without a deferred state."""
-        return (self.model.tp.world == 1 and not self.model.capture_layers
+        sequence and 2.9 ms at 256.  On one rank only, for rows without a deferred state, and not where something follows the
+        layers' work step by step, or the layers read the contexts' lengths on the host (a sparse-attention indexer)."""
+        return (self.model.tp.world == 1 and not self.model.observed and not self.model.cfg.indexer_heads
                 and all(c.want_logits == 1 and not c.defer_state and c.parents is None for c in chunks))
 
     def _key_splits(self, n: int) -> int:

@@ -965,6 +965,12 @@ class Model:
                 y = ops.add(y, s)
         return y, ("partial" if routed_partial else "full")
 
+    @property
+    def observed(self) -> bool:
+        """Something follows the layers' work step by step: hidden rows kept for a drafter, routing statistics (which would count a captured
+        step's padding), dumps, phase timers."""
+        return bool(self.capture_layers or self.heat is not None or _DUMP_DIR or _PROFILE_PHASES)
+
     # ------------------------------------------------------------------ head
     def final_hidden(self, x: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
         if rows is not None:

@@ -1,0 +1,46 @@
+"""Which decode steps with logits may replay a captured step: the engine's rules, which need no GPU."""
+import pytest
+import torch
+
+from blaze_b200.config import named_config
+from blaze_b200.llm import LLM
+from blaze_b200.models import qwen3
+
+
+def _engine(name="tiny", **kw):
+    return LLM(named_config(name), device="cpu", dtype=torch.float32, max_seqs=4, max_model_len=128, seed=0, **kw).engine
+
+
+def _decode_step(eng):
+    return eng.plan([(eng.open_from(), [1], 1) for _ in range(2)])
+
+
+def test_steps_that_something_follows_are_launched_one_by_one(monkeypatch):
+    """Dumps, phase timers, routing statistics and kept hidden rows come from the layer loop itself, and an indexer reads the contexts'
+    lengths on the host: a replayed step would leave them out, count its padding, or select keys for other lengths."""
+    eng = _engine()
+    step = _decode_step(eng)
+    assert eng._logits_graphable(step)
+    for name, value in (("_DUMP_DIR", "/nowhere"), ("_PROFILE_PHASES", True)):
+        with monkeypatch.context() as m:
+            m.setattr(qwen3, name, value)
+            assert not eng._logits_graphable(step), name
+    for obj, name, value in ((eng.model, "capture_layers", [0]), (eng.model, "heat", object()), (eng.model.cfg, "indexer_heads", 2)):
+        with monkeypatch.context() as m:
+            m.setattr(obj, name, value)
+            assert not eng._logits_graphable(step), name
+    assert eng._logits_graphable(step)
+
+
+def test_routing_statistics_keep_sampled_steps_uncaptured():
+    eng = _engine("tiny-hybrid", expert_heat=True)
+    assert eng.model.heat is not None and not eng._logits_graphable(_decode_step(eng))
+
+
+@pytest.mark.parametrize("change", [{"want_logits": 0}, {"defer_state": True}, {"parents": [-1]}])
+def test_rows_that_a_captured_step_does_not_hold(change):
+    eng = _engine()
+    step = _decode_step(eng)
+    for k, v in change.items():
+        setattr(step[1], k, v)
+    assert not eng._logits_graphable(step)
