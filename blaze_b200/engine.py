@@ -12,7 +12,7 @@ from __future__ import annotations
 import threading
 import time
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Sequence, Tuple
+from typing import Dict, List, Optional, Sequence, Set, Tuple
 
 import numpy as np
 import torch
@@ -151,6 +151,7 @@ class Engine:
         self.seqs: Dict[int, Seq] = {}
         self._graphs: Dict[Tuple, "_Graph"] = {}
         self._seen: Dict[Tuple, int] = {}
+        self._limits: Optional[Set[int]] = None      # see _expert_limits
         self._pinned = None
         if self.device.type == "cuda":
             self._pinned = [torch.empty(1 << 19, dtype=torch.int32, pin_memory=True) for _ in range(2)]
@@ -462,6 +463,26 @@ class Engine:
         return (self.model.tp.world == 1 and not self.model.observed and not self.model.cfg.indexer_heads
                 and all(c.want_logits == 1 and not c.defer_state and c.parents is None for c in chunks))
 
+    def _sampled_bucket(self, n: int) -> int:
+        """Rows of the captured step with logits for ``n`` sequences: ``n`` itself up to 16, above in eighths of a power of two.  The rows
+        that fill a step up are computed and routed like the others, and what such a step replaces was not padded, only launched one
+        by one: with powers of two alone 65 sequences would compute 128 rows, and five take up to a fifth more experts' weights.  The
+        kernels choose their forms at powers of two and, for experts, at the row limits below, so a step's form does not depend on
+        its padding either.  Per step, us, launched one by one / replayed in these buckets / in powers of two, contexts of 300 - 600:
+        12 layers of the 8B shape, NVFP4: 5 sequences 1968 / 1276 / 1322, 65: 2306 / 1579 / 1606, 257: 3700 / 2740 / 3056; in bf16 65:
+        2475 / 2247 / 2278, 257: 4030 / 3713 / 4358; 6 layers with 128 experts, NVFP4: 5: 1704 / 878 / 911, 129: 2543 / 1294 / 1480, 257:
+        3412 / 1717 / 1968."""
+        if n <= 16:
+            return n
+        step = 1 << ((n - 1).bit_length() - 4)
+        return min([-(-n // step) * step] + [r for r in self._expert_limits() if r >= n])
+
+    def _expert_limits(self) -> Set[int]:
+        if self._limits is None:
+            ops, moe = self.model.ops, [L.mlp for L in self.model.layers if getattr(L.mlp, "experts", None) is not None]
+            self._limits = {ops.moe_narrow_tokens(M.experts, M.top_k) for M in moe}
+        return self._limits
+
     def _key_splits(self, n: int) -> int:
         """Runs the attention kernels cut the keys of a decode step of ``n`` sequences into.  A captured step with logits keeps the
         number that ``n`` sequences get, not the one of its padded batch: partial sums are rounded, so the logits of a step would
@@ -475,7 +496,7 @@ class Engine:
 
     def _forward_graph(self, chunks: Sequence[SeqChunk], feedback: bool = False, rows_per_seq: int = 1, mode: str = "greedy"):
         B = len(chunks)
-        bucket = self._bucket(B)
+        bucket = self._sampled_bucket(B) if mode == "logits" else self._bucket(B)
         key = (("decode", bucket) if rows_per_seq == 1 and mode == "greedy" else
                ("logits", bucket, self._key_splits(B)) if mode == "logits" else ("verify", bucket, rows_per_seq, mode))
         g = self._graphs.get(key)

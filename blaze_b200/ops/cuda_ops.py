@@ -1405,6 +1405,11 @@ class CudaOps:
                     "moe_combine")
         return out
 
+    def moe_narrow_tokens(self, experts, k: int) -> int:
+        """The most tokens of a step whose routed rows (``k`` per token) take the narrow expert kernel."""
+        rows = self.MOE_NARROW_ROWS * 8 // 3 if self.pack_experts(experts)["gate_up"]["kind"] == 2 else self.MOE_NARROW_ROWS
+        return rows * experts.count // k
+
     def moe_rows(self, x, topk_w, topk_id, experts, shared=None, gate=None) -> RoutedRows:
         """The routed experts' outputs as rows (:meth:`branch_norm` and :meth:`branch_step` sum them up, with ``shared`` added, there times
         the sigmoid of the logits ``gate``)."""
@@ -1429,8 +1434,7 @@ class CudaOps:
         row_map = torch.empty(T, k, dtype=torch.int32, device=dev)
         self._check(self.lib.blz_moe_plan(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), n_exp,
                                           max_tiles, self._stream()), "moe_plan")
-        narrow_rows = self.MOE_NARROW_ROWS * 8 // 3 if gu["kind"] == 2 else self.MOE_NARROW_ROWS
-        narrow = T * k <= narrow_rows * n_exp and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
+        narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)
         if mode:
             proxy = Linear(gu["fmt"], gu["N"], gu["K"])

@@ -20,8 +20,8 @@ def _rel(a, b):
 
 
 def test_logits_steps_replay_a_captured_step():
-    """A decode step with logits: the first of a batch size runs launch by launch, the others replay it; the tensors handed out
-    stay as they were."""
+    """A decode step with logits: the first of a batch size runs launch by launch, the others replay it; what a step handed out stays as
+    it was when the next one runs."""
     from blaze_b200.llm import LLM
     cfg = ModelConfig(vocab_size=2048, hidden_size=512, num_layers=2, num_heads=8, num_kv_heads=2, head_dim=128, intermediate_size=1024,
                       rope=RopeConfig(theta=1e6))
@@ -35,11 +35,64 @@ def test_logits_steps_replay_a_captured_step():
         for s, n in zip(seqs, base):
             s.length = n
         outs.append(eng.forward(eng.plan([(s, [tok], 1) for s in seqs]), "logits"))
-    assert any(k[:2] == ("logits", 4) for k in eng._graphs) and outs[0].shape == (3, 2048) and outs[0].dtype == torch.float32
-    assert torch.equal(outs[1], outs[2]) and not torch.equal(outs[2], outs[3])
-    assert torch.equal(outs[1], outs[0])           # launch by launch and replayed: the keys are split alike
+        kept = outs[-1].clone() if len(outs) == 3 else kept if len(outs) > 3 else None
+    assert any(k[:2] == ("logits", 3) for k in eng._graphs) and outs[0].shape == (3, 2048) and outs[0].dtype == torch.float32
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2]) and not torch.equal(outs[2], outs[3]) and torch.equal(outs[2], kept)
     some = eng.forward(eng.plan([(seqs[0], [1], 1), (seqs[1], [1], 0)]), "logits")
     assert some.shape[0] == 1                      # rows without logits: not a step of that kind
+
+
+def _steps_engine(kind):
+    """A small model of a kind with 32 sequences open, their contexts (60 to 1400 tokens) filled with random keys, values and states."""
+    from blaze_b200.llm import LLM
+    D = 256 if kind == "recurrent" else 128
+    cfg = ModelConfig(vocab_size=2048, hidden_size=512, num_layers=2, num_heads=8, num_kv_heads={"dense": 8, "experts": 4, "recurrent": 1}[kind], head_dim=D,
+                      intermediate_size=1024, rope=RopeConfig(theta=1e6))
+    cfg.layer_types = ["full_attention"] * 2
+    if kind == "experts":
+        cfg.num_experts, cfg.num_experts_per_tok, cfg.moe_intermediate_size = 16, 4, 256
+    if kind == "recurrent":
+        cfg.layer_types = ["linear_attention", "full_attention"]
+        cfg.linear_num_key_heads, cfg.linear_num_value_heads, cfg.linear_key_head_dim, cfg.linear_value_head_dim = 2, 4, 128, 128
+        cfg.linear_conv_kernel_dim = 4
+    eng = LLM(cfg, weight_format="mxfp8" if kind == "recurrent" else "nvfp4", max_seqs=32, max_model_len=2048, kv_tokens=33 * 1536, seed=4).engine
+    g = torch.Generator(device=DEV).manual_seed(1)
+    ctxs = [60 + (i * 743) % 1341 for i in range(32)]
+    seqs = [eng.open_from() for _ in ctxs]
+    for s, c in zip(seqs, ctxs):
+        eng.reserve(s, c + 1)
+    for p in eng.kv.kv.values():
+        p.copy_(torch.randn(p.shape, generator=g, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8))
+    states = [*eng.kv.conv_state.values(), *eng.kv.rec_state.values()]
+    for t in states:
+        t.normal_(0.0, 0.1, generator=g)
+    before = [t.clone() for t in states]
+
+    def step(n, graphs):
+        eng.ecfg.use_graphs = graphs
+        for t, b in zip(states, before):
+            t.copy_(b)
+        for s, c in zip(seqs, ctxs):
+            s.length = c
+        out = eng.forward(eng.plan([(s, [7 * i + 1], 1) for i, s in enumerate(seqs[:n])]), "logits")
+        return [out.clone()] + [t.clone() for t in states]
+    return eng, step
+
+
+@pytest.mark.parametrize("kind", ["dense", "experts", "recurrent"])
+def test_logits_do_not_depend_on_how_a_step_was_launched(kind):
+    """Padded and whole batches, replayed and launched one by one: the same bits, and the same states.  Keys are cut as the sequences'
+    number asks for, not as the padded batch's would, and batches that differ in that alone have captured steps of their own."""
+    eng, step = _steps_engine(kind)
+    sizes = [n for n in range(17, 33) if eng._sampled_bucket(n) != n]
+    apart = [n for n in sizes if eng._key_splits(n) != eng._key_splits(eng._sampled_bucket(n))]
+    shared = [n for n in range(17, 32) if (eng._sampled_bucket(n), eng._key_splits(n)) == (eng._sampled_bucket(n + 1), eng._key_splits(n + 1))][0]
+    assert sizes and apart                         # (a step's form is that of its own number, whatever the SMs of the device)
+    for n in {1, 3, sizes[0], apart[0], apart[-1], shared, shared + 1}:
+        want = step(n, False)
+        for _ in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(step(n, True), want)), n
+    assert sum(k[:2] == ("logits", eng._sampled_bucket(shared)) and k[2] == eng._key_splits(shared) for k in eng._graphs) == 1
 
 
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [

@@ -44,3 +44,16 @@ def test_rows_that_a_captured_step_does_not_hold(change):
     for k, v in change.items():
         setattr(step[1], k, v)
     assert not eng._logits_graphable(step)
+
+
+def test_buckets_of_sampled_steps():
+    """No padding up to 16 sequences and an eighth at most above; no bucket crosses a power of two, a row tile or a limit of the expert
+    kernels, where products take other forms; a few buckets for every doubling."""
+    eng = _engine()
+    for limits in (set(), {21, 192, 768}):
+        eng._limits = limits
+        for n in range(1, 2049):
+            b = eng._sampled_bucket(n)
+            assert n <= b <= n * 9 // 8 and eng._sampled_bucket(b) == b
+            assert not any(n <= r < b for r in [24, *limits, *(1 << i for i in range(12)), *range(128, 1025, 128)]), (n, b)
+        assert len({eng._sampled_bucket(n) for n in range(17, 1025)}) <= 8 * 6 + len(limits)
