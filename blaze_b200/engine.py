@@ -459,8 +459,11 @@ class Engine:
         tensor of its own (the logits of a large batch would otherwise stay allocated for every bucket, or be copied out).  Issuing
         a step's launches one by one takes 2.0 ms of host time for 12 layers of the 8B shape, against 1.2 ms on the GPU at one
         sequence and 2.9 ms at 256.  On one rank only, for rows without a deferred state, and not where something follows the
-        layers' work step by step, or the layers read the contexts' lengths on the host (a sparse-attention indexer)."""
-        return (self.model.tp.world == 1 and not self.model.observed and not self.model.cfg.indexer_heads
+        layers' work step by step, or the layers read the contexts' lengths on the host: a sparse-attention indexer, and the attention
+        kernels of layer-by-layer designs, which cut keys by pages into as many runs as the longest context has tiles.  (A captured
+        step, which does not know that, would cut them otherwise, and its logits would differ by the roundings.)"""
+        cfg = self.model.cfg
+        return (self.model.tp.world == 1 and not self.model.observed and not cfg.indexer_heads and not cfg.layer_specs
                 and all(c.want_logits == 1 and not c.defer_state and c.parents is None for c in chunks))
 
     def _sampled_bucket(self, n: int) -> int:
@@ -486,7 +489,8 @@ class Engine:
     def _key_splits(self, n: int) -> int:
         """Runs the attention kernels cut the keys of a decode step of ``n`` sequences into.  A captured step with logits keeps the
         number that ``n`` sequences get, not the one of its padded batch: partial sums are rounded, so the logits of a step would
-        otherwise depend on whether it was replayed."""
+        otherwise depend on whether it was replayed.  (They are cut by tiles, so the tiles of the longest context, which a captured
+        step does not know, only end runs that would be empty.)"""
         heads = n * self.model.cfg.num_kv_heads
         if self.attn_group == 0:
             return 1

@@ -43,29 +43,33 @@ def test_logits_steps_replay_a_captured_step():
 
 
 def _steps_engine(kind):
-    """A small model of a kind with 32 sequences open, their contexts (60 to 1400 tokens) filled with random keys, values and states."""
+    """A small model of a kind with 40 sequences open, whose contexts (60 to 1400 tokens) are in the cache."""
+    from blaze_b200.config import named_config
     from blaze_b200.llm import LLM
-    D = 256 if kind == "recurrent" else 128
-    cfg = ModelConfig(vocab_size=2048, hidden_size=512, num_layers=2, num_heads=8, num_kv_heads={"dense": 8, "experts": 4, "recurrent": 1}[kind], head_dim=D,
-                      intermediate_size=1024, rope=RopeConfig(theta=1e6))
-    cfg.layer_types = ["full_attention"] * 2
+    if kind.startswith("tiny-"):
+        cfg, fmt = named_config(kind), "bf16"
+        for spec in cfg.layer_specs:               # contexts of one key tile would not be cut at all
+            if spec.attn is not None and spec.attn.window:
+                spec.attn.window = 0
+    else:
+        fmt = "mxfp8" if kind == "recurrent" else "nvfp4"
+        cfg = ModelConfig(vocab_size=2048, hidden_size=512, num_layers=2, num_heads=8, num_kv_heads={"dense": 8, "experts": 4, "recurrent": 1}[kind],
+                          head_dim=256 if kind == "recurrent" else 128, intermediate_size=1024, rope=RopeConfig(theta=1e6))
+        cfg.layer_types = ["full_attention"] * 2
     if kind == "experts":
         cfg.num_experts, cfg.num_experts_per_tok, cfg.moe_intermediate_size = 16, 4, 256
     if kind == "recurrent":
         cfg.layer_types = ["linear_attention", "full_attention"]
         cfg.linear_num_key_heads, cfg.linear_num_value_heads, cfg.linear_key_head_dim, cfg.linear_value_head_dim = 2, 4, 128, 128
         cfg.linear_conv_kernel_dim = 4
-    eng = LLM(cfg, weight_format="mxfp8" if kind == "recurrent" else "nvfp4", max_seqs=32, max_model_len=2048, kv_tokens=33 * 1536, seed=4).engine
-    g = torch.Generator(device=DEV).manual_seed(1)
-    ctxs = [60 + (i * 743) % 1341 for i in range(32)]
+    eng = LLM(cfg, weight_format=fmt, max_seqs=40, max_model_len=4096, kv_tokens=41 * 1536, seed=4).engine
+    gen = torch.Generator().manual_seed(1)
+    ctxs = [60 + (i * 743) % 1341 for i in range(40)]
     seqs = [eng.open_from() for _ in ctxs]
-    for s, c in zip(seqs, ctxs):
-        eng.reserve(s, c + 1)
-    for p in eng.kv.kv.values():
-        p.copy_(torch.randn(p.shape, generator=g, device=DEV).to(torch.float8_e4m3fn).view(torch.uint8))
-    states = [*eng.kv.conv_state.values(), *eng.kv.rec_state.values()]
-    for t in states:
-        t.normal_(0.0, 0.1, generator=g)
+    for i in range(0, 40, 8):
+        eng.forward(eng.plan([(s, torch.randint(0, 1000, (c,), generator=gen).tolist(), 0) for s, c in zip(seqs[i:i + 8], ctxs[i:i + 8])]), "none")
+    kv = eng.kv
+    states = [t for d in (kv.conv_state, kv.rec_state, kv.qkv_state, kv.input_state) for t in d.values()]
     before = [t.clone() for t in states]
 
     def step(n, graphs):
@@ -79,20 +83,22 @@ def _steps_engine(kind):
     return eng, step
 
 
-@pytest.mark.parametrize("kind", ["dense", "experts", "recurrent"])
+@pytest.mark.parametrize("kind", ["dense", "experts", "recurrent", "tiny-sevevik", "tiny-niletar", "tiny-rapisun", "tiny-medodra"])
 def test_logits_do_not_depend_on_how_a_step_was_launched(kind):
-    """Padded and whole batches, replayed and launched one by one: the same bits, and the same states.  Keys are cut as the sequences'
-    number asks for, not as the padded batch's would, and batches that differ in that alone have captured steps of their own."""
+    """Padded and whole batches, replayed (where the design's steps are) and launched one by one: the same bits, and the same states.
+    Keys are cut as the sequences' number asks for, not as the padded batch's would, and batches that differ in that alone have captured
+    steps of their own."""
     eng, step = _steps_engine(kind)
-    sizes = [n for n in range(17, 33) if eng._sampled_bucket(n) != n]
-    apart = [n for n in sizes if eng._key_splits(n) != eng._key_splits(eng._sampled_bucket(n))]
-    shared = [n for n in range(17, 32) if (eng._sampled_bucket(n), eng._key_splits(n)) == (eng._sampled_bucket(n + 1), eng._key_splits(n + 1))][0]
-    assert sizes and apart                         # (a step's form is that of its own number, whatever the SMs of the device)
-    for n in {1, 3, sizes[0], apart[0], apart[-1], shared, shared + 1}:
+    bucket, splits = eng._sampled_bucket, eng._key_splits
+    padded = [n for n in range(17, 41) if bucket(n) != n]
+    apart = [n for n in padded if splits(n) != splits(bucket(n))]
+    shared = [n for n in range(17, 40) if (bucket(n), splits(n)) == (bucket(n + 1), splits(n + 1))][0]
+    for n in sorted({1, 3, padded[0], *apart, 37, shared, shared + 1}):
         want = step(n, False)
         for _ in range(3):
             assert all(torch.equal(a, b) for a, b in zip(step(n, True), want)), n
-    assert sum(k[:2] == ("logits", eng._sampled_bucket(shared)) and k[2] == eng._key_splits(shared) for k in eng._graphs) == 1
+    if not kind.startswith("tiny-"):
+        assert apart and sum(k == ("logits", bucket(shared), splits(shared)) for k in eng._graphs) == 1
 
 
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [

@@ -37,6 +37,13 @@ def test_routing_statistics_keep_sampled_steps_uncaptured():
     assert eng.model.heat is not None and not eng._logits_graphable(_decode_step(eng))
 
 
+@pytest.mark.parametrize("name", ["tiny-sevevik", "tiny-niletar", "tiny-rapisun", "tiny-medodra"])
+def test_designs_whose_keys_are_cut_by_the_longest_context(name):
+    """Their kernels' runs of keys depend on a length that a captured step does not know: launched one by one, always."""
+    eng = _engine(name)
+    assert not eng._logits_graphable(_decode_step(eng))
+
+
 @pytest.mark.parametrize("change", [{"want_logits": 0}, {"defer_state": True}, {"parents": [-1]}])
 def test_rows_that_a_captured_step_does_not_hold(change):
     eng = _engine()
