@@ -152,6 +152,9 @@ class Engine:
         self._graphs: Dict[Tuple, "_Graph"] = {}
         self._seen: Dict[Tuple, int] = {}
         self._limits: Optional[Set[int]] = None      # see _expert_limits
+        # Memory of the captured steps with logits, of which there are many: they share it, since what one leaves behind (its final
+        # hidden rows) is read by the head before another runs.
+        self._sampled_pool = None
         self._pinned = None
         if self.device.type == "cuda":
             self._pinned = [torch.empty(1 << 19, dtype=torch.int32, pin_memory=True) for _ in range(2)]
@@ -498,11 +501,14 @@ class Engine:
             return self.model.ops.row_block_splits(heads, 8)
         return self.model.ops.decode_splits(heads * ((self.attn_group + 15) // 16), 8)
 
+    def _sampled_key(self, n: int) -> Tuple:
+        return "logits", self._sampled_bucket(n), self._key_splits(n)
+
     def _forward_graph(self, chunks: Sequence[SeqChunk], feedback: bool = False, rows_per_seq: int = 1, mode: str = "greedy"):
         B = len(chunks)
         bucket = self._sampled_bucket(B) if mode == "logits" else self._bucket(B)
-        key = (("decode", bucket) if rows_per_seq == 1 and mode == "greedy" else
-               ("logits", bucket, self._key_splits(B)) if mode == "logits" else ("verify", bucket, rows_per_seq, mode))
+        key = (self._sampled_key(B) if mode == "logits" else ("decode", bucket) if rows_per_seq == 1 and mode == "greedy" else
+               ("verify", bucket, rows_per_seq, mode))
         g = self._graphs.get(key)
         if g is None:
             seen = self._seen.get(key, 0)
@@ -516,31 +522,39 @@ class Engine:
         return g.replay(chunks, feedback)
 
     def capture_decode_graphs(self, max_batch: Optional[int] = None) -> int:
-        """Capture the decode-step graph of every batch bucket up front (server start-up), so that no request pays for a
-        capture.  Uses scratch sequences that are closed again; returns the number of graphs captured."""
+        """Capture the decode steps of every batch size up front (server start-up), greedy ones and those with logits, so that no plain
+        decode step of a request pays for a capture (verify steps are captured when they come).  Uses scratch sequences that are
+        closed again; returns the number of steps captured."""
         if not (self.ecfg.use_graphs and self.device.type == "cuda" and self.model.ops.is_cuda
                 and self.model.is_first_stage and self.model.is_last_stage):
             return 0
         cap = min(max_batch or self.ecfg.max_seqs, len(self.free_rows), max(self.pages.free_count, 0))
-        n = 0
-        for b in self.ecfg.graph_buckets:
-            if b > cap:
-                break
-            if ("decode", b) in self._graphs:
-                continue
+        before = len(self._graphs)
+
+        def capture(b: int, mode: str) -> bool:
             seqs = [self.open_from() for _ in range(b)]
             try:
                 for _ in range(2):      # first sight runs eagerly, second sight captures
                     for s in seqs:
                         s.length = 0
-                    self.forward(self.plan([(s, [0], 1) for s in seqs]), "greedy")
-                n += 1
+                    chunks = self.plan([(s, [0], 1) for s in seqs])
+                    if mode == "logits" and not self._logits_graphable(chunks):
+                        return False
+                    self.forward(chunks, mode)
+                return True
             finally:
                 for s in seqs:
                     self.close(s)
+        for b in self.ecfg.graph_buckets:
+            if b <= cap and ("decode", b) not in self._graphs:
+                capture(b, "greedy")
+        # the largest first: the others then find their memory in the pool that these steps share
+        for b in range(cap, 0, -1):
+            if self._sampled_key(b) not in self._graphs and not capture(b, "logits"):
+                break
         if self.device.type == "cuda":
             torch.cuda.synchronize(self.device)
-        return n
+        return len(self._graphs) - before
 
     def graph_kernel_count(self) -> int:
         """Kernels of this library inside one captured decode step (the largest captured bucket)."""
@@ -688,7 +702,10 @@ class _Graph:
             torch.cuda.synchronize()
             self.graph = torch.cuda.CUDAGraph()
             l0 = self.eng.model.ops.launches
-            with torch.cuda.graph(self.graph):
+            pool = None
+            if self.mode == "logits":
+                pool = self.eng._sampled_pool = self.eng._sampled_pool or torch.cuda.graph_pool_handle()
+            with torch.cuda.graph(self.graph, pool=pool):
                 self.out = self.eng._run(self.batch, "hidden" if self.mode == "logits" else self.mode)
             self.kernels = self.eng.model.ops.launches - l0
         self.graph.replay()

@@ -101,6 +101,23 @@ def test_logits_do_not_depend_on_how_a_step_was_launched(kind):
         assert apart and sum(k == ("logits", bucket(shared), splits(shared)) for k in eng._graphs) == 1
 
 
+def test_captured_steps_are_there_from_the_start():
+    """With ``warm_graphs`` no decode step of any batch size captures anything; the steps with logits share their memory, which holds
+    when they are replayed in any order."""
+    eng, step = _steps_engine("dense")
+    for s in list(eng.seqs.values())[24:]:
+        eng.close(s)                               # (16 rows for the scratch sequences)
+    want = {n: step(n, False) for n in (16, 3, 11)}
+    eng.ecfg.use_graphs = True
+    made = eng.capture_decode_graphs()
+    keys = set(eng._graphs)
+    assert made == len(keys) and keys == {("decode", b) for b in (1, 2, 4, 8, 16)} | {eng._sampled_key(n) for n in range(1, 17)}
+    assert len({eng._graphs[k].graph.pool() for k in keys if k[0] == "logits"}) == 1
+    for n in (3, 16, 11, 3, 11, 16):
+        assert all(torch.equal(a, b) for a, b in zip(step(n, True), want[n])), n
+    assert set(eng._graphs) == keys
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [
     (32, 8, [1], 1), (32, 8, [129], 1), (32, 8, [5000, 3, 128, 1291], 1),          # fewer items than CTAs: runs of tiles
     (16, 2, [2600, 40, 1025], 1), (32, 4, [700], 2), (32, 8, [900, 260], 5), (32, 4, [1500, 64], 8),      # 8, 16, 20 and 64 rows
