@@ -143,9 +143,12 @@ class CudaOps:
         lib.blz_swiglu_live.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, VP, VP]
         # routed rows per expert up to this: the expert GEMMs put the features on the tensor-core lanes and only the live rows on its
         # columns (blz_moe_gemm), which streams the weights; above it the 128-row tiles of the grouped GEMM are full enough
-        # (BLAZE_MOE_NARROW=0: never).  MXFP8 weights up to 8/3 of it, a whole tile of rows: twice the bytes to stream for the same
-        # tiles.  Measured per step, narrow / tiles: 80 rows per expert (512 experts, MXFP8, 4096 tokens) 6.29 / 6.83 ms, 256 rows per
-        # expert (128 experts, NVFP4, 4096 tokens) 4.30 / 4.20 ms.
+        # (BLAZE_MOE_NARROW=0: never).  MXFP8 weights of 2048 feature tiles and more up to 8/3 of it, a whole tile of rows: twice the
+        # bytes of NVFP4 to stream for the same tiles, on all SMs.  Narrow over tiles, MXFP8, routed experts of a layer as a whole, at
+        # 48 / 80 / 128 rows per expert: 512 x 1024 features (4096 tiles) of 2048 0.66 / 0.77 / 0.83, 128 x 3072 of 4096 (3072 tiles)
+        # 0.73 / 0.82 / 0.80, but 64 x 2816 of 2048 (1408) 0.90 / 1.01 / 1.22, 128 x 1024 of 2048 (1024) 0.84 / 0.98 / 0.97 (1.04 at
+        # 112), 32 x 3072 of 4096 (768) 0.90 / 0.96 / 1.03, 8 x 3072 of 4096 (192) 1.42 / 1.87 / 1.54.  NVFP4, 256 rows per expert of
+        # 128: 4.30 / 4.20 ms a step.
         self.MOE_NARROW_ROWS = 48 if os.environ.get("BLAZE_MOE_NARROW", "1") != "0" else 0
         lib.blz_moe_scatter.argtypes = [_c.c_int, VP, VP, VP, VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                         _c.c_int, VP, _c.c_int, VP]
@@ -1407,7 +1410,9 @@ class CudaOps:
 
     def moe_narrow_tokens(self, experts, k: int) -> int:
         """The most tokens of a step whose routed rows (``k`` per token) take the narrow expert kernel."""
-        rows = self.MOE_NARROW_ROWS * 8 // 3 if self.pack_experts(experts)["gate_up"]["kind"] == 2 else self.MOE_NARROW_ROWS
+        gu, rows = self.pack_experts(experts)["gate_up"], self.MOE_NARROW_ROWS
+        if gu["kind"] == 2 and experts.count * gu["N"] >= 2048 * 128:
+            rows = rows * 8 // 3
         return rows * experts.count // k
 
     def moe_rows(self, x, topk_w, topk_id, experts, shared=None, gate=None) -> RoutedRows:

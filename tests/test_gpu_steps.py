@@ -333,6 +333,14 @@ def test_expert_product_of_up_to_a_tile_of_rows(ops, fmt, T, E, k, H, I):      #
     assert _rel(outs[0], ref.moe_forward(x, w, ids, ex.forward_one, E)) < 0.08
 
 
+@pytest.mark.parametrize("kind,E,N,k,most", [(2, 512, 1024, 10, 6553), (2, 128, 2048, 8, 2048), (2, 127, 2048, 8, 762), (2, 8, 6144, 2, 192), (1, 512, 1024, 10, 2457)])
+def test_which_steps_take_the_narrow_expert_kernel(ops, kind, E, N, k, most):      # noqa: F811
+    """48 routed rows per expert, 128 where MXFP8 experts have 2048 feature tiles together."""
+    ex = _A()
+    ex.count, ex.cuda_pack = E, {"gate_up": {"kind": kind, "N": N}}
+    assert ops.moe_narrow_tokens(ex, k) == most
+
+
 @pytest.mark.parametrize("E,T,k", [(1, 5, 1), (33, 300, 4), (512, 700, 10)])
 def test_expert_plan(ops, E, T, k):      # noqa: F811
     """Offsets of the experts' rows in tiles of 128 and each tile's expert and live rows."""
