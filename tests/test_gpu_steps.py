@@ -385,3 +385,16 @@ def test_gated_norm(ops, T, Hv, DV, flags):      # noqa: F811
     # half a step of bf16 (8 bits: up to 2^-8 of the value), and the fast exponential: 2 ulp and, of its argument, 88 * 2^-24
     err = (outs[0].double().view_as(want) - want).abs()
     assert (err <= want.abs() * (2.0 ** -8 + 2e-5) + 1e-40).all()
+
+
+def test_silu_of_every_gate(ops):      # noqa: F811
+    """The activation's quotient over all 16-bit gates: rounded as the division is, up to where e^-x overflows, with its infinities."""
+    x = torch.arange(1 << 16, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).view(16, 4096)
+    got = ops.silu_mul(torch.cat([x, torch.ones_like(x)], 1)).double()
+    xd = x.double()
+    want = torch.where(xd < -88.72, 0.0, xd * xd.sigmoid())       # e^-x is infinite there: x / inf
+    assert torch.equal(got.isnan(), xd.isnan() | (xd == -torch.inf)) and (got[xd == torch.inf] == torch.inf).all()
+    ok = xd.isfinite()
+    step = torch.exp2(torch.frexp(want.abs().clamp_min(2.0 ** -126))[1].double() - 8)      # of bf16 (8 bits) at that size
+    # half a step, and in front of the rounding the fast exponential: 2 ulp and, of its argument, 88 * 2^-24, of 2^8 steps
+    assert ((got - want).abs()[ok] <= step[ok] * (0.5 + 256 * (88 + 4) * 2.0 ** -24)).all()
