@@ -36,8 +36,10 @@ namespace blz {
 
 constexpr int kOrdered = 64;          // sequences that a launch with splits takes by their length (more: as they come)
 
-// NMAX = MMA N (rows per work item); RMAX = rows kept in registers by the softmax threads (4, 8 or 16, >= live rows).
-template <int NMAX, int RMAX>
+constexpr int NMAX = 16;              // MMA N: rows per work item
+
+// RMAX = rows kept in registers by the softmax threads (4, 8 or 16, >= live rows).
+template <int RMAX>
 struct DecCfg {
   static constexpr int D = 128;
   static constexpr int PAGE_BYTES = 16 * D;
@@ -96,14 +98,13 @@ template <int N>
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&r)[N]) {
   if constexpr (N == 4) tmem_ld4(taddr, r);
   else if constexpr (N == 8) tmem_ld8(taddr, r);
-  else if constexpr (N == 16) tmem_ld16(taddr, r);
-  else tmem_ld32(taddr, r);
+  else tmem_ld16(taddr, r);
 }
 
-template <int NMAX, int RMAX>
-__global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_decode_kernel(AttnParams p) {
+template <int RMAX>
+__global__ void __launch_bounds__(320, (DecCfg<RMAX>::CTAS_PER_SM)) attn_decode_kernel(AttnParams p) {
   pdl_trigger();
-  using Cfg = DecCfg<NMAX, RMAX>;
+  using Cfg = DecCfg<RMAX>;
   constexpr int ST = Cfg::STAGES, D = Cfg::D, NB = Cfg::NB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
         // rows and K tiles while the V half is still waiting for ring slots of this one.  (The rows beyond RMAX of both Q
         // buffers are zeroed once, before the loop.)
         constexpr bool HALF = RMAX <= 8;
-        constexpr int LPR = RMAX <= 4 ? 4 : RMAX <= 8 ? 2 : (32 / NMAX == 0 ? 1 : 32 / NMAX);   // lanes per row
+        constexpr int LPR = RMAX <= 4 ? 4 : 2;              // lanes per row
         constexpr int DPL = D / LPR;                               // dims per lane
         constexpr uint32_t QMASK = HALF ? 0x0000FFFFu : 0xFFFFFFFFu;
         if (!HALF || lane < 16) {
@@ -550,7 +551,7 @@ __global__ void __launch_bounds__(320, (DecCfg<NMAX, RMAX>::CTAS_PER_SM)) attn_d
 // side by side, and the runs' sums are added up (in their order) by loads that do not wait for one another; with a thread per
 // dim, a row after the other and a branch around every run it took 10.5 us for 48 items of 8 runs, now 5.3.
 // WIDE: the caller's arrays and output lie on 16 bytes (else they are read and written by elements).
-template <int NMAX, bool WIDE>
+template <bool WIDE>
 __global__ void __launch_bounds__(512) attn_decode_combine_kernel(AttnParams p) {
   pdl_trigger();
   pdl_wait();
@@ -613,15 +614,15 @@ static cudaError_t launch_form(K kernel, PerDeviceOnce& configured, const AttnPa
   e = launch_pdl(kernel, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, p);
   if (e != cudaSuccess || p.splits == 1) return e;
   const bool wide = !((reinterpret_cast<uintptr_t>(p.part_o) | reinterpret_cast<uintptr_t>(p.part_ml) | reinterpret_cast<uintptr_t>(p.out)) & 15);
-  return launch_pdl(wide ? attn_decode_combine_kernel<16, true> : attn_decode_combine_kernel<16, false>, dim3(items), dim3(512), 0, stream, p);
+  return launch_pdl(wide ? attn_decode_combine_kernel<true> : attn_decode_combine_kernel<false>, dim3(items), dim3(512), 0, stream, p);
 }
 
 // The most rows of any work item choose the kernel (16 rows an item).  Draft trees need the mask that the 4-row one leaves out.
 static cudaError_t launch_decode(const AttnParams& p, int max_ctas, cudaStream_t stream) {
   static PerDeviceOnce four, eight, sixteen;
-  if (p.max_rows <= 4 && !p.tree_mask) return launch_form<DecCfg<16, 4>>(attn_decode_kernel<16, 4>, four, p, max_ctas, stream);
-  if (p.max_rows <= 8) return launch_form<DecCfg<16, 8>>(attn_decode_kernel<16, 8>, eight, p, max_ctas, stream);
-  return launch_form<DecCfg<16, 16>>(attn_decode_kernel<16, 16>, sixteen, p, max_ctas, stream);
+  if (p.max_rows <= 4 && !p.tree_mask) return launch_form<DecCfg<4>>(attn_decode_kernel<4>, four, p, max_ctas, stream);
+  if (p.max_rows <= 8) return launch_form<DecCfg<8>>(attn_decode_kernel<8>, eight, p, max_ctas, stream);
+  return launch_form<DecCfg<16>>(attn_decode_kernel<16>, sixteen, p, max_ctas, stream);
 }
 
 }  // namespace blz
