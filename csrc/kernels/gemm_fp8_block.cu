@@ -270,6 +270,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   pdl_trigger();
   if (ks > 1) cluster_arrive();            // the peers' barriers are initialised before anyone arrives on them remotely
   const uint32_t tmem = *tmem_slot;
+  int issued = 0;                          // thread 0: blocks whose copies have been started
 
   if (warp == 0) {
     if (lane == 0) {
@@ -292,6 +293,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         mbar_expect_tx(&sa_full[slot], sa_bytes);
         bulk_load(sSA + slot * 64, p.sa + (size_t)(kb0 + i) * p.ld_sa, sa_bytes, &sa_full[slot]);
         if (++s == STAGES) { s = 0; ph ^= 1; }
+        issued = i + 1;
       }
     }
   } else if (warp == 1) {
@@ -406,6 +408,19 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) {
+    // a wait ran out: the copies that are still on their way write to this CTA's memory (these waits are limited, too)
+    *abort_flag = 0;
+    for (int i = max(issued - STAGES, 0); i < issued; ++i) mbar_wait(&full[i % STAGES], (uint32_t)((i / STAGES) & 1), abort_flag, p.status);
+    for (int i = max(issued - Cfg::SA_SLOTS, 0); i < issued; ++i)
+      mbar_wait(&sa_full[i % Cfg::SA_SLOTS], (uint32_t)((i / Cfg::SA_SLOTS) & 1), abort_flag, p.status);
+  }
+  if (ks > 1) {
+    // ... and a peer whose waits ran out later still writes and arrives here: nobody leaves before all are done
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, Cfg::TMEM_COLS);

@@ -31,3 +31,15 @@ def test_scales_of_few_rows_are_read_before_their_slot_is_filled_again():
         return seen
     for i in range(slots, n):
         assert ("read", i - slots) in earlier(("copy", i)), f"block {i} overwrites scales that may not have been read"
+
+
+def test_few_rows_ctas_leave_after_their_copies_and_their_peers():
+    """After a wait that ran out, too: behind the last access to a peer's memory, and before a CTA gives up its own, it waits for the
+    copies that it has started and for the peers."""
+    text = open(SRC).read()
+    body = text[text.index("gemm_fp8_rows_kernel("):]
+    body = body[:body.index("\n}\n")]
+    end = body[body.rindex("mbar_arrive_remote("):]
+    order = [end.index(s) for s in ("__syncthreads();", "if (threadIdx.x == 0 && *abort_flag)", "mbar_wait(&full[", "mbar_wait(&sa_full[",
+                                    "cluster_arrive();", "cluster_wait();", "tmem_dealloc(")]
+    assert order == sorted(order)
