@@ -258,10 +258,12 @@ __device__ __forceinline__ uint32_t pack_e4m3x4_f(float a, float b, float c, flo
 
 // Quantise this thread's 8 elements [e0, e0+8) of row t, neighbouring lanes holding neighbouring elements (a warp starts at a
 // multiple of 256).  Every lane of the warp must call it (shuffles); `valid` gates the stores.
-// A scale byte stored by itself costs the memory system a sector, as a full one does: four of them (neighbours in the 128x4 tiles)
-// make one store, and those of a row's padded columns are written as 0.  8192 rows of 12288 activations: 101 -> 82 us, together
-// with the registers that the plain form of the kernel below no longer carries.
-template <int QUANT>
+// PACK: a scale byte stored by itself costs the memory system a sector, as a full one does; four of them (neighbours in the 128x4
+// tiles) make one store, and those of a row's padded columns are written as 0.  8192 rows of 12288 activations, NVFP4: 97 -> 78 us
+// (with the registers that the plain form of the kernel below no longer carries).  Where the arithmetic in front sets the pace the
+// two more shuffles cost more than they save: norms of 8192 x 4096 46.2 -> 47.6 us, gated activations of the same in MXFP8 42.6 ->
+// 47.6.
+template <int QUANT, bool PACK>
 __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, int t, int e0, int W, float g, uint8_t* q_out,
                                              uint8_t* sf_out, int ct) {
   const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&packed);
@@ -274,13 +276,17 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
   if (QUANT == 1) {
     const uint8_t sf = f2e4m3(bm / 6.f / g);           // (ties between two scales are common: the same roundings as ever)
     const float denom = e4m32f(sf) * g;
-    const float inv = denom > 0.f ? __frcp_rn(denom) : 0.f;
+    const float inv = denom > 0.f ? 1.f / denom : 0.f;
     const uint32_t codes = pack_e2m1x8(v, inv);
     if (valid) *reinterpret_cast<uint32_t*>(q_out + (size_t)t * (W / 2) + e0 / 2) = codes;
-    uint32_t four = valid ? (uint32_t)sf << (8 * ((lane >> 1) & 3)) : 0u;
-    four |= __shfl_xor_sync(0xffffffffu, four, 2);
-    four |= __shfl_xor_sync(0xffffffffu, four, 4);
-    if (valid && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 4, ct)) = four;
+    if constexpr (PACK) {
+      uint32_t four = valid ? (uint32_t)sf << (8 * ((lane >> 1) & 3)) : 0u;
+      four |= __shfl_xor_sync(0xffffffffu, four, 2);
+      four |= __shfl_xor_sync(0xffffffffu, four, 4);
+      if (valid && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 4, ct)) = four;
+    } else if (valid && (e0 & 15) == 0) {
+      sf_out[sf_offset(t, e0 >> 4, ct)] = sf;
+    }
   } else {
     bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 2));
     bm = fmaxf(bm, 1.17549435e-38f);
@@ -292,10 +298,14 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
           make_uint2(pack_e4m3x4_f(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv),
                      pack_e4m3x4_f(v[4] * inv, v[5] * inv, v[6] * inv, v[7] * inv));
     }
-    uint32_t four = valid ? (uint32_t)(ex + 127) << (8 * ((lane >> 2) & 3)) : 0u;
-    four |= __shfl_xor_sync(0xffffffffu, four, 4);
-    four |= __shfl_xor_sync(0xffffffffu, four, 8);
-    if (valid && (lane & 15) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 5, ct)) = four;
+    if constexpr (PACK) {
+      uint32_t four = valid ? (uint32_t)(ex + 127) << (8 * ((lane >> 2) & 3)) : 0u;
+      four |= __shfl_xor_sync(0xffffffffu, four, 4);
+      four |= __shfl_xor_sync(0xffffffffu, four, 8);
+      if (valid && (lane & 15) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 5, ct)) = four;
+    } else if (valid && (e0 & 31) == 0) {
+      sf_out[sf_offset(t, e0 >> 5, ct)] = (uint8_t)(ex + 127);
+    }
   }
 }
 
@@ -365,7 +375,7 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
-    quant_store8<QUANT>(u[c], i < H, t, i, H, g, q_out, sf_out, sf_col_tiles);
+    quant_store8<QUANT, false>(u[c], i < H, t, i, H, g, q_out, sf_out, sf_col_tiles);
   }
 }
 
@@ -421,7 +431,7 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
-    quant_store8<MODE>(a[c], i < I, t, i, I, gs, q_out, sf_out, sf_col_tiles);
+    quant_store8<MODE, ACT>(a[c], i < I, t, i, I, gs, q_out, sf_out, sf_col_tiles);
   }
 }
 
@@ -477,7 +487,7 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const __nv_bfloat16* _
     gs = fmaxf(m / (6.f * 448.f), 1e-30f);
     if (live && in_row == 0) row_scale[t] = gs;
   }
-  quant_store8<MODE>(a, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
+  quant_store8<MODE, false>(a, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
 }
 
 // ---------------------------------------------------------------------------------------------- attention prep
