@@ -791,44 +791,40 @@ __global__ void __launch_bounds__(512) attn_prep_heads_kernel(const __nv_bfloat1
   }
 }
 
-// Elementwise kernels on bf16, eight elements per thread and step where pointers and sizes allow 16-byte accesses (one element
-// per thread took 80 us for a sum of 8192 x 4096, now 40; the bytes take 31 at copy bandwidth).
-template <typename F>
-__device__ __forceinline__ uint4 each8(const uint4& a, const uint4& b, F f) {
-  uint4 o;
-  const __nv_bfloat16 *x = reinterpret_cast<const __nv_bfloat16*>(&a), *y = reinterpret_cast<const __nv_bfloat16*>(&b);
-  __nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(&o);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) z[j] = __float2bfloat16(f(bf2f(x[j]), bf2f(y[j])));
-  return o;
-}
-__device__ __forceinline__ bool aligned16(const void* a, const void* b, const void* c) {
-  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
-}
+// Elementwise kernels on bf16, V elements per access: 8 or 4 where pointers and sizes allow, else 1 (see each_width).
+template <int V> struct EachWord { typedef uint4 type; };
+template <> struct EachWord<4> { typedef uint2 type; };
+template <> struct EachWord<1> { typedef __nv_bfloat16 type; };
 // out[i] = f(a[i], b[i]) for i < n (out may be a)
-template <typename F>
+template <int V, typename F>
 __device__ __forceinline__ void each(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, size_t n, size_t first, size_t step, F f) {
-  size_t done = 0;
-  if (aligned16(a, b, out)) {
-    for (size_t i = first; i < n / 8; i += step)
-      reinterpret_cast<uint4*>(out)[i] = each8(reinterpret_cast<const uint4*>(a)[i], reinterpret_cast<const uint4*>(b)[i], f);
-    done = n / 8 * 8;
+  typedef typename EachWord<V>::type W;
+  for (size_t i = first; i < n / V; i += step) {
+    const W wa = reinterpret_cast<const W*>(a)[i], wb = reinterpret_cast<const W*>(b)[i];
+    W wo;
+    const __nv_bfloat16 *x = reinterpret_cast<const __nv_bfloat16*>(&wa), *y = reinterpret_cast<const __nv_bfloat16*>(&wb);
+    __nv_bfloat16* z = reinterpret_cast<__nv_bfloat16*>(&wo);
+#pragma unroll
+    for (int j = 0; j < V; ++j) z[j] = __float2bfloat16(f(bf2f(x[j]), bf2f(y[j])));
+    reinterpret_cast<W*>(out)[i] = wo;
   }
-  for (size_t i = done + first; i < n; i += step) out[i] = __float2bfloat16(f(bf2f(a[i]), bf2f(b[i])));
 }
-__global__ void mul_sigmoid_kernel(__nv_bfloat16* x, const __nv_bfloat16* gate, size_t n) {
-  each(x, gate, x, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x,
-       [](float v, float g) { return v / (1.f + __expf(-g)); });
+// (the division sets the pace: wider accesses make a thread's divisions wait for one another, 1.1 - 1.4 times as long up to 10 M elements)
+__global__ void mul_sigmoid_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ gate, size_t n) {
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    x[i] = __float2bfloat16(bf2f(x[i]) / (1.f + __expf(-bf2f(gate[i]))));
 }
+template <int V>
 __global__ void add_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, size_t n) {
-  each(a, b, out, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, [](float x, float y) { return x + y; });
+  each<V>(a, b, out, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, [](float x, float y) { return x + y; });
 }
 // out[t, :] = a[t, :] + b[t, :] * bf16(sigmoid(gate_logit[t]))
+template <int V>
 __global__ void add_sigmoid_scaled_kernel(const __nv_bfloat16* a, const __nv_bfloat16* b, const __nv_bfloat16* gl,
                                           __nv_bfloat16* out, int H) {
   const size_t row = (size_t)blockIdx.x * H;
   const float s = bf2f(__float2bfloat16(1.f / (1.f + __expf(-bf2f(gl[blockIdx.x])))));
-  each(a + row, b + row, out + row, H, threadIdx.x, blockDim.x, [s](float x, float y) { return x + y * s; });
+  each<V>(a + row, b + row, out + row, H, threadIdx.x, blockDim.x, [s](float x, float y) { return x + y * s; });
 }
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ rows,
                                    __nv_bfloat16* __restrict__ out, int H) {
@@ -1105,6 +1101,14 @@ BLZ_API int blz_kv_move_rows(void* pool, const int* src, const int* dst, const i
   return (int)cudaGetLastError();
 }
 
+// Elements per access that n elements at these places allow.  One block per 256 accesses and rows' blocks without idle passes: sum of
+// 256 x 4096 2.5 us with single elements, 2.3 with eight (3.3 with a grid for single elements), 8192 x 4096 78 and 32; rows with a
+// gate 1000 x 5120 7.2 and 5.4 (8.8 in blocks of 256 threads), 8192 x 4096 75 and 41.
+static int each_width(long long n, const void* a, const void* b, const void* c) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c);
+  return n % 8 == 0 && !(at & 15) ? 8 : n % 4 == 0 && !(at & 7) ? 4 : 1;
+}
+#define BLZ_EACH(V, CALL) { if (V == 8) { constexpr int W = 8; CALL; } else if (V == 4) { constexpr int W = 4; CALL; } else { constexpr int W = 1; CALL; } }
 BLZ_API int blz_mul_sigmoid(void* x, const void* gate, long long n, cudaStream_t s) {
   if (n == 0) return 0;
   mul_sigmoid_kernel<<<(int)((n + 1023) / 1024 > 4096 ? 4096 : (n + 1023) / 1024), 256, 0, s>>>((bf16*)x, (const bf16*)gate, (size_t)n);
@@ -1112,14 +1116,20 @@ BLZ_API int blz_mul_sigmoid(void* x, const void* gate, long long n, cudaStream_t
 }
 BLZ_API int blz_add(const void* a, const void* b, void* out, long long n, cudaStream_t s) {
   if (n == 0) return 0;
-  add_kernel<<<(int)((n + 1023) / 1024 > 4096 ? 4096 : (n + 1023) / 1024), 256, 0, s>>>((const bf16*)a, (const bf16*)b, (bf16*)out, (size_t)n);
+  const int v = each_width(n, a, b, out);
+  const long long blocks = (n / v + 255) / 256, most = 1 << 20;
+  BLZ_EACH(v, (add_kernel<W><<<(unsigned)(blocks < most ? blocks : most), 256, 0, s>>>((const bf16*)a, (const bf16*)b, (bf16*)out, (size_t)n)))
   return (int)cudaGetLastError();
 }
 BLZ_API int blz_add_sigmoid_scaled(const void* a, const void* b, const void* gl, void* out, int T, int H, cudaStream_t s) {
   if (T == 0) return 0;
-  add_sigmoid_scaled_kernel<<<T, 256, 0, s>>>((const bf16*)a, (const bf16*)b, (const bf16*)gl, (bf16*)out, H);
+  // blocks of up to 512 threads, of 256 where there are rows for all SMs several times over
+  const int v = each_width(H, a, b, out), items = H / v, most = T >= 2048 ? 256 : 512, passes = (items + most - 1) / most;
+  const int threads = passes ? ((items + passes - 1) / passes + 31) / 32 * 32 : 32;
+  BLZ_EACH(v, (add_sigmoid_scaled_kernel<W><<<T, threads, 0, s>>>((const bf16*)a, (const bf16*)b, (const bf16*)gl, (bf16*)out, H)))
   return (int)cudaGetLastError();
 }
+#undef BLZ_EACH
 BLZ_API int blz_gather_rows(const void* x, const int* rows, void* out, int R, int H, cudaStream_t s) {
   if (R == 0) return 0;
   if (H % 8) return (int)cudaErrorInvalidValue;

@@ -281,7 +281,7 @@ def test_quantised_rows(ops, fmt, T, K):      # noqa: F811
     assert (got != want).float().mean().item() < 1e-3 and _rel(got, want) < 1e-2
 
 
-@pytest.mark.parametrize("T,H,shift", [(1, 8, 0), (3, 20, 0), (7, 2048, 0), (5, 4096, 1), (1, 33, 3)])
+@pytest.mark.parametrize("T,H,shift", [(1, 8, 0), (3, 20, 0), (7, 2048, 0), (5, 4096, 1), (1, 33, 3), (300, 5120, 0), (2100, 4096, 0), (2, 12, 4), (3, 20, 4)])
 def test_elementwise(ops, T, H, shift):      # noqa: F811
     g = torch.Generator(device=DEV).manual_seed(5)
     a, b = [torch.randn(T * H + shift, generator=g, device=DEV).bfloat16()[shift:].view(T, H) for _ in range(2)]
