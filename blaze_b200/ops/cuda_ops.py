@@ -111,9 +111,9 @@ class CudaOps:
         lib.blz_embed.argtypes = [VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, VP]
         lib.blz_rmsnorm.argtypes = [VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_float, _c.c_int, _c.c_int, _c.c_int, VP]
         lib.blz_swiglu.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, VP]
-        lib.blz_attn_prep.argtypes = [VP, VP, VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
+        lib.blz_attn_prep_runs.argtypes = [VP, VP, VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                       _c.c_float, _c.c_float, _c.c_int, _c.c_int, _c.c_float, _c.c_float, _c.c_longlong,
-                                      _c.c_longlong, _c.c_int, _c.c_longlong, _c.c_int, _c.c_int, VP]
+                                      _c.c_longlong, _c.c_int, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int, VP]
         lib.blz_attn_tc.argtypes = [VP, VP, VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
                                     _c.c_longlong, _c.c_longlong, _c.c_float, _c.c_float, _c.c_float, _c.c_int, VP, VP, _c.c_int, VP]
         lib.blz_attn_decode_tree.argtypes = [VP, VP, VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int,
@@ -715,12 +715,12 @@ class CudaOps:
                 m0, m1 = int(sec[0]), int(sec[0]) + int(sec[1])
             else:
                 m0 = m1 = cfg.rotary_dim // 2          # no sections: every frequency follows the first stream
-        self._check(self.lib.blz_attn_prep(_ptr(qkv), _ptr(q), _ptr(gate), _ptr(kv.kv[layer_idx]), _ptr(pos),
-                                           _ptr(batch.slot_mapping), _ptr(model.inv_freq), _ptr(attn.q_norm), _ptr(attn.k_norm),
-                                           T, attn.heads, attn.kv_heads, D, cfg.rotary_dim, cfg.rms_norm_eps,
-                                           model.rope_scale, int(cfg.attn_output_gate), int(cfg.zero_centered_norm),
-                                           1.0, 1.0, kv.kv[layer_idx].stride(0), kv.kv[layer_idx].stride(1),
-                                           int(getattr(model, "kv_rotate", False)), pos_stride, m0, m1, self._stream()),
+        self._check(self.lib.blz_attn_prep_runs(_ptr(qkv), _ptr(q), _ptr(gate), _ptr(kv.kv[layer_idx]), _ptr(pos),
+                                                _ptr(batch.slot_mapping), _ptr(model.inv_freq), _ptr(attn.q_norm), _ptr(attn.k_norm),
+                                                T, attn.heads, attn.kv_heads, D, cfg.rotary_dim, cfg.rms_norm_eps,
+                                                model.rope_scale, int(cfg.attn_output_gate), int(cfg.zero_centered_norm),
+                                                1.0, 1.0, kv.kv[layer_idx].stride(0), kv.kv[layer_idx].stride(1),
+                                                int(getattr(model, "kv_rotate", False)), pos_stride, m0, m1, int(batch.max_q_len), self._stream()),
                     "attn_prep")
         return q, gate
 

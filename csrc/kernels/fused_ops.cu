@@ -1024,11 +1024,12 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   return (int)cudaGetLastError();
 }
 
-BLZ_API int blz_attn_prep(const void* qkv, void* q_out, void* gate_out, void* kv_pool, const int* positions,
-                          const int* slot_mapping, const float* inv_freq, const void* q_norm_w, const void* k_norm_w,
-                          int T, int Hq, int Hkv, int D, int rot_dim, float eps, float rope_scale, int gated,
-                          int zero_centered, float k_scale, float v_scale, long long page_stride, long long head_stride,
-                          int rotate, long long pos_stride, int mrope0, int mrope1, cudaStream_t s) {
+// longest: the most new tokens of a sequence (host knowledge): a page that one step fills takes 16.
+BLZ_API int blz_attn_prep_runs(const void* qkv, void* q_out, void* gate_out, void* kv_pool, const int* positions,
+                               const int* slot_mapping, const float* inv_freq, const void* q_norm_w, const void* k_norm_w,
+                               int T, int Hq, int Hkv, int D, int rot_dim, float eps, float rope_scale, int gated,
+                               int zero_centered, float k_scale, float v_scale, long long page_stride, long long head_stride,
+                               int rotate, long long pos_stride, int mrope0, int mrope1, int longest, cudaStream_t s) {
   if (T == 0) return 0;
   const int half = rot_dim / 2, vpl = D / 32;
   if ((D != 64 && D != 128 && D != 256) || rot_dim > D || half % vpl || ((half / vpl) & (half / vpl - 1)) || half / vpl > 16)
@@ -1040,12 +1041,19 @@ BLZ_API int blz_attn_prep(const void* qkv, void* q_out, void* gate_out, void* kv
   // 8 dims per lane: head_dim 128 and 256, no rotation, the rotated pairs a whole number of lanes apart, rows on 16 bytes
   const bool on16 = !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(gate_out) |
                        reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w) | reinterpret_cast<uintptr_t>(kv_pool)) & 15);
-  if (D != 64 && !rotate && half % 8 == 0 && half > 0 && on16 && page_stride % 16 == 0 && head_stride % 16 == 0) {
-    // Values in blocks of their own from 64 tokens on (fewer: hardly a page is filled).  Few tokens take a warp for every pass over
-    // the heads, so that nothing waits in turn; many keep blocks of four warps.
-    const int v_blocks = T >= 64 ? (T + 15) / 16 : 0, hpw = 256 / D;
-    const int passes = (Hq + 2 * Hkv + hpw - 1) / hpw;
-    const int warps = T > 1024 ? 4 : passes < 4 ? 4 : passes > 16 ? 16 : passes;
+  // ... except for many single tokens of few heads, which the kernel by single heads spreads over more warps (8 + 2 x 8 heads of 128,
+  // 700 tokens of decode steps: 11.0 us there, 12.2 here).
+  const int heads = Hq + 2 * Hkv, sms = sm_count();
+  if (D != 64 && !rotate && half % 8 == 0 && half > 0 && on16 && page_stride % 16 == 0 && head_stride % 16 == 0 &&
+      (longest >= 16 || heads > 24 || T <= sms)) {
+    // Values in blocks of their own where the step may fill pages, from 64 tokens on.  A warp for every pass over the heads as long as
+    // there is a block per SM, so that nothing waits in turn; then blocks of eight warps, and of four from some four blocks per SM
+    // on.  Over the kernel by single heads, 4 / 8 / 12 / 16 warps: 32 + 2 x 8 heads of 128, prompts of 128 tokens 0.85 / 0.73 / 0.66 /
+    // 0.70, 384 tokens 0.61 / 0.59 / 0.82 / 0.78, 1024 tokens 0.48 / 0.56 / 0.73 / 0.79; 700 single tokens 1.01 / 1.02 / 1.11 / 1.15;
+    // 16 + 2 x 2 gated heads of 256, 700 tokens 0.50 / 0.63 / 0.77 / 1.07.
+    const int v_blocks = T >= 64 && longest >= 16 ? (T + 15) / 16 : 0, hpw = 256 / D;
+    const int passes = (heads + hpw - 1) / hpw, most = T <= sms ? 12 : T <= 4 * sms ? 8 : 4;
+    const int warps = passes < 4 ? 4 : passes > most ? most : passes;
 #define BLZ_PREP(DD)                                                                                                 \
   launch_pdl(attn_prep_heads_kernel<DD>, dim3(T + v_blocks), dim3(warps * 32), 0, s, (const bf16*)qkv, (bf16*)q_out,     \
              (bf16*)gate_out, (uint8_t*)kv_pool, positions, slot_mapping, inv_freq, (const bf16*)q_norm_w,              \
@@ -1066,6 +1074,16 @@ BLZ_API int blz_attn_prep(const void* qkv, void* q_out, void* gate_out, void* kv
   if (D == 64) BLZ_PREP(64); else if (D == 128) BLZ_PREP(128); else BLZ_PREP(256);
 #undef BLZ_PREP
   return (int)cudaGetLastError();
+}
+
+BLZ_API int blz_attn_prep(const void* qkv, void* q_out, void* gate_out, void* kv_pool, const int* positions,
+                          const int* slot_mapping, const float* inv_freq, const void* q_norm_w, const void* k_norm_w,
+                          int T, int Hq, int Hkv, int D, int rot_dim, float eps, float rope_scale, int gated,
+                          int zero_centered, float k_scale, float v_scale, long long page_stride, long long head_stride,
+                          int rotate, long long pos_stride, int mrope0, int mrope1, cudaStream_t s) {
+  return blz_attn_prep_runs(qkv, q_out, gate_out, kv_pool, positions, slot_mapping, inv_freq, q_norm_w, k_norm_w, T, Hq, Hkv, D, rot_dim,
+                            eps, rope_scale, gated, zero_centered, k_scale, v_scale, page_stride, head_stride, rotate, pos_stride, mrope0,
+                            mrope1, T, s);
 }
 
 namespace blz {

@@ -209,8 +209,9 @@ def test_prompt_attention(ops, Hq, Hkv, ctxs, qlens, splits):      # noqa: F811
     assert err.max().item() < 0.15
 
 
-@pytest.mark.parametrize("D,Hq,Hkv,rot,gated", [(128, 8, 2, 128, False), (128, 6, 3, 64, True), (256, 4, 2, 64, True), (256, 2, 1, 256, False)])
-@pytest.mark.parametrize("chunks", [[(0, 64)], [(11, 90), (0, 17)], [(5, 1)] * 3 + [(16, 70), (15, 1), (0, 40)], [(3, 20)], [(0, 1100)]])
+@pytest.mark.parametrize("D,Hq,Hkv,rot,gated", [(128, 8, 2, 128, False), (128, 16, 8, 128, False), (128, 6, 3, 64, True), (256, 4, 2, 64, True), (256, 2, 1, 256, False)])
+@pytest.mark.parametrize("chunks", [[(0, 64)], [(11, 90), (0, 17)], [(5, 1)] * 3 + [(16, 70), (15, 1), (0, 40)], [(3, 20)], [(0, 1100)], [(i % 17, 1) for i in range(170)],
+                                    [(3, 15)] * 20, [(5, 300), (0, 3)]])
 def test_attention_preparation_writes_pages(ops, D, Hq, Hkv, rot, gated, chunks):      # noqa: F811
     """Queries, keys and values of steps with whole pages, parts of pages and single tokens: every page byte as the reference has
     it, nothing written for rows without a slot."""
