@@ -10,7 +10,10 @@
 // layout, so one 1-D bulk copy per page and operand feeds the tensor core with no register pass.  The online-softmax state
 // (max, sum, output row) stays in registers: one thread per query row.
 //
-// head_dim 128: attn_prompt_kernel, two CTAs of four warps per SM, see there.
+// head_dim 128, more blocks than SMs: attn_prompt_kernel, two CTAs of four warps per SM, see there.
+// attn_tc_kernel: one CTA per SM with warps of their own for loads and MMAs.
+// head_dim 128, as many blocks as SMs at most (192 threads): warp 0 loads pages (block-table walk + bulk copies), warp 1 issues MMAs,
+// warps 2-5 run softmax / accumulation on TMEM lane quadrant (warp & 3), S and O_t are double-buffered.
 // head_dim 256 (384 threads = three warpgroups): an output row has 256 fp32 accumulators, too many for one thread, so
 // warps 0-3 run softmax and accumulate output columns 0-127, warps 4-7 accumulate columns 128-255 (they get each tile's
 // rescale factor and the final row sum through shared memory), warp 8 loads, warp 9 issues MMAs.  The register file is
@@ -347,15 +350,18 @@ __global__ void __launch_bounds__(PromptCfg::THREADS, 2) attn_prompt_kernel(Attn
   }
 }
 
-struct WideCfg {                                    // head_dim 256
-  static constexpr int D = 256;
+template <int D>
+struct AttnCfg {
+  static constexpr int TILE = 128;                 // tokens per KV tile
   static constexpr int PAGE_BYTES = 16 * D;        // one operand (K or V^T) of one page and head
   static constexpr int TILE_BYTES = 8 * PAGE_BYTES;
-  static constexpr int STAGES = 2;
+  static constexpr int STAGES = D == 128 ? 4 : 2;
   static constexpr int Q_BYTES = 128 * D;
   static constexpr int P_BYTES = 128 * 128;
-  static constexpr int THREADS = 384;
-  static constexpr int XCH_BYTES = (4 * 128 + 2 * 128 * 2) * 4;   // rescale factors [4][128], (max, sum) [2][128][2]
+  static constexpr bool WIDE = D > 128;            // two accumulator warpgroups, one output buffer in TMEM
+  static constexpr int THREADS = WIDE ? 384 : 192;
+  static constexpr int OBUF = WIDE ? 1 : 2;
+  static constexpr int XCH_BYTES = WIDE ? (4 * 128 + 2 * 128 * 2) * 4 : 0;   // rescale factors [4][128], (max, sum) [2][128][2]
   static constexpr int SMEM = Q_BYTES + STAGES * 2 * TILE_BYTES + 2 * P_BYTES + XCH_BYTES + 1024 + 512;
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
 };
@@ -363,18 +369,21 @@ struct WideCfg {                                    // head_dim 256
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
-__global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnParams p) {
-  using Cfg = WideCfg;
-  constexpr int ST = Cfg::STAGES, D = Cfg::D;
-  constexpr int ACC = 128;                         // output columns accumulated by one thread
+template <int D>
+__global__ void __launch_bounds__(AttnCfg<D>::THREADS, 1) attn_tc_kernel(AttnParams p) {
+  using Cfg = AttnCfg<D>;
+  constexpr int ST = Cfg::STAGES;
+  constexpr bool WIDE = Cfg::WIDE;
+  constexpr int OBUF = Cfg::OBUF;
+  constexpr int ACC = WIDE ? 128 : D;              // output columns accumulated by one thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + Cfg::Q_BYTES;
   uint8_t* sV = sK + ST * Cfg::TILE_BYTES;
   uint8_t* sP = sV + ST * Cfg::TILE_BYTES;
-  float* s_alpha = reinterpret_cast<float*>(sP + 2 * Cfg::P_BYTES);     // [4][128] rescale factor of (tile & 3, row)
-  float* s_fin = s_alpha + 4 * 128;                                     // [2][128][2] (max, sum) of (item & 1, row)
+  float* s_alpha = reinterpret_cast<float*>(sP + 2 * Cfg::P_BYTES);     // WIDE: [4][128] rescale factor of (tile & 3, row)
+  float* s_fin = s_alpha + 4 * 128;                                     // WIDE: [2][128][2] (max, sum) of (item & 1, row)
   uint64_t* bars = reinterpret_cast<uint64_t*>(sP + 2 * Cfg::P_BYTES + Cfg::XCH_BYTES);
   uint64_t* k_full = bars;                 // [ST]
   uint64_t* v_full = k_full + ST;          // [ST]
@@ -382,24 +391,25 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
   uint64_t* s_full = kv_empty + ST;        // [2]
   uint64_t* s_empty = s_full + 2;          // [2]
   uint64_t* p_full = s_empty + 2;          // [2]
-  uint64_t* o_full = p_full + 2;           // [1]
-  uint64_t* o_empty = o_full + 1;          // [1]
-  uint64_t* q_full = o_empty + 1;          // [1]
+  uint64_t* o_full = p_full + 2;           // [2]
+  uint64_t* o_empty = o_full + 2;          // [2]
+  uint64_t* q_full = o_empty + 2;          // [1]
   uint64_t* q_empty = q_full + 1;          // [1]
-  uint64_t* fin_full = q_empty + 1;        // [2] the softmax warps have published (max, sum) of an item
+  uint64_t* fin_full = q_empty + 1;        // [2] WIDE: the softmax warps have published (max, sum) of an item
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fin_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // role of this warp
-  const bool is_loader = warp == 8, is_mma = warp == 9;
+  const bool is_loader = warp == (WIDE ? 8 : 0), is_mma = warp == (WIDE ? 9 : 1);
+  const bool is_softmax = WIDE ? warp < 4 : (warp >= 2 && warp < 6);
   if (threadIdx.x == 0) {
     for (int i = 0; i < ST; ++i) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&kv_empty[i], 1); }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s_full[i], 1); mbar_init(&s_empty[i], 4); mbar_init(&p_full[i], 4);
+      mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], WIDE ? 8 : 4);
       mbar_init(&fin_full[i], 4);
     }
-    mbar_init(o_full, 1); mbar_init(o_empty, 8);
     mbar_init(q_full, 4); mbar_init(q_empty, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -409,6 +419,10 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // output accumulator buffer, its barrier index and barrier parity for global tile number gj
+  auto o_buf = [&](int gj) -> int { return OBUF == 2 ? (gj & 1) : 0; };
+  auto o_par = [&](int gj) -> uint32_t { return (uint32_t)(OBUF == 2 ? ((gj >> 1) & 1) : (gj & 1)); };
+
   const int group = p.Hq / p.Hkv;
   const int total = p.num_items * p.Hkv * p.splits;
 
@@ -474,15 +488,16 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
           const int s = gj % ST, pb = gj & 1;
           if (!mbar_wait(&v_full[s], (gj / ST) & 1, abort_flag, p.status)) return false;
           if (!mbar_wait(&p_full[pb], (gj >> 1) & 1, abort_flag, p.status)) return false;
-          if (!mbar_wait(o_empty, (gj & 1) ^ 1, abort_flag, p.status)) return false;
+          const int ob = o_buf(gj);
+          if (!mbar_wait(&o_empty[ob], o_par(gj) ^ 1, abort_flag, p.status)) return false;
           tc_fence_after();
           const uint32_t pa = smem_u32(sP + pb * Cfg::P_BYTES), va = smem_u32(sV + s * Cfg::TILE_BYTES);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
-            mma_f8(tmem + 256, make_smem_desc(pa + ks * 256, 128, 1024, kSwzNone),
+            mma_f8(tmem + 256 + ob * 128, make_smem_desc(pa + ks * 256, 128, 1024, kSwzNone),
                    make_smem_desc(va + ks * 2 * Cfg::PAGE_BYTES, Cfg::PAGE_BYTES, 128, kSwzNone),
                    make_idesc(0, 0, 128, D), ks > 0);
-          mma_commit(o_full);
+          mma_commit(&o_full[ob]);
           mma_commit(&kv_empty[s]);
           return true;
         };
@@ -503,7 +518,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
         if (ok) mma_commit(q_empty);
       }
     } else if constexpr (ROLE == R_UPPER) {
-      // -------------------------------------------------------------- output columns 128..255
+      // -------------------------------------------------------------- output columns 128..255 (head_dim 256 only)
       const int qd = warp & 3;
       const int r = qd * 32 + lane;
       const bool live = r < nrows;
@@ -515,7 +530,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
       bool ok = true;
       for (int i = 0; i < n && ok; ++i) {
         const int gj = g + i;
-        ok = __all_sync(0xffffffffu, mbar_wait(o_full, gj & 1, abort_flag, p.status));
+        ok = __all_sync(0xffffffffu, mbar_wait(&o_full[0], o_par(gj), abort_flag, p.status));
         if (!ok) break;
         tc_fence_after();
         const float alpha = s_alpha[(gj & 3) * 128 + r];     // written before the row's probabilities were handed over
@@ -529,7 +544,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(o_empty);
+        if (lane == 0) mbar_arrive(&o_empty[0]);
       }
       if (n > 0 && ok) ok = mbar_wait(&fin_full[item_it & 1], (uint32_t)((item_it >> 1) & 1), abort_flag, p.status);
       if (ok && live && n > 0) {
@@ -574,20 +589,21 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
       float alpha_prev = 1.f;
       bool ok = true;
       auto accumulate = [&](int gj, float alpha) -> bool {
+        const int ob = o_buf(gj);
         // tcgen05.ld is warp-collective: the wait's outcome is made warp-uniform before any lane loads
-        if (!__all_sync(0xffffffffu, mbar_wait(o_full, gj & 1, abort_flag, p.status))) return false;
+        if (!__all_sync(0xffffffffu, mbar_wait(&o_full[ob], o_par(gj), abort_flag, p.status))) return false;
         tc_fence_after();
 #pragma unroll
         for (int cch = 0; cch < ACC / 32; ++cch) {
           uint32_t v[32];
-          tmem_ld32(tmem + 256 + cch * 32 + ((uint32_t)(qd * 32) << 16), v);
+          tmem_ld32(tmem + 256 + ob * 128 + cch * 32 + ((uint32_t)(qd * 32) << 16), v);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[cch * 32 + i] = acc[cch * 32 + i] * alpha + __uint_as_float(v[i]);
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(o_empty);
+        if (lane == 0) mbar_arrive(&o_empty[ob]);
         return true;
       };
       for (int i = 0; i < n && ok; ++i) {
@@ -647,7 +663,7 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
         }
         l_run = l_run * alpha + rs;
         m_run = m_new;
-        s_alpha[(gi & 3) * 128 + r] = alpha;   // for the warps that accumulate the other output half
+        if constexpr (WIDE) s_alpha[(gi & 3) * 128 + r] = alpha;   // for the warps that accumulate the other output half
         fence_async_smem();
         tc_fence_before();
         __syncwarp();
@@ -656,11 +672,13 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
         alpha_prev = alpha;
       }
       if (ok && n > 0) ok = accumulate(g + n - 1, alpha_prev);
-      if (n > 0) {             // (also after a failed wait: the other warpgroup's bounded wait then ends at once, via the abort flag)
-        s_fin[((item_it & 1) * 128 + r) * 2] = m_run;
-        s_fin[((item_it & 1) * 128 + r) * 2 + 1] = l_run;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&fin_full[item_it & 1]);
+      if constexpr (WIDE) {
+        if (n > 0) {           // (also after a failed wait: the other warpgroup's bounded wait then ends at once, via the abort flag)
+          s_fin[((item_it & 1) * 128 + r) * 2] = m_run;
+          s_fin[((item_it & 1) * 128 + r) * 2 + 1] = l_run;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&fin_full[item_it & 1]);
+        }
       }
       // ---- write out
       if (ok && live) {
@@ -688,17 +706,23 @@ __global__ void __launch_bounds__(WideCfg::THREADS, 1) attn_wide_kernel(AttnPara
   }
   };   // run
 
-  // 384 threads start with 168 registers each; the loader / MMA warpgroup hands most of its share to the other two
-  if (warp >= 8) {
-    reg_dec<64>();
+  if constexpr (WIDE) {
+    // 384 threads start with 168 registers each; the loader / MMA warpgroup hands most of its share to the other two
+    if (warp >= 8) {
+      reg_dec<64>();
+      if (is_loader) run(std::integral_constant<int, R_LOAD>{});
+      else if (is_mma) run(std::integral_constant<int, R_MMA>{});
+    } else if (warp >= 4) {
+      reg_inc<200>();
+      run(std::integral_constant<int, R_UPPER>{});
+    } else {
+      reg_inc<240>();
+      run(std::integral_constant<int, R_SOFTMAX>{});
+    }
+  } else {
     if (is_loader) run(std::integral_constant<int, R_LOAD>{});
     else if (is_mma) run(std::integral_constant<int, R_MMA>{});
-  } else if (warp >= 4) {
-    reg_inc<200>();
-    run(std::integral_constant<int, R_UPPER>{});
-  } else {
-    reg_inc<240>();
-    run(std::integral_constant<int, R_SOFTMAX>{});
+    else if (is_softmax) run(std::integral_constant<int, R_SOFTMAX>{});
   }
   tc_fence_before();
   __syncthreads();
@@ -769,18 +793,24 @@ BLZ_API int blz_attn_tc(const void* q, void* out, const void* pool, const int* b
   p.tokens_per_block = 128 / (Hq / Hkv);
   p.status = status_word();
   p.min_rows = 0; p.max_rows = 1 << 30; p.row_blocks = 1; p.prof = nullptr;
-  static PerDeviceOnce configured, configured_wide;
+  // With a CTA per SM or less nobody covers the waits of attn_prompt_kernel's four warps, and the kernel with warps for loads and MMAs is
+  // the faster one: 256 tokens after 15000, 32 + 8 heads (128 CTAs) 137 us there, 173 here; 100 tokens of a prompt 10.5 and 11.1; with
+  // 8 prompts of 1024 tokens (2048 blocks) 217 and 163.
+  const int total = num_items * Hkv * splits;
+  const bool pairs = D == 128 && total > sm_count();
+  static PerDeviceOnce configured, configured_one, configured_wide;
   {
-    cudaError_t e = D == 128 ? configured.smem_limit(attn_prompt_kernel, PromptCfg::SMEM)
-                             : configured_wide.smem_limit(attn_wide_kernel, WideCfg::SMEM);
+    cudaError_t e = D == 256 ? configured_wide.smem_limit(attn_tc_kernel<256>, AttnCfg<256>::SMEM)
+                    : pairs  ? configured.smem_limit(attn_prompt_kernel, PromptCfg::SMEM)
+                             : configured_one.smem_limit(attn_tc_kernel<128>, AttnCfg<128>::SMEM);
     if (e != cudaSuccess) return (int)e;
   }
-  const int total = num_items * Hkv * splits;
-  const int fit = (D == 128 ? 2 : 1) * sm_count();
+  const int fit = (pairs ? 2 : 1) * sm_count();
   int grid = total < fit ? total : fit;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  if (D == 128) attn_prompt_kernel<<<grid, PromptCfg::THREADS, PromptCfg::SMEM, stream>>>(p);
-  else attn_wide_kernel<<<grid, WideCfg::THREADS, WideCfg::SMEM, stream>>>(p);
+  if (D == 256) attn_tc_kernel<256><<<grid, AttnCfg<256>::THREADS, AttnCfg<256>::SMEM, stream>>>(p);
+  else if (pairs) attn_prompt_kernel<<<grid, PromptCfg::THREADS, PromptCfg::SMEM, stream>>>(p);
+  else attn_tc_kernel<128><<<grid, AttnCfg<128>::THREADS, AttnCfg<128>::SMEM, stream>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (splits > 1) {

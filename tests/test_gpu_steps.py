@@ -200,6 +200,8 @@ def test_decode_attention_runs_that_are_not_a_number(ops):      # noqa: F811
 @pytest.mark.parametrize("Hq,Hkv,ctxs,qlens,splits", [
     (8, 2, [17], [17], 0), (32, 8, [128, 129, 33], [128, 129, 33], 0), (8, 1, [1100, 40], [300, 40], 1),      # blocks of 128 rows and parts
     (4, 4, [700], [513], 1), (16, 2, [2000, 90], [70, 60], 3), (32, 4, [300], [40], 8),                        # split key ranges, some empty
+    # the same with more blocks than SMs: two CTAs of four warps each
+    (32, 8, [700, 129, 33], [700, 129, 33], 0), (8, 1, [2600], [2500], 1), (4, 4, [5200], [5000], 0), (16, 2, [2000, 90], [520, 60], 3), (32, 4, [300], [200], 8),
 ])
 def test_prompt_attention(ops, Hq, Hkv, ctxs, qlens, splits):      # noqa: F811
     """Blocks whose rows see no key of a tile, few keys of it, or all; runs of tiles whose maxima grow and do not."""
