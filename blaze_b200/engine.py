@@ -9,6 +9,7 @@ control group.
 """
 from __future__ import annotations
 
+import gc
 import threading
 import time
 from dataclasses import dataclass, field
@@ -705,8 +706,15 @@ class _Graph:
             pool = None
             if self.mode == "logits":
                 pool = self.eng._sampled_pool = self.eng._sampled_pool or torch.cuda.graph_pool_handle()
-            with torch.cuda.graph(self.graph, pool=pool):
-                self.out = self.eng._run(self.batch, "hidden" if self.mode == "logits" else self.mode)
+            # no collection of garbage meanwhile: a captured step of an engine that is gone, given back during a capture, ends it
+            collects = gc.isenabled()
+            gc.disable()
+            try:
+                with torch.cuda.graph(self.graph, pool=pool):
+                    self.out = self.eng._run(self.batch, "hidden" if self.mode == "logits" else self.mode)
+            finally:
+                if collects:
+                    gc.enable()
             self.kernels = self.eng.model.ops.launches - l0
         self.graph.replay()
         R = B * self.L

@@ -118,6 +118,39 @@ def test_captured_steps_are_there_from_the_start():
     assert set(eng._graphs) == keys
 
 
+def test_capture_while_garbage_holds_a_captured_step():
+    """A captured step that only a reference cycle keeps is not given back in the middle of another step's capture."""
+    import gc
+    eng, step = _steps_engine("dense")
+    want = step(3, False)
+    run, old, lists = eng._run, gc.get_threshold(), []
+
+    def collecting(batch, mode, hidden_in=None):
+        gc.set_threshold(1, 1, 1)
+        lists.extend([[i] for i in range(4)])      # a collection would come now
+        try:
+            return run(batch, mode, hidden_in)
+        finally:
+            gc.set_threshold(1 << 30)
+    gc.collect()
+    gc.set_threshold(1 << 30)                      # none until the steps run
+    try:
+        g, x = torch.cuda.CUDAGraph(), torch.zeros(8, device=DEV)
+        with torch.cuda.graph(g):
+            x += 1
+        cycle = [g]
+        cycle.append(cycle)
+        step(3, True)                              # launched one by one
+        del g, cycle
+        eng._run = collecting
+        got = step(3, True)                        # captured
+    finally:
+        eng._run = run
+        gc.set_threshold(*old)
+    assert ("logits", 3, eng._key_splits(3)) in eng._graphs and gc.isenabled()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [
     (32, 8, [1], 1), (32, 8, [129], 1), (32, 8, [5000, 3, 128, 1291], 1),          # fewer items than CTAs: runs of tiles
     (16, 2, [2600, 40, 1025], 1), (32, 4, [700], 2), (32, 8, [900, 260], 5), (32, 4, [1500, 64], 8),      # 8, 16, 20 and 64 rows
