@@ -154,7 +154,8 @@ def test_capture_while_garbage_holds_a_captured_step():
 @pytest.mark.parametrize("Hq,Hkv,ctxs,q", [
     (32, 8, [1], 1), (32, 8, [129], 1), (32, 8, [5000, 3, 128, 1291], 1),          # fewer items than CTAs: runs of tiles
     (16, 2, [2600, 40, 1025], 1), (32, 4, [700], 2), (32, 8, [900, 260], 5), (32, 4, [1500, 64], 8),      # 8, 16, 20 and 64 rows
-    (32, 8, [33 + 7 * i for i in range(40)], 1), (64, 8, [200 + i for i in range(19)], 3),                 # more items than CTAs
+    (8, 8, [129, 1500], 1), (16, 8, [700, 40], 1), (24, 8, [900, 260], 3), (40, 8, [1291], 2), (12, 4, [513, 77], 4),      # 1, 2, 9, 10 and 12 rows
+    (32, 8, [33 + 7 * i for i in range(40)], 1), (24, 8, [33 + 7 * i for i in range(40)], 3), (64, 8, [200 + i for i in range(19)], 3),                 # more items than CTAs
 ])
 def test_decode_attention_runs_of_tiles(ops, Hq, Hkv, ctxs, q):      # noqa: F811
     got, want = _attention_case(ops, Hq, Hkv, ctxs, [q] * len(ctxs))
