@@ -27,7 +27,7 @@
 // and conversion from overlapping), tiles that no mask touches skip the masks, and what is done once per item is short: code
 // that runs once per item comes from beyond the instruction caches.  256 sequences of 1.2 K tokens, 8 kv heads of 4 rows:
 // 120 -> 113 us; 4 kv heads of 8 rows: 99 -> 77 us; 64 sequences, 8 kv heads of 8 rows: 52 -> 36 us; 16 sequences of 1.0 K to
-// 2.1 K tokens with 20 rows: 86 -> 59 us.
+// 2.1 K tokens with 20 rows: 86 -> 51 us (with the loaders).
 // (Warp MMAs with the rows as M and probabilities in half precision need no word between warps until an item ends and took
 // 43 us there, but 189 instead of 113 us for 4 rows; and a token verified in one kernel and decoded in the other would see its
 // probabilities rounded differently.)

@@ -794,8 +794,9 @@ BLZ_API int blz_attn_tc(const void* q, void* out, const void* pool, const int* b
   p.status = status_word();
   p.min_rows = 0; p.max_rows = 1 << 30; p.row_blocks = 1; p.prof = nullptr;
   // With a CTA per SM or less nobody covers the waits of attn_prompt_kernel's four warps, and the kernel with warps for loads and MMAs is
-  // the faster one: 256 tokens after 15000, 32 + 8 heads (128 CTAs) 137 us there, 173 here; 100 tokens of a prompt 10.5 and 11.1; with
-  // 8 prompts of 1024 tokens (2048 blocks) 217 and 163.
+  // the faster one: 256 tokens after 15000, 32 + 8 heads (128 CTAs) 137 us there, 173 here; 100 tokens of a prompt 10.5 and 11.1.  From
+  // there on this one is: 23 launches of 152 to 2048 blocks take 0.79 - 0.98 of the time there (600 tokens 28.7 and 26.6 us, 640 after
+  // 15000 440 and 348, 4096 tokens 279 and 233, 8 prompts of 1024 217 and 172).
   const int total = num_items * Hkv * splits;
   const bool pairs = D == 128 && total > sm_count();
   static PerDeviceOnce configured, configured_one, configured_wide;
