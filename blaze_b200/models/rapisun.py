@@ -28,7 +28,7 @@ def _up(n: int, m: int) -> int:
 
 
 class Rapisun(Model):
-    kernel_sources = ("host", "fused_ops", "gemm_tc", "gemm_sk", "gemm_wide", "moe_gemm", "gemm_simple", "streams", "attn_maps",
+    kernel_sources = ("host", "fused_ops", "gemm_tc", "gemm_sk", "gemm_wide", "gemm_pair", "moe_gemm", "gemm_simple", "streams", "attn_maps",
                       "attn_maps_tc", "latent", "recurrent", "moe", "sampling")
     cuda_dtypes = (torch.bfloat16, torch.float32)
     fp8_pages = False

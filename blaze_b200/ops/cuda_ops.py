@@ -102,6 +102,11 @@ class CudaOps:
         self._sk_ok = os.environ.get("BLAZE_GEMM_SK", "1") != "0"
         self.SK_MAX_ROWS = 512
         self.tuning = None         # optional tune.Tuning: per-shape kernel choices measured on this device
+        lib.blz_gemm_pair.restype = _c.c_int
+        lib.blz_gemm_pair.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
+                                      VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_float, VP]
+        lib.blz_gemm_pair_columns.restype = _c.c_int
+        lib.blz_gemm_pair_columns.argtypes = [_c.c_int] * 5
         lib.blz_gemm_wide_ksplit.restype = _c.c_int
         lib.blz_gemm_wide_ksplit.argtypes = [_c.c_int, _c.c_int, _c.c_int]
         self._wide_ok = os.environ.get("BLAZE_GEMM_WIDE", "1") != "0"
@@ -603,7 +608,8 @@ class CudaOps:
                 # fp32 partials through distributed shared memory (about 5 us per 64 KB tile) costs what the split saves.
                 # A tuning table measured on this device (tune.tune_linear) overrides the rule.
                 tiles = ((M + 127) // 128) * ((lin.N + 127) // 128)
-                sk = lin.K >= 8192 and tiles <= 2 * self._sm // 2
+                # Above 256 rows the pairs of CTAs are faster (512 x 4096 x 12288: 35.8 against 29.7 us).
+                sk = M <= 256 and lin.K >= 8192 and tiles <= 2 * self._sm // 2
                 if self.tuning is not None:
                     from ..tune import bucket
                     hit = self.tuning.get(f"gemm{kind}", lin.N, lin.K, bucket(M))
@@ -616,6 +622,17 @@ class CudaOps:
             self._check(self.lib.blz_gemm_sk(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K,
                                              _ptr(rs), _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]),
                                              ks, act, limit, self._stream()), f"gemm_sk kind {kind}")
+            return out
+        # More than 256 rows: pairs of CTAs, the same sums in the same order.  Measured on B200 (us, single-CTA kernels / pairs): bf16 300 x
+        # 6144 x 4096 33 / 31, 1600 rows 84 / 61, 8192 rows 328 / 254; NVFP4 300 rows 20.5 / 17.2, 1600 rows 38 / 30, 8192 rows 115 / 92;
+        # MXFP8 300 x 12352 x 2048 22.5 / 22.4, 4096 rows 140 / 90.  Gated block-scaled products of few rows stay on wide tiles of one
+        # CTA, whose epilogue has a thread per token (NVFP4 x 24576 x 4096: 300 rows 33 / 35, 825 rows 55 / 57, 1200 rows 74 / 68).
+        if (wide is None and self._wide_ok and bn == 0 and M > 256 and kind in (0, 1, 2) and lin.N >= 512 and not kt and pending is None
+                and argmax_parts is None and max_ctas != 1 and not relu2 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0))
+                and (not swiglu or (lin.N % 32 == 0 and (kind == 0 or M > 1024)))):
+            self._check(self.lib.blz_gemm_pair(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
+                                               _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), int(f32), 0, max_ctas, act, limit,
+                                               self._stream()), f"gemm_pair kind {kind}")
             return out
         if wide is None:
             # Measured on B200 (Qwen3-8B shapes, captured-graph timing): 256-feature tiles win for block-scaled prefill GEMMs

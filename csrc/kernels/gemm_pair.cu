@@ -1,0 +1,432 @@
+// GEMM of many rows on CTA pairs:  C[tokens, features] = X[tokens, K] · W[features, K]^T.
+//
+// A pair (a cluster of two CTAs on neighbouring SMs) computes 256 features x up to 256 tokens with one tcgen05.mma.cta_group::2 per
+// K step: features are the MMA lanes (128 in each CTA), tokens its columns, half of their rows in either CTA's shared memory.  Per 128
+// bytes of K an SM so fetches 16 KB of weights and at most 16 KB of activations, where a CTA by itself fetches 16 + 32 KB for a tile of
+// the same work (128 x 256): the path from L2 to shared memory, about 64 bytes per clock and SM, is what bounds these products, not
+// the tensor pipe.  Tokens as columns: a tile is as wide as the rows need (a multiple of 64), features are whole tiles in practice.
+//
+// Two accumulators per CTA, so that the epilogue of a tile runs beside the next tile's MMAs.  Scale factors of the block-scaled kinds take
+// 48 (NVFP4) or 12 columns of tensor memory (copied anew for every stage: copies and MMAs of one issuer run in order), so at 256
+// columns the two accumulators share as many: the epilogue reads the shared ones first, and the next tile waits for those alone.
+//
+// 448 threads: warp 0 = TMA producer (one per CTA, its own half of the tile), warp 1 = MMA issuer (first CTA of the pair only), warps
+// 2-13 = epilogue.  Persistent, one pair per two SMs.  Barriers: `full` lives in the first CTA and counts both CTAs' bytes; `empty` and
+// `acc_full` are in both and raised by multicast commits; `acc_free` is in the first and counts both CTAs' epilogue warps.  Every wait is bounded;
+// the hardware cluster barrier is used at the start and, by all threads, at the end.  No load is multicast.
+//
+// Measured against one CTA per tile of 128 x 256 (gemm_wide.cu, gemm_tc.cu; device time of a call, L2 flushed): 8192 rows, NVFP4 x 4096 x
+// 12288 177 -> 138 us (6.0 PFLOP/s), x 6144 x 4096 115 -> 92, x 24576 x 4096 with the gated activation 380 -> 360; bf16 x 6144 x 4096
+// 328 -> 254; MXFP8 x 12352 x 2048 266 -> 171.  In a long run the chip's power limit takes a part of that back.  Of an NVFP4 tile's K
+// block at 256 columns (387 ns) the MMAs alone need 333.  Twelve epilogue warps: eight did not keep up with a gated tile of K 4096
+// (390 -> 371 us), sixteen have too few registers.  A loop of one thread that built each descriptor anew issued a K block in 330 ns
+// whatever its columns (371 -> 350).
+//
+// Counterpart in the reference: the tiled kernels of kernels/src/cuda/nvfp4_gemm.cu.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include "blaze/glu.cuh"
+#include "blaze/host.h"
+#include "blaze/sm100.cuh"
+
+namespace blz {
+
+bool gemm_oneshot_take_unsupported();   // gemm_tc.cu
+
+struct PairParams {
+  int M, N, K;                // tokens, features, elements
+  void* C;                    // [tokens, ldc] bf16 or fp32
+  long long ldc;
+  int out_f32;
+  const float* row_scale;     // per token, or null
+  const float* alpha;         // per feature, or null
+  const __nv_bfloat16* bias;  // per feature, or null
+  int sf_col_tiles;           // 4-column scale tiles per 128-row tile
+  int cn;                     // columns (tokens) of a tile
+  int acc1;                   // first tensor-memory column of the second accumulator
+  int act;                    // 1, 2: rows of W are [16 gate | 16 up] groups; C = gated activation, bf16 [tokens, N/2]
+  float act_limit;            // act 2: the clamp of glu.cuh
+  int* status;
+};
+
+template <int KIND> struct PKind;
+template <> struct PKind<0> { static constexpr int KMMA = 16, SF_ATOMS = 0; };
+template <> struct PKind<1> { static constexpr int KMMA = 64, SF_ATOMS = 4; };
+template <> struct PKind<2> { static constexpr int KMMA = 32, SF_ATOMS = 1; };
+
+template <int KIND>
+struct PairCfg {
+  static constexpr int KMMA = PKind<KIND>::KMMA;
+  static constexpr int BK = KMMA * 4;                       // 128 bytes of K per row and stage
+  static constexpr int SF_ATOMS = PKind<KIND>::SF_ATOMS;
+  static constexpr int A_BYTES = 128 * 128, B_BYTES = 128 * 128;
+  static constexpr int SF_BYTES = SF_ATOMS * 512;           // scales of 128 rows and one stage
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + 3 * SF_BYTES;
+  static constexpr int STAGES = (216 * 1024) / STAGE_BYTES;
+  static constexpr int SF_COLS = SF_ATOMS * 4 * 3;
+  static constexpr int SF_COL0 = 512 - SF_COLS;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 512 + 2 * 256 * 4;
+  static constexpr int EPI = 12;                            // epilogue warps
+  static constexpr int THREADS = 64 + EPI * 32;
+  static_assert((2 * STAGES + 5) * 8 + 8 <= 512 && SMEM <= 227 * 1024, "shared memory");
+  static_assert(SF_COLS <= 64, "the accumulators may share two chunks of 32 columns at most");
+};
+
+template <int KIND>
+__global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                                                            const __grid_constant__ CUtensorMap tmSW, const __grid_constant__ CUtensorMap tmSX,
+                                                            const PairParams p) {
+  using Cfg = PairCfg<KIND>;
+  constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS;
+  pdl_trigger();
+  extern __shared__ uint8_t smem_raw[];
+  // both CTAs of a pair round the same way: dynamic shared memory starts at the same offset in each
+  uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint8_t* sA = base;
+  uint8_t* sB = sA + STAGES * Cfg::A_BYTES;
+  uint8_t* sSFA = sB + STAGES * Cfg::B_BYTES;
+  uint8_t* sSFB = sSFA + STAGES * Cfg::SF_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sSFB + STAGES * 2 * Cfg::SF_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;      // [2]
+  uint64_t* acc_free = acc_full + 2;        // [2]
+  uint64_t* drain = acc_free + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  float* s_rs = reinterpret_cast<float*>(full + 64);        // [2][256] row scales of a tile's tokens (after 512 bytes of barriers)
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int cn = p.cn;
+  const int tiles_f = (p.N + 255) / 256, tiles_t = (p.M + cn - 1) / cn;
+  const int k_tiles = (p.K + BK - 1) / BK;
+  const int tiles = tiles_f * tiles_t;
+  const int groups = cn > 128 ? 2 : 1;      // 128-row scale tiles under a tile's tokens (tiles of 64 and 192 start in the middle of one)
+  const bool shared_cols = p.acc1 < cn;     // the accumulators overlap
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_free[i], 2 * Cfg::EPI); }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    prefetch_tmap(&tmW);
+    prefetch_tmap(&tmX);
+    if (ATOMS) { prefetch_tmap(&tmSW); prefetch_tmap(&tmSX); }
+  }
+  __syncwarp();
+  if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  cluster_arrive();                         // the peer's barriers are initialised before anything signals them
+  cluster_wait();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+
+  // tile u -> (feature tile, token tile): bands of eight token tiles, so that the pairs at work at one time share both operands in L2
+  auto decode = [&](int u, int& ft, int& tt) {
+    const int per_band = 8 * tiles_f, band = u / per_band, in = u - band * per_band;
+    const int width = min(8, tiles_t - band * 8);
+    ft = in / width;
+    tt = band * 8 + in - ft * width;
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer: this CTA's half of the operands
+    if (lane == 0) {
+      int s = 0; uint32_t ph = 0;
+      uint32_t used = 0, last = 0;          // stages filled so far, and the parity of their latest fill
+      bool ok = true;
+      for (int u = pair; u < tiles && ok; u += pairs) {
+        int ft, tt;
+        decode(u, ft, tt);
+        const int frow = ft * 256 + (int)rank * 128, t0 = tt * cn, trow = t0 + (int)rank * (cn >> 1);
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) { ok = false; break; }
+          const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
+          if (rank == 0) mbar_expect_tx(&full[s], 2u * (Cfg::A_BYTES + (uint32_t)cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
+          const int kc = KIND == 0 ? kt * BK : kt * 128;
+          tma_load_2d_pair(sA + s * Cfg::A_BYTES, &tmW, kc, frow, bar);
+          tma_load_2d_pair(sB + s * Cfg::B_BYTES, &tmX, kc, trow, bar);
+          if constexpr (ATOMS > 0) {
+            tma_load_3d_pair(sSFA + s * Cfg::SF_BYTES, &tmSW, 0, kt * ATOMS, frow >> 7, bar);
+            tma_load_3d_pair(sSFB + s * 2 * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, t0 >> 7, bar);
+          }
+          used |= 1u << s;
+          last = (last & ~(1u << s)) | (ph << s);
+          if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+      }
+      if (!ok && rank == 0)                 // no copy of either CTA is in flight when the pair leaves
+        for (int i = 0; i < STAGES; ++i)
+          if (used >> i & 1) mbar_drain(&full[i], last >> i & 1);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer of the pair.  The whole warp walks the loop, so that
+    // the descriptors stay in uniform registers, and one thread issues; they are built from their lower halves, which alone change.
+    if (rank == 0) {
+      int s = 0; uint32_t ph = 0;
+      int it = 0;
+      bool ok = true;
+      const bool leader = elect_one();
+      const uint32_t idesc = KIND == 0 ? make_idesc(1, 1, 256, cn) : make_idesc_bs(KIND == 1, KIND == 1, KIND == 2, 256, cn);
+      const uint32_t a_lo0 = (uint32_t)desc_sw128(smem_u32(sA)), b_lo0 = (uint32_t)desc_sw128(smem_u32(sB));
+      const uint32_t sa_lo0 = (uint32_t)make_smem_desc(smem_u32(sSFA), 0, 128, kSwzNone);
+      const uint32_t sb_lo0 = (uint32_t)make_smem_desc(smem_u32(sSFB), 0, 128, kSwzNone);
+      constexpr uint32_t OP_HI = (1024u >> 4) | 1u << 14 | (uint32_t)kSwz128 << 29, SF_HI = (128u >> 4) | 1u << 14;
+      auto desc = [](uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; };
+      for (int u = pair; u < tiles && ok; u += pairs, ++it) {
+        int ft, tt;
+        decode(u, ft, tt);
+        // Overlapping accumulators: the tile before this one has been read as far as the two overlap (and the one before that
+        // altogether).  Separate ones: the tile before the last has been read.
+        const int prev = shared_cols ? it - 1 : it - 2;
+        if (prev >= 0 && !mbar_wait_cluster(&acc_free[prev & 1], (prev >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t d = tmem + (it & 1 ? p.acc1 : 0);
+        const uint32_t sfa = tmem + Cfg::SF_COL0, sfb = sfa + ATOMS * 4, sfb0 = sfb + (((tt * cn) & 127) >> 5);
+        for (int kt = 0; kt < k_tiles; ++kt) {
+          if (!mbar_wait(&full[s], ph, abort_flag, p.status)) { ok = false; break; }
+          tc_fence_after();
+          const int nblk = min(4, (p.K - kt * BK + Cfg::KMMA - 1) / Cfg::KMMA);
+          const uint32_t a_lo = a_lo0 + s * (Cfg::A_BYTES >> 4), b_lo = b_lo0 + s * (Cfg::B_BYTES >> 4);
+          if (leader) {
+            if constexpr (ATOMS > 0) {
+              const uint32_t sa_lo = sa_lo0 + s * (Cfg::SF_BYTES >> 4), sb_lo = sb_lo0 + s * (2 * Cfg::SF_BYTES >> 4);
+#pragma unroll
+              for (int a = 0; a < ATOMS; ++a) {
+                tmem_cp_sf_pair(sfa + a * 4, desc(sa_lo + a * 32, SF_HI));
+                tmem_cp_sf_pair(sfb + a * 8, desc(sb_lo + a * 32, SF_HI));
+              }
+              if (groups == 2) {
+#pragma unroll
+                for (int a = 0; a < ATOMS; ++a) tmem_cp_sf_pair(sfb + a * 8 + 4, desc(sb_lo + (ATOMS + a) * 32, SF_HI));
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (j < nblk) {
+                const uint64_t da = desc(a_lo + j * 2, OP_HI), db = desc(b_lo + j * 2, OP_HI);
+                const uint32_t acc = (kt > 0 || j > 0) ? 1u : 0u;
+                if constexpr (KIND == 0) mma_f16_pair(d, da, db, idesc, acc);
+                else if constexpr (KIND == 1) mma_nvfp4_pair(d, da, db, idesc, sfa + j * 4, sfb0 + j * 8, acc);
+                else mma_mxf8_pair(d, da, db, idesc | make_idesc_bs(0, 0, 0, 0, 0, j, j), sfa, sfb0, acc);
+              }
+            }
+            mma_commit_pair(&empty[s]);
+          }
+          __syncwarp();
+          if (++s == STAGES) { s = 0; ph ^= 1; }
+        }
+        if (ok && leader) mma_commit_pair(&acc_full[it & 1]);
+        __syncwarp();
+      }
+      if (!ok && leader) {                  // the MMAs in flight end before their operands' memory goes
+        mma_commit_pair(drain);
+        mbar_drain(drain, 0);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue: lane = feature, column = token
+    const int q = warp & 3, part = (warp - 2) >> 2, etid = threadIdx.x - 64;
+    const uint32_t quad = (uint32_t)(q * 32) << 16;
+    const bool odd = lane & 1, hi = lane >= 16;
+    bool ok = true;
+    int it = 0;
+    for (int u = pair; u < tiles; u += pairs, ++it) {
+      int ft, tt;
+      decode(u, ft, tt);
+      const int b = it & 1, t0 = tt * cn;
+      float* rs = s_rs + b * 256;
+      if (etid < cn) rs[etid] = (p.row_scale && t0 + etid < p.M) ? __ldg(p.row_scale + t0 + etid) : 1.0f;
+      const int feat = ft * 256 + (int)rank * 128 + q * 32 + lane;
+      const bool feat_ok = feat < p.N;
+      const float al = (p.alpha && feat_ok) ? __ldg(p.alpha + feat) : 1.0f;
+      const float bs = (p.bias && feat_ok) ? bf2f(p.bias[feat]) : 0.0f;
+      // the row scales are complete, and the warps agree on whether a wait ran out, so that none is left at a barrier
+      if (!bar_red_and(1, Cfg::EPI * 32, ok)) break;
+      ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, p.status);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) continue;
+      tc_fence_after();
+      // chunks of 32 columns, a round of one per warp at a time, the end that the accumulators share first
+      constexpr int PARTS = Cfg::EPI / 4;
+      const int chunks = cn >> 5, rounds = (chunks + PARTS - 1) / PARTS;
+      for (int i = 0; i < rounds; ++i) {
+        const int ch = b ? i * PARTS + part : chunks - 1 - i * PARTS - part;
+        const bool mine = ch >= 0 && ch < chunks;
+        const int c = ch * 32;
+        uint32_t r[32];
+        if (mine) {
+          tmem_ld32(tmem + (b ? p.acc1 : 0) + c + quad, r);
+          tmem_ld_wait();
+        }
+        if (i == (shared_cols ? 0 : rounds - 1)) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&acc_free[b]), 0));
+        }
+        if (!mine) break;
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          const float4 s4 = *reinterpret_cast<const float4*>(rs + c + j);
+          v[j] = fmaf(__uint_as_float(r[j]) * s4.x, al, bs);
+          v[j + 1] = fmaf(__uint_as_float(r[j + 1]) * s4.y, al, bs);
+          v[j + 2] = fmaf(__uint_as_float(r[j + 2]) * s4.z, al, bs);
+          v[j + 3] = fmaf(__uint_as_float(r[j + 3]) * s4.w, al, bs);
+        }
+        const int tc = t0 + c;              // token of the chunk's first column
+        if (p.out_f32) {
+          float* C = reinterpret_cast<float*>(p.C) + feat;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (feat_ok && tc + j < p.M) C[(size_t)(tc + j) * p.ldc] = v[j];
+        } else if (p.act) {
+          // lanes 0-15 hold the gates and 16-31 the up values of 16 features: one exchange gives the lower lanes a token and the upper
+          // ones the next, a second one pairs two features per store
+          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + ((ft * 256 + (int)rank * 128 + q * 32) >> 1) + (lane & 14);
+          auto gated = [&](auto act) {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              float a[2];
+#pragma unroll
+              for (int k = 0; k < 2; ++k) {
+                const float lo = v[j + 2 * k], up = v[j + 2 * k + 1];
+                const float got = __shfl_xor_sync(0xffffffffu, hi ? lo : up, 16);
+                a[k] = act(hi ? got : lo, hi ? up : got);
+              }
+              const float got = __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 1);
+              const int tok = tc + j + (odd ? 2 : 0) + (hi ? 1 : 0);
+              if (tok < p.M && feat_ok)
+                *reinterpret_cast<uint32_t*>(C + (size_t)tok * p.ldc) = odd ? pack_bf16x2(got, a[1]) : pack_bf16x2(a[0], got);
+            }
+          };
+          if (p.act == 2) {
+            gated([&](float gf, float uf) { return clamped_glu_fast(gf, uf, p.act_limit); });
+          } else {
+            gated([](float gf, float uf) {
+              const float g = bf2f(__float2bfloat16(gf)), up = bf2f(__float2bfloat16(uf));
+              return silu(g) * up;
+            });
+          }
+        } else {
+          // neighbouring lanes trade every other token so that each writes two adjacent features at once
+          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + (feat & ~1);
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+            const int tok = tc + j + (odd ? 1 : 0);
+            if (tok < p.M && feat_ok)
+              *reinterpret_cast<uint32_t*>(C + (size_t)tok * p.ldc) = odd ? pack_bf16x2(got, v[j + 1]) : pack_bf16x2(v[j], got);
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncwarp();
+  cluster_arrive();                         // neither CTA leaves while the other still reads its memory or signals its barriers
+  cluster_wait();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem, 512);
+  }
+}
+
+template <int KIND>
+static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW, const CUtensorMap& tmSX,
+                               const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
+  using Cfg = PairCfg<KIND>;
+  auto kern = gemm_pair_kernel<KIND>;
+  static PerDeviceOnce configured;
+  cudaError_t e = configured.smem_limit(kern, Cfg::SMEM);
+  if (e != cudaSuccess) return e;
+  int pairs = sm_count() / 2;
+  if (max_ctas > 1 && pairs > max_ctas / 2) pairs = max_ctas / 2;
+  if (pairs > tiles) pairs = tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(pairs * 2));
+  cfg.blockDim = dim3(Cfg::THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
+}
+
+}  // namespace blz
+
+// Columns of a tile: the multiple of 64 with the least rounds x time of a round.  Nanoseconds per K block measured at 8192 x 4096 x 12288
+// (NVFP4 and bf16; more columns than the MMAs of a block can hide behind its bytes and its issue cost little), and about a microsecond per tile
+// for the accumulators' hand-over.
+BLZ_API int blz_gemm_pair_columns(int kind, int M, int N, int K, int sms) {
+  static const int scaled[] = {294, 313, 338, 387}, plain[] = {237, 255, 296, 385};
+  const int tiles_f = (N + 255) / 256, pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int k_tiles = (K + (kind == 0 ? 63 : kind == 1 ? 255 : 127)) / (kind == 0 ? 64 : kind == 1 ? 256 : 128);
+  int best = 256;
+  long best_cost = 1L << 60;
+  for (int cn = 256; cn >= 64; cn -= 64) {
+    const long tiles = (long)tiles_f * ((M + cn - 1) / cn);
+    const long cost = ((tiles + pairs - 1) / pairs) * ((long)k_tiles * (kind ? scaled : plain)[cn / 64 - 1] + 1000);
+    if (cost < best_cost) { best_cost = cost; best = cn; }
+  }
+  return best;
+}
+
+// C[M, N] = X[M, K] · W[N, K]^T with the operand conventions of blz_gemm_tc (ldx / ldw in BYTES, ldc in elements).  kind: 0 bf16,
+// 1 NVFP4, 2 MXFP8.  N even, or a multiple of 32 with act (bf16 out, [M, N/2]).  cn: tokens per tile, 64 / 128 / 192 / 256, or 0 to choose.
+BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N,
+                          int K, const float* row_scale, const float* alpha, const void* bias, const void* sfx, const void* sfw,
+                          int out_f32, int cn, int max_ctas, int act, float act_limit, cudaStream_t stream) {
+  using namespace blz;
+  // this kernel has no fused all-reduce / peer-wait / arg-max epilogue: a call armed for one is refused (and disarmed)
+  if (gemm_oneshot_take_unsupported()) return (int)cudaErrorNotSupported;
+  if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || cn < 0 || cn > 256 || cn % 64) return (int)cudaErrorInvalidValue;
+  const int kmma = kind == 0 ? 16 : kind == 1 ? 64 : 32;
+  if (K % kmma) return (int)cudaErrorInvalidValue;
+  if (kind && (!sfx || !sfw)) return (int)cudaErrorInvalidValue;
+  if (act < 0 || act > 2 || (act && (out_f32 || N % 32))) return (int)cudaErrorInvalidValue;
+  if (!out_f32 && ((N & 1) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3))) return (int)cudaErrorInvalidValue;
+  PairParams p;
+  p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_f32 = out_f32;
+  p.row_scale = row_scale; p.alpha = alpha; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
+  p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
+  p.cn = cn ? cn : blz_gemm_pair_columns(kind, M, N, K, sm_count());
+  const int room = kind == 0 ? PairCfg<0>::SF_COL0 : kind == 1 ? PairCfg<1>::SF_COL0 : PairCfg<2>::SF_COL0;
+  p.acc1 = room - p.cn < 256 ? room - p.cn : 256;
+  p.act = act; p.act_limit = act_limit;
+  p.status = status_word();
+  CUtensorMap tmW, tmX, tmSW, tmSX;
+  const int es = kind == 0 ? 2 : 1;                                   // bytes per tensor-map element
+  const uint64_t inner = kind == 1 ? (uint64_t)K / 2 : (uint64_t)K;
+  cudaError_t e = encode_tmap(&tmW, W, es, inner, N, ldw, 128 / es, 128, 3);
+  if (e == cudaSuccess) e = encode_tmap(&tmX, X, es, inner, M, ldx, 128 / es, p.cn / 2, 3);
+  if (e != cudaSuccess) return (int)e;
+  tmSW = tmW; tmSX = tmX;
+  if (kind) {
+    // Scales of 128 rows and 4 columns are 512 bytes: a map of [row tiles][scale tiles][128 words], so that a stage's scales of one
+    // operand come with one instruction.  Copies of their own (cp.async.bulk of 2 KB) or a map of 256-byte rows, one instruction per row
+    // tile, held the ring up: 8192 x 4096 x 12288 in NVFP4 275 and 166 us, so 141.
+    const uint64_t atoms = (uint64_t)p.sf_col_tiles;
+    const uint32_t box = kind == 1 ? 4 : 1;
+    e = encode_tmap(&tmSW, sfw, 4, 128, atoms, 512, 128, box, 0, (uint64_t)((N + 127) / 128), atoms * 512, 1);
+    if (e == cudaSuccess) e = encode_tmap(&tmSX, sfx, 4, 128, atoms, 512, 128, box, 0, (uint64_t)((M + 127) / 128), atoms * 512, p.cn > 128 ? 2 : 1);
+    if (e != cudaSuccess) return (int)e;
+  }
+  const int tiles = ((N + 255) / 256) * ((M + p.cn - 1) / p.cn);
+  if (kind == 0) return (int)launch_pair<0>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  if (kind == 1) return (int)launch_pair<1>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  return (int)launch_pair<2>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+}

@@ -112,6 +112,38 @@ def test_gemm_wide(ops, fmt, M, N, K, ksplit):
     assert rel < 0.05
 
 
+@pytest.mark.parametrize("fmt,M,N,K,act", [
+    ("bf16", 257, 512, 16, 0), ("bf16", 300, 514, 320, 0), ("bf16", 1601, 1216, 1024, 0), ("bf16", 825, 1056, 192, 1), ("bf16", 700, 544, 64, 2),
+    ("nvfp4", 257, 512, 64, 0), ("nvfp4", 321, 1216, 320, 0), ("nvfp4", 20000, 768, 512, 0), ("nvfp4", 1025, 1024, 4096, 1),
+    ("mxfp8", 300, 12352, 160, 0), ("mxfp8", 513, 640, 2048, 0), ("mxfp8", 1100, 576, 384, 1)])
+def test_gemm_pair(ops, fmt, M, N, K, act):
+    """CTA pairs: every tile width at ragged rows, features and K; one tile per pair and several.  The same products summed in the same
+    order as by the 128-column kernel, so the same bits."""
+    g = torch.Generator(device=DEV).manual_seed(31)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    f = {"nvfp4": Format.NVFP4, "mxfp8": Format.MXFP8, "bf16": Format.DENSE}[fmt]
+    lin = Linear.from_dense(torch.randn(N, K, generator=g, device=DEV) * 0.05, f)
+    if not act:
+        lin.bias = (torch.randn(N, generator=g, device=DEV) * 0.1).bfloat16()
+    kw = {"swiglu": True, "glu_limit": 7.0 if act == 2 else None} if act else {}
+    pk = ops.pack(lin, swiglu=bool(act))
+    xin = ops.quantize_rows(x, lin) if ops._qmode(lin) else x
+    want = ops.linear(lin, xin, wide=False, sk=False, **kw)
+    assert torch.equal(ops.linear(lin, xin, **kw), want)
+    a, sf, rs = (xin.data, xin.sf, xin.row_scale) if ops._qmode(lin) else (x, None, None)
+    p = lambda t: t.data_ptr() if t is not None else 0      # noqa: E731
+    for f32 in (False, True) if not act else (False,):
+        if f32:
+            want = ops.linear(lin, xin, out_dtype=torch.float32, wide=False, sk=False)
+        for cn, ctas in ((64, 0), (128, 6), (192, 4), (256, 2)):
+            out = torch.full_like(want, float("nan"))
+            rc = ops.lib.blz_gemm_pair(pk["kind"], p(a), a.shape[1] * a.element_size(), p(pk["w"]), pk["w"].shape[1] * pk["w"].element_size(), p(out),
+                                       out.stride(0), M, N, K, p(rs), p(pk["alpha"]), p(pk["bias"]), p(sf), p(pk["sf"]), int(f32), cn, ctas, act,
+                                       7.0, ops._stream())
+            assert rc == 0 and ops.take_status() == 0
+            assert torch.equal(out, want), (cn, ctas, f32)
+
+
 @pytest.mark.parametrize("fmt,M,N,K,ks", [
     ("nvfp4", 256, 6144, 4096, 0), ("nvfp4", 256, 4096, 4096, 4), ("nvfp4", 256, 768, 4096, 8), ("nvfp4", 256, 4096, 512, 2),
     ("nvfp4", 200, 1024, 12288, 3), ("nvfp4", 77, 520, 1024, 4), ("nvfp4", 1, 384, 512, 2), ("nvfp4", 130, 256, 320, 5),
