@@ -31,9 +31,7 @@ struct SkParams {
   const float* row_scale;    // [M] or null
   const float* alpha;        // [N] or null
   const __nv_bfloat16* bias; // [N] or null
-  const uint8_t* sfa;        // scale factors, 128x4-tiled (kinds 1, 2)
-  const uint8_t* sfb;
-  int sf_col_tiles;          // 4-column scale tiles per 128-row tile along K
+  int sf_col_tiles;          // 4-column scale tiles per 128-row tile along K (kinds 1, 2)
   int ks;                    // cluster size = number of K slices
   int act;                   // 1: B rows are [16 gate | 16 up] groups, C = silu(gate) * up, bf16 [M, N/2] (ks must be 1)
   float act_limit;           // act 2: the clamp of glu.cuh
@@ -85,7 +83,8 @@ __device__ __forceinline__ float silu_mul_bf16(float g, float u) {
 
 template <int KIND>
 __global__ void __launch_bounds__(192, 2)
-gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, SkParams p) {
+gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmSA,
+               const __grid_constant__ CUtensorMap tmSB, SkParams p) {
   using Cfg = SkCfg<KIND>;
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -125,6 +124,7 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     mbar_fence_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
+    if (Cfg::SF_ATOMS > 0) { prefetch_tmap(&tmSA); prefetch_tmap(&tmSB); }
   }
   if (threadIdx.x == 0) SK_MARK(1);
   if (warp == 1) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -143,21 +143,17 @@ gemm_sk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
       auto issue = [&](int s, int kt, int what) {
-        int atoms = 0;
-        if constexpr (Cfg::SF_ATOMS > 0) atoms = min(Cfg::SF_ATOMS, p.sf_col_tiles - kt * Cfg::SF_ATOMS);
         const int kc = (KIND == 0) ? kt * BK : kt * 128;
         if (what & 1) {
-          mbar_expect_tx(&full[s], Cfg::A_BYTES + Cfg::B_BYTES + (uint32_t)atoms * 1024u);
+          mbar_expect_tx(&full[s], Cfg::A_BYTES + Cfg::B_BYTES + 2u * Cfg::SF_BYTES);
           tma_load_2d(sB + s * Cfg::B_BYTES, &tmB, kc, nt * BN, &full[s]);
           if constexpr (Cfg::SF_ATOMS > 0)
-            bulk_load(sSFB + s * Cfg::SF_BYTES, p.sfb + ((size_t)nt * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512,
-                      atoms * 512, &full[s]);
+            tma_load_3d(sSFB + s * Cfg::SF_BYTES, &tmSB, 0, kt * Cfg::SF_ATOMS, nt, &full[s]);
         }
         if (what & 2) {
           tma_load_2d(sA + s * Cfg::A_BYTES, &tmA, kc, mt * BM, &full[s]);
           if constexpr (Cfg::SF_ATOMS > 0)
-            bulk_load(sSFA + s * Cfg::SF_BYTES, p.sfa + ((size_t)mt * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512,
-                      atoms * 512, &full[s]);
+            tma_load_3d(sSFA + s * Cfg::SF_BYTES, &tmSA, 0, kt * Cfg::SF_ATOMS, mt, &full[s]);
         }
       };
       // the weights do not depend on the kernel before this one: their first tiles go out before the dependency wait
@@ -390,7 +386,14 @@ static void fill_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int 
 }
 
 template <int KIND>
-static cudaError_t launch_sk(const CUtensorMap& tmA, const CUtensorMap& tmB, const SkParams& p, cudaStream_t stream) {
+static cudaError_t launch_sk(const CUtensorMap& tmA, const CUtensorMap& tmB, const void* sfa, const void* sfb, const SkParams& p,
+                             cudaStream_t stream) {
+  CUtensorMap tmSA = tmA, tmSB = tmB;
+  if (SkCfg<KIND>::SF_ATOMS > 0) {
+    cudaError_t e = encode_sf_tmap(&tmSA, sfa, (p.M + 127) / 128, p.sf_col_tiles, SkCfg<KIND>::SF_ATOMS);
+    if (e == cudaSuccess) e = encode_sf_tmap(&tmSB, sfb, (p.N + 127) / 128, p.sf_col_tiles, SkCfg<KIND>::SF_ATOMS);
+    if (e != cudaSuccess) return e;
+  }
   auto kern = gemm_sk_kernel<KIND>;
   static PerDeviceOnce configured;
   {
@@ -401,7 +404,7 @@ static cudaError_t launch_sk(const CUtensorMap& tmA, const CUtensorMap& tmB, con
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   fill_config<KIND>(cfg, attr, tiles * p.ks, p.ks, stream);
-  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p);
+  return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmSA, tmSB, p);
 }
 
 // How many CTAs of this kernel run at the same time on the current device when launched in clusters of `ks` (clusters are
@@ -497,7 +500,6 @@ BLZ_API int blz_gemm_sk(int kind, const void* A, long long lda, const void* B, l
   SkParams p;
   p.M = M; p.N = N; p.K = K; p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
   p.row_scale = row_scale; p.alpha = alpha; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
-  p.sfa = reinterpret_cast<const uint8_t*>(sfa); p.sfb = reinterpret_cast<const uint8_t*>(sfb);
   p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
   p.ks = ks; p.act = act; p.act_limit = act_limit;
   p.status = status_word();
@@ -519,9 +521,9 @@ BLZ_API int blz_gemm_sk(int kind, const void* A, long long lda, const void* B, l
   }
   if (e != cudaSuccess) return (int)e;
   switch (kind) {
-    case 0: return (int)launch_sk<0>(tmA, tmB, p, stream);
-    case 1: return (int)launch_sk<1>(tmA, tmB, p, stream);
-    case 2: return (int)launch_sk<2>(tmA, tmB, p, stream);
-    default: return (int)launch_sk<3>(tmA, tmB, p, stream);
+    case 0: return (int)launch_sk<0>(tmA, tmB, sfa, sfb, p, stream);
+    case 1: return (int)launch_sk<1>(tmA, tmB, sfa, sfb, p, stream);
+    case 2: return (int)launch_sk<2>(tmA, tmB, sfa, sfb, p, stream);
+    default: return (int)launch_sk<3>(tmA, tmB, sfa, sfb, p, stream);
   }
 }

@@ -34,9 +34,7 @@ struct GemmParams {
   const float* row_scale;    // [M] or null
   const float* alpha;        // [N] or null
   const __nv_bfloat16* bias; // [N] or null
-  const uint8_t* sfa;        // scale factors of A, 128x4-tiled (kinds 1, 2)
-  const uint8_t* sfb;
-  int sfa_col_tiles;         // number of 4-column tiles per 128-row tile in sfa / sfb
+  int sfa_col_tiles;         // scale factors (kinds 1, 2): number of 4-column tiles per 128-row tile, of A and B
   // fused all-reduce (OUT mode 2): the epilogue adds this rank's partial tile into every rank's output through the
   // NVSwitch (multimem.red); the last CTA then meets the other ranks at a flag barrier, so kernel completion means
   // the summed output is complete in local memory.
@@ -54,7 +52,7 @@ struct GemmParams {
   uint32_t* push_flag[8];
   int push_rows_per;
   long long* stamps;         // optional diagnostics: [gridDim.x][8] global-timer stamps of the pushed epilogue (null = off)
-  const int* tile_expert;    // grouped GEMM: expert of every 128-row M tile (-1 = skip); B / alpha / sfb rows are offset by expert * N
+  const int* tile_expert;    // grouped GEMM: expert of every 128-row M tile (-1 = skip); B / alpha / scale rows are offset by expert * N
   // activations still in flight from the peers (fused all-reduce + norm that signals instead of waiting): the producer
   // sends the first weight tiles, then waits until counter[r] >= *wait_expect for every rank r, then loads A
   const uint32_t* wait_pad;  // own arrival counters, one uint32 per source rank (peers add to them)
@@ -100,7 +98,8 @@ struct GemmCfg {
 
 template <int KIND, int BN, bool OUT_F32>
 __global__ void __launch_bounds__(192, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmParams p) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmSA,
+               const __grid_constant__ CUtensorMap tmSB, GemmParams p) {
   pdl_trigger();
   using Cfg = GemmCfg<KIND, BN>;
   constexpr int BM = Cfg::BM, BK = Cfg::BK, STAGES = Cfg::STAGES, ACC = Cfg::ACC_BUFS;
@@ -133,6 +132,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     mbar_fence_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
+    if (Cfg::SF_ATOMS > 0) { prefetch_tmap(&tmSA); prefetch_tmap(&tmSB); }
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
@@ -145,13 +145,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ------------------------------------------------------------------ producer
     // what: 1 = the B tile (+ its scales) and the stage's byte count, 2 = the A tile (+ its scales), 3 = both
     auto issue = [&](int s, int mt, int nt, int ex, int kt, int what) {
-      int atoms = 0;
-      if constexpr (Cfg::SF_ATOMS > 0) atoms = min(Cfg::SF_ATOMS, p.sfa_col_tiles - kt * Cfg::SF_ATOMS);
       const int kc = (KIND == 0) ? kt * BK : kt * 128;   // coordinate in map elements (bf16 or bytes)
       if (what & 1) {
-        uint32_t bytes = Cfg::A_BYTES + Cfg::B_BYTES;
-        if constexpr (Cfg::SF_ATOMS > 0) bytes += atoms * 512 * (1 + BN / 128);
-        mbar_expect_tx(&full[s], bytes);
+        mbar_expect_tx(&full[s], Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES);
         const int brow = ex * p.N + nt * BN;                  // first B row of this tile
         if (p.b_kt > 0) {
           // tile-major weights: every 128-row x 128-byte tile is stored as its swizzled shared-memory image, one
@@ -163,20 +159,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         } else {
           tma_load_2d(sB + s * Cfg::B_BYTES, &tmB, kc, brow, &full[s]);
         }
-        if constexpr (Cfg::SF_ATOMS > 0) {
-#pragma unroll
-          for (int h = 0; h < BN / 128; ++h) {
-            const size_t b_off = ((size_t)(brow / 128 + h) * p.sfa_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512;
-            bulk_load(sSFB + s * Cfg::SFB_BYTES + h * Cfg::SFA_BYTES, p.sfb + b_off, atoms * 512, &full[s]);
-          }
-        }
+        if constexpr (Cfg::SF_ATOMS > 0) tma_load_3d(sSFB + s * Cfg::SFB_BYTES, &tmSB, 0, kt * Cfg::SF_ATOMS, brow / 128, &full[s]);
       }
       if (what & 2) {
         tma_load_2d(sA + s * Cfg::A_BYTES, &tmA, kc, mt * BM, &full[s]);
-        if constexpr (Cfg::SF_ATOMS > 0) {
-          const size_t a_off = ((size_t)mt * p.sfa_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512;
-          bulk_load(sSFA + s * Cfg::SFA_BYTES, p.sfa + a_off, atoms * 512, &full[s]);
-        }
+        if constexpr (Cfg::SF_ATOMS > 0) tma_load_3d(sSFA + s * Cfg::SFA_BYTES, &tmSA, 0, kt * Cfg::SF_ATOMS, mt, &full[s]);
       }
     };
     // The weights do not depend on the kernel before this one: the first tile's B stages go out first, then the producer
@@ -513,9 +500,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 template <int KIND, int BN, bool OUT_F32>
-static cudaError_t launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmParams& p, int max_ctas,
-                          cudaStream_t stream) {
+static cudaError_t launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const void* sfa, const void* sfb, uint64_t b_rows,
+                          const GemmParams& p, int max_ctas, cudaStream_t stream) {
   using Cfg = GemmCfg<KIND, BN>;
+  CUtensorMap tmSA = tmA, tmSB = tmB;
+  if (Cfg::SF_ATOMS > 0) {
+    cudaError_t e = encode_sf_tmap(&tmSA, sfa, (p.M + 127) / 128, p.sfa_col_tiles, Cfg::SF_ATOMS);
+    if (e == cudaSuccess) e = encode_sf_tmap(&tmSB, sfb, (b_rows + 127) / 128, p.sfa_col_tiles, Cfg::SF_ATOMS, BN / 128);
+    if (e != cudaSuccess) return e;
+  }
   auto kern = gemm_tc_kernel<KIND, BN, OUT_F32>;
   static PerDeviceOnce configured;
   {
@@ -525,7 +518,7 @@ static cudaError_t launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const 
   const int tiles = ((p.M + 127) / 128) * ((p.N + BN - 1) / BN);
   int grid = tiles < sm_count() ? tiles : sm_count();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  return launch_pdl(kern, dim3(grid), dim3(192), Cfg::SMEM, stream, tmA, tmB, p);
+  return launch_pdl(kern, dim3(grid), dim3(192), Cfg::SMEM, stream, tmA, tmB, tmSA, tmSB, p);
 }
 
 }  // namespace blz
@@ -667,7 +660,6 @@ BLZ_API int blz_gemm_tc(int kind, const void* A, long long lda, const void* B, l
   GemmParams p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.row_scale = row_scale; p.alpha = alpha;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
-  p.sfa = reinterpret_cast<const uint8_t*>(sfa); p.sfb = reinterpret_cast<const uint8_t*>(sfb);
   p.sfa_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
   p.status = status_word();
   p.tile_expert = tile_expert;
@@ -721,8 +713,8 @@ BLZ_API int blz_gemm_tc(int kind, const void* A, long long lda, const void* B, l
   if (e != cudaSuccess) return (int)e;
 #define BLZ_GEMM_CASE(KD, BNV)                                                                        \
   if (kind == KD && bn == BNV)                                                                        \
-    return (int)(out_f32 ? launch<KD, BNV, true>(tmA, tmB, p, max_ctas, stream)                       \
-                         : launch<KD, BNV, false>(tmA, tmB, p, max_ctas, stream));
+    return (int)(out_f32 ? launch<KD, BNV, true>(tmA, tmB, sfa, sfb, b_rows, p, max_ctas, stream)                       \
+                         : launch<KD, BNV, false>(tmA, tmB, sfa, sfb, b_rows, p, max_ctas, stream));
   BLZ_GEMM_CASE(0, 128) BLZ_GEMM_CASE(0, 256) BLZ_GEMM_CASE(1, 128) BLZ_GEMM_CASE(1, 256)
   BLZ_GEMM_CASE(2, 128) BLZ_GEMM_CASE(2, 256) BLZ_GEMM_CASE(3, 128) BLZ_GEMM_CASE(3, 256)
 #undef BLZ_GEMM_CASE

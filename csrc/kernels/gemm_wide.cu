@@ -37,9 +37,7 @@ struct WideParams {
   const float* lane_scale;    // per lane-operand row, or null
   const float* col_scale;     // per column-operand row, or null
   const __nv_bfloat16* bias;  // per feature, or null
-  const uint8_t* sf_lane;     // 128x4-tiled scale factors of the lane operand (block-scaled kinds)
-  const uint8_t* sf_col;
-  int sf_col_tiles;           // 4-column scale tiles per 128-row tile
+  int sf_col_tiles;           // scale factors (block-scaled kinds): 4-column tiles per 128-row tile
   int ksplit;                 // CTAs sharing one output tile along K
   float* ws;                  // [tiles * ksplit][128][BN] fp32 partial tiles (ksplit > 1)
   unsigned* ctr;              // [tiles] arrival counters, zero between launches
@@ -81,8 +79,9 @@ struct WideCfg {
 };
 
 template <int KIND, int BN, bool SWAP>
-__global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                            const __grid_constant__ CUtensorMap tmB, const WideParams p) {
+__global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                                                            const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSB,
+                                                            const WideParams p) {
   pdl_trigger();
   using Cfg = WideCfg<KIND, BN>;
   constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, CPT = Cfg::CPT;
@@ -118,6 +117,7 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
     mbar_fence_init();
     prefetch_tmap(&tmA);
     prefetch_tmap(&tmB);
+    if (Cfg::SF_ATOMS > 0) { prefetch_tmap(&tmSA); prefetch_tmap(&tmSB); }
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
@@ -146,13 +146,7 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
         const int kt0 = ks * kb_per, kt1 = min(k_tiles, kt0 + kb_per);
         for (int kt = kt0; kt < kt1; ++kt) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) goto producer_done;
-          uint32_t bytes = Cfg::A_BYTES + Cfg::B_BYTES;
-          int atoms = 0;
-          if constexpr (Cfg::SF_ATOMS > 0) {
-            atoms = min(Cfg::SF_ATOMS, p.sf_col_tiles - kt * Cfg::SF_ATOMS);
-            bytes += atoms * 512 * (1 + Cfg::NB);
-          }
-          mbar_expect_tx(&full[s], bytes);
+          mbar_expect_tx(&full[s], Cfg::A_BYTES + Cfg::B_BYTES + Cfg::SFA_BYTES + Cfg::SFB_BYTES);
           const int kc = (KIND == 0) ? kt * BK : kt * 128;
           if (p.w_kt > 0 && SWAP) {
             bulk_load(sA + s * Cfg::A_BYTES, p.w_raw + ((size_t)lt * p.w_kt + kt) * 16384, 16384, &full[s]);
@@ -168,13 +162,8 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
             tma_load_2d(sB + s * Cfg::B_BYTES, &tmB, kc, ct * BN, &full[s]);
           }
           if constexpr (Cfg::SF_ATOMS > 0) {
-            const size_t a_off = ((size_t)lt * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512;
-            bulk_load(sSFA + s * Cfg::SFA_BYTES, p.sf_lane + a_off, atoms * 512, &full[s]);
-#pragma unroll
-            for (int h = 0; h < Cfg::NB; ++h) {
-              const size_t b_off = ((size_t)((ct * BN) / 128 + h) * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512;
-              bulk_load(sSFB + s * Cfg::SFB_BYTES + h * Cfg::SFA_BYTES, p.sf_col + b_off, atoms * 512, &full[s]);
-            }
+            tma_load_3d(sSFA + s * Cfg::SFA_BYTES, &tmSA, 0, kt * Cfg::SF_ATOMS, lt, &full[s]);
+            tma_load_3d(sSFB + s * Cfg::SFB_BYTES, &tmSB, 0, kt * Cfg::SF_ATOMS, (ct * BN) / 128, &full[s]);
           }
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
@@ -427,9 +416,15 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
 }
 
 template <int KIND, int BN, bool SWAP>
-static cudaError_t launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, const WideParams& p, int units, int max_ctas,
-                               cudaStream_t stream) {
+static cudaError_t launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, const void* sf_lane, const void* sf_col,
+                               const WideParams& p, int units, int max_ctas, cudaStream_t stream) {
   using Cfg = WideCfg<KIND, BN>;
+  CUtensorMap tmSA = tmA, tmSB = tmB;
+  if (Cfg::SF_ATOMS > 0) {
+    cudaError_t e = encode_sf_tmap(&tmSA, sf_lane, (p.lanes_total + 127) / 128, p.sf_col_tiles, Cfg::SF_ATOMS);
+    if (e == cudaSuccess) e = encode_sf_tmap(&tmSB, sf_col, (p.cols_total + 127) / 128, p.sf_col_tiles, Cfg::SF_ATOMS, Cfg::NB);
+    if (e != cudaSuccess) return e;
+  }
   auto kern = gemm_wide_kernel<KIND, BN, SWAP>;
   static PerDeviceOnce configured;
   {
@@ -438,7 +433,7 @@ static cudaError_t launch_wide(const CUtensorMap& tmA, const CUtensorMap& tmB, c
   }
   int grid = units < sm_count() ? units : sm_count();
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  return launch_pdl(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, tmA, tmB, p);
+  return launch_pdl(kern, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM, stream, tmA, tmB, tmSA, tmSB, p);
 }
 
 }  // namespace blz
@@ -498,12 +493,10 @@ BLZ_API int blz_gemm_wide(int kind, const void* X, long long ldx, const void* W,
   if (swap) {
     p.lanes_total = N; p.cols_total = M;
     p.lane_scale = alpha; p.col_scale = row_scale;
-    p.sf_lane = reinterpret_cast<const uint8_t*>(sfw); p.sf_col = reinterpret_cast<const uint8_t*>(sfx);
     A = W; lda = ldw; B = X; ldb = ldx;
   } else {
     p.lanes_total = M; p.cols_total = N;
     p.lane_scale = row_scale; p.col_scale = alpha;
-    p.sf_lane = reinterpret_cast<const uint8_t*>(sfx); p.sf_col = reinterpret_cast<const uint8_t*>(sfw);
     A = X; lda = ldx; B = W; ldb = ldw;
   }
   const int tiles = ((p.lanes_total + 127) / 128) * ((p.cols_total + bn - 1) / bn);
@@ -535,7 +528,7 @@ BLZ_API int blz_gemm_wide(int kind, const void* X, long long ldx, const void* W,
   if (e != cudaSuccess) return (int)e;
   const int units = tiles * ksplit;
 #define BLZ_WIDE_CASE(KD, BNV, SW) \
-  if (kind == KD && bn == BNV && (swap != 0) == SW) return (int)launch_wide<KD, BNV, SW>(tmA, tmB, p, units, max_ctas, stream);
+  if (kind == KD && bn == BNV && (swap != 0) == SW) return (int)launch_wide<KD, BNV, SW>(tmA, tmB, swap ? sfw : sfx, swap ? sfx : sfw, p, units, max_ctas, stream);
   BLZ_WIDE_CASE(0, 64, true) BLZ_WIDE_CASE(0, 128, true) BLZ_WIDE_CASE(0, 256, true) BLZ_WIDE_CASE(0, 256, false)
   BLZ_WIDE_CASE(1, 64, true) BLZ_WIDE_CASE(1, 128, true) BLZ_WIDE_CASE(1, 256, true) BLZ_WIDE_CASE(1, 256, false)
   BLZ_WIDE_CASE(2, 64, true) BLZ_WIDE_CASE(2, 128, true) BLZ_WIDE_CASE(2, 256, true) BLZ_WIDE_CASE(2, 256, false)

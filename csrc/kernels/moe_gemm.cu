@@ -39,9 +39,7 @@ struct MoeGemmParams {
   long long ldc;
   const float* row_scale;    // [padded rows] or null
   const float* alpha;        // [experts * N] or null
-  const uint8_t* sfw;        // weight scale factors, 128x4-tiled over [experts * N] rows
-  const uint8_t* sfx;        // activation scale factors, 128x4-tiled over the padded rows
-  int sf_col_tiles;
+  int sf_col_tiles;          // scale factors: 4-column tiles per 128-row tile
   const int* tile_expert;    // [row tiles] expert of the tile, -1 = unused; null = dense layer (one row tile of `rows` rows)
   const int* tile_rows;      // [row tiles] live rows of the tile
   int rows;                  // dense layer: rows of the activation matrix (<= 128)
@@ -85,7 +83,8 @@ __device__ __forceinline__ float mg_silu_mul(float g, float u) {
 
 template <int KIND>
 __global__ void __launch_bounds__(192, 2)
-moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, MoeGemmParams p) {
+moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmSW,
+                const __grid_constant__ CUtensorMap tmSX, MoeGemmParams p) {
   using Cfg = MgCfg<KIND>;
   constexpr int BK = Cfg::BK, STAGES = Cfg::STAGES;
   const int tiles_n = p.N / 128;
@@ -133,6 +132,7 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     mbar_fence_init();
     prefetch_tmap(&tmW);
     prefetch_tmap(&tmX);
+    if (Cfg::SF_ATOMS > 0) { prefetch_tmap(&tmSW); prefetch_tmap(&tmSX); }
   }
   if (warp == 1) tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
   tc_fence_before();
@@ -146,22 +146,18 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
       auto issue = [&](int s, int kt, int what, size_t wrow0) {
-        int atoms = 0;
-        if constexpr (Cfg::SF_ATOMS > 0) atoms = min(Cfg::SF_ATOMS, p.sf_col_tiles - kt * Cfg::SF_ATOMS);
         const int kc = (KIND == 0) ? kt * BK : kt * 128;
         if (what & 1) {       // weights: do not depend on the kernel before this one
-          mbar_expect_tx(&full[s], Cfg::W_BYTES + (uint32_t)ncols * 128u + (uint32_t)atoms * 1024u);
+          mbar_expect_tx(&full[s], Cfg::W_BYTES + (uint32_t)ncols * 128u + 2u * Cfg::SF_BYTES);
           tma_load_2d(sW + s * Cfg::W_BYTES, &tmW, kc, (int)wrow0, &full[s]);
           if constexpr (Cfg::SF_ATOMS > 0)
-            bulk_load(sSFW + s * Cfg::SF_BYTES, p.sfw + ((wrow0 >> 7) * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512,
-                      atoms * 512, &full[s]);
+            tma_load_3d(sSFW + s * Cfg::SF_BYTES, &tmSW, 0, kt * Cfg::SF_ATOMS, (int)(wrow0 >> 7), &full[s]);
         }
         if (what & 2) {       // routed rows, 32 at a time
           for (int c = 0; c < ncols; c += 32)
             tma_load_2d(sX + s * Cfg::X_BYTES + c * 128, &tmX, kc, mt * 128 + c, &full[s]);
           if constexpr (Cfg::SF_ATOMS > 0)
-            bulk_load(sSFX + s * Cfg::SF_BYTES, p.sfx + ((size_t)mt * p.sf_col_tiles + (size_t)kt * Cfg::SF_ATOMS) * 512,
-                      atoms * 512, &full[s]);
+            tma_load_3d(sSFX + s * Cfg::SF_BYTES, &tmSX, 0, kt * Cfg::SF_ATOMS, mt, &full[s]);
         }
       };
       const int pre = min(STAGES, nkb);
@@ -359,8 +355,14 @@ moe_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
 }
 
 template <int KIND>
-static cudaError_t launch_moe_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, const MoeGemmParams& p, int row_tiles,
-                                   cudaStream_t stream) {
+static cudaError_t launch_moe_gemm(const CUtensorMap& tmW, const CUtensorMap& tmX, const MoeGemmParams& p, int row_tiles, int experts,
+                                   const void* sfw, const void* sfx, cudaStream_t stream) {
+  CUtensorMap tmSW = tmW, tmSX = tmX;
+  if (MgCfg<KIND>::SF_ATOMS > 0) {
+    cudaError_t e = encode_sf_tmap(&tmSW, sfw, (uint64_t)experts * p.N / 128, p.sf_col_tiles, MgCfg<KIND>::SF_ATOMS);
+    if (e == cudaSuccess) e = encode_sf_tmap(&tmSX, sfx, row_tiles, p.sf_col_tiles, MgCfg<KIND>::SF_ATOMS);
+    if (e != cudaSuccess) return e;
+  }
   const int ks = p.ks;
   auto kern = moe_gemm_kernel<KIND>;
   static PerDeviceOnce configured;
@@ -388,7 +390,7 @@ static cudaError_t launch_moe_gemm(const CUtensorMap& tmW, const CUtensorMap& tm
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p);
+  return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
 }
 
 }  // namespace blz
@@ -409,7 +411,6 @@ BLZ_API int blz_moe_gemm(int kind, const void* X, long long ldx, const void* W, 
   MoeGemmParams p;
   p.N = N; p.K = K; p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
   p.row_scale = row_scale; p.alpha = alpha;
-  p.sfw = reinterpret_cast<const uint8_t*>(sfw); p.sfx = reinterpret_cast<const uint8_t*>(sfx);
   p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
   p.tile_expert = tile_expert; p.tile_rows = tile_rows; p.act = act; p.act_limit = 0.f;
   p.rows = 0; p.bias = nullptr; p.ks = 1;
@@ -437,9 +438,9 @@ BLZ_API int blz_moe_gemm(int kind, const void* X, long long ldx, const void* W, 
   }
   if (e != cudaSuccess) return (int)e;
   switch (kind) {
-    case 0: return (int)launch_moe_gemm<0>(tmW, tmX, p, row_tiles, stream);
-    case 1: return (int)launch_moe_gemm<1>(tmW, tmX, p, row_tiles, stream);
-    default: return (int)launch_moe_gemm<2>(tmW, tmX, p, row_tiles, stream);
+    case 0: return (int)launch_moe_gemm<0>(tmW, tmX, p, row_tiles, experts, sfw, sfx, stream);
+    case 1: return (int)launch_moe_gemm<1>(tmW, tmX, p, row_tiles, experts, sfw, sfx, stream);
+    default: return (int)launch_moe_gemm<2>(tmW, tmX, p, row_tiles, experts, sfw, sfx, stream);
   }
 }
 
@@ -467,7 +468,6 @@ BLZ_API int blz_gemm_narrow(int kind, const void* X, long long ldx, const void* 
   MoeGemmParams p;
   p.N = N; p.K = K; p.C = reinterpret_cast<__nv_bfloat16*>(C); p.ldc = ldc;
   p.row_scale = row_scale; p.alpha = alpha;
-  p.sfw = reinterpret_cast<const uint8_t*>(sfw); p.sfx = reinterpret_cast<const uint8_t*>(sfx);
   p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
   p.tile_expert = nullptr; p.tile_rows = nullptr; p.rows = M; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.ks = ks; p.act = act; p.act_limit = act_limit; p.ft_per = 1;
@@ -487,8 +487,8 @@ BLZ_API int blz_gemm_narrow(int kind, const void* X, long long ldx, const void* 
   }
   if (e != cudaSuccess) return (int)e;
   switch (kind) {
-    case 0: return (int)launch_moe_gemm<0>(tmW, tmX, p, 1, stream);
-    case 1: return (int)launch_moe_gemm<1>(tmW, tmX, p, 1, stream);
-    default: return (int)launch_moe_gemm<2>(tmW, tmX, p, 1, stream);
+    case 0: return (int)launch_moe_gemm<0>(tmW, tmX, p, 1, 1, sfw, sfx, stream);
+    case 1: return (int)launch_moe_gemm<1>(tmW, tmX, p, 1, 1, sfw, sfx, stream);
+    default: return (int)launch_moe_gemm<2>(tmW, tmX, p, 1, 1, sfw, sfx, stream);
   }
 }
