@@ -132,23 +132,24 @@ class CudaOps:
         lib.blz_argmax.argtypes = [VP, VP, VP, _c.c_int, _c.c_int, _c.c_longlong, _c.c_int, VP]
         lib.blz_moe_route.argtypes = [VP, _c.c_longlong, VP, VP, VP] + [_c.c_int] * 7 + [VP]
         lib.blz_moe_plan.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, VP]
+        lib.blz_moe_plan_runs.argtypes = [VP] * 6 + [_c.c_int] * 3 + [VP]
+        lib.blz_gemm_pair_experts.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
+                                              _c.c_int] + [VP] * 5 + [_c.c_int, _c.c_int, VP]
         lib.blz_moe_gemm.restype = _c.c_int
         lib.blz_moe_gemm.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
                                      _c.c_int, VP, VP, VP, VP, VP, VP, _c.c_int, VP]
         lib.blz_gemm_narrow.restype = _c.c_int
         lib.blz_gemm_narrow.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
                                         VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_float, VP]
-        # dense layers with few rows (single-user decoding, verify steps) and a large weight take the features-on-lanes kernel
-        # with the K range split over a cluster (blz_gemm_narrow).  Measured on B200, NVFP4, captured-graph timing, against the
-        # one-CTA-per-tile kernel: 1-32 rows 24576x4096 21 -> 16 us, 4096x12288 19 -> 16 us, 17408x5120 18 -> 16 us, 6144x4096
-        # equal, 4096x4096 11.3 -> 12.0 us (loses); at 64 rows only the 24576-wide layer still wins, at 128 rows none does: both
-        # kernels sit on a floor of about 10 us (launch, set-up, first load, reduction) at these sizes.  0 = never.
+        # dense layers with few rows, a long K and few features take the features-on-lanes kernel with the K range split over a
+        # cluster (blz_gemm_narrow; _linear_pair says which).  0 = never.
         self.NARROW_ROWS = int(os.environ.get("BLAZE_GEMM_NARROW_ROWS", "64"))
         self.NARROW_ALWAYS = os.environ.get("BLAZE_GEMM_NARROW_ALWAYS", "0") == "1"
         lib.blz_swiglu_live.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, VP, VP]
-        # routed rows per expert up to this: the expert GEMMs put the features on the tensor-core lanes and only the live rows on its
-        # columns (blz_moe_gemm), which streams the weights; above it the 128-row tiles of the grouped GEMM are full enough
-        # (BLAZE_MOE_NARROW=0: never).  MXFP8 weights of 2048 feature tiles and more up to 8/3 of it, a whole tile of rows: twice the
+        # Experts that the pair kernel does not take (bf16, or features that are no multiple of 256): routed rows per expert up to this,
+        # the expert GEMMs put the features on the tensor-core lanes and only the live rows on its columns (blz_moe_gemm), which streams
+        # the weights; above it the 128-row tiles of the grouped GEMM are full enough (BLAZE_MOE_NARROW=0: never; 1 << 20: always, also
+        # before the pair kernel).  MXFP8 weights of 2048 feature tiles and more up to 8/3 of it, a whole tile of rows: twice the
         # bytes of NVFP4 to stream for the same tiles, on all SMs.  Narrow over tiles, MXFP8, routed experts of a layer as a whole, at
         # 48 / 80 / 128 rows per expert: 512 x 1024 features (4096 tiles) of 2048 0.66 / 0.77 / 0.83, 128 x 3072 of 4096 (3072 tiles)
         # 0.73 / 0.82 / 0.80, but 64 x 2816 of 2048 (1408) 0.90 / 1.01 / 1.22, 128 x 1024 of 2048 (1024) 0.84 / 0.98 / 0.97 (1.04 at
@@ -590,11 +591,20 @@ class CudaOps:
             if rc != 0:
                 raise CudaError(f"blz_gemm_wait_flags failed: {rc}")
             x.wait = None
-        big = self.NARROW_ALWAYS or (lin.N * lin.K >= 6144 * 4096 if M <= 32 else lin.N >= 16384)
-        narrow = (M <= self.NARROW_ROWS and big and kind in (0, 1, 2) and lin.N % 128 == 0 and not f32 and argmax_parts is None
+        narrow = (M <= self.NARROW_ROWS and kind in (0, 1, 2) and lin.N % 128 == 0 and not f32 and argmax_parts is None
                   and pending is None and not kt and (wide is None or relu2) and bn == 0 and (sk is None or sk is False)
                   and (not swiglu or ld_out % 8 == 0) and (sfa is None or sfa.numel() >= 512))
-        if narrow:
+        pair = (wide is None and self._wide_ok and bn == 0 and kind in (0, 1, 2) and lin.N >= 128 and not kt and pending is None
+                and argmax_parts is None and max_ctas != 1 and not relu2 and (sk is None or sk is False)
+                and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0)) and (not swiglu or lin.N % 32 == 0))
+        # Pairs of CTAs stream a weight fastest (us of a call, NVFP4, one CTA per tile or K over a cluster / pairs, 1, 64, 256, 8192 rows:
+        # x 6144 x 4096 12.1, 12.5, 13.5, 115 / 8.9, 9.0, 10.3, 75; x 24576 x 4096 gated 20.7, 28, 30, 380 / 19.6, 19.6, 25, 306; bf16 x
+        # 6144 x 4096 19.9, 26.5, 27.3, 328 / 18.9, 19.5, 21.3, 249; head of 151936 x 4096 216, 228, 315 / 210, 212, 254) but where few
+        # feature tiles have a long K: NVFP4 x 4096 x 12288 14.0, 20.4, 24.0 / 18.9, 18.2, 18.0, bf16 39.9, 39.8, 56 / 74, 43.7, 45.4
+        # (128 rows 40.6 / 44.3).  Those split K over a cluster up to 32 rows (bf16: 128).
+        long_k = lin.N <= 4096 and lin.K >= (8192 if kind == 0 else 10240 if kind == 1 else 5120) and M <= (128 if kind == 0 else 32)
+        big = lin.N * lin.K >= 6144 * 4096 if M <= 32 else lin.N >= 16384
+        if narrow and (self.NARROW_ALWAYS or (big and (long_k or not pair))):
             self._check(self.lib.blz_gemm_narrow(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
                                                  _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), 0, act, limit,
                                                  self._stream()), f"gemm_narrow kind {kind}")
@@ -603,13 +613,10 @@ class CudaOps:
         if sk is None:
             sk = False
             if self._sk_ok and sk_able and wide is None and bn == 0 and M <= self.SK_MAX_ROWS:
-                # Measured on B200 (NVFP4, 256 rows, captured-graph timing): splitting K over a cluster pays when the K range
-                # is long and the tiles are few (4096 x 12288: 23.7 -> 22.2 us); for the other decode shapes the exchange of
-                # fp32 partials through distributed shared memory (about 5 us per 64 KB tile) costs what the split saves.
-                # A tuning table measured on this device (tune.tune_linear) overrides the rule.
+                # Splitting K over a cluster pays where K is long and the tiles are few.  A tuning table measured on this device
+                # (tune.tune_linear) overrides the rule.
                 tiles = ((M + 127) // 128) * ((lin.N + 127) // 128)
-                # Above 256 rows the pairs of CTAs are faster (512 x 4096 x 12288: 35.8 against 29.7 us).
-                sk = M <= 256 and lin.K >= 8192 and tiles <= 2 * self._sm // 2
+                sk = (long_k or not pair) and lin.K >= 8192 and tiles <= 2 * self._sm // 2
                 if self.tuning is not None:
                     from ..tune import bucket
                     hit = self.tuning.get(f"gemm{kind}", lin.N, lin.K, bucket(M))
@@ -623,21 +630,14 @@ class CudaOps:
                                              _ptr(rs), _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]),
                                              ks, act, limit, self._stream()), f"gemm_sk kind {kind}")
             return out
-        # More than 256 rows: pairs of CTAs, the same sums in the same order.  Measured on B200 (us, single-CTA kernels / pairs): bf16 300 x
-        # 6144 x 4096 33 / 31, 1600 rows 84 / 61, 8192 rows 328 / 254; NVFP4 300 rows 20.5 / 17.2, 1600 rows 38 / 30, 8192 rows 115 / 92;
-        # MXFP8 300 x 12352 x 2048 22.5 / 22.4, 4096 rows 140 / 90.  Gated block-scaled products of few rows stay on wide tiles of one
-        # CTA, whose epilogue has a thread per token (NVFP4 x 24576 x 4096: 300 rows 33 / 35, 825 rows 55 / 57, 1200 rows 74 / 68).
-        if (wide is None and self._wide_ok and bn == 0 and M > 256 and kind in (0, 1, 2) and lin.N >= 512 and not kt and pending is None
-                and argmax_parts is None and max_ctas != 1 and not relu2 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0))
-                and (not swiglu or (lin.N % 32 == 0 and (kind == 0 or M > 1024)))):
+        if pair:
             self._check(self.lib.blz_gemm_pair(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
                                                _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), int(f32), 0, max_ctas, act, limit,
                                                self._stream()), f"gemm_pair kind {kind}")
             return out
         if wide is None:
-            # Measured on B200 (Qwen3-8B shapes, captured-graph timing): 256-feature tiles win for block-scaled prefill GEMMs
-            # (NVFP4 2048x24576x4096: 156 -> 119 us); the swapped orientation wins for the very wide bf16 head
-            # (256x151936x4096: 346 -> 315 us) but not for the per-layer decode GEMMs, which stay on the 128-column kernel.
+            # what the pairs do not take (tile-major weights, one CTA at most): 256-feature tiles for block-scaled kinds, the swapped
+            # orientation for a very wide bf16 head, which fetches each weight once
             wide = self._wide_ok and bn == 0 and ((M <= 256 and kind == 0 and lin.N >= 32768 and not swiglu)
                                                   or (kind in (1, 2) and lin.N % 256 == 0 and M > 256))
         if wide:
@@ -1401,7 +1401,9 @@ class CudaOps:
         ex.cuda_pack = {"gate_up": stack(up), "down": stack(down)}
         return ex.cuda_pack
 
-    def _grouped_gemm(self, pk, a, M_pad, tile_expert, n_exp, out, act: int = 0):
+    def _grouped_gemm(self, pk, a, M_pad, tile_expert, n_exp, out, act: int = 0, runs=None):
+        """Expert GEMM over the padded row space: runs of rows on pairs of CTAs (``runs``: the plan's list, rows per run) where every expert's
+        features are whole tiles of 256, else tiles of 128 x 128."""
         kind = pk["kind"]
         if kind in (1, 2):
             data, sfa, rs = a.data, a.sf, a.row_scale
@@ -1410,6 +1412,11 @@ class CudaOps:
             data, sfa, rs = a, None, None
             lda = a.shape[1] * 2
         w = pk["w"]
+        if runs is not None and kind in (0, 1, 2) and pk["N"] % 256 == 0 and act in (0, 1):
+            self._check(self.lib.blz_gemm_pair_experts(kind, _ptr(data), lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
+                                                       M_pad // 128, pk["N"], pk["K"], n_exp, _ptr(rs), _ptr(pk["alpha"]), _ptr(sfa), _ptr(pk["sf"]),
+                                                       _ptr(runs[0]), runs[1], act, self._stream()), "grouped gemm")
+            return out
         self._check(self.lib.blz_gemm_tc(kind, _ptr(data), lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
                                          M_pad, pk["N"], pk["K"], _ptr(rs), _ptr(pk["alpha"]), VP(0), _ptr(sfa), _ptr(pk["sf"]),
                                          0, 128, 0, _ptr(tile_expert), n_exp, 0, act, 0.0, self._stream()), "grouped gemm")
@@ -1454,9 +1461,17 @@ class CudaOps:
         tile_expert = torch.empty(max_tiles, dtype=torch.int32, device=dev)
         tile_rows = torch.empty(max_tiles, dtype=torch.int32, device=dev)
         row_map = torch.empty(T, k, dtype=torch.int32, device=dev)
-        self._check(self.lib.blz_moe_plan(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), n_exp,
-                                          max_tiles, self._stream()), "moe_plan")
+        # rows per tile of the pair kernel by the rows that an expert gets on average: beyond them its weights are read again
+        run = 64 if T * k <= 32 * n_exp else 128 if T * k <= 96 * n_exp else 256
+        runs = (torch.empty(T * k // run + n_exp + 1, 4, dtype=torch.int32, device=dev), run)
+        self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(runs[0]), run, n_exp,
+                                               max_tiles, self._stream()), "moe_plan")
         narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
+        # The pair kernel beats the narrow one for block-scaled experts at any number of rows (us, both products of a layer, narrow / tiles
+        # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 101 / 146 / 94, 4096 277 / 266 / 153; MXFP8, 512
+        # experts of 1024 x 2048, 1 token 43 / 53 / 27, 64 245 / 418 / 238, 1024 322 / 597 / 320, 4096 427 / 585 / 368)
+        if gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2" and self.MOE_NARROW_ROWS < 1 << 20:
+            narrow = False
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)
         if mode:
             proxy = Linear(gu["fmt"], gu["N"], gu["K"])
@@ -1490,7 +1505,7 @@ class CudaOps:
                     if narrow:
                         self._moe_gemm(w, src, max_tiles, tile_expert, tile_rows, n_exp, dst, act=int(dst is g))
                     else:
-                        self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act=int(dst is g))
+                        self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act=int(dst is g), runs=runs)
             return RoutedRows(y, row_map, weights, shared, gate)
         g = torch.empty(M_pad, gu["N"], dtype=x.dtype, device=dev)
         if experts.act == "relu2":
@@ -1515,10 +1530,10 @@ class CudaOps:
             act = self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map)
             self._moe_gemm(dn, act, max_tiles, tile_expert, tile_rows, n_exp, y)
         else:
-            self._grouped_gemm(gu, a, M_pad, tile_expert, n_exp, g)
+            self._grouped_gemm(gu, a, M_pad, tile_expert, n_exp, g, runs=runs)
             # only the routed rows: the padded row space is up to (1 + experts * 128 / routed rows) times larger
             act = self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map)
-            self._grouped_gemm(dn, act, M_pad, tile_expert, n_exp, y)
+            self._grouped_gemm(dn, act, M_pad, tile_expert, n_exp, y, runs=runs)
         return RoutedRows(y, row_map, weights, shared, gate)
 
     def _moe_gemm(self, pk, a, row_tiles, tile_expert, tile_rows, n_exp, out, act: int = 0):

@@ -115,6 +115,10 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t mapped_bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
 }
+// the same for what lies in tensor memory alone: ordered by the tcgen05 fences, so earlier global stores are not waited for
+__device__ __forceinline__ void mbar_arrive_remote_tmem(uint32_t mapped_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(mapped_bar) : "memory");
+}
 __device__ __forceinline__ void fence_acq_rel_cluster() { asm volatile("fence.acq_rel.cluster;" ::: "memory"); }
 __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t mapped_addr) {
   float4 v;

@@ -10,17 +10,23 @@
 // 48 (NVFP4) or 12 columns of tensor memory (copied anew for every stage: copies and MMAs of one issuer run in order), so at 256
 // columns the two accumulators share as many: the epilogue reads the shared ones first, and the next tile waits for those alone.
 //
+// Few tokens: tiles of 64 or 128 columns take less of a stage, so that up to ten stages are in flight, which is what a weight that is read
+// once needs (NVFP4 x 4096 x 4096, 64 rows 12.7 -> 9.1 us).  Experts (GROUPED): a tile is a run of one expert's routed rows.
+//
 // 448 threads: warp 0 = TMA producer (one per CTA, its own half of the tile), warp 1 = MMA issuer (first CTA of the pair only), warps
 // 2-13 = epilogue.  Persistent, one pair per two SMs.  Barriers: `full` lives in the first CTA and counts both CTAs' bytes; `empty` and
-// `acc_full` are in both and raised by multicast commits; `acc_free` is in the first and counts both CTAs' epilogue warps.  Every wait is bounded;
+// `acc_full` are in both and raised by multicast commits; `acc_early`
+// and `acc_free` are in the first and count both CTAs' epilogue warps.  Every wait is bounded;
 // the hardware cluster barrier is used at the start and, by all threads, at the end.  No load is multicast.
 //
-// Measured against one CTA per tile of 128 x 256 (gemm_wide.cu, gemm_tc.cu; device time of a call, L2 flushed): 8192 rows, NVFP4 x 4096 x
-// 12288 177 -> 138 us (6.0 PFLOP/s), x 6144 x 4096 115 -> 92, x 24576 x 4096 with the gated activation 380 -> 360; bf16 x 6144 x 4096
-// 328 -> 254; MXFP8 x 12352 x 2048 266 -> 171.  In a long run the chip's power limit takes a part of that back.  Of an NVFP4 tile's K
-// block at 256 columns (387 ns) the MMAs alone need 333.  Twelve epilogue warps: eight did not keep up with a gated tile of K 4096
-// (390 -> 371 us), sixteen have too few registers.  A loop of one thread that built each descriptor anew issued a K block in 330 ns
-// whatever its columns (371 -> 350).
+// Measured against one CTA per tile of 128 x 256 (gemm_wide.cu, gemm_tc.cu; back to back in a graph, inputs from memory): 8192 rows, NVFP4
+// x 4096 x 12288 177 -> 126 us (6.6 PFLOP/s), x 6144 x 4096 115 -> 75, x 24576 x 4096 with the gated activation 380 -> 306; bf16 x
+// 6144 x 4096 328 -> 249; MXFP8 x 12352 x 2048 266 -> 142.  In a long run the chip's power limit takes a part of that back.  What the
+// stages of the loop cost: of an NVFP4 K block at 256 columns (360 ns) the MMAs and scale copies alone need 350.  One thread that built
+// each descriptor anew issued a block in 330 ns whatever its columns (gated 371 -> 350 us).  Arrivals that release global stores to the
+// cluster made every warp wait for its stores twice per tile, some 1200 clocks each, and 64-bit addresses and exchanges per store
+// another 1800 per 32 columns, so that short tiles hung on the epilogue (gated 350 -> 309 us, K 512 x 2048 27.5 -> 16.6).  Twelve
+// epilogue warps: eight did not keep up with a gated tile, sixteen have too few registers.
 //
 // Counterpart in the reference: the tiled kernels of kernels/src/cuda/nvfp4_gemm.cu.
 #include <cuda.h>
@@ -46,6 +52,7 @@ struct PairParams {
   int sf_col_tiles;           // 4-column scale tiles per 128-row tile
   int cn;                     // columns (tokens) of a tile
   int acc1;                   // first tensor-memory column of the second accumulator
+  const int4* heads;          // experts (grouped kernel): [0].x = number of tiles, then {first row, live rows, expert, 0} of each
   int act;                    // 1, 2: rows of W are [16 gate | 16 up] groups; C = gated activation, bf16 [tokens, N/2]
   float act_limit;            // act 2: the clamp of glu.cuh
   int* status;
@@ -56,29 +63,50 @@ template <> struct PKind<0> { static constexpr int KMMA = 16, SF_ATOMS = 0; };
 template <> struct PKind<1> { static constexpr int KMMA = 64, SF_ATOMS = 4; };
 template <> struct PKind<2> { static constexpr int KMMA = 32, SF_ATOMS = 1; };
 
-template <int KIND>
+// CN: most columns of a tile (64, 128 or 256).  Narrow tiles leave room for more stages: what a weight that is read once needs.
+template <int KIND, int CN>
 struct PairCfg {
   static constexpr int KMMA = PKind<KIND>::KMMA;
   static constexpr int BK = KMMA * 4;                       // 128 bytes of K per row and stage
   static constexpr int SF_ATOMS = PKind<KIND>::SF_ATOMS;
-  static constexpr int A_BYTES = 128 * 128, B_BYTES = 128 * 128;
+  static constexpr int A_BYTES = 128 * 128, B_BYTES = CN * 64;
+  static constexpr int GROUPS = CN > 128 ? 2 : 1;           // 128-row scale tiles under a tile's tokens
   static constexpr int SF_BYTES = SF_ATOMS * 512;           // scales of 128 rows and one stage
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + 3 * SF_BYTES;
+  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + (1 + GROUPS) * SF_BYTES;
   static constexpr int STAGES = (216 * 1024) / STAGE_BYTES;
   static constexpr int SF_COLS = SF_ATOMS * 4 * 3;
   static constexpr int SF_COL0 = 512 - SF_COLS;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 512 + 2 * 256 * 4;
   static constexpr int EPI = 12;                            // epilogue warps
   static constexpr int THREADS = 64 + EPI * 32;
-  static_assert((2 * STAGES + 5) * 8 + 8 <= 512 && SMEM <= 227 * 1024, "shared memory");
+  static_assert((2 * STAGES + 7) * 8 + 8 <= 512 && STAGES <= 32 && SMEM <= 227 * 1024, "shared memory");
   static_assert(SF_COLS <= 64, "the accumulators may share two chunks of 32 columns at most");
 };
 
-template <int KIND>
-__global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+// (x * s) * a + b of two neighbours at once, each rounded as by fmaf(x * s, a, b)
+__device__ __forceinline__ void scale_pair(uint32_t x0, uint32_t x1, float s0, float s1, float a, float b, float& y0, float& y1) {
+  asm("{\n\t.reg .b64 x, s, a, b;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\tmov.b64 a, {%6, %6};\n\tmov.b64 b, {%7, %7};\n\t"
+      "mul.rn.f32x2 x, x, s;\n\tfma.rn.f32x2 x, x, a, b;\n\tmov.b64 {%0, %1}, x;\n\t}\n"
+      : "=f"(y0), "=f"(y1)
+      : "r"(x0), "r"(x1), "f"(s0), "f"(s1), "f"(a), "f"(b));
+}
+
+// A tile as its roles see it.
+struct PairTile {
+  int frow;      // first row of W
+  int feat;      // first feature
+  int t0;        // first token (row of X and of C)
+  int cn;        // columns: live tokens, rounded up to 64
+  int end;       // first row past the live ones
+  int wbase;     // first row of W of the tile's expert (0 for one weight)
+};
+
+template <int KIND, int CN, bool GROUPED>
+__global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                                                             const __grid_constant__ CUtensorMap tmSW, const __grid_constant__ CUtensorMap tmSX,
                                                             const PairParams p) {
-  using Cfg = PairCfg<KIND>;
+  using Cfg = PairCfg<KIND, CN>;
   constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS;
   pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
@@ -88,10 +116,11 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
   uint8_t* sB = sA + STAGES * Cfg::A_BYTES;
   uint8_t* sSFA = sB + STAGES * Cfg::B_BYTES;
   uint8_t* sSFB = sSFA + STAGES * Cfg::SF_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sSFB + STAGES * 2 * Cfg::SF_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(sSFB + STAGES * Cfg::GROUPS * Cfg::SF_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;      // [2]
-  uint64_t* acc_free = acc_full + 2;        // [2]
+  uint64_t* acc_early = acc_full + 2;       // [2] an accumulator has been read as far as the two overlap
+  uint64_t* acc_free = acc_early + 2;       // [2] and altogether
   uint64_t* drain = acc_free + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -100,16 +129,12 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int cn = p.cn;
-  const int tiles_f = (p.N + 255) / 256, tiles_t = (p.M + cn - 1) / cn;
+  const int tiles_f = (p.N + 255) / 256;
   const int k_tiles = (p.K + BK - 1) / BK;
-  const int tiles = tiles_f * tiles_t;
-  const int groups = cn > 128 ? 2 : 1;      // 128-row scale tiles under a tile's tokens (tiles of 64 and 192 start in the middle of one)
-  const bool shared_cols = p.acc1 < cn;     // the accumulators overlap
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_free[i], 2 * Cfg::EPI); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_early[i], 2 * Cfg::EPI); mbar_init(&acc_free[i], 2 * Cfg::EPI); }
     mbar_init(drain, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -127,12 +152,33 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
 
-  // tile u -> (feature tile, token tile): bands of eight token tiles, so that the pairs at work at one time share both operands in L2
-  auto decode = [&](int u, int& ft, int& tt) {
-    const int per_band = 8 * tiles_f, band = u / per_band, in = u - band * per_band;
-    const int width = min(8, tiles_t - band * 8);
-    ft = in / width;
-    tt = band * 8 + in - ft * width;
+  const int tiles_t = GROUPED ? p.heads[0].x : (p.M + p.cn - 1) / p.cn;
+  const int tiles = tiles_f * tiles_t;
+  // Tile u.  One weight: bands of eight token tiles, so that the pairs at work at one time share both operands in L2.  Experts: all
+  // features of a run of rows, then the next.  The roles ask for a tile while they are at the one before it.
+  auto tile_at = [&](int u) {
+    PairTile t = {0, 0, 0, 64, 0, 0};
+    if (u >= tiles) return t;
+    int ft;
+    if constexpr (GROUPED) {
+      const int h = u / tiles_f;
+      ft = u - h * tiles_f;
+      const int4 e = __ldg(p.heads + 1 + h);
+      t.t0 = e.x;
+      t.cn = (e.y + 63) & ~63;
+      t.end = t.t0 + e.y;
+      t.wbase = e.z * p.N;
+    } else {
+      const int per_band = 8 * tiles_f, band = u / per_band, in = u - band * per_band;
+      const int width = min(8, tiles_t - band * 8);
+      ft = in / width;
+      t.t0 = (band * 8 + in - ft * width) * p.cn;
+      t.cn = p.cn;
+      t.end = p.M;
+    }
+    t.feat = ft * 256;
+    t.frow = t.wbase + t.feat;
+    return t;
   };
 
   if (warp == 0) {
@@ -141,20 +187,28 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
       int s = 0; uint32_t ph = 0;
       uint32_t used = 0, last = 0;          // stages filled so far, and the parity of their latest fill
       bool ok = true;
+      PairTile next = tile_at(pair);
       for (int u = pair; u < tiles && ok; u += pairs) {
-        int ft, tt;
-        decode(u, ft, tt);
-        const int frow = ft * 256 + (int)rank * 128, t0 = tt * cn, trow = t0 + (int)rank * (cn >> 1);
+        const PairTile t = next;
+        next = tile_at(u + pairs);
+        const int frow = t.frow + (int)rank * 128, trow = t.t0 + (int)rank * (t.cn >> 1);
+        const int groups = t.cn > 128 ? 2 : 1;      // tiles of 64 and 192 may start in the middle of a scale tile, but not end past the second
         for (int kt = 0; kt < k_tiles; ++kt) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) { ok = false; break; }
           const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
-          if (rank == 0) mbar_expect_tx(&full[s], 2u * (Cfg::A_BYTES + (uint32_t)cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
+          if (rank == 0) mbar_expect_tx(&full[s], 2u * (Cfg::A_BYTES + (uint32_t)t.cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
           const int kc = KIND == 0 ? kt * BK : kt * 128;
           tma_load_2d_pair(sA + s * Cfg::A_BYTES, &tmW, kc, frow, bar);
-          tma_load_2d_pair(sB + s * Cfg::B_BYTES, &tmX, kc, trow, bar);
+          if constexpr (GROUPED) {
+            for (int r = 0; r < t.cn >> 1; r += 32) tma_load_2d_pair(sB + s * Cfg::B_BYTES + r * 128, &tmX, kc, trow + r, bar);
+          } else {
+            tma_load_2d_pair(sB + s * Cfg::B_BYTES, &tmX, kc, trow, bar);
+          }
           if constexpr (ATOMS > 0) {
             tma_load_3d_pair(sSFA + s * Cfg::SF_BYTES, &tmSW, 0, kt * ATOMS, frow >> 7, bar);
-            tma_load_3d_pair(sSFB + s * 2 * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, t0 >> 7, bar);
+            tma_load_3d_pair(sSFB + s * Cfg::GROUPS * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, t.t0 >> 7, bar);
+            if (GROUPED && Cfg::GROUPS == 2 && groups == 2)
+              tma_load_3d_pair(sSFB + (s * 2 + 1) * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, (t.t0 >> 7) + 1, bar);
           }
           used |= 1u << s;
           last = (last & ~(1u << s)) | (ph << s);
@@ -173,22 +227,25 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
       int it = 0;
       bool ok = true;
       const bool leader = elect_one();
-      const uint32_t idesc = KIND == 0 ? make_idesc(1, 1, 256, cn) : make_idesc_bs(KIND == 1, KIND == 1, KIND == 2, 256, cn);
       const uint32_t a_lo0 = (uint32_t)desc_sw128(smem_u32(sA)), b_lo0 = (uint32_t)desc_sw128(smem_u32(sB));
       const uint32_t sa_lo0 = (uint32_t)make_smem_desc(smem_u32(sSFA), 0, 128, kSwzNone);
       const uint32_t sb_lo0 = (uint32_t)make_smem_desc(smem_u32(sSFB), 0, 128, kSwzNone);
       constexpr uint32_t OP_HI = (1024u >> 4) | 1u << 14 | (uint32_t)kSwz128 << 29, SF_HI = (128u >> 4) | 1u << 14;
       auto desc = [](uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; };
+      PairTile next = tile_at(pair);
+      int before = 0;                       // columns of the tile before
       for (int u = pair; u < tiles && ok; u += pairs, ++it) {
-        int ft, tt;
-        decode(u, ft, tt);
-        // Overlapping accumulators: the tile before this one has been read as far as the two overlap (and the one before that
-        // altogether).  Separate ones: the tile before the last has been read.
-        const int prev = shared_cols ? it - 1 : it - 2;
-        if (prev >= 0 && !mbar_wait_cluster(&acc_free[prev & 1], (prev >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+        const PairTile t = next;
+        next = tile_at(u + pairs);
+        const int b = it & 1;
+        const uint32_t idesc = KIND == 0 ? make_idesc(1, 1, 256, t.cn) : make_idesc_bs(KIND == 1, KIND == 1, KIND == 2, 256, t.cn);
+        // this accumulator has been read by the tile before the last, and where it reaches into the other one, that by the last
+        if (it >= 2 && !mbar_wait_cluster(&acc_free[b], ((it >> 1) - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+        if (it >= 1 && (b ? before : t.cn) > p.acc1 && !mbar_wait_cluster(&acc_early[b ^ 1], ((it - 1) >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+        before = t.cn;
         tc_fence_after();
-        const uint32_t d = tmem + (it & 1 ? p.acc1 : 0);
-        const uint32_t sfa = tmem + Cfg::SF_COL0, sfb = sfa + ATOMS * 4, sfb0 = sfb + (((tt * cn) & 127) >> 5);
+        const uint32_t d = tmem + (b ? p.acc1 : 0);
+        const uint32_t sfa = tmem + Cfg::SF_COL0, sfb = sfa + ATOMS * 4, sfb0 = sfb + ((t.t0 & 127) >> 5);
         for (int kt = 0; kt < k_tiles; ++kt) {
           if (!mbar_wait(&full[s], ph, abort_flag, p.status)) { ok = false; break; }
           tc_fence_after();
@@ -196,13 +253,13 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
           const uint32_t a_lo = a_lo0 + s * (Cfg::A_BYTES >> 4), b_lo = b_lo0 + s * (Cfg::B_BYTES >> 4);
           if (leader) {
             if constexpr (ATOMS > 0) {
-              const uint32_t sa_lo = sa_lo0 + s * (Cfg::SF_BYTES >> 4), sb_lo = sb_lo0 + s * (2 * Cfg::SF_BYTES >> 4);
+              const uint32_t sa_lo = sa_lo0 + s * (Cfg::SF_BYTES >> 4), sb_lo = sb_lo0 + s * (Cfg::GROUPS * Cfg::SF_BYTES >> 4);
 #pragma unroll
               for (int a = 0; a < ATOMS; ++a) {
                 tmem_cp_sf_pair(sfa + a * 4, desc(sa_lo + a * 32, SF_HI));
                 tmem_cp_sf_pair(sfb + a * 8, desc(sb_lo + a * 32, SF_HI));
               }
-              if (groups == 2) {
+              if (Cfg::GROUPS == 2 && t.cn > 128) {
 #pragma unroll
                 for (int a = 0; a < ATOMS; ++a) tmem_cp_sf_pair(sfb + a * 8 + 4, desc(sb_lo + (ATOMS + a) * 32, SF_HI));
               }
@@ -235,17 +292,19 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
     const int q = warp & 3, part = (warp - 2) >> 2, etid = threadIdx.x - 64;
     const uint32_t quad = (uint32_t)(q * 32) << 16;
     const bool odd = lane & 1, hi = lane >= 16;
+    const uint32_t pick = odd ? 0x3276u : 0x5410u;      // even lanes: both lower halves, odd lanes: both upper halves
     bool ok = true;
     int it = 0;
+    PairTile next = tile_at(pair);
     for (int u = pair; u < tiles; u += pairs, ++it) {
-      int ft, tt;
-      decode(u, ft, tt);
-      const int b = it & 1, t0 = tt * cn;
+      const PairTile t = next;
+      next = tile_at(u + pairs);
+      const int b = it & 1, t0 = t.t0, cn = t.cn;
       float* rs = s_rs + b * 256;
-      if (etid < cn) rs[etid] = (p.row_scale && t0 + etid < p.M) ? __ldg(p.row_scale + t0 + etid) : 1.0f;
-      const int feat = ft * 256 + (int)rank * 128 + q * 32 + lane;
+      if (etid < cn) rs[etid] = (p.row_scale && t0 + etid < t.end) ? __ldg(p.row_scale + t0 + etid) : 1.0f;
+      const int fl = (int)rank * 128 + q * 32 + lane, feat = t.feat + fl;
       const bool feat_ok = feat < p.N;
-      const float al = (p.alpha && feat_ok) ? __ldg(p.alpha + feat) : 1.0f;
+      const float al = (p.alpha && feat_ok) ? __ldg(p.alpha + t.frow + fl) : 1.0f;
       const float bs = (p.bias && feat_ok) ? bf2f(p.bias[feat]) : 0.0f;
       // the row scales are complete, and the warps agree on whether a wait ran out, so that none is left at a barrier
       if (!bar_red_and(1, Cfg::EPI * 32, ok)) break;
@@ -265,31 +324,32 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
           tmem_ld32(tmem + (b ? p.acc1 : 0) + c + quad, r);
           tmem_ld_wait();
         }
-        if (i == (shared_cols ? 0 : rounds - 1)) {
+        if (i == 0 || i == rounds - 1) {
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_remote(mapa_shared(smem_u32(&acc_free[b]), 0));
+          if (lane == 0 && i == 0) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_early[b]), 0));
+          if (lane == 0 && i == rounds - 1) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_free[b]), 0));
         }
         if (!mine) break;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           const float4 s4 = *reinterpret_cast<const float4*>(rs + c + j);
-          v[j] = fmaf(__uint_as_float(r[j]) * s4.x, al, bs);
-          v[j + 1] = fmaf(__uint_as_float(r[j + 1]) * s4.y, al, bs);
-          v[j + 2] = fmaf(__uint_as_float(r[j + 2]) * s4.z, al, bs);
-          v[j + 3] = fmaf(__uint_as_float(r[j + 3]) * s4.w, al, bs);
+          scale_pair(r[j], r[j + 1], s4.x, s4.y, al, bs, v[j], v[j + 1]);
+          scale_pair(r[j + 2], r[j + 3], s4.z, s4.w, al, bs, v[j + 2], v[j + 3]);
         }
         const int tc = t0 + c;              // token of the chunk's first column
         if (p.out_f32) {
           float* C = reinterpret_cast<float*>(p.C) + feat;
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (feat_ok && tc + j < p.M) C[(size_t)(tc + j) * p.ldc] = v[j];
+            if (feat_ok && tc + j < t.end) C[(size_t)(tc + j) * p.ldc] = v[j];
         } else if (p.act) {
           // lanes 0-15 hold the gates and 16-31 the up values of 16 features: one exchange gives the lower lanes a token and the upper
           // ones the next, a second one pairs two features per store
-          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + ((ft * 256 + (int)rank * 128 + q * 32) >> 1) + (lane & 14);
+          const int first = tc + (odd ? 2 : 0) + (hi ? 1 : 0), left = feat_ok ? t.end - first : 0;
+          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)first * p.ldc + ((t.feat + (int)rank * 128 + q * 32) >> 1) + (lane & 14);
+          const size_t step = (size_t)p.ldc * 4;
           auto gated = [&](auto act) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
@@ -300,10 +360,10 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
                 const float got = __shfl_xor_sync(0xffffffffu, hi ? lo : up, 16);
                 a[k] = act(hi ? got : lo, hi ? up : got);
               }
-              const float got = __shfl_xor_sync(0xffffffffu, odd ? a[0] : a[1], 1);
-              const int tok = tc + j + (odd ? 2 : 0) + (hi ? 1 : 0);
-              if (tok < p.M && feat_ok)
-                *reinterpret_cast<uint32_t*>(C + (size_t)tok * p.ldc) = odd ? pack_bf16x2(got, a[1]) : pack_bf16x2(a[0], got);
+              const uint32_t own = pack_bf16x2(a[0], a[1]);
+              const uint32_t two = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), pick);
+              if (j < left) *reinterpret_cast<uint32_t*>(C) = two;
+              C += step;
             }
           };
           if (p.act == 2) {
@@ -316,13 +376,15 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
           }
         } else {
           // neighbouring lanes trade every other token so that each writes two adjacent features at once
-          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + (feat & ~1);
+          const int first = tc + (odd ? 1 : 0), left = feat_ok ? t.end - first : 0;
+          __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)first * p.ldc + (feat & ~1);
+          const size_t step = (size_t)p.ldc * 2;
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
-            const int tok = tc + j + (odd ? 1 : 0);
-            if (tok < p.M && feat_ok)
-              *reinterpret_cast<uint32_t*>(C + (size_t)tok * p.ldc) = odd ? pack_bf16x2(got, v[j + 1]) : pack_bf16x2(v[j], got);
+            const uint32_t own = pack_bf16x2(v[j], v[j + 1]);
+            const uint32_t two = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), pick);
+            if (j < left) *reinterpret_cast<uint32_t*>(C) = two;
+            C += step;
           }
         }
       }
@@ -338,17 +400,17 @@ __global__ void __launch_bounds__(PairCfg<KIND>::THREADS, 1) gemm_pair_kernel(co
   }
 }
 
-template <int KIND>
+template <int KIND, int CN, bool GROUPED>
 static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW, const CUtensorMap& tmSX,
                                const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
-  using Cfg = PairCfg<KIND>;
-  auto kern = gemm_pair_kernel<KIND>;
+  using Cfg = PairCfg<KIND, CN>;
+  auto kern = gemm_pair_kernel<KIND, CN, GROUPED>;
   static PerDeviceOnce configured;
   cudaError_t e = configured.smem_limit(kern, Cfg::SMEM);
   if (e != cudaSuccess) return e;
   int pairs = sm_count() / 2;
   if (max_ctas > 1 && pairs > max_ctas / 2) pairs = max_ctas / 2;
-  if (pairs > tiles) pairs = tiles;
+  if (!GROUPED && pairs > tiles) pairs = tiles;          // the experts' tiles are counted on the device
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(pairs * 2));
   cfg.blockDim = dim3(Cfg::THREADS);
@@ -364,6 +426,29 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
+}
+
+template <bool GROUPED>
+static cudaError_t launch_pair_kind(int kind, int most, const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW,
+                                    const CUtensorMap& tmSX, const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
+#define BLZ_PAIR_CASE(KD, CN) \
+  if (kind == KD && most <= CN) return launch_pair<KD, CN, GROUPED>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  BLZ_PAIR_CASE(0, 64) BLZ_PAIR_CASE(0, 128) BLZ_PAIR_CASE(0, 256)
+  BLZ_PAIR_CASE(1, 64) BLZ_PAIR_CASE(1, 128) BLZ_PAIR_CASE(1, 256)
+  BLZ_PAIR_CASE(2, 64) BLZ_PAIR_CASE(2, 128) BLZ_PAIR_CASE(2, 256)
+#undef BLZ_PAIR_CASE
+  return cudaErrorInvalidValue;
+}
+
+static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, const float* row_scale, const float* alpha, int act, float act_limit) {
+  PairParams p = {};
+  p.N = N; p.K = K; p.C = C; p.ldc = ldc;
+  p.row_scale = row_scale; p.alpha = alpha;
+  p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
+  p.acc1 = (kind == 0 ? PairCfg<0, 256>::SF_COL0 : kind == 1 ? PairCfg<1, 256>::SF_COL0 : PairCfg<2, 256>::SF_COL0) - 256;
+  p.act = act; p.act_limit = act_limit;
+  p.status = status_word();
+  return p;
 }
 
 }  // namespace blz
@@ -399,15 +484,11 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
   if (kind && (!sfx || !sfw)) return (int)cudaErrorInvalidValue;
   if (act < 0 || act > 2 || (act && (out_f32 || N % 32))) return (int)cudaErrorInvalidValue;
   if (!out_f32 && ((N & 1) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3))) return (int)cudaErrorInvalidValue;
-  PairParams p;
-  p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_f32 = out_f32;
-  p.row_scale = row_scale; p.alpha = alpha; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
-  p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
+  PairParams p = pair_params(kind, N, K, C, ldc, row_scale, alpha, act, act_limit);
+  p.M = M; p.out_f32 = out_f32;
+  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.cn = cn ? cn : blz_gemm_pair_columns(kind, M, N, K, sm_count());
-  const int room = kind == 0 ? PairCfg<0>::SF_COL0 : kind == 1 ? PairCfg<1>::SF_COL0 : PairCfg<2>::SF_COL0;
-  p.acc1 = room - p.cn < 256 ? room - p.cn : 256;
-  p.act = act; p.act_limit = act_limit;
-  p.status = status_word();
+  p.acc1 = p.acc1 + 256 - p.cn < 256 ? p.acc1 + 256 - p.cn : 256;               // narrower tiles overlap less
   CUtensorMap tmW, tmX, tmSW, tmSX;
   const int es = kind == 0 ? 2 : 1;                                   // bytes per tensor-map element
   const uint64_t inner = kind == 1 ? (uint64_t)K / 2 : (uint64_t)K;
@@ -416,17 +497,40 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
   if (e != cudaSuccess) return (int)e;
   tmSW = tmW; tmSX = tmX;
   if (kind) {
-    // Scales of 128 rows and 4 columns are 512 bytes: a map of [row tiles][scale tiles][128 words], so that a stage's scales of one
-    // operand come with one instruction.  Copies of their own (cp.async.bulk of 2 KB) or a map of 256-byte rows, one instruction per row
-    // tile, held the ring up: 8192 x 4096 x 12288 in NVFP4 275 and 166 us, so 141.
-    const uint64_t atoms = (uint64_t)p.sf_col_tiles;
-    const uint32_t box = kind == 1 ? 4 : 1;
-    e = encode_tmap(&tmSW, sfw, 4, 128, atoms, 512, 128, box, 0, (uint64_t)((N + 127) / 128), atoms * 512, 1);
-    if (e == cudaSuccess) e = encode_tmap(&tmSX, sfx, 4, 128, atoms, 512, 128, box, 0, (uint64_t)((M + 127) / 128), atoms * 512, p.cn > 128 ? 2 : 1);
+    // with copies of 2 KB on barriers of each CTA, or a map of 256-byte rows with a load per row tile, 8192 x 4096 x 12288 in NVFP4 took
+    // 275 and 166 us, so 141
+    const uint32_t atoms = kind == 1 ? 4 : 1;
+    e = encode_sf_tmap(&tmSW, sfw, (uint64_t)((N + 127) / 128), p.sf_col_tiles, atoms);
+    if (e == cudaSuccess) e = encode_sf_tmap(&tmSX, sfx, (uint64_t)((M + 127) / 128), p.sf_col_tiles, atoms, p.cn > 128 ? 2 : 1);
     if (e != cudaSuccess) return (int)e;
   }
   const int tiles = ((N + 255) / 256) * ((M + p.cn - 1) / p.cn);
-  if (kind == 0) return (int)launch_pair<0>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
-  if (kind == 1) return (int)launch_pair<1>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
-  return (int)launch_pair<2>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  return (int)launch_pair_kind<false>(kind, p.cn, tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+}
+
+// The routed rows of `experts` experts: X and C are in the padded row space of moe.cu (row_tiles x 128 rows), `heads` comes from
+// blz_moe_plan_runs with the same `run` (64, 128 or 256 rows at most per tile), W holds the experts' weights one after the other, [experts * N, K].  N % 256 == 0; act 0, or 1 (rows of each
+// expert's W in [16 gate | 16 up] groups).
+BLZ_API int blz_gemm_pair_experts(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int row_tiles,
+                                  int N, int K, int experts, const float* row_scale, const float* alpha, const void* sfx, const void* sfw,
+                                  const void* heads, int run, int act, cudaStream_t stream) {
+  using namespace blz;
+  if (row_tiles <= 0) return 0;
+  if (N <= 0 || N % 256 || K <= 0 || kind < 0 || kind > 2 || experts <= 0 || !heads || (run != 64 && run != 128 && run != 256) || act < 0 || act > 1) return (int)cudaErrorInvalidValue;
+  const int kmma = kind == 0 ? 16 : kind == 1 ? 64 : 32;
+  if (K % kmma || (kind && (!sfx || !sfw)) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3)) return (int)cudaErrorInvalidValue;
+  if ((long long)experts * N > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
+  PairParams p = pair_params(kind, N, K, C, ldc, row_scale, alpha, act, 0.f);
+  p.heads = reinterpret_cast<const int4*>(heads);
+  CUtensorMap tmW, tmX, tmSW, tmSX;
+  const int es = kind == 0 ? 2 : 1;
+  const uint64_t inner = kind == 1 ? (uint64_t)K / 2 : (uint64_t)K;
+  cudaError_t e = encode_tmap(&tmW, W, es, inner, (uint64_t)experts * N, ldw, 128 / es, 128, 3);
+  if (e == cudaSuccess) e = encode_tmap(&tmX, X, es, inner, (uint64_t)row_tiles * 128, ldx, 128 / es, 32, 3);
+  tmSW = tmW; tmSX = tmX;
+  const uint32_t atoms = kind == 1 ? 4 : 1;
+  if (e == cudaSuccess && kind) e = encode_sf_tmap(&tmSW, sfw, (uint64_t)experts * N / 128, p.sf_col_tiles, atoms);
+  if (e == cudaSuccess && kind) e = encode_sf_tmap(&tmSX, sfx, row_tiles, p.sf_col_tiles, atoms);
+  if (e != cudaSuccess) return (int)e;
+  return (int)launch_pair_kind<true>(kind, run, tmW, tmX, tmSW, tmSX, p, 0, 0, stream);
 }

@@ -69,19 +69,29 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, float* __rest
 // Single block.  offsets[e] = first row of expert e in the padded row space; tile_expert[m_tile] = local expert or -1.
 // The experts' padded counts are summed up by a scan over the block (one thread walking 512 experts took 16 us, now 3).
 __global__ void __launch_bounds__(512) moe_plan_kernel(const int* __restrict__ counts, int* __restrict__ offsets, int* __restrict__ fill,
-                                int* __restrict__ tile_expert, int* __restrict__ tile_rows, int local_n, int max_tiles) {
+                                int* __restrict__ tile_expert, int* __restrict__ tile_rows, int4* __restrict__ heads, int run, int local_n, int max_tiles) {
   __shared__ int s_off[513];
-  __shared__ int s_warp[16];
+  __shared__ int s_warp[16], s_warp_h[16];
   {
+    // the row tiles of the experts before this one, and their runs of up to `run` rows
     const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-    int sum = e < local_n ? (counts[e] + 127) / 128 * 128 : 0;
+    const int n = e < local_n ? counts[e] : 0, runs = (n + run - 1) / run;
+    int sum = (n + 127) / 128 * 128, before = runs;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, sum, o); if (lane >= o) sum += v; }
-    if (lane == 31) s_warp[warp] = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o), h = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) { sum += v; before += h; }
+    }
+    if (lane == 31) { s_warp[warp] = sum; s_warp_h[warp] = before; }
     __syncthreads();
-    for (int w = 0; w < warp; ++w) sum += s_warp[w];
+    for (int w = 0; w < warp; ++w) { sum += s_warp[w]; before += s_warp_h[w]; }
     if (e == 0) s_off[0] = 0;
     if (e < local_n) s_off[e + 1] = sum;
+    if (heads) {
+      const int first = sum - (n + 127) / 128 * 128;
+      for (int i = 0; i < runs; ++i) heads[1 + before - runs + i] = make_int4(first + run * i, min(run, n - run * i), e, 0);
+      if (e == 511) heads[0] = make_int4(before, 0, 0, 0);
+    }
   }
   __syncthreads();
   for (int e = threadIdx.x; e < local_n; e += blockDim.x) {
@@ -207,11 +217,18 @@ BLZ_API int blz_moe_route(const float* logits, long long ld, float* topk_w, int*
   return (int)cudaGetLastError();
 }
 
+// heads (16-byte entries, or null): the number of runs, then {first row, rows, expert, 0} of the experts' runs of up to `run` rows (64, 128 or
+// 256), what blz_gemm_pair_experts computes at a time.  At most routed rows / run + experts of them.
+BLZ_API int blz_moe_plan_runs(const int* counts, int* offsets, int* fill, int* tile_expert, int* tile_rows, void* heads, int run,
+                              int local_n, int max_tiles, cudaStream_t s) {
+  if (local_n > 512 || (reinterpret_cast<uintptr_t>(heads) & 15) || (run != 64 && run != 128 && run != 256)) return (int)cudaErrorInvalidValue;
+  moe_plan_kernel<<<1, 512, 0, s>>>(counts, offsets, fill, tile_expert, tile_rows, (int4*)heads, run, local_n, max_tiles);
+  return (int)cudaGetLastError();
+}
+
 BLZ_API int blz_moe_plan(const int* counts, int* offsets, int* fill, int* tile_expert, int* tile_rows, int local_n,
                          int max_tiles, cudaStream_t s) {
-  if (local_n > 512) return (int)cudaErrorInvalidValue;
-  moe_plan_kernel<<<1, 512, 0, s>>>(counts, offsets, fill, tile_expert, tile_rows, local_n, max_tiles);
-  return (int)cudaGetLastError();
+  return blz_moe_plan_runs(counts, offsets, fill, tile_expert, tile_rows, nullptr, 256, local_n, max_tiles, s);
 }
 
 // weights (qk 0 only; [T, k] or null): a row is multiplied by its weight on the way; f32: the rows are fp32 (K counts 16-bit elements).

@@ -144,6 +144,37 @@ def test_gemm_pair(ops, fmt, M, N, K, act):
             assert torch.equal(out, want), (cn, ctas, f32)
 
 
+@pytest.mark.parametrize("run", [64, 128, 256])
+@pytest.mark.parametrize("fmt,N,K", [("nvfp4", 512, 320), ("mxfp8", 256, 2048), ("bf16", 768, 48)])
+@pytest.mark.parametrize("counts", [[0, 1, 0, 64, 65, 0], [700, 128, 129, 256, 257, 31], [0, 0, 0, 0, 0, 0], [5000, 0, 1, 0, 0, 513]])
+def test_grouped_gemm_pair(ops, fmt, N, K, counts, run):
+    """Runs of routed rows on CTA pairs: experts without rows, one, whole runs and one row more; the same bits as in tiles of 128."""
+    g = torch.Generator(device=DEV).manual_seed(41)
+    f = {"nvfp4": Format.NVFP4, "mxfp8": Format.MXFP8, "bf16": Format.DENSE}[fmt]
+    E, tiles = len(counts), sum(-(-c // 128) for c in counts) + 2
+
+    class Ex:
+        act, fused_act, cuda_pack, count, first = "swiglu", False, None, E, 0
+        gate_up = [Linear.from_dense(torch.randn(N, K, generator=g, device=DEV) * 0.05, f) for _ in range(E)]
+        down = gate_up
+    pk = ops.pack_experts(Ex)["gate_up"]
+    c = torch.tensor(counts, dtype=torch.int32, device=DEV)
+    off, fill = torch.empty_like(c), torch.empty_like(c)
+    te, tr = [torch.empty(tiles, dtype=torch.int32, device=DEV) for _ in range(2)]
+    heads = torch.full((sum(counts) // run + E + 1, 4), -7, dtype=torch.int32, device=DEV)
+    ptr = [t.data_ptr() for t in (c, off, fill, te, tr, heads)]
+    assert ops.lib.blz_moe_plan_runs(*ptr, run, E, tiles, ops._stream()) == 0
+    want = [[at + run * i, min(run, n - run * i), e, 0] for e, (n, at) in enumerate(zip(counts, off.tolist())) for i in range(-(-n // run))]
+    assert heads[0, 0].item() == len(want) and heads[1:len(want) + 1].tolist() == want
+    x = torch.randn(tiles * 128, K, generator=g, device=DEV).bfloat16()
+    a = ops.quantize_rows(x, Ex.gate_up[0]) if pk["kind"] else x
+    outs = [ops._grouped_gemm(pk, a, tiles * 128, te, E, torch.zeros(tiles * 128, N, dtype=torch.bfloat16, device=DEV), runs=r) for r in (None, (heads, run))]
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
+    for n, at in zip(counts, off.tolist()):
+        assert torch.equal(outs[0][at:at + n], outs[1][at:at + n])
+
+
 @pytest.mark.parametrize("fmt,M,N,K,ks", [
     ("nvfp4", 256, 6144, 4096, 0), ("nvfp4", 256, 4096, 4096, 4), ("nvfp4", 256, 768, 4096, 8), ("nvfp4", 256, 4096, 512, 2),
     ("nvfp4", 200, 1024, 12288, 3), ("nvfp4", 77, 520, 1024, 4), ("nvfp4", 1, 384, 512, 2), ("nvfp4", 130, 256, 320, 5),
