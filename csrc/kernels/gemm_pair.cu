@@ -421,10 +421,14 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  // The set-up (barriers, tensor memory, tensor maps, cluster) runs while the kernel before this one ends; nothing is read before
+  // pdl_wait.  With it 8b decode steps of 1, 256 and 80 rows take 1109, 2652, 1617 us, without 1146, 2688, 1674.  Fetching the first
+  // weights ahead into L2 as well cost 3 % (the copy engine serves those first), and the same attribute on the norms and quantisers
+  // gained 2 % at one row and lost as much elsewhere.
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
 }
 
