@@ -258,16 +258,10 @@ __device__ __forceinline__ uint32_t pack_e4m3x4_f(float a, float b, float c, flo
 
 // Quantise this thread's 8 elements [e0, e0+8) of row t, neighbouring lanes holding neighbouring elements (a warp starts at a
 // multiple of 256).  Every lane of the warp must call it (shuffles); `valid` gates the stores.
-// PACK: a scale byte stored by itself costs the memory system a sector, as a full one does; four of them (neighbours in the 128x4
-// tiles) make one store, and those of a row's padded columns are written as 0.  8192 rows of 12288 activations, NVFP4: 97 -> 78 us
-// (with the registers that the plain form of the kernel below no longer carries).  Where the arithmetic in front sets the pace the
-// two more shuffles cost more than they save: norms of 8192 x 4096 46.2 -> 47.6 us, gated activations of the same in MXFP8 42.6 ->
-// 47.6.
-template <int QUANT, bool PACK>
+template <int QUANT>
 __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, int t, int e0, int W, float g, uint8_t* q_out,
                                              uint8_t* sf_out, int ct) {
   const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&packed);
-  const int lane = threadIdx.x & 31;
   float v[8];
   float bm = 0.f;
 #pragma unroll
@@ -279,12 +273,7 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
     const float inv = denom > 0.f ? 1.f / denom : 0.f;
     const uint32_t codes = pack_e2m1x8(v, inv);
     if (valid) *reinterpret_cast<uint32_t*>(q_out + (size_t)t * (W / 2) + e0 / 2) = codes;
-    if constexpr (PACK) {
-      uint32_t four = valid ? (uint32_t)sf << (8 * ((lane >> 1) & 3)) : 0u;
-      four |= __shfl_xor_sync(0xffffffffu, four, 2);
-      four |= __shfl_xor_sync(0xffffffffu, four, 4);
-      if (valid && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 4, ct)) = four;
-    } else if (valid && (e0 & 15) == 0) {
+    if (valid && (e0 & 15) == 0) {
       sf_out[sf_offset(t, e0 >> 4, ct)] = sf;
     }
   } else {
@@ -298,23 +287,216 @@ __device__ __forceinline__ void quant_store8(const uint4& packed, bool valid, in
           make_uint2(pack_e4m3x4_f(v[0] * inv, v[1] * inv, v[2] * inv, v[3] * inv),
                      pack_e4m3x4_f(v[4] * inv, v[5] * inv, v[6] * inv, v[7] * inv));
     }
-    if constexpr (PACK) {
-      uint32_t four = valid ? (uint32_t)(ex + 127) << (8 * ((lane >> 2) & 3)) : 0u;
-      four |= __shfl_xor_sync(0xffffffffu, four, 4);
-      four |= __shfl_xor_sync(0xffffffffu, four, 8);
-      if (valid && (lane & 15) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 5, ct)) = four;
-    } else if (valid && (e0 & 31) == 0) {
+    if (valid && (e0 & 31) == 0) {
       sf_out[sf_offset(t, e0 >> 5, ct)] = (uint8_t)(ex + 127);
     }
   }
 }
 
+// ---- Rows of many tokens: 16 neighbouring elements per thread, so that an NVFP4 block is one thread's (an MXFP8 block two threads').  The
+// quantisers are bound by their instructions, and most of those are per block: two divisions for the scale, one for its reciprocal.
+// Magnitudes are compared two at a time on the 16-bit values, and the largest of a block serves the row's maximum too.
+__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+// largest magnitude of 16 bf16 values (those that are not numbers do not count, as with fmaxf)
+__device__ __forceinline__ float amax16(const uint32_t (&w)[8]) {
+  __nv_bfloat162 m = __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[0]));
+#pragma unroll
+  for (int j = 1; j < 8; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+  return fmaxf(fmaxf(0.f, __low2float(m)), __high2float(m));
+}
+__device__ __forceinline__ void load16(uint32_t (&w)[8], const __nv_bfloat16* src, bool valid) {
+  const uint4 z = make_uint4(0, 0, 0, 0);
+  const uint4 a = valid ? reinterpret_cast<const uint4*>(src)[0] : z, b = valid ? reinterpret_cast<const uint4*>(src)[1] : z;
+  w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+  w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+}
+// Quantise 16 elements [e0, e0 + 16) of row t, of which `bm` is the largest magnitude; every lane of the warp calls it, a warp starts at a
+// multiple of 512.  Four scales of neighbours make one store.
+template <int QUANT>
+__device__ __forceinline__ void quant_store16(const uint32_t (&w)[8], float bm, bool valid, int t, int e0, int W, float g, uint8_t* q_out,
+                                              uint8_t* sf_out, int ct) {
+  const int lane = threadIdx.x & 31;
+  if (QUANT == 1) {
+    const uint8_t sf = f2e4m3(bm / 6.f / g);           // the same roundings as quant_store8
+    const float denom = e4m32f(sf) * g;
+    const float inv = denom > 0.f ? 1.f / denom : 0.f;
+    uint32_t codes[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { v[2 * j] = lo_f(w[4 * h + j]); v[2 * j + 1] = hi_f(w[4 * h + j]); }
+      codes[h] = pack_e2m1x8(v, inv);
+    }
+    if (valid) *reinterpret_cast<uint2*>(q_out + (size_t)t * (W / 2) + e0 / 2) = make_uint2(codes[0], codes[1]);
+    uint32_t four = valid ? (uint32_t)sf << (8 * (lane & 3)) : 0u;
+    four |= __shfl_xor_sync(0xffffffffu, four, 1);
+    four |= __shfl_xor_sync(0xffffffffu, four, 2);
+    if (valid && (lane & 3) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 4, ct)) = four;
+  } else {
+    bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 1));
+    bm = fmaxf(bm, 1.17549435e-38f);
+    int ex = (int)ceilf(log2f(bm / 448.f));
+    ex = max(-127, min(127, ex));
+    const float inv = exp2f((float)-ex);
+    uint32_t q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = pack_e4m3x4_f(lo_f(w[2 * j]) * inv, hi_f(w[2 * j]) * inv, lo_f(w[2 * j + 1]) * inv, hi_f(w[2 * j + 1]) * inv);
+    if (valid) *reinterpret_cast<uint4*>(q_out + (size_t)t * W + e0) = make_uint4(q[0], q[1], q[2], q[3]);
+    uint32_t four = valid ? (uint32_t)(ex + 127) << (8 * ((lane >> 1) & 3)) : 0u;
+    four |= __shfl_xor_sync(0xffffffffu, four, 2);
+    four |= __shfl_xor_sync(0xffffffffu, four, 4);
+    if (valid && (lane & 7) == 0) *reinterpret_cast<uint32_t*>(sf_out + sf_offset(t, e0 >> 5, ct)) = four;
+  }
+}
+
 template <int QUANT, int CH>
+__global__ void __launch_bounds__(256) rmsnorm_row16_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
+                                                              const __nv_bfloat16* __restrict__ w, uint8_t* __restrict__ q_out,
+                                                              uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int H,
+                                                              float eps, int zero_centered, int sf_col_tiles, int zero_src) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[32];
+  const int t = blockIdx.x;
+  __nv_bfloat16* xr = x + (size_t)t * H;
+  __nv_bfloat16* rr = residual ? residual + (size_t)t * H : nullptr;
+  uint32_t u[CH][8];
+  float ss = 0.f;
+  {
+    uint32_t r[CH][8];
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 16;
+      load16(u[c], xr + i, i < H);
+      if (rr) load16(r[c], rr + i, i < H);
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int i = (c * blockDim.x + threadIdx.x) * 16;
+      if (i < H && zero_src) {
+        reinterpret_cast<uint4*>(xr + i)[0] = make_uint4(0, 0, 0, 0);
+        reinterpret_cast<uint4*>(xr + i)[1] = make_uint4(0, 0, 0, 0);
+      }
+      if (rr) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u[c][j] = pack_bf16x2(lo_f(u[c][j]) + lo_f(r[c][j]), hi_f(u[c][j]) + hi_f(r[c][j]));
+        if (i < H) {
+          reinterpret_cast<uint4*>(rr + i)[0] = make_uint4(u[c][0], u[c][1], u[c][2], u[c][3]);
+          reinterpret_cast<uint4*>(rr + i)[1] = make_uint4(u[c][4], u[c][5], u[c][6], u[c][7]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { ss = fmaf(lo_f(u[c][j]), lo_f(u[c][j]), ss); ss = fmaf(hi_f(u[c][j]), hi_f(u[c][j]), ss); }
+    }
+  }
+  ss = block_reduce(ss, red, false);
+  const float rstd = rsqrtf(ss / H + eps);
+  float bm[CH], amax = 0.f;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 16;
+    uint32_t uw[8];
+    load16(uw, w + i, i < H);
+    const float one = zero_centered ? 1.f : 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      u[c][j] = pack_bf16x2(lo_f(u[c][j]) * rstd * (lo_f(uw[j]) + one), hi_f(u[c][j]) * rstd * (hi_f(uw[j]) + one));
+    bm[c] = amax16(u[c]);
+    amax = fmaxf(amax, bm[c]);
+  }
+  float g = 1.f;
+  if (QUANT == 1) {
+    amax = block_reduce(amax, red, true);
+    g = fmaxf(amax / (6.f * 448.f), 1e-30f);
+    if (threadIdx.x == 0) row_scale[t] = g;
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 16;
+    quant_store16<QUANT>(u[c], bm[c], i < H, t, i, H, g, q_out, sf_out, sf_col_tiles);
+  }
+}
+
+// ACT: the source rows are activations already (no up half).
+template <int MODE, int CH, bool ACT>
+__global__ void __launch_bounds__(256) swiglu_row16_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ q_out,
+                                                             uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int I,
+                                                             int sf_col_tiles, const int* __restrict__ row_list) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[32];
+  const int t = row_list ? row_list[blockIdx.x] : (int)blockIdx.x;
+  if (t < 0) return;
+  const __nv_bfloat16* src = gu + (size_t)t * (ACT ? I : 2 * I);
+  uint32_t a[CH][8], b[ACT ? 1 : CH][8];
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 16;
+    load16(a[c], src + i, i < I);
+    if constexpr (!ACT) load16(b[c], src + I + i, i < I);
+  }
+  float bm[CH], amax = 0.f;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    if constexpr (!ACT) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[c][j] = pack_bf16x2(silu(lo_f(a[c][j])) * lo_f(b[c][j]), silu(hi_f(a[c][j])) * hi_f(b[c][j]));
+    }
+    bm[c] = amax16(a[c]);
+    amax = fmaxf(amax, bm[c]);
+  }
+  float gs = 1.f;
+  if (MODE == 1) {
+    amax = block_reduce(amax, red, true);
+    gs = fmaxf(amax / (6.f * 448.f), 1e-30f);
+    if (threadIdx.x == 0) row_scale[t] = gs;
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 16;
+    quant_store16<MODE>(a[c], bm[c], i < I, t, i, I, gs, q_out, sf_out, sf_col_tiles);
+  }
+}
+
+// Rows of at most 1024 activations, several per CTA (see swiglu_rows_kernel): a warp, or two, per row.
+template <int MODE>
+__global__ void __launch_bounds__(256) quant_rows16_kernel(const __nv_bfloat16* __restrict__ act, uint8_t* __restrict__ q_out,
+                                                             uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int I,
+                                                             int sf_col_tiles, const int* __restrict__ row_list, int n_rows, int tpr) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[8];
+  const int sub = threadIdx.x / tpr, in_row = threadIdx.x - sub * tpr;
+  const int r = blockIdx.x * (blockDim.x / tpr) + sub;
+  int t = -1;
+  if (r < n_rows) t = row_list ? row_list[r] : r;
+  const bool live = t >= 0;
+  const int i = in_row * 16;
+  const bool valid = live && i < I;
+  uint32_t a[8];
+  load16(a, act + (size_t)(live ? t : 0) * I + i, valid);
+  const float bm = amax16(a);
+  float gs = 1.f;
+  if (MODE == 1) {
+    float m = warp_max(bm);
+    if (tpr > 32) {
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+      __syncthreads();
+      m = 0.f;
+      for (int k = 0; k < (tpr >> 5); ++k) m = fmaxf(m, red[((sub * tpr) >> 5) + k]);
+    }
+    gs = fmaxf(m / (6.f * 448.f), 1e-30f);
+    if (live && in_row == 0) row_scale[t] = gs;
+  }
+  quant_store16<MODE>(a, bm, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
+}
+
+template <int CH>
 __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                                             const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
-                                                            uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
-                                                            float* __restrict__ row_scale, int H, float eps, int zero_centered,
-                                                            int sf_col_tiles, int zero_src) {
+                                                            int H, float eps, int zero_centered, int zero_src) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[32];
@@ -350,7 +532,6 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
   }
   ss = block_reduce(ss, red, false);
   const float rstd = rsqrtf(ss / H + eps);
-  float amax = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
@@ -361,25 +542,12 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
     for (int j = 0; j < 8; ++j) {
       const float wf = bf2f(ew[j]) + (zero_centered ? 1.f : 0.f);
       e[j] = __float2bfloat16(bf2f(e[j]) * rstd * wf);
-      amax = fmaxf(amax, fabsf(bf2f(e[j])));
     }
-    if (QUANT == 0 && i < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + i) = u[c];
-  }
-  if (QUANT == 0) return;
-  float g = 1.f;
-  if (QUANT == 1) {
-    amax = block_reduce(amax, red, true);
-    g = fmaxf(amax / (6.f * 448.f), 1e-30f);
-    if (threadIdx.x == 0) row_scale[t] = g;
-  }
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int i = (c * blockDim.x + threadIdx.x) * 8;
-    quant_store8<QUANT, false>(u[c], i < H, t, i, H, g, q_out, sf_out, sf_col_tiles);
+    if (i < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + i) = u[c];
   }
 }
 
-// ACT: the source rows are activations already (no up half): without its registers twice the rows are in flight per SM.
+// Gated rows; ACT (bf16 out only): the source rows are activations already.
 template <int MODE, int CH, bool ACT>
 __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                                            uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
@@ -431,7 +599,7 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
-    quant_store8<MODE, ACT>(a[c], i < I, t, i, I, gs, q_out, sf_out, sf_col_tiles);
+    quant_store8<MODE>(a[c], i < I, t, i, I, gs, q_out, sf_out, sf_col_tiles);
   }
 }
 
@@ -487,7 +655,7 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const __nv_bfloat16* _
     gs = fmaxf(m / (6.f * 448.f), 1e-30f);
     if (live && in_row == 0) row_scale[t] = gs;
   }
-  quant_store8<MODE, false>(a, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
+  quant_store8<MODE>(a, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
 }
 
 // ---------------------------------------------------------------------------------------------- attention prep
@@ -934,6 +1102,13 @@ static inline void reg_shape(int W, int T, int* threads, int* chunks) {
     case 5: CALL(5); break; default: CALL(6); break;                                                \
   }
 
+// The quantising row kernels with 16 elements per thread: rows of up to 6 chunks of 256 threads.  At any number of rows where rows are
+// normed or are activations already (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norm of 8192
+// x 4096 48 / 40, of 1 row 3.3 / 2.5), for gated rows from 512 on (825 rows of 12288 19.8 / 17.1, 256 rows 7.6 / 8.3: their
+// activation is the longer chain per thread there; the experts' short gated rows likewise 43.7 / 46.2).
+constexpr int ROW16_MOST = 6 * 256 * 16;
+static inline int row16_threads(int W, int chunks) { return (W / 16 + chunks * 32 - 1) / (chunks * 32) * 32; }
+
 static inline int norm_threads(int H) {
   int t = H / 8;
   t = (t + 31) / 32 * 32;
@@ -957,11 +1132,17 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
   const int ct = quant == 1 ? (H + 63) / 64 : (H + 127) / 128;
   int rt, ch;
   reg_shape(H, T, &rt, &ch);
-  if (ch) {
+  if (quant && H <= ROW16_MOST) {
+    const int c16 = (H + 4095) / 4096;
 #define BLZ_RN(C)                                                                                                              \
-  if (quant == 0) launch_pdl(rmsnorm_reg_kernel<0, C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, H, eps, zero_centered, 0, zero_src); \
-  else if (quant == 1) launch_pdl(rmsnorm_reg_kernel<1, C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src); \
-  else launch_pdl(rmsnorm_reg_kernel<2, C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src)
+  if (quant == 1) launch_pdl(rmsnorm_row16_kernel<1, C>, dim3(T), dim3(row16_threads(H, C)), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src); \
+  else launch_pdl(rmsnorm_row16_kernel<2, C>, dim3(T), dim3(row16_threads(H, C)), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src)
+    BLZ_CH_SWITCH(c16, BLZ_RN)
+#undef BLZ_RN
+    return (int)cudaGetLastError();
+  }
+  if (!quant && ch) {
+#define BLZ_RN(C) launch_pdl(rmsnorm_reg_kernel<C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)out, H, eps, zero_centered, zero_src)
     BLZ_CH_SWITCH(ch, BLZ_RN)
 #undef BLZ_RN
     return (int)cudaGetLastError();
@@ -996,6 +1177,14 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   const int ct = mode == 1 ? (I + 63) / 64 : (I + 127) / 128;
   configure_once();
   {
+    const int tpr16 = (I / 16 + 31) / 32 * 32;
+    if (mode && src_is_act && I <= 1024) {
+      const int per = 256 / tpr16;
+      const dim3 grid((T + per - 1) / per), block(per * tpr16);
+      if (mode == 1) launch_pdl(quant_rows16_kernel<1>, grid, block, 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list, T, tpr16);
+      else launch_pdl(quant_rows16_kernel<2>, grid, block, 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list, T, tpr16);
+      return (int)cudaGetLastError();
+    }
     const int tpr = (I / 8 + 31) / 32 * 32, rows_per = tpr <= 128 ? 256 / tpr : 1;
     if (I <= 1024 && rows_per >= 2) {
       const dim3 grid((T + rows_per - 1) / rows_per), block(rows_per * tpr);
@@ -1007,15 +1196,23 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   }
   int rt, ch;
   reg_shape(I, T, &rt, &ch);
-  if (ch) {
-#define BLZ_SW2(C, ACT)                                                                                                        \
-  if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
-  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list); \
-  else launch_pdl(swiglu_reg_kernel<2, C, ACT>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
-#define BLZ_SW(C) if (src_is_act) { BLZ_SW2(C, true); } else { BLZ_SW2(C, false); }
-    BLZ_CH_SWITCH(ch, BLZ_SW)
+  if (mode && I <= ROW16_MOST && (src_is_act || T >= 512)) {
+    const int c16 = (I + 4095) / 4096;
+#define BLZ_SW2(Q, C, ACT) launch_pdl(swiglu_row16_kernel<Q, C, ACT>, dim3(T), dim3(row16_threads(I, C)), 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
+#define BLZ_SW(C) if (mode == 1) { if (src_is_act) BLZ_SW2(1, C, true); else BLZ_SW2(1, C, false); } else { if (src_is_act) BLZ_SW2(2, C, true); else BLZ_SW2(2, C, false); }
+    BLZ_CH_SWITCH(c16, BLZ_SW)
 #undef BLZ_SW
 #undef BLZ_SW2
+    return (int)cudaGetLastError();
+  }
+  if (ch && !(mode && src_is_act)) {
+#define BLZ_SW(C)                                                                                                              \
+  if (src_is_act) launch_pdl(swiglu_reg_kernel<0, C, true>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
+  else if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
+  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list); \
+  else launch_pdl(swiglu_reg_kernel<2, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
+    BLZ_CH_SWITCH(ch, BLZ_SW)
+#undef BLZ_SW
     return (int)cudaGetLastError();
   }
   if (mode == 0) swiglu_kernel<0><<<T, thr, 0, s>>>((const bf16*)gu, (bf16*)out, nullptr, nullptr, nullptr, I, src_is_act, 0, row_list);
