@@ -1359,29 +1359,38 @@ class CudaOps:
                 out.append(Linear.from_dense(w, dtype=l.w.dtype))
             return out
 
-        def stack(lins):
-            pk0 = self.pack(lins[0], tiled=False, exact_fp8=False)
-            kind = pk0["kind"]
-            w = torch.cat([self.pack(l, tiled=False, exact_fp8=False)["w"] for l in lins])
-            alpha = torch.cat([self.pack(l, tiled=False, exact_fp8=False)["alpha"] for l in lins]) if pk0["alpha"] is not None else None
+        def stack(lins, swiglu=False):
+            """``swiglu``: block-scaled rows in the order of the SwiGLU epilogue."""
+            l0, E, dev = lins[0], len(lins), self.device
+            swiglu = swiglu and l0.fmt in (Format.NVFP4, Format.MXFP8, Format.FP8_BLOCK) and l0.N % 32 == 0
+            order = self.swiglu_order(l0.N).to(dev) if swiglu else None
+
+            def rows(ts, dtype=None):        # every expert's rows one after the other, in that order
+                t = torch.cat([t.to(dev) if dtype is None else t.to(dev, dtype) for t in ts])
+                return t if order is None else t.view(E, l0.N, -1)[:, order].reshape(t.shape)
+
+            if l0.fmt in (Format.NVFP4, Format.MXFP8):
+                kind = 1 if l0.fmt == Format.NVFP4 else 2
+                w, alpha = rows([l.w.view(torch.uint8) for l in lins]), rows([l.alpha for l in lins], torch.float32)
+                raw = rows([l.sf.view(torch.uint8) for l in lins])
+            else:
+                packs = [self.pack(l, tiled=False, swiglu=swiglu, exact_fp8=False) for l in lins]
+                kind = packs[0]["kind"]
+                w = torch.cat([p["w"] for p in packs])
+                alpha = torch.cat([p["alpha"] for p in packs]) if packs[0]["alpha"] is not None else None
+                if kind == 2:
+                    raw = torch.cat([quant.unswizzle_sf_128x4(p["sf"], (l0.N + 255) // 256 * 256, l0.K // 32)[:l0.N] for p in packs])
             sf = None
             if kind in (1, 2):
-                l0 = lins[0]
                 if l0.N % 128:
                     raise CudaError("grouped GEMM needs expert output dims that are multiples of 128")
-                per = l0.K // (16 if kind == 1 else 32)
-                if kind == 1:
-                    raw = torch.cat([l.sf.to(self.device).view(torch.uint8) for l in lins])
-                else:
-                    raw = torch.cat([quant.unswizzle_sf_128x4(self.pack(l, tiled=False, exact_fp8=False)["sf"], (l.N + 255) // 256 * 256, per)[:l.N] for l in lins])
-                rows = (raw.shape[0] + 255) // 256 * 256
-                buf = torch.zeros(rows, per, dtype=torch.uint8, device=self.device)
+                buf = torch.zeros((raw.shape[0] + 255) // 256 * 256, l0.K // (16 if kind == 1 else 32), dtype=torch.uint8, device=dev)
                 buf[:raw.shape[0]] = raw
                 sf = quant.swizzle_sf_128x4(buf)
             for l in lins:
                 l.cuda_pack = None          # the stacked copy replaces the per-expert ones
-            return {"kind": kind, "w": w.contiguous(), "sf": sf, "alpha": alpha, "N": lins[0].N, "K": lins[0].K,
-                    "fmt": lins[0].fmt, "act_quant": lins[0].act_quant}
+            return {"kind": kind, "w": w.contiguous(), "sf": sf, "alpha": alpha, "N": l0.N, "K": l0.K,
+                    "fmt": l0.fmt, "act_quant": l0.act_quant, "swiglu": swiglu}
         if fused:
             # [gate | up] rows, each half rounded up to 64 features, in the order of the SwiGLU epilogue
             ff, K = ex.down[0].K, ex.gate_up[0].K
@@ -1398,7 +1407,7 @@ class CudaOps:
                                 "K": w[0].shape[1], "fmt": Format.DENSE, "act_quant": False} for n, w in (("gate_up", ws), ("down", downs))}
             return ex.cuda_pack
         up, down = (padded(ex.gate_up, True, False), padded(ex.down, True, True)) if relu2 else (ex.gate_up, ex.down)
-        ex.cuda_pack = {"gate_up": stack(up), "down": stack(down)}
+        ex.cuda_pack = {"gate_up": stack(up, swiglu=ex.act == "swiglu"), "down": stack(down)}
         return ex.cuda_pack
 
     def _grouped_gemm(self, pk, a, M_pad, tile_expert, n_exp, out, act: int = 0, runs=None):
@@ -1507,7 +1516,8 @@ class CudaOps:
                     else:
                         self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act=int(dst is g), runs=runs)
             return RoutedRows(y, row_map, weights, shared, gate)
-        g = torch.empty(M_pad, gu["N"], dtype=x.dtype, device=dev)
+        act = bool(gu["swiglu"]) if experts.act != "relu2" else False      # the gated activation is in the product's epilogue
+        g = torch.empty(M_pad, gu["N"] // 2 if act else gu["N"], dtype=x.dtype, device=dev)
         if experts.act == "relu2":
             y = torch.empty(M_pad, dn["N"], dtype=x.dtype, device=dev)
             for w, src, dst in ((gu, a, g), (dn, g, y)):
@@ -1525,15 +1535,14 @@ class CudaOps:
         proxy_d = Linear(dn["fmt"], dn["N"], dn["K"])
         proxy_d.act_quant = dn["act_quant"]
         y = torch.empty(M_pad, dn["N"], dtype=torch.bfloat16, device=dev)
-        if narrow:
-            self._moe_gemm(gu, a, max_tiles, tile_expert, tile_rows, n_exp, g)
-            act = self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map)
-            self._moe_gemm(dn, act, max_tiles, tile_expert, tile_rows, n_exp, y)
-        else:
-            self._grouped_gemm(gu, a, M_pad, tile_expert, n_exp, g, runs=runs)
-            # only the routed rows: the padded row space is up to (1 + experts * 128 / routed rows) times larger
-            act = self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map)
-            self._grouped_gemm(dn, act, M_pad, tile_expert, n_exp, y, runs=runs)
+        def product(w, src, dst, act=0):
+            if narrow:
+                self._moe_gemm(w, src, max_tiles, tile_expert, tile_rows, n_exp, dst, act)
+            else:
+                self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act, runs=runs)
+        product(gu, a, g, int(act))
+        # only the routed rows: the padded row space is up to (1 + experts * 128 / routed rows) times larger
+        product(dn, self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map, act), y)
         return RoutedRows(y, row_map, weights, shared, gate)
 
     def _moe_gemm(self, pk, a, row_tiles, tile_expert, tile_rows, n_exp, out, act: int = 0):
@@ -1550,20 +1559,21 @@ class CudaOps:
                                           row_tiles, pk["N"], pk["K"], n_exp, _ptr(rs), _ptr(pk["alpha"]), _ptr(sfa), _ptr(pk["sf"]),
                                           _ptr(tile_expert), _ptr(tile_rows), act, self._stream()), f"moe_gemm kind {kind}")
 
-    def _silu_mul_live(self, gu, quant_for, row_list):
+    def _silu_mul_live(self, gu, quant_for, row_list, is_act: bool = False):
         """``silu_mul`` over the padded row space of the routed rows: only the rows named in ``row_list`` (-1 = none) are
-        touched, one CTA each."""
-        T, I2 = gu.shape
-        I = I2 // 2
+        touched, one CTA each.  ``is_act``: the rows are gated activations already, which are only quantised."""
+        T, I = gu.shape[0], gu.shape[1] if is_act else gu.shape[1] // 2
         n = row_list.numel()
         mode = self._qmode(quant_for)
         if mode == 0:
+            if is_act:
+                return gu
             out = torch.empty(T, I, dtype=torch.bfloat16, device=self.device)
             self._check(self.lib.blz_swiglu_live(_ptr(gu), _ptr(out), VP(0), VP(0), VP(0), n, I, 0, 0, _ptr(row_list), self._stream()),
                         "swiglu_live")
             return out
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, I)
-        self._check(self.lib.blz_swiglu_live(_ptr(gu), VP(0), _ptr(qa.data), _ptr(qa.sf), _ptr(qa.row_scale), n, I, mode, 0,
+        self._check(self.lib.blz_swiglu_live(_ptr(gu), VP(0), _ptr(qa.data), _ptr(qa.sf), _ptr(qa.row_scale), n, I, mode, int(is_act),
                                              _ptr(row_list), self._stream()), "swiglu_live_q")
         return qa
 

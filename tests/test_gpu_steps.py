@@ -435,3 +435,63 @@ def test_silu_of_every_gate(ops):      # noqa: F811
     step = torch.exp2(torch.frexp(want.abs().clamp_min(2.0 ** -126))[1].double() - 8)      # of bf16 (8 bits) at that size
     # half a step, and in front of the rounding the fast exponential: 2 ulp and, of its argument, 88 * 2^-24, of 2^8 steps
     assert ((got - want).abs()[ok] <= step[ok] * (0.5 + 256 * (88 + 4) * 2.0 ** -24)).all()
+
+
+@pytest.mark.parametrize("mode", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("W", [32, 96, 480, 1024, 1056, 4096, 4128, 12288, 12320, 24576, 24608])
+def test_quantised_rows_of_sixteen_elements_per_thread(ops, mode, W):      # noqa: F811
+    """Rows of the quantisers with 16 elements per thread (part of a warp, whole chunks, one block more, the widest, and the kernel
+    behind it) against those with 8: activations, gated rows of 511 and 512 tokens, norms whose sums are exact; the same codes, scales
+    and row scales, also in rows with infinities and values that are not numbers."""
+    g = torch.Generator(device=DEV).manual_seed(4)
+    lin = Linear(mode, 128, W)
+    lin.act_quant = True
+    per = 16 if mode == Format.NVFP4 else 32
+
+    def same(a, b, n):
+        sf = [quant.unswizzle_sf_128x4(q.sf, q.rows, W // per)[:n] for q in (a, b)]
+        rs = a.row_scale is None or torch.equal(a.row_scale[:n].view(torch.int32), b.row_scale[:n].view(torch.int32))
+        return torch.equal(a.data[:n], b.data[:n]) and torch.equal(*sf) and rs
+    gu = torch.randn(512, 2 * W, generator=g, device=DEV).bfloat16()
+    gu[3, 5], gu[4, 7], gu[5, W + 9], gu[6, :] = float("nan"), float("inf"), float("-inf"), 0.0
+    wide = W <= 24576                              # beyond, one kernel takes all of them
+    few, many = ops.silu_mul(gu[:511], lin), ops.silu_mul(gu, lin)
+    assert same(few, many, 511)
+    if wide:
+        assert same(ops.quantize_rows(ops.silu_mul(gu[:511]), lin), few, 511)
+    x = torch.randint(-4, 5, (33, W), generator=g, device=DEV).bfloat16() / 2
+    r = torch.randint(-4, 5, (33, W), generator=g, device=DEV).bfloat16() / 4
+    w = (1 + 0.1 * torch.randn(W, generator=g, device=DEV)).bfloat16()
+    for zero in (False, True):
+        r1, r2, x1 = r.clone(), r.clone(), x.clone()
+        plain, _ = ops.norm(x.clone(), r1, w, 1e-6, zero_centered=zero)
+        q, _ = ops.norm(x1, r2, w, 1e-6, zero_centered=zero, quant_for=lin, zero_src=True)
+        assert torch.equal(r1, r2) and not x1.any()
+        if wide:
+            assert same(q, ops.quantize_rows(plain, lin), 33)
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
+
+
+@pytest.mark.parametrize("fmt", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("T,E,k,H,I", [(5, 3, 1, 256, 128), (300, 4, 2, 512, 256), (130, 8, 4, 256, 192)])
+def test_experts_with_the_activation_in_the_product(ops, fmt, T, E, k, H, I):      # noqa: F811
+    """Interleaved gate and up rows: the pairs', the narrow and the 128-column product give the rounded gate and up sums' activation."""
+    g = torch.Generator(device=DEV).manual_seed(8)
+    x = torch.randn(T, H, generator=g, device=DEV).bfloat16()
+    logits = torch.randn(T, E, generator=g, device=DEV)
+    outs, old = [], ops.MOE_NARROW_ROWS
+    try:
+        for rows in (48, 1 << 20, 0):
+            ex = _experts(E, H, I, fmt, 9)
+            ops.MOE_NARROW_ROWS = rows
+            w, ids = ops.router_topk(logits, k, True, 0, E)
+            outs.append(ops.moe(x, w, ids, ex))
+            assert ex.cuda_pack["gate_up"]["swiglu"]
+    finally:
+        ops.MOE_NARROW_ROWS = old
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
+    for o in outs:
+        assert _rel(o, outs[0]) < 2e-3             # one may round a sum to the neighbouring bf16
+        assert _rel(o, ref.moe_forward(x, w, ids, ex.forward_one, E)) < 0.08
