@@ -104,9 +104,7 @@ class CudaOps:
         self.tuning = None         # optional tune.Tuning: per-shape kernel choices measured on this device
         lib.blz_gemm_pair.restype = _c.c_int
         lib.blz_gemm_pair.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
-                                      VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_float, VP]
-        lib.blz_gemm_pair_columns.restype = _c.c_int
-        lib.blz_gemm_pair_columns.argtypes = [_c.c_int] * 5
+                                      VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_float, VP]
         lib.blz_gemm_wide_ksplit.restype = _c.c_int
         lib.blz_gemm_wide_ksplit.argtypes = [_c.c_int, _c.c_int, _c.c_int]
         self._wide_ok = os.environ.get("BLAZE_GEMM_WIDE", "1") != "0"
@@ -141,8 +139,8 @@ class CudaOps:
         lib.blz_gemm_narrow.restype = _c.c_int
         lib.blz_gemm_narrow.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
                                         VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_float, VP]
-        # dense layers with few rows, a long K and few features take the features-on-lanes kernel with the K range split over a
-        # cluster (blz_gemm_narrow; _linear_pair says which).  0 = never.
+        # dense layers with few rows that the pair kernel does not take: features on the lanes, K split over a cluster
+        # (blz_gemm_narrow).  0 = never.
         self.NARROW_ROWS = int(os.environ.get("BLAZE_GEMM_NARROW_ROWS", "64"))
         self.NARROW_ALWAYS = os.environ.get("BLAZE_GEMM_NARROW_ALWAYS", "0") == "1"
         lib.blz_swiglu_live.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, VP, VP]
@@ -598,13 +596,11 @@ class CudaOps:
                 and argmax_parts is None and max_ctas != 1 and not relu2 and (sk is None or sk is False)
                 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0)) and (not swiglu or lin.N % 32 == 0))
         # Pairs of CTAs stream a weight fastest (us of a call, NVFP4, one CTA per tile or K over a cluster / pairs, 1, 64, 256, 8192 rows:
-        # x 6144 x 4096 12.1, 12.5, 13.5, 115 / 8.9, 9.0, 10.3, 75; x 24576 x 4096 gated 20.7, 28, 30, 380 / 19.6, 19.6, 25, 306; bf16 x
-        # 6144 x 4096 19.9, 26.5, 27.3, 328 / 18.9, 19.5, 21.3, 249; head of 151936 x 4096 216, 228, 315 / 210, 212, 254) but where few
-        # feature tiles have a long K: NVFP4 x 4096 x 12288 14.0, 20.4, 24.0 / 18.9, 18.2, 18.0, bf16 39.9, 39.8, 56 / 74, 43.7, 45.4
-        # (128 rows 40.6 / 44.3).  Those split K over a cluster up to 32 rows (bf16: 128).
-        long_k = lin.N <= 4096 and lin.K >= (8192 if kind == 0 else 10240 if kind == 1 else 5120) and M <= (128 if kind == 0 else 32)
+        # x 6144 x 4096 12.1, 12.5, 13.5, 115 / 8.9, 9.0, 10.3, 75; x 24576 x 4096 gated 20.7, 28, 30, 380 / 19.6, 19.6, 25, 306; x 4096 x
+        # 12288 15.9, 20.4, 24, 177 / 14.2, 14.3, 16.7, 126; bf16 x 6144 x 4096 19.9, 26.5, 27.3, 328 / 17.7, 18.1, 22.7, 249; head of
+        # 151936 x 4096 216, 228, 315 / 210, 212, 254).
         big = lin.N * lin.K >= 6144 * 4096 if M <= 32 else lin.N >= 16384
-        if narrow and (self.NARROW_ALWAYS or (big and (long_k or not pair))):
+        if narrow and (self.NARROW_ALWAYS or (big and not pair)):
             self._check(self.lib.blz_gemm_narrow(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
                                                  _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), 0, act, limit,
                                                  self._stream()), f"gemm_narrow kind {kind}")
@@ -616,7 +612,7 @@ class CudaOps:
                 # Splitting K over a cluster pays where K is long and the tiles are few.  A tuning table measured on this device
                 # (tune.tune_linear) overrides the rule.
                 tiles = ((M + 127) // 128) * ((lin.N + 127) // 128)
-                sk = (long_k or not pair) and lin.K >= 8192 and tiles <= 2 * self._sm // 2
+                sk = not pair and lin.K >= 8192 and tiles <= 2 * self._sm // 2
                 if self.tuning is not None:
                     from ..tune import bucket
                     hit = self.tuning.get(f"gemm{kind}", lin.N, lin.K, bucket(M))
@@ -632,7 +628,7 @@ class CudaOps:
             return out
         if pair:
             self._check(self.lib.blz_gemm_pair(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
-                                               _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), int(f32), 0, max_ctas, act, limit,
+                                               _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), int(f32), 0, 0, max_ctas, act, limit,
                                                self._stream()), f"gemm_pair kind {kind}")
             return out
         if wide is None:

@@ -21,8 +21,7 @@ cudaError_t encode_tmap(CUtensorMap* out, const void* base, int dtype_bytes, uin
                         uint64_t stride2_bytes = 0, uint32_t box2 = 1);
 
 // Scale factors of `row_tiles` x 128 rows in 4-column tiles of 512 bytes, [row tiles][col tiles][128 words]: a load takes the `atoms`
-// scale tiles of one K block for `box_tiles` row tiles.  One such load per operand and stage: copies of their own (cp.async.bulk of
-// 2 KB) take several times as long and hold the operand ring up.
+// scale tiles of one K block for `box_tiles` row tiles: one load per operand and stage, on any barrier of a CTA pair.
 inline cudaError_t encode_sf_tmap(CUtensorMap* out, const void* base, uint64_t row_tiles, uint64_t col_tiles, uint32_t atoms, uint32_t box_tiles = 1) {
   return encode_tmap(out, base, 4, 128, col_tiles, 512, 128, atoms, 0, row_tiles, col_tiles * 512, box_tiles);
 }

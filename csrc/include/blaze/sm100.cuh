@@ -275,8 +275,8 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 // ------------------------------------------------------------------------------------------ CTA pairs
-// One MMA over the two CTAs of a cluster of two: 256 rows of the lane operand (128 in each CTA's shared memory), the column operand's
-// rows half in each; every CTA gets its 128 lanes of the accumulator.  Issued by the CTA of rank 0 alone, for both: shared and tensor
+// One MMA over two neighbouring CTAs of a cluster (ranks 2 i and 2 i + 1): 256 rows of the lane operand (128 in each CTA's shared memory), the column operand's
+// rows half in each; every CTA gets its 128 lanes of the accumulator.  Issued by the CTA of even rank alone, for both: shared and tensor
 // memory hold the same things at the same addresses in both CTAs.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
@@ -308,10 +308,10 @@ __device__ __forceinline__ void mma_mxf8_pair(uint32_t d_tmem, uint64_t a, uint6
       ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(sfa), "r"(sfb), "r"(acc)
       : "memory");
 }
-// All previously issued pair MMAs of this thread arrive on the barrier at this offset in both CTAs when they complete.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
+// All previously issued pair MMAs of this thread arrive on the barrier at this offset in both CTAs (of ranks lead, lead + 1) when they complete.
+__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint32_t lead) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((uint16_t)3)
+               ::"r"(smem_u32(bar)), "h"((uint16_t)(3u << lead))
                : "memory");
 }
 // Scale-factor atoms of both CTAs, each from its own shared into its own tensor memory.

@@ -10,6 +10,9 @@
 // 48 (NVFP4) or 12 columns of tensor memory (copied anew for every stage: copies and MMAs of one issuer run in order), so at 256
 // columns the two accumulators share as many: the epilogue reads the shared ones first, and the next tile waits for those alone.
 //
+// Few tiles and a long K: a cluster of up to four pairs shares a tile's K, and the CTAs of one rank exchange their partial sums through
+// distributed shared memory (each owns some columns and adds the parts up in the pairs' order, so results do not depend on timing).
+//
 // Few tokens: tiles of 64 or 128 columns take less of a stage, so that up to ten stages are in flight, which is what a weight that is read
 // once needs (NVFP4 x 4096 x 4096, 64 rows 12.7 -> 9.1 us).  Experts (GROUPED): a tile is a run of one expert's routed rows.
 //
@@ -51,6 +54,7 @@ struct PairParams {
   const __nv_bfloat16* bias;  // per feature, or null
   int sf_col_tiles;           // 4-column scale tiles per 128-row tile
   int cn;                     // columns (tokens) of a tile
+  int ks;                     // pairs that share a tile's K (split kernel), else 1
   int acc1;                   // first tensor-memory column of the second accumulator
   const int4* heads;          // experts (grouped kernel): [0].x = number of tiles, then {first row, live rows, expert, 0} of each
   int act;                    // 1, 2: rows of W are [16 gate | 16 up] groups; C = gated activation, bf16 [tokens, N/2]
@@ -79,7 +83,7 @@ struct PairCfg {
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 512 + 2 * 256 * 4;
   static constexpr int EPI = 12;                            // epilogue warps
   static constexpr int THREADS = 64 + EPI * 32;
-  static_assert((2 * STAGES + 7) * 8 + 8 <= 512 && STAGES <= 32 && SMEM <= 227 * 1024, "shared memory");
+  static_assert((2 * STAGES + 9) * 8 + 8 <= 512 && STAGES <= 32 && SMEM <= 227 * 1024, "shared memory");
   static_assert(SF_COLS <= 64, "the accumulators may share two chunks of 32 columns at most");
 };
 
@@ -102,12 +106,15 @@ struct PairTile {
   int wbase;     // first row of W of the tile's expert (0 for one weight)
 };
 
-template <int KIND, int CN, bool GROUPED>
+// MODE: one weight, the routed rows of several experts, or one weight with K split over the pairs of a cluster.
+enum { kPairDense = 0, kPairExperts = 1, kPairSplit = 2 };
+template <int KIND, int CN, int MODE>
 __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                                                             const __grid_constant__ CUtensorMap tmSW, const __grid_constant__ CUtensorMap tmSX,
                                                             const PairParams p) {
   using Cfg = PairCfg<KIND, CN>;
   constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS;
+  constexpr bool GROUPED = MODE == kPairExperts, SPLIT = MODE == kPairSplit;
   pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   // both CTAs of a pair round the same way: dynamic shared memory starts at the same offset in each
@@ -122,20 +129,26 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
   uint64_t* acc_early = acc_full + 2;       // [2] an accumulator has been read as far as the two overlap
   uint64_t* acc_free = acc_early + 2;       // [2] and altogether
   uint64_t* drain = acc_free + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  uint64_t* ring_free = drain + 1;          // every CTA of the split is done with its operands (its ring may be written)
+  uint64_t* part_ready = ring_free + 1;     // and has handed out its partial sums
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part_ready + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* s_rs = reinterpret_cast<float*>(full + 64);        // [2][256] row scales of a tile's tokens (after 512 bytes of barriers)
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // warp-uniform to the compiler
-  const uint32_t rank = cluster_ctarank();
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_ctarank(), rank = crank & 1, lead = crank & ~1u;       // lead: the pair's first CTA
+  const int ks = SPLIT ? p.ks : 1, kp = SPLIT ? (int)(crank >> 1) : 0;                   // this pair's share of K
+  const int pair = blockIdx.x / (2 * ks), pairs = gridDim.x / (2 * ks);
   const int tiles_f = (p.N + 255) / 256;
   const int k_tiles = (p.K + BK - 1) / BK;
+  const int kb0 = kp * k_tiles / ks, kb1 = (kp + 1) * k_tiles / ks;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_early[i], 2 * Cfg::EPI); mbar_init(&acc_free[i], 2 * Cfg::EPI); }
     mbar_init(drain, 1);
+    mbar_init(ring_free, ks);
+    mbar_init(part_ready, ks);
     *abort_flag = 0;
     mbar_fence_init();
     prefetch_tmap(&tmW);
@@ -193,9 +206,9 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
         next = tile_at(u + pairs);
         const int frow = t.frow + (int)rank * 128, trow = t.t0 + (int)rank * (t.cn >> 1);
         const int groups = t.cn > 128 ? 2 : 1;      // tiles of 64 and 192 may start in the middle of a scale tile, but not end past the second
-        for (int kt = 0; kt < k_tiles; ++kt) {
+        for (int kt = kb0; kt < kb1; ++kt) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) { ok = false; break; }
-          const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
+          const uint32_t bar = mapa_shared(smem_u32(&full[s]), lead);
           if (rank == 0) mbar_expect_tx(&full[s], 2u * (Cfg::A_BYTES + (uint32_t)t.cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
           const int kc = KIND == 0 ? kt * BK : kt * 128;
           tma_load_2d_pair(sA + s * Cfg::A_BYTES, &tmW, kc, frow, bar);
@@ -246,7 +259,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
         tc_fence_after();
         const uint32_t d = tmem + (b ? p.acc1 : 0);
         const uint32_t sfa = tmem + Cfg::SF_COL0, sfb = sfa + ATOMS * 4, sfb0 = sfb + ((t.t0 & 127) >> 5);
-        for (int kt = 0; kt < k_tiles; ++kt) {
+        for (int kt = kb0; kt < kb1; ++kt) {
           if (!mbar_wait(&full[s], ph, abort_flag, p.status)) { ok = false; break; }
           tc_fence_after();
           const int nblk = min(4, (p.K - kt * BK + Cfg::KMMA - 1) / Cfg::KMMA);
@@ -268,22 +281,22 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
             for (int j = 0; j < 4; ++j) {
               if (j < nblk) {
                 const uint64_t da = desc(a_lo + j * 2, OP_HI), db = desc(b_lo + j * 2, OP_HI);
-                const uint32_t acc = (kt > 0 || j > 0) ? 1u : 0u;
+                const uint32_t acc = (kt > kb0 || j > 0) ? 1u : 0u;
                 if constexpr (KIND == 0) mma_f16_pair(d, da, db, idesc, acc);
                 else if constexpr (KIND == 1) mma_nvfp4_pair(d, da, db, idesc, sfa + j * 4, sfb0 + j * 8, acc);
                 else mma_mxf8_pair(d, da, db, idesc | make_idesc_bs(0, 0, 0, 0, 0, j, j), sfa, sfb0, acc);
               }
             }
-            mma_commit_pair(&empty[s]);
+            mma_commit_pair(&empty[s], lead);
           }
           __syncwarp();
           if (++s == STAGES) { s = 0; ph ^= 1; }
         }
-        if (ok && leader) mma_commit_pair(&acc_full[it & 1]);
+        if (ok && leader) mma_commit_pair(&acc_full[it & 1], lead);
         __syncwarp();
       }
       if (!ok && leader) {                  // the MMAs in flight end before their operands' memory goes
-        mma_commit_pair(drain);
+        mma_commit_pair(drain, lead);
         mbar_drain(drain, 0);
       }
     }
@@ -306,43 +319,21 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
       const bool feat_ok = feat < p.N;
       const float al = (p.alpha && feat_ok) ? __ldg(p.alpha + t.frow + fl) : 1.0f;
       const float bs = (p.bias && feat_ok) ? bf2f(p.bias[feat]) : 0.0f;
-      // the row scales are complete, and the warps agree on whether a wait ran out, so that none is left at a barrier
-      if (!bar_red_and(1, Cfg::EPI * 32, ok)) break;
-      ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, p.status);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) continue;
-      tc_fence_after();
-      // chunks of 32 columns, a round of one per warp at a time, the end that the accumulators share first
-      constexpr int PARTS = Cfg::EPI / 4;
-      const int chunks = cn >> 5, rounds = (chunks + PARTS - 1) / PARTS;
-      for (int i = 0; i < rounds; ++i) {
-        const int ch = b ? i * PARTS + part : chunks - 1 - i * PARTS - part;
-        const bool mine = ch >= 0 && ch < chunks;
-        const int c = ch * 32;
-        uint32_t r[32];
-        if (mine) {
-          tmem_ld32(tmem + (b ? p.acc1 : 0) + c + quad, r);
-          tmem_ld_wait();
-        }
-        if (i == 0 || i == rounds - 1) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0 && i == 0) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_early[b]), 0));
-          if (lane == 0 && i == rounds - 1) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_free[b]), 0));
-        }
-        if (!mine) break;
-        float v[32];
+      // sums of the columns [c, c + NC) of the tile, as they come from tensor memory: scales, bias, activation, store
+      auto finish = [&](const auto& r, int c) {
+        constexpr int NC = sizeof(r) / sizeof(r[0]);
+        const int tc = t0 + c;              // token of the first column
+        float v[NC];
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
+        for (int j = 0; j < NC; j += 4) {
           const float4 s4 = *reinterpret_cast<const float4*>(rs + c + j);
           scale_pair(r[j], r[j + 1], s4.x, s4.y, al, bs, v[j], v[j + 1]);
           scale_pair(r[j + 2], r[j + 3], s4.z, s4.w, al, bs, v[j + 2], v[j + 3]);
         }
-        const int tc = t0 + c;              // token of the chunk's first column
         if (p.out_f32) {
           float* C = reinterpret_cast<float*>(p.C) + feat;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
+          for (int j = 0; j < NC; ++j)
             if (feat_ok && tc + j < t.end) C[(size_t)(tc + j) * p.ldc] = v[j];
         } else if (p.act) {
           // lanes 0-15 hold the gates and 16-31 the up values of 16 features: one exchange gives the lower lanes a token and the upper
@@ -352,7 +343,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
           const size_t step = (size_t)p.ldc * 4;
           auto gated = [&](auto act) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
+            for (int j = 0; j < NC; j += 4) {
               float a[2];
 #pragma unroll
               for (int k = 0; k < 2; ++k) {
@@ -380,12 +371,86 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
           __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)first * p.ldc + (feat & ~1);
           const size_t step = (size_t)p.ldc * 2;
 #pragma unroll
-          for (int j = 0; j < 32; j += 2) {
+          for (int j = 0; j < NC; j += 2) {
             const uint32_t own = pack_bf16x2(v[j], v[j + 1]);
             const uint32_t two = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), pick);
             if (j < left) *reinterpret_cast<uint32_t*>(C) = two;
             C += step;
           }
+        }
+      };
+      // the row scales are complete, and the warps agree on whether a wait ran out, so that none is left at a barrier
+      if (!bar_red_and(1, Cfg::EPI * 32, ok)) break;
+      ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, p.status);
+      ok = __all_sync(0xffffffffu, ok);
+      constexpr int PARTS = Cfg::EPI / 4;
+      if constexpr (SPLIT) {
+        // The CTAs of one rank exchange their partial sums: of the tile's groups of 16 columns pair i owns [i * ng / ks, (i + 1) * ng /
+        // ks), whose sums all pairs push into its ring (free once all are done with theirs), slot [source][group][quad of columns]
+        // [feature]; it adds them up in the pairs' order.  A CTA whose wait ran out still arrives, so that none waits for it.
+        const int ng = cn >> 4, most = (ng + ks - 1) / ks, f = q * 32 + lane;
+        if (etid == 0)
+          for (int i = 0; i < ks; ++i) mbar_arrive_remote(mapa_shared(smem_u32(ring_free), 2 * i + rank));
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(ring_free, 0, abort_flag, p.status)) && ok;
+        if (ok) {
+          tc_fence_after();
+          for (int ch = part; ch < cn >> 5; ch += PARTS) {
+            uint32_t r[32];
+            tmem_ld32(tmem + ch * 32 + quad, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int g = ch * 2 + h, owner = (g * ks + ks - 1) / ng, gl = g - owner * ng / ks;
+              const uint32_t dst = mapa_shared(smem_u32(base) + (uint32_t)(((kp * most + gl) * 4 * 128 + f) * 16), 2 * owner + rank);
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                st_dsmem_f4(dst + k * 2048, __uint_as_float(r[h * 16 + k * 4]), __uint_as_float(r[h * 16 + k * 4 + 1]),
+                            __uint_as_float(r[h * 16 + k * 4 + 2]), __uint_as_float(r[h * 16 + k * 4 + 3]));
+            }
+          }
+        }
+        fence_acq_rel_cluster();
+        bar_sync(2, Cfg::EPI * 32);
+        if (etid == 0)
+          for (int i = 0; i < ks; ++i) mbar_arrive_remote(mapa_shared(smem_u32(part_ready), 2 * i + rank));
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(part_ready, 0, abort_flag, p.status)) && ok;
+        if (!ok || *abort_flag) break;
+        const int g0 = kp * ng / ks, g1 = (kp + 1) * ng / ks;
+        for (int g = g0 + part; g < g1; g += PARTS) {
+          uint32_t r[16];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int i = 0; i < ks; ++i) {
+              const float4 v = reinterpret_cast<const float4*>(base)[((i * most + g - g0) * 4 + k) * 128 + f];
+              a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+            }
+            r[4 * k] = __float_as_uint(a.x); r[4 * k + 1] = __float_as_uint(a.y);
+            r[4 * k + 2] = __float_as_uint(a.z); r[4 * k + 3] = __float_as_uint(a.w);
+          }
+          finish(r, g * 16);
+        }
+      } else {
+        if (!ok) continue;
+        tc_fence_after();
+        // chunks of 32 columns, a round of one per warp at a time, the end that the accumulators share first
+        const int chunks = cn >> 5, rounds = (chunks + PARTS - 1) / PARTS;
+        for (int i = 0; i < rounds; ++i) {
+          const int ch = b ? i * PARTS + part : chunks - 1 - i * PARTS - part;
+          const bool mine = ch >= 0 && ch < chunks;
+          uint32_t r[32];
+          if (mine) {
+            tmem_ld32(tmem + (b ? p.acc1 : 0) + ch * 32 + quad, r);
+            tmem_ld_wait();
+          }
+          if (i == 0 || i == rounds - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0 && i == 0) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_early[b]), lead));
+            if (lane == 0 && i == rounds - 1) mbar_arrive_remote_tmem(mapa_shared(smem_u32(&acc_free[b]), lead));
+          }
+          if (!mine) break;
+          finish(r, ch * 32);
         }
       }
     }
@@ -400,17 +465,18 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
   }
 }
 
-template <int KIND, int CN, bool GROUPED>
+template <int KIND, int CN, int MODE>
 static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW, const CUtensorMap& tmSX,
                                const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
   using Cfg = PairCfg<KIND, CN>;
-  auto kern = gemm_pair_kernel<KIND, CN, GROUPED>;
+  auto kern = gemm_pair_kernel<KIND, CN, MODE>;
   static PerDeviceOnce configured;
   cudaError_t e = configured.smem_limit(kern, Cfg::SMEM);
   if (e != cudaSuccess) return e;
   int pairs = sm_count() / 2;
   if (max_ctas > 1 && pairs > max_ctas / 2) pairs = max_ctas / 2;
-  if (!GROUPED && pairs > tiles) pairs = tiles;          // the experts' tiles are counted on the device
+  if (MODE != kPairExperts && pairs > tiles) pairs = tiles;          // the experts' tiles are counted on the device
+  if (MODE == kPairSplit) pairs = tiles * p.ks;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(pairs * 2));
   cfg.blockDim = dim3(Cfg::THREADS);
@@ -418,7 +484,7 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = 2 * p.ks;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   // The set-up (barriers, tensor memory, tensor maps, cluster) runs while the kernel before this one ends; nothing is read before
@@ -432,11 +498,11 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
 }
 
-template <bool GROUPED>
+template <int MODE>
 static cudaError_t launch_pair_kind(int kind, int most, const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW,
                                     const CUtensorMap& tmSX, const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
 #define BLZ_PAIR_CASE(KD, CN) \
-  if (kind == KD && most <= CN) return launch_pair<KD, CN, GROUPED>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  if (kind == KD && most <= CN) return launch_pair<KD, CN, MODE>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
   BLZ_PAIR_CASE(0, 64) BLZ_PAIR_CASE(0, 128) BLZ_PAIR_CASE(0, 256)
   BLZ_PAIR_CASE(1, 64) BLZ_PAIR_CASE(1, 128) BLZ_PAIR_CASE(1, 256)
   BLZ_PAIR_CASE(2, 64) BLZ_PAIR_CASE(2, 128) BLZ_PAIR_CASE(2, 256)
@@ -446,7 +512,7 @@ static cudaError_t launch_pair_kind(int kind, int most, const CUtensorMap& tmW, 
 
 static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, const float* row_scale, const float* alpha, int act, float act_limit) {
   PairParams p = {};
-  p.N = N; p.K = K; p.C = C; p.ldc = ldc;
+  p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.ks = 1;
   p.row_scale = row_scale; p.alpha = alpha;
   p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
   p.acc1 = (kind == 0 ? PairCfg<0, 256>::SF_COL0 : kind == 1 ? PairCfg<1, 256>::SF_COL0 : PairCfg<2, 256>::SF_COL0) - 256;
@@ -455,43 +521,81 @@ static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, co
   return p;
 }
 
-}  // namespace blz
-
-// Columns of a tile: the multiple of 64 with the least rounds x time of a round.  Nanoseconds per K block measured at 8192 x 4096 x 12288
-// (NVFP4 and bf16; more columns than the MMAs of a block can hide behind its bytes and its issue cost little), and about a microsecond per tile
-// for the accumulators' hand-over.
-BLZ_API int blz_gemm_pair_columns(int kind, int M, int N, int K, int sms) {
-  static const int scaled[] = {294, 313, 338, 387}, plain[] = {237, 255, 296, 385};
-  const int tiles_f = (N + 255) / 256, pairs = sms / 2 > 0 ? sms / 2 : 1;
-  const int k_tiles = (K + (kind == 0 ? 63 : kind == 1 ? 255 : 127)) / (kind == 0 ? 64 : kind == 1 ? 256 : 128);
-  int best = 256;
-  long best_cost = 1L << 60;
-  for (int cn = 256; cn >= 64; cn -= 64) {
-    const long tiles = (long)tiles_f * ((M + cn - 1) / cn);
-    const long cost = ((tiles + pairs - 1) / pairs) * ((long)k_tiles * (kind ? scaled : plain)[cn / 64 - 1] + 1000);
-    if (cost < best_cost) { best_cost = cost; best = cn; }
-  }
-  return best;
+// Clusters of `ctas` CTAs that run at the same time on the current device (whole within a GPC each; one CTA fits an SM, whatever the kind).
+static int cluster_room(int ctas) {
+  static int cache[64][9] = {{0}};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || ctas < 2 || ctas > 8) return 0;
+  if (cache[dev][ctas]) return cache[dev][ctas];
+  auto kern = gemm_pair_kernel<1, 64, kPairSplit>;
+  static PerDeviceOnce configured;
+  if (configured.smem_limit(kern, PairCfg<1, 64>::SMEM) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ctas * sm_count()));
+  cfg.blockDim = dim3(PairCfg<1, 64>::THREADS);
+  cfg.dynamicSmemBytes = PairCfg<1, 64>::SMEM;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)ctas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) n = 1;
+  return cache[dev][ctas] = n;
 }
 
+// Columns of a tile (a multiple of 64) and pairs that share its K: the least rounds x time of a round.  Nanoseconds per K block measured at
+// 8192 x 4096 x 12288 (NVFP4 and bf16; more columns than the MMAs of a block can hide behind its bytes and its issue cost little), a
+// microsecond per tile for the accumulators' hand-over, and some four for the exchange of a split, which only pays where all clusters
+// run at once: us of one pair per tile / of the split chosen here, 64 rows: NVFP4 4096 x 12288 17.3 / 14.3 (3 pairs; over a cluster
+// of single CTAs 20), 4096 x 4096 8.2 / 9.6 (not chosen), bf16 4096 x 12288 43 / 31, 4096 x 4096 17.4 / 15, MXFP8 2048 x 4096 12.9 /
+// 10.6; 16 tiles of 4 pairs do not fit the chip at once: 24.9.
+static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
+  static const int scaled[] = {294, 313, 338, 387}, plain[] = {237, 255, 296, 385};
+  const int tiles_f = (N + 255) / 256, sms = sm_count(), pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const int k_tiles = (K + (kind == 0 ? 63 : kind == 1 ? 255 : 127)) / (kind == 0 ? 64 : kind == 1 ? 256 : 128);
+  long best = 1L << 60;
+  int best_cn = 256, best_ks = 1;
+  for (int c = 256; c >= 64; c -= 64) {
+    if (*cn && c != *cn) continue;
+    const long tiles = (long)tiles_f * ((M + c - 1) / c);
+    const long block = (kind ? scaled : plain)[c / 64 - 1];
+    for (int k = 1; k <= 4 && k <= k_tiles; ++k) {
+      if (*ks && k != *ks) continue;
+      if (k > 1 && !*ks && (tiles * k > pairs || tiles > cluster_room(2 * k))) continue;
+      const long cost = k == 1 ? ((tiles + pairs - 1) / pairs) * (k_tiles * block + 1000) : (k_tiles + k - 1) / k * block + 5000 + 10 * c;
+      if (cost < best) { best = cost; best_cn = c; best_ks = k; }
+    }
+  }
+  *cn = best_cn;
+  *ks = best_ks;
+}
+
+}  // namespace blz
+
 // C[M, N] = X[M, K] · W[N, K]^T with the operand conventions of blz_gemm_tc (ldx / ldw in BYTES, ldc in elements).  kind: 0 bf16,
-// 1 NVFP4, 2 MXFP8.  N even, or a multiple of 32 with act (bf16 out, [M, N/2]).  cn: tokens per tile, 64 / 128 / 192 / 256, or 0 to choose.
+// 1 NVFP4, 2 MXFP8.  N even, or a multiple of 32 with act (bf16 out, [M, N/2]).  cn: tokens per tile, 64 / 128 / 192 / 256, and
+// ks: pairs that share a tile's K, 1 - 4 (at most one per K block); 0 to choose.
 BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N,
                           int K, const float* row_scale, const float* alpha, const void* bias, const void* sfx, const void* sfw,
-                          int out_f32, int cn, int max_ctas, int act, float act_limit, cudaStream_t stream) {
+                          int out_f32, int cn, int ks, int max_ctas, int act, float act_limit, cudaStream_t stream) {
   using namespace blz;
   // this kernel has no fused all-reduce / peer-wait / arg-max epilogue: a call armed for one is refused (and disarmed)
   if (gemm_oneshot_take_unsupported()) return (int)cudaErrorNotSupported;
-  if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || cn < 0 || cn > 256 || cn % 64) return (int)cudaErrorInvalidValue;
+  if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || cn < 0 || cn > 256 || cn % 64 || ks < 0 || ks > 4) return (int)cudaErrorInvalidValue;
   const int kmma = kind == 0 ? 16 : kind == 1 ? 64 : 32;
-  if (K % kmma) return (int)cudaErrorInvalidValue;
+  if (K % kmma || ks > (K + 4 * kmma - 1) / (4 * kmma)) return (int)cudaErrorInvalidValue;
   if (kind && (!sfx || !sfw)) return (int)cudaErrorInvalidValue;
   if (act < 0 || act > 2 || (act && (out_f32 || N % 32))) return (int)cudaErrorInvalidValue;
   if (!out_f32 && ((N & 1) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3))) return (int)cudaErrorInvalidValue;
   PairParams p = pair_params(kind, N, K, C, ldc, row_scale, alpha, act, act_limit);
   p.M = M; p.out_f32 = out_f32;
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
-  p.cn = cn ? cn : blz_gemm_pair_columns(kind, M, N, K, sm_count());
+  if (max_ctas > 0) ks = 1;                  // a split is one round of clusters
+  pair_shape(kind, M, N, K, &cn, &ks);
+  p.cn = cn; p.ks = ks;
   p.acc1 = p.acc1 + 256 - p.cn < 256 ? p.acc1 + 256 - p.cn : 256;               // narrower tiles overlap less
   CUtensorMap tmW, tmX, tmSW, tmSX;
   const int es = kind == 0 ? 2 : 1;                                   // bytes per tensor-map element
@@ -509,7 +613,8 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
     if (e != cudaSuccess) return (int)e;
   }
   const int tiles = ((N + 255) / 256) * ((M + p.cn - 1) / p.cn);
-  return (int)launch_pair_kind<false>(kind, p.cn, tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  if (p.ks > 1) return (int)launch_pair_kind<kPairSplit>(kind, p.cn, tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
+  return (int)launch_pair_kind<kPairDense>(kind, p.cn, tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
 }
 
 // The routed rows of `experts` experts: X and C are in the padded row space of moe.cu (row_tiles x 128 rows), `heads` comes from
@@ -536,5 +641,5 @@ BLZ_API int blz_gemm_pair_experts(int kind, const void* X, long long ldx, const 
   if (e == cudaSuccess && kind) e = encode_sf_tmap(&tmSW, sfw, (uint64_t)experts * N / 128, p.sf_col_tiles, atoms);
   if (e == cudaSuccess && kind) e = encode_sf_tmap(&tmSX, sfx, row_tiles, p.sf_col_tiles, atoms);
   if (e != cudaSuccess) return (int)e;
-  return (int)launch_pair_kind<true>(kind, run, tmW, tmX, tmSW, tmSX, p, 0, 0, stream);
+  return (int)launch_pair_kind<kPairExperts>(kind, run, tmW, tmX, tmSW, tmSX, p, 0, 0, stream);
 }
