@@ -89,6 +89,9 @@ class CudaOps:
         lib.blz_gemm_fp8_block.restype = _c.c_int
         lib.blz_gemm_fp8_block.argtypes = [VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
                                            VP, _c.c_longlong, VP, VP, _c.c_int, VP]
+        lib.blz_gemm_fp8_pair.restype = _c.c_int
+        lib.blz_gemm_fp8_pair.argtypes = [VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
+                                          VP, _c.c_longlong, VP, VP, _c.c_int, _c.c_int, _c.c_int, VP]
         lib.blz_quant_fp8_block.restype = _c.c_int
         lib.blz_quant_fp8_block.argtypes = [VP, _c.c_longlong, VP, VP, _c.c_longlong, _c.c_int, _c.c_int, VP]
         # FP8 checkpoints with 128x128 fp32 block scales: "exact" keeps the stored codes and scales and promotes every K block

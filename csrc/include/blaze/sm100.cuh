@@ -292,6 +292,13 @@ __device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a, uint64
       ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
+__device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      : "memory");
+}
 __device__ __forceinline__ void mma_nvfp4_pair(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                                uint32_t acc) {
   asm volatile(
@@ -417,6 +424,15 @@ __device__ __forceinline__ bool bar_red_and(int id, int threads, bool pred) {
   asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.and.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}"
                : "=r"(out) : "r"((uint32_t)pred), "r"(id), "r"(threads) : "memory");
   return out != 0;
+}
+
+// y += x * (s * w) of two neighbours at once, each rounded as by fmaf(x, s * w, y)
+__device__ __forceinline__ void fma_scaled_pair(float& y0, float& y1, uint32_t x0, uint32_t x1, float s0, float s1, float w) {
+  asm("{\n\t.reg .b64 x, s, w, y;\n\t"
+      "mov.b64 x, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\tmov.b64 w, {%6, %6};\n\tmov.b64 y, {%0, %1};\n\t"
+      "mul.rn.f32x2 s, s, w;\n\tfma.rn.f32x2 y, x, s, y;\n\tmov.b64 {%0, %1}, y;\n\t}\n"
+      : "+f"(y0), "+f"(y1)
+      : "r"(x0), "r"(x1), "f"(s0), "f"(s1), "f"(w));
 }
 
 __device__ __forceinline__ float bf2f(__nv_bfloat16 v) { return __bfloat162float(v); }

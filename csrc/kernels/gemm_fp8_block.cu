@@ -15,6 +15,8 @@
 // warp per scheduler the tensor pipe sat at 32 % and the FMA pipe at 19 %).  Every wait is a bounded mbarrier wait that
 // reports through the status word.  No TMA load is cluster-multicast.
 //
+// Both kernels here are what calls take that gemm_fp8_pair.cu does not (see blz_gemm_fp8_block).
+//
 // Reference counterpart: the FP8 block-scale linear of kernels/src/cuda/fp8_linear.cu (fp8_block_* kernels: dequantise to
 // bf16 and run a bf16 GEMM, or 1x128-quantised activations with per-block fp32 rescale on mma.sync), routed from
 // crates/blaze/src/linear.rs (Fp8Block variants).
@@ -22,6 +24,10 @@
 #include "blaze/sm100.cuh"
 
 namespace blz {
+
+cudaError_t gemm_fp8_pair(const void* A, long long lda, const void* B, long long ldb, void* C, long long ldc, int M, int N, int K,
+                          const float* sa, long long ld_sa, const float* sb, const void* bias, int out_f32, int cn, int ks, cudaStream_t stream);   // gemm_fp8_pair.cu
+int pair_cluster_room(int ctas);           // gemm_pair.cu
 
 struct FbParams {
   int M, N, K;
@@ -527,12 +533,16 @@ BLZ_API int blz_gemm_fp8_block(const void* A, long long lda, const void* B, long
                                cudaStream_t stream) {
   using namespace blz;
   if (M <= 0 || N <= 0 || K <= 0 || K % 128 || !sa || !sb || ld_sa < M) return (int)cudaErrorInvalidValue;
+  // The pairs' kernel is the faster one at any size; it fetches the token scales by a tensor map, which start and step on 16 bytes
+  // (blz_quant_fp8_block's do), and needs a context with room for two neighbouring CTAs.
+  const bool on16 = ld_sa % 4 == 0 && (reinterpret_cast<uintptr_t>(sa) & 15) == 0;
+  if (on16 && pair_cluster_room(2) > 0)
+    return (int)gemm_fp8_pair(A, lda, B, ldb, C, ldc, M, N, K, sa, ld_sa, sb, bias, out_f32, 0, 0, stream);
   FbParams p;
   p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.out_f32 = out_f32;
   p.sa = sa; p.ld_sa = ld_sa; p.sb = sb; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias);
   p.status = status_word();
-  // the scales' rows are copied by 16 bytes: they start and step on them (blz_quant_fp8_block's do)
-  if (M <= 64 && ld_sa % 4 == 0 && (reinterpret_cast<uintptr_t>(sa) & 15) == 0) {
+  if (M <= 64 && on16) {                     // the scales' rows are copied by 16 bytes
     const int ks = fp8_rows_ks(p);
     if (ks > 0) return (int)launch_fp8_rows(p, ks, A, lda, B, ldb, stream);
   }

@@ -522,12 +522,12 @@ static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, co
 }
 
 // Clusters of `ctas` CTAs that run at the same time on the current device (whole within a GPC each; one CTA fits an SM, whatever the kind).
-static int cluster_room(int ctas) {
+int pair_cluster_room(int ctas) {
   static int cache[64][9] = {{0}};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || ctas < 2 || ctas > 8) return 0;
-  if (cache[dev][ctas]) return cache[dev][ctas];
+  if (cache[dev][ctas]) return cache[dev][ctas] - 1;
   auto kern = gemm_pair_kernel<1, 64, kPairSplit>;
   static PerDeviceOnce configured;
   if (configured.smem_limit(kern, PairCfg<1, 64>::SMEM) != cudaSuccess) return 0;
@@ -542,8 +542,9 @@ static int cluster_room(int ctas) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) n = 1;
-  return cache[dev][ctas] = n;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) return 0;
+  cache[dev][ctas] = n + 1;
+  return n;
 }
 
 // Columns of a tile (a multiple of 64) and pairs that share its K: the least rounds x time of a round.  Nanoseconds per K block measured at
@@ -564,7 +565,7 @@ static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
     const long block = (kind ? scaled : plain)[c / 64 - 1];
     for (int k = 1; k <= 4 && k <= k_tiles; ++k) {
       if (*ks && k != *ks) continue;
-      if (k > 1 && !*ks && (tiles * k > pairs || tiles > cluster_room(2 * k))) continue;
+      if (k > 1 && !*ks && (tiles * k > pairs || tiles > pair_cluster_room(2 * k))) continue;
       const long cost = k == 1 ? ((tiles + pairs - 1) / pairs) * (k_tiles * block + 1000) : (k_tiles + k - 1) / k * block + 5000 + 10 * c;
       if (cost < best) { best = cost; best_cn = c; best_ks = k; }
     }

@@ -495,3 +495,33 @@ def test_experts_with_the_activation_in_the_product(ops, fmt, T, E, k, H, I):   
     for o in outs:
         assert _rel(o, outs[0]) < 2e-3             # one may round a sum to the neighbouring bf16
         assert _rel(o, ref.moe_forward(x, w, ids, ex.forward_one, E)) < 0.08
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (64, 200, 384), (65, 131, 256), (129, 640, 1152), (300, 1000, 640), (20000, 384, 256)])
+def test_fp8_block_product_on_cta_pairs(ops, M, N, K):      # noqa: F811
+    """Both tile widths, K whole and split over 2 to 4 pairs, odd numbers of blocks, features that are no whole tiles: against the kernel of
+    one CTA per tile, which adds the blocks in the same order, so the same bits where K is not split."""
+    from blaze_b200.ops.cuda_ops import VP, _ptr
+    g = torch.Generator(device=DEV).manual_seed(12)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    lin = Linear.from_dense(torch.randn(N, K, generator=g, device=DEV) * 0.02, Format.FP8_BLOCK)
+    lin.bias = torch.randn(N, generator=g, device=DEV).bfloat16()
+    pk = ops.pack(lin)
+    q, sc = ops.quantize_fp8_block(x)
+    odd = torch.zeros(K // 128, M + 1 - M % 2, dtype=torch.float32, device=DEV)        # rows off 16 bytes: the other kernel
+    odd[:, :M] = sc[:, :M]
+    for dt in (torch.float32, torch.bfloat16):
+        want, out = torch.empty(M, N, dtype=dt, device=DEV), torch.empty(M, N, dtype=dt, device=DEV)
+        shape = (_ptr(q), K, _ptr(pk["w"]), K)
+        rest = (_ptr(pk["sf"]), _ptr(pk["bias"]), int(dt == torch.float32))
+        assert ops.lib.blz_gemm_fp8_block(*shape, _ptr(want), N, M, N, K, _ptr(odd), odd.stride(0), *rest, VP(0)) == 0
+        for cn in (64, 128):
+            for ks in range(1, min(4, (K + 255) // 256) + 1):
+                if ks > 1 and M > 1000:
+                    continue
+                out.fill_(float("nan"))
+                assert ops.lib.blz_gemm_fp8_pair(*shape, _ptr(out), N, M, N, K, _ptr(sc), sc.stride(0), *rest, cn, ks, VP(0)) == 0
+                torch.cuda.synchronize()
+                assert ops.take_status() == 0
+                # parts of K add in another order: up to 2^-24 of the terms' size per addition
+                assert torch.equal(out, want) if ks == 1 else _rel(out, want) < (1e-6 if dt == torch.float32 else 2e-3), (cn, ks)
