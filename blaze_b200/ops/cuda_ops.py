@@ -1470,14 +1470,14 @@ class CudaOps:
         tile_rows = torch.empty(max_tiles, dtype=torch.int32, device=dev)
         row_map = torch.empty(T, k, dtype=torch.int32, device=dev)
         # rows per tile of the pair kernel by the rows that an expert gets on average: beyond them its weights are read again
-        run = 64 if T * k <= 32 * n_exp else 128 if T * k <= 96 * n_exp else 256
+        run = 128 if T * k <= 96 * n_exp else 256
         runs = (torch.empty(T * k // run + n_exp + 1, 4, dtype=torch.int32, device=dev), run)
         self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(runs[0]), run, n_exp,
                                                max_tiles, self._stream()), "moe_plan")
         narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
         # The pair kernel beats the narrow one for block-scaled experts at any number of rows (us, both products of a layer, narrow / tiles
-        # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 101 / 146 / 94, 4096 277 / 266 / 153; MXFP8, 512
-        # experts of 1024 x 2048, 1 token 43 / 53 / 27, 64 245 / 418 / 238, 1024 322 / 597 / 320, 4096 427 / 585 / 368)
+        # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 102 / 145 / 94, 4096 278 / 264 / 147; MXFP8, 512
+        # experts of 1024 x 2048, 1 token 43 / 51 / 29, 256 313 / 575 / 307, 1024 322 / 580 / 313, 4096 428 / 580 / 352)
         if gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2" and self.MOE_NARROW_ROWS < 1 << 20:
             narrow = False
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)

@@ -67,8 +67,11 @@ template <> struct PKind<0> { static constexpr int KMMA = 16, SF_ATOMS = 0; };
 template <> struct PKind<1> { static constexpr int KMMA = 64, SF_ATOMS = 4; };
 template <> struct PKind<2> { static constexpr int KMMA = 32, SF_ATOMS = 1; };
 
+// MODE: one weight, the routed rows of several experts, or one weight with K split over the pairs of a cluster.
+enum { kPairDense = 0, kPairExperts = 1, kPairSplit = 2 };
+
 // CN: most columns of a tile (64, 128 or 256).  Narrow tiles leave room for more stages: what a weight that is read once needs.
-template <int KIND, int CN>
+template <int KIND, int CN, int MODE>
 struct PairCfg {
   static constexpr int KMMA = PKind<KIND>::KMMA;
   static constexpr int BK = KMMA * 4;                       // 128 bytes of K per row and stage
@@ -76,7 +79,11 @@ struct PairCfg {
   static constexpr int A_BYTES = 128 * 128, B_BYTES = CN * 64;
   static constexpr int GROUPS = CN > 128 ? 2 : 1;           // 128-row scale tiles under a tile's tokens
   static constexpr int SF_BYTES = SF_ATOMS * 512;           // scales of 128 rows and one stage
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + (1 + GROUPS) * SF_BYTES;
+  // K blocks per stage.  Waits and commits cost as much as the products of 64 columns (one / two blocks: NVFP4 64 x 4096 x 12288 17.3 / 15.1
+  // us, MXFP8 64 x 2048 x 4096 12.5 / 10.7); at 128 the stages are worth more (17.6 / 18.4, bf16 45 / 48), but for experts, whose tiles
+  // are mostly not full (512 MXFP8 experts, both products of 256 tokens 314 / 307).
+  static constexpr int UB = CN == 64 || (CN == 128 && MODE == kPairExperts) ? 2 : 1;
+  static constexpr int STAGE_BYTES = UB * (A_BYTES + B_BYTES + (1 + GROUPS) * SF_BYTES);
   static constexpr int STAGES = (216 * 1024) / STAGE_BYTES;
   static constexpr int SF_COLS = SF_ATOMS * 4 * 3;
   static constexpr int SF_COL0 = 512 - SF_COLS;
@@ -106,24 +113,22 @@ struct PairTile {
   int wbase;     // first row of W of the tile's expert (0 for one weight)
 };
 
-// MODE: one weight, the routed rows of several experts, or one weight with K split over the pairs of a cluster.
-enum { kPairDense = 0, kPairExperts = 1, kPairSplit = 2 };
 template <int KIND, int CN, int MODE>
-__global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+__global__ void __launch_bounds__(PairCfg<KIND, CN, MODE>::THREADS, 1) gemm_pair_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
                                                             const __grid_constant__ CUtensorMap tmSW, const __grid_constant__ CUtensorMap tmSX,
                                                             const PairParams p) {
-  using Cfg = PairCfg<KIND, CN>;
-  constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS;
+  using Cfg = PairCfg<KIND, CN, MODE>;
+  constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS, UB = Cfg::UB;
   constexpr bool GROUPED = MODE == kPairExperts, SPLIT = MODE == kPairSplit;
   pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   // both CTAs of a pair round the same way: dynamic shared memory starts at the same offset in each
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sA = base;
-  uint8_t* sB = sA + STAGES * Cfg::A_BYTES;
-  uint8_t* sSFA = sB + STAGES * Cfg::B_BYTES;
-  uint8_t* sSFB = sSFA + STAGES * Cfg::SF_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sSFB + STAGES * Cfg::GROUPS * Cfg::SF_BYTES);
+  uint8_t* sB = sA + STAGES * UB * Cfg::A_BYTES;
+  uint8_t* sSFA = sB + STAGES * UB * Cfg::B_BYTES;
+  uint8_t* sSFB = sSFA + STAGES * UB * Cfg::SF_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(sSFB + STAGES * UB * Cfg::GROUPS * Cfg::SF_BYTES);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;      // [2]
   uint64_t* acc_early = acc_full + 2;       // [2] an accumulator has been read as far as the two overlap
@@ -140,7 +145,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
   const int ks = SPLIT ? p.ks : 1, kp = SPLIT ? (int)(crank >> 1) : 0;                   // this pair's share of K
   const int pair = blockIdx.x / (2 * ks), pairs = gridDim.x / (2 * ks);
   const int tiles_f = (p.N + 255) / 256;
-  const int k_tiles = (p.K + BK - 1) / BK;
+  const int k_tiles = (p.K + BK * UB - 1) / (BK * UB);      // stages along K
   const int kb0 = kp * k_tiles / ks, kb1 = (kp + 1) * k_tiles / ks;
 
   if (threadIdx.x == 0) {
@@ -209,19 +214,22 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
         for (int kt = kb0; kt < kb1; ++kt) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) { ok = false; break; }
           const uint32_t bar = mapa_shared(smem_u32(&full[s]), lead);
-          if (rank == 0) mbar_expect_tx(&full[s], 2u * (Cfg::A_BYTES + (uint32_t)t.cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
-          const int kc = KIND == 0 ? kt * BK : kt * 128;
-          tma_load_2d_pair(sA + s * Cfg::A_BYTES, &tmW, kc, frow, bar);
-          if constexpr (GROUPED) {
-            for (int r = 0; r < t.cn >> 1; r += 32) tma_load_2d_pair(sB + s * Cfg::B_BYTES + r * 128, &tmX, kc, trow + r, bar);
-          } else {
-            tma_load_2d_pair(sB + s * Cfg::B_BYTES, &tmX, kc, trow, bar);
-          }
-          if constexpr (ATOMS > 0) {
-            tma_load_3d_pair(sSFA + s * Cfg::SF_BYTES, &tmSW, 0, kt * ATOMS, frow >> 7, bar);
-            tma_load_3d_pair(sSFB + s * Cfg::GROUPS * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, t.t0 >> 7, bar);
-            if (GROUPED && Cfg::GROUPS == 2 && groups == 2)
-              tma_load_3d_pair(sSFB + (s * 2 + 1) * Cfg::SF_BYTES, &tmSX, 0, kt * ATOMS, (t.t0 >> 7) + 1, bar);
+          if (rank == 0) mbar_expect_tx(&full[s], 2u * UB * (Cfg::A_BYTES + (uint32_t)t.cn * 64u + (uint32_t)(1 + groups) * Cfg::SF_BYTES));
+#pragma unroll
+          for (int h = 0; h < UB; ++h) {         // (a block beyond K is filled with zeros and not used)
+            const int kk = kt * UB + h, kc = KIND == 0 ? kk * BK : kk * 128, sh = s * UB + h;
+            tma_load_2d_pair(sA + sh * Cfg::A_BYTES, &tmW, kc, frow, bar);
+            if constexpr (GROUPED) {
+              for (int r = 0; r < t.cn >> 1; r += 32) tma_load_2d_pair(sB + sh * Cfg::B_BYTES + r * 128, &tmX, kc, trow + r, bar);
+            } else {
+              tma_load_2d_pair(sB + sh * Cfg::B_BYTES, &tmX, kc, trow, bar);
+            }
+            if constexpr (ATOMS > 0) {
+              tma_load_3d_pair(sSFA + sh * Cfg::SF_BYTES, &tmSW, 0, kk * ATOMS, frow >> 7, bar);
+              tma_load_3d_pair(sSFB + sh * Cfg::GROUPS * Cfg::SF_BYTES, &tmSX, 0, kk * ATOMS, t.t0 >> 7, bar);
+              if (GROUPED && Cfg::GROUPS == 2 && groups == 2)
+                tma_load_3d_pair(sSFB + (sh * 2 + 1) * Cfg::SF_BYTES, &tmSX, 0, kk * ATOMS, (t.t0 >> 7) + 1, bar);
+            }
           }
           used |= 1u << s;
           last = (last & ~(1u << s)) | (ph << s);
@@ -262,29 +270,34 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
         for (int kt = kb0; kt < kb1; ++kt) {
           if (!mbar_wait(&full[s], ph, abort_flag, p.status)) { ok = false; break; }
           tc_fence_after();
-          const int nblk = min(4, (p.K - kt * BK + Cfg::KMMA - 1) / Cfg::KMMA);
-          const uint32_t a_lo = a_lo0 + s * (Cfg::A_BYTES >> 4), b_lo = b_lo0 + s * (Cfg::B_BYTES >> 4);
           if (leader) {
-            if constexpr (ATOMS > 0) {
-              const uint32_t sa_lo = sa_lo0 + s * (Cfg::SF_BYTES >> 4), sb_lo = sb_lo0 + s * (Cfg::GROUPS * Cfg::SF_BYTES >> 4);
 #pragma unroll
-              for (int a = 0; a < ATOMS; ++a) {
-                tmem_cp_sf_pair(sfa + a * 4, desc(sa_lo + a * 32, SF_HI));
-                tmem_cp_sf_pair(sfb + a * 8, desc(sb_lo + a * 32, SF_HI));
+            for (int u2 = 0; u2 < UB; ++u2) {
+              const int kk = kt * UB + u2, sh = s * UB + u2;
+              const int nblk = min(4, (p.K - kk * BK + Cfg::KMMA - 1) / Cfg::KMMA);
+              if (nblk <= 0) break;
+              const uint32_t a_lo = a_lo0 + sh * (Cfg::A_BYTES >> 4), b_lo = b_lo0 + sh * (Cfg::B_BYTES >> 4);
+              if constexpr (ATOMS > 0) {
+                const uint32_t sa_lo = sa_lo0 + sh * (Cfg::SF_BYTES >> 4), sb_lo = sb_lo0 + sh * (Cfg::GROUPS * Cfg::SF_BYTES >> 4);
+#pragma unroll
+                for (int a = 0; a < ATOMS; ++a) {
+                  tmem_cp_sf_pair(sfa + a * 4, desc(sa_lo + a * 32, SF_HI));
+                  tmem_cp_sf_pair(sfb + a * 8, desc(sb_lo + a * 32, SF_HI));
+                }
+                if (Cfg::GROUPS == 2 && t.cn > 128) {
+#pragma unroll
+                  for (int a = 0; a < ATOMS; ++a) tmem_cp_sf_pair(sfb + a * 8 + 4, desc(sb_lo + (ATOMS + a) * 32, SF_HI));
+                }
               }
-              if (Cfg::GROUPS == 2 && t.cn > 128) {
 #pragma unroll
-                for (int a = 0; a < ATOMS; ++a) tmem_cp_sf_pair(sfb + a * 8 + 4, desc(sb_lo + (ATOMS + a) * 32, SF_HI));
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (j < nblk) {
-                const uint64_t da = desc(a_lo + j * 2, OP_HI), db = desc(b_lo + j * 2, OP_HI);
-                const uint32_t acc = (kt > kb0 || j > 0) ? 1u : 0u;
-                if constexpr (KIND == 0) mma_f16_pair(d, da, db, idesc, acc);
-                else if constexpr (KIND == 1) mma_nvfp4_pair(d, da, db, idesc, sfa + j * 4, sfb0 + j * 8, acc);
-                else mma_mxf8_pair(d, da, db, idesc | make_idesc_bs(0, 0, 0, 0, 0, j, j), sfa, sfb0, acc);
+              for (int j = 0; j < 4; ++j) {
+                if (j < nblk) {
+                  const uint64_t da = desc(a_lo + j * 2, OP_HI), db = desc(b_lo + j * 2, OP_HI);
+                  const uint32_t acc = (kt > kb0 || u2 > 0 || j > 0) ? 1u : 0u;
+                  if constexpr (KIND == 0) mma_f16_pair(d, da, db, idesc, acc);
+                  else if constexpr (KIND == 1) mma_nvfp4_pair(d, da, db, idesc, sfa + j * 4, sfb0 + j * 8, acc);
+                  else mma_mxf8_pair(d, da, db, idesc | make_idesc_bs(0, 0, 0, 0, 0, j, j), sfa, sfb0, acc);
+                }
               }
             }
             mma_commit_pair(&empty[s], lead);
@@ -468,7 +481,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN>::THREADS, 1) gemm_pair_kerne
 template <int KIND, int CN, int MODE>
 static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, const CUtensorMap& tmSW, const CUtensorMap& tmSX,
                                const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
-  using Cfg = PairCfg<KIND, CN>;
+  using Cfg = PairCfg<KIND, CN, MODE>;
   auto kern = gemm_pair_kernel<KIND, CN, MODE>;
   static PerDeviceOnce configured;
   cudaError_t e = configured.smem_limit(kern, Cfg::SMEM);
@@ -503,9 +516,9 @@ static cudaError_t launch_pair_kind(int kind, int most, const CUtensorMap& tmW, 
                                     const CUtensorMap& tmSX, const PairParams& p, int tiles, int max_ctas, cudaStream_t stream) {
 #define BLZ_PAIR_CASE(KD, CN) \
   if (kind == KD && most <= CN) return launch_pair<KD, CN, MODE>(tmW, tmX, tmSW, tmSX, p, tiles, max_ctas, stream);
-  BLZ_PAIR_CASE(0, 64) BLZ_PAIR_CASE(0, 128) BLZ_PAIR_CASE(0, 256)
-  BLZ_PAIR_CASE(1, 64) BLZ_PAIR_CASE(1, 128) BLZ_PAIR_CASE(1, 256)
-  BLZ_PAIR_CASE(2, 64) BLZ_PAIR_CASE(2, 128) BLZ_PAIR_CASE(2, 256)
+  if constexpr (MODE != kPairExperts) { BLZ_PAIR_CASE(0, 64) BLZ_PAIR_CASE(1, 64) BLZ_PAIR_CASE(2, 64) }
+  BLZ_PAIR_CASE(0, 128) BLZ_PAIR_CASE(1, 128) BLZ_PAIR_CASE(2, 128)
+  BLZ_PAIR_CASE(0, 256) BLZ_PAIR_CASE(1, 256) BLZ_PAIR_CASE(2, 256)
 #undef BLZ_PAIR_CASE
   return cudaErrorInvalidValue;
 }
@@ -515,7 +528,7 @@ static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, co
   p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.ks = 1;
   p.row_scale = row_scale; p.alpha = alpha;
   p.sf_col_tiles = kind == 1 ? (K + 63) / 64 : kind == 2 ? (K + 127) / 128 : 0;
-  p.acc1 = (kind == 0 ? PairCfg<0, 256>::SF_COL0 : kind == 1 ? PairCfg<1, 256>::SF_COL0 : PairCfg<2, 256>::SF_COL0) - 256;
+  p.acc1 = (kind == 0 ? PairCfg<0, 256, kPairDense>::SF_COL0 : kind == 1 ? PairCfg<1, 256, kPairDense>::SF_COL0 : PairCfg<2, 256, kPairDense>::SF_COL0) - 256;
   p.act = act; p.act_limit = act_limit;
   p.status = status_word();
   return p;
@@ -530,11 +543,11 @@ int pair_cluster_room(int ctas) {
   if (cache[dev][ctas]) return cache[dev][ctas] - 1;
   auto kern = gemm_pair_kernel<1, 64, kPairSplit>;
   static PerDeviceOnce configured;
-  if (configured.smem_limit(kern, PairCfg<1, 64>::SMEM) != cudaSuccess) return 0;
+  if (configured.smem_limit(kern, PairCfg<1, 64, kPairSplit>::SMEM) != cudaSuccess) return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ctas * sm_count()));
-  cfg.blockDim = dim3(PairCfg<1, 64>::THREADS);
-  cfg.dynamicSmemBytes = PairCfg<1, 64>::SMEM;
+  cfg.blockDim = dim3(PairCfg<1, 64, kPairSplit>::THREADS);
+  cfg.dynamicSmemBytes = PairCfg<1, 64, kPairSplit>::SMEM;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = (unsigned)ctas;
@@ -548,13 +561,13 @@ int pair_cluster_room(int ctas) {
 }
 
 // Columns of a tile (a multiple of 64) and pairs that share its K: the least rounds x time of a round.  Nanoseconds per K block measured at
-// 8192 x 4096 x 12288 (NVFP4 and bf16; more columns than the MMAs of a block can hide behind its bytes and its issue cost little), a
-// microsecond per tile for the accumulators' hand-over, and some four for the exchange of a split, which only pays where all clusters
-// run at once: us of one pair per tile / of the split chosen here, 64 rows: NVFP4 4096 x 12288 17.3 / 14.3 (3 pairs; over a cluster
-// of single CTAs 20), 4096 x 4096 8.2 / 9.6 (not chosen), bf16 4096 x 12288 43 / 31, 4096 x 4096 17.4 / 15, MXFP8 2048 x 4096 12.9 /
-// 10.6; 16 tiles of 4 pairs do not fit the chip at once: 24.9.
+// 8192 x 4096 x 12288 (NVFP4 and bf16, 64 columns: 64 rows; more columns than the MMAs of a block can hide behind its bytes and its issue
+// cost little), a microsecond per tile for the accumulators' hand-over, and some six for the exchange of a split, which only pays where
+// all clusters run at once: us of one pair per tile / of two / of three, 64 rows: NVFP4 4096 x 12288 15.1 / 14.1 / 14.5 (over a
+// cluster of single CTAs 20), 4096 x 4096 8.6 / 9.9 / 10.5, bf16 4096 x 12288 41 / 32 / 31, 4096 x 4096 16.3 / 15.1 / 15.0; 16 tiles
+// of 4 pairs do not fit the chip at once: 24.3.
 static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
-  static const int scaled[] = {294, 313, 338, 387}, plain[] = {237, 255, 296, 385};
+  static const int scaled[] = {230, 313, 338, 387}, plain[] = {195, 255, 296, 385};
   const int tiles_f = (N + 255) / 256, sms = sm_count(), pairs = sms / 2 > 0 ? sms / 2 : 1;
   const int k_tiles = (K + (kind == 0 ? 63 : kind == 1 ? 255 : 127)) / (kind == 0 ? 64 : kind == 1 ? 256 : 128);
   long best = 1L << 60;
@@ -563,10 +576,10 @@ static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
     if (*cn && c != *cn) continue;
     const long tiles = (long)tiles_f * ((M + c - 1) / c);
     const long block = (kind ? scaled : plain)[c / 64 - 1];
-    for (int k = 1; k <= 4 && k <= k_tiles; ++k) {
+    for (int k = 1; k <= 4 && k <= (k_tiles + 1) / 2; ++k) {
       if (*ks && k != *ks) continue;
       if (k > 1 && !*ks && (tiles * k > pairs || tiles > pair_cluster_room(2 * k))) continue;
-      const long cost = k == 1 ? ((tiles + pairs - 1) / pairs) * (k_tiles * block + 1000) : (k_tiles + k - 1) / k * block + 5000 + 10 * c;
+      const long cost = k == 1 ? ((tiles + pairs - 1) / pairs) * (k_tiles * block + 1000) : (k_tiles + k - 1) / k * block + 1300 + 2000 * k + 10 * c;
       if (cost < best) { best = cost; best_cn = c; best_ks = k; }
     }
   }
@@ -578,7 +591,7 @@ static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
 
 // C[M, N] = X[M, K] · W[N, K]^T with the operand conventions of blz_gemm_tc (ldx / ldw in BYTES, ldc in elements).  kind: 0 bf16,
 // 1 NVFP4, 2 MXFP8.  N even, or a multiple of 32 with act (bf16 out, [M, N/2]).  cn: tokens per tile, 64 / 128 / 192 / 256, and
-// ks: pairs that share a tile's K, 1 - 4 (at most one per K block); 0 to choose.
+// ks: pairs that share a tile's K, 1 - 4 (at most one per two K blocks); 0 to choose.
 BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int M, int N,
                           int K, const float* row_scale, const float* alpha, const void* bias, const void* sfx, const void* sfw,
                           int out_f32, int cn, int ks, int max_ctas, int act, float act_limit, cudaStream_t stream) {
@@ -587,7 +600,7 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
   if (gemm_oneshot_take_unsupported()) return (int)cudaErrorNotSupported;
   if (M <= 0 || N <= 0 || K <= 0 || kind < 0 || kind > 2 || cn < 0 || cn > 256 || cn % 64 || ks < 0 || ks > 4) return (int)cudaErrorInvalidValue;
   const int kmma = kind == 0 ? 16 : kind == 1 ? 64 : 32;
-  if (K % kmma || ks > (K + 4 * kmma - 1) / (4 * kmma)) return (int)cudaErrorInvalidValue;
+  if (K % kmma || (ks > 1 && ks > (K + 8 * kmma - 1) / (8 * kmma))) return (int)cudaErrorInvalidValue;
   if (kind && (!sfx || !sfw)) return (int)cudaErrorInvalidValue;
   if (act < 0 || act > 2 || (act && (out_f32 || N % 32))) return (int)cudaErrorInvalidValue;
   if (!out_f32 && ((N & 1) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3))) return (int)cudaErrorInvalidValue;
@@ -619,14 +632,14 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
 }
 
 // The routed rows of `experts` experts: X and C are in the padded row space of moe.cu (row_tiles x 128 rows), `heads` comes from
-// blz_moe_plan_runs with the same `run` (64, 128 or 256 rows at most per tile), W holds the experts' weights one after the other, [experts * N, K].  N % 256 == 0; act 0, or 1 (rows of each
+// blz_moe_plan_runs with the same `run` (128 or 256 rows at most per tile), W holds the experts' weights one after the other, [experts * N, K].  N % 256 == 0; act 0, or 1 (rows of each
 // expert's W in [16 gate | 16 up] groups).
 BLZ_API int blz_gemm_pair_experts(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int row_tiles,
                                   int N, int K, int experts, const float* row_scale, const float* alpha, const void* sfx, const void* sfw,
                                   const void* heads, int run, int act, cudaStream_t stream) {
   using namespace blz;
   if (row_tiles <= 0) return 0;
-  if (N <= 0 || N % 256 || K <= 0 || kind < 0 || kind > 2 || experts <= 0 || !heads || (run != 64 && run != 128 && run != 256) || act < 0 || act > 1) return (int)cudaErrorInvalidValue;
+  if (N <= 0 || N % 256 || K <= 0 || kind < 0 || kind > 2 || experts <= 0 || !heads || (run != 128 && run != 256) || act < 0 || act > 1) return (int)cudaErrorInvalidValue;
   const int kmma = kind == 0 ? 16 : kind == 1 ? 64 : 32;
   if (K % kmma || (kind && (!sfx || !sfw)) || (ldc & 1) || (reinterpret_cast<uintptr_t>(C) & 3)) return (int)cudaErrorInvalidValue;
   if ((long long)experts * N > 0x7fffffffLL) return (int)cudaErrorInvalidValue;

@@ -217,11 +217,11 @@ BLZ_API int blz_moe_route(const float* logits, long long ld, float* topk_w, int*
   return (int)cudaGetLastError();
 }
 
-// heads (16-byte entries, or null): the number of runs, then {first row, rows, expert, 0} of the experts' runs of up to `run` rows (64, 128 or
+// heads (16-byte entries, or null): the number of runs, then {first row, rows, expert, 0} of the experts' runs of up to `run` rows (128 or
 // 256), what blz_gemm_pair_experts computes at a time.  At most routed rows / run + experts of them.
 BLZ_API int blz_moe_plan_runs(const int* counts, int* offsets, int* fill, int* tile_expert, int* tile_rows, void* heads, int run,
                               int local_n, int max_tiles, cudaStream_t s) {
-  if (local_n > 512 || (reinterpret_cast<uintptr_t>(heads) & 15) || (run != 64 && run != 128 && run != 256)) return (int)cudaErrorInvalidValue;
+  if (local_n > 512 || (reinterpret_cast<uintptr_t>(heads) & 15) || (run != 128 && run != 256)) return (int)cudaErrorInvalidValue;
   moe_plan_kernel<<<1, 512, 0, s>>>(counts, offsets, fill, tile_expert, tile_rows, (int4*)heads, run, local_n, max_tiles);
   return (int)cudaGetLastError();
 }

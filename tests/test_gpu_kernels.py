@@ -136,7 +136,7 @@ def test_gemm_pair(ops, fmt, M, N, K, act):
         if f32:
             want = ops.linear(lin, xin, out_dtype=torch.float32, wide=False, sk=False)
         for cn, ks, ctas in ((64, 1, 0), (128, 1, 6), (192, 1, 4), (256, 1, 2), (64, 2, 0), (128, 3, 0), (192, 4, 0), (256, 2, 0)):
-            if ks > -(-K // {"bf16": 64, "nvfp4": 256, "mxfp8": 128}[fmt]):
+            if ks > 1 and ks > -(-K // {"bf16": 128, "nvfp4": 512, "mxfp8": 256}[fmt]):
                 continue
             out = torch.full_like(want, float("nan"))
             rc = ops.lib.blz_gemm_pair(pk["kind"], p(a), a.shape[1] * a.element_size(), p(pk["w"]), pk["w"].shape[1] * pk["w"].element_size(), p(out),
@@ -149,7 +149,7 @@ def test_gemm_pair(ops, fmt, M, N, K, act):
                 assert _report(f"pair split {ks}", out, want)[1] < (2e-6 if f32 else 2e-3), (cn, ks, f32)
 
 
-@pytest.mark.parametrize("run", [64, 128, 256])
+@pytest.mark.parametrize("run", [128, 256])
 @pytest.mark.parametrize("fmt,N,K", [("nvfp4", 512, 320), ("mxfp8", 256, 2048), ("bf16", 768, 48)])
 @pytest.mark.parametrize("counts", [[0, 1, 0, 64, 65, 0], [700, 128, 129, 256, 257, 31], [0, 0, 0, 0, 0, 0], [5000, 0, 1, 0, 0, 513]])
 def test_grouped_gemm_pair(ops, fmt, N, K, counts, run):
