@@ -195,14 +195,9 @@ def build_batch(chunks: Sequence[SeqChunk], block_table_host: np.ndarray, device
     else:
         stage = torch.empty(total, dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
     sn = stage.numpy()
-    off = 0
-    offs = []
-    for p in parts:
-        sn[off:off + p.size] = p
-        offs.append((off, p.size))
-        off += p.size
+    np.concatenate(parts, out=sn)
     dev = stage.to(device, non_blocking=True)
-    v = [dev[o:o + n] for o, n in offs]
+    v = dev.split([p.size for p in parts])
     return StepBatch(tokens=v[0], positions=v[1], slot_mapping=v[2], seq_of_row=v[3], slots=v[4], q_start=v[5],
                      ctx_len=v[6], logit_rows=v[7], item_seq=v[8] if items_s else None,
                      item_q0=v[9] if items_s else None, tree_mask=v[10] if has_tree else None,

@@ -43,6 +43,50 @@ class QuantAct:
         # GEMM that consumes it waits for the flags inside its producer warp
         self.wait = None
 
+    def addresses(self):
+        """Addresses of the codes, the block scales and the row scales, for a launch made while this object lives."""
+        rs = self.row_scale
+        return self.data.data_ptr(), self.sf.data_ptr(), None if rs is None else rs.data_ptr()
+
+    @property
+    def row_bytes(self) -> int:
+        return self.data.shape[1]
+
+
+class PackedAct(QuantAct):
+    """NVFP4 or MXFP8 rows in one allocation: codes, block scales in the tensor core's order, row scales (NVFP4).  The tensors
+    are made when they are asked for: a step's kernels take the addresses (three allocations take 5 us of host time, as much as a
+    launch)."""
+    __slots__ = ("buf", "off_sf", "off_rs")
+
+    def __init__(self, fmt, rows, cols, device):
+        fp4 = fmt == Format.NVFP4
+        per = 64 if fp4 else 128
+        self.off_sf = (rows * (cols // 2 if fp4 else cols) + 255) // 256 * 256
+        self.off_rs = self.off_sf + (rows + 127) // 128 * ((cols + per - 1) // per) * 512
+        self.buf = torch.empty(self.off_rs + (4 * rows if fp4 else 0), dtype=torch.uint8, device=device)
+        self.fmt, self.rows, self.cols, self.dense, self.wait = fmt, rows, cols, None, None
+
+    def addresses(self):
+        p = self.buf.data_ptr()
+        return p, p + self.off_sf, p + self.off_rs if self.fmt == Format.NVFP4 else None
+
+    @property
+    def row_bytes(self) -> int:
+        return self.cols // 2 if self.fmt == Format.NVFP4 else self.cols
+
+    @property
+    def data(self):
+        return self.buf[:self.rows * self.row_bytes].view(self.rows, self.row_bytes)
+
+    @property
+    def sf(self):
+        return self.buf[self.off_sf:self.off_rs]
+
+    @property
+    def row_scale(self):
+        return self.buf[self.off_rs:].view(torch.float32) if self.fmt == Format.NVFP4 else None
+
 
 class Linear:
     """``y = x @ W^T`` with W ``[N, K]`` held in one of the storage formats."""

@@ -16,7 +16,7 @@ import torch
 
 from .. import quant
 from .._native import kernels
-from ..linear import Linear, QuantAct
+from ..linear import Linear, PackedAct, QuantAct
 from ..quant import Format
 
 _c = ctypes
@@ -27,8 +27,15 @@ class CudaError(RuntimeError):
     pass
 
 
-def _ptr(t: Optional[torch.Tensor]) -> VP:
-    return VP(0) if t is None else VP(t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
+    """A tensor's address for a ``c_void_p`` parameter (the entry points have their types declared; a plain integer is converted
+    faster than an object made for it)."""
+    return None if t is None else t.data_ptr()
+
+
+def _rows(T: int, W: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+    """An uninitialised matrix (1.4 us of host time; ``torch.empty`` of two sizes takes 2.1)."""
+    return torch.empty_strided((T, W), (W, 1), dtype=dtype, device=device)
 
 
 class _Symbols:
@@ -381,16 +388,7 @@ class CudaOps:
 
     # ------------------------------------------------------------------ activation quantisation
     def _alloc_qact(self, fmt: Format, T: int, K: int) -> QuantAct:
-        dev = self.device
-        if fmt == Format.NVFP4:
-            data = torch.empty(T, K // 2, dtype=torch.uint8, device=dev)
-            sf = torch.empty(((T + 127) // 128) * ((K + 63) // 64) * 512, dtype=torch.uint8, device=dev)
-            rs = torch.empty(T, dtype=torch.float32, device=dev)
-        else:
-            data = torch.empty(T, K, dtype=torch.uint8, device=dev)
-            sf = torch.empty(((T + 127) // 128) * ((K + 127) // 128) * 512, dtype=torch.uint8, device=dev)
-            rs = None
-        return QuantAct(fmt, data, sf, rs, T, K)
+        return PackedAct(fmt, T, K, self.device)
 
     def _qmode(self, lin: Optional[Linear]) -> int:
         """Activation format the producer's epilogue should emit for ``lin``: 0 bf16, 1 NVFP4, 2 MXFP8.  (The exact FP8
@@ -420,10 +418,12 @@ class CudaOps:
     def quantize_rows(self, x: torch.Tensor, lin: Linear) -> QuantAct:
         """bf16 ``[T, K]`` → the activation format ``lin`` consumes."""
         mode = self._qmode(lin)
+        return self._quantize(x, mode)
+
+    def _quantize(self, x: torch.Tensor, mode: int) -> QuantAct:
         T, K = x.shape
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, K)
-        self._check(self.lib.blz_swiglu(_ptr(x), VP(0), _ptr(qa.data), _ptr(qa.sf), _ptr(qa.row_scale), T, K, mode, 1,
-                                        self._stream()), "quantize_rows")
+        self._check(self.lib.blz_swiglu(x.data_ptr(), None, *qa.addresses(), T, K, mode, 1, self._stream()), "quantize_rows")
         return qa
 
     # ------------------------------------------------------------------ basics
@@ -440,12 +440,12 @@ class CudaOps:
         new_res = residual if residual is not None else x
         if mode == 0:
             out = torch.empty_like(x)
-            self._check(self.lib.blz_rmsnorm(_ptr(x), _ptr(residual), _ptr(w), _ptr(out), VP(0), VP(0), VP(0), T, H, eps,
+            self._check(self.lib.blz_rmsnorm(_ptr(x), _ptr(residual), _ptr(w), _ptr(out), None, None, None, T, H, eps,
                                              int(zero_centered), 0, int(zero_src), self._stream()), "rmsnorm")
             return out, new_res
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, H)
-        self._check(self.lib.blz_rmsnorm(_ptr(x), _ptr(residual), _ptr(w), VP(0), _ptr(qa.data), _ptr(qa.sf),
-                                         _ptr(qa.row_scale), T, H, eps, int(zero_centered), mode, int(zero_src), self._stream()), "rmsnorm_q")
+        self._check(self.lib.blz_rmsnorm(_ptr(x), _ptr(residual), _ptr(w), None, *qa.addresses(), T, H, eps, int(zero_centered), mode,
+                                         int(zero_src), self._stream()), "rmsnorm_q")
         return qa, new_res
 
     WIDE_WS_BYTES = 40 << 20
@@ -558,27 +558,28 @@ class CudaOps:
         if kind in (1, 2):
             if not isinstance(x, QuantAct):
                 x = self.quantize_rows(x.contiguous(), lin)
-            a, sfa, rs, M = x.data, x.sf, x.row_scale, x.rows
-            lda = a.shape[1]
+            M, lda = x.rows, x.row_bytes
+            a, sfa, rs = x.addresses()
         elif kind == 3:
             xt = x.dense if isinstance(x, QuantAct) else x
             q, s = quant.fp8_rowwise_quantize(xt)
-            a, rs, M = q.view(torch.uint8).contiguous(), s.float().contiguous(), xt.shape[0]
-            lda = a.shape[1]
+            q, s = q.view(torch.uint8).contiguous(), s.float().contiguous()
+            a, rs, M, lda = q.data_ptr(), s.data_ptr(), xt.shape[0], q.shape[1]
         else:
             # rows may be a run of columns of a wider matrix where TMA can start and step on 16 bytes
-            a = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 else x.contiguous()
-            M, lda = a.shape[0], a.stride(0) * 2
+            if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+                x = x.contiguous()
+            a, M, lda = x.data_ptr(), x.shape[0], x.stride(0) * 2
         if argmax_parts is not None:
             out = argmax_parts[0]            # the logits are not written; any valid pointer will do
             ld_out = n_out
         elif out is None:
-            out = torch.empty(M, n_out, dtype=torch.float32 if f32 else torch.bfloat16, device=self.device)
-        if argmax_parts is None:
+            out, ld_out = _rows(M, n_out, torch.float32 if f32 else torch.bfloat16, self.device), n_out
+        else:
             ld_out = out.stride(0)
         if M == 0:
             return out
-        w = pk["w"]
+        w, bias, sfw = pk["w"], pk["bias"], pk["sf"]
         kt = pk.get("kt", 0)
         ldb = 128 if kt else w.shape[1] * w.element_size()
         pending = getattr(x, "wait", None) if isinstance(x, QuantAct) else None
@@ -592,9 +593,6 @@ class CudaOps:
             if rc != 0:
                 raise CudaError(f"blz_gemm_wait_flags failed: {rc}")
             x.wait = None
-        narrow = (M <= self.NARROW_ROWS and kind in (0, 1, 2) and lin.N % 128 == 0 and not f32 and argmax_parts is None
-                  and pending is None and not kt and (wide is None or relu2) and bn == 0 and (sk is None or sk is False)
-                  and (not swiglu or ld_out % 8 == 0) and (sfa is None or sfa.numel() >= 512))
         pair = (wide is None and self._wide_ok and bn == 0 and kind in (0, 1, 2) and lin.N >= 128 and not kt and pending is None
                 and argmax_parts is None and max_ctas != 1 and not relu2 and (sk is None or sk is False)
                 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0)) and (not swiglu or lin.N % 32 == 0))
@@ -602,10 +600,14 @@ class CudaOps:
         # x 6144 x 4096 12.1, 12.5, 13.5, 115 / 8.9, 9.0, 10.3, 75; x 24576 x 4096 gated 20.7, 28, 30, 380 / 19.6, 19.6, 25, 306; x 4096 x
         # 12288 15.9, 20.4, 24, 177 / 14.2, 14.3, 16.7, 126; bf16 x 6144 x 4096 19.9, 26.5, 27.3, 328 / 17.7, 18.1, 22.7, 249; head of
         # 151936 x 4096 216, 228, 315 / 210, 212, 254).
-        big = lin.N * lin.K >= 6144 * 4096 if M <= 32 else lin.N >= 16384
-        if narrow and (self.NARROW_ALWAYS or (big and not pair)):
-            self._check(self.lib.blz_gemm_narrow(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
-                                                 _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), 0, act, limit,
+        narrow = (self.NARROW_ALWAYS or not pair) and (
+            M <= self.NARROW_ROWS and kind in (0, 1, 2) and lin.N % 128 == 0 and not f32 and argmax_parts is None
+            and pending is None and not kt and (wide is None or relu2) and bn == 0 and (sk is None or sk is False)
+            and (not swiglu or ld_out % 8 == 0) and (sfa is None or x.sf.numel() >= 512)
+            and (self.NARROW_ALWAYS or (lin.N * lin.K >= 6144 * 4096 if M <= 32 else lin.N >= 16384)))
+        if narrow:
+            self._check(self.lib.blz_gemm_narrow(kind, a, lda, w.data_ptr(), ldb, _ptr(out), ld_out, M, lin.N, lin.K, rs,
+                                                 _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw), 0, act, limit,
                                                  self._stream()), f"gemm_narrow kind {kind}")
             return out
         sk_able = not f32 and argmax_parts is None and pending is None and not kt
@@ -625,13 +627,13 @@ class CudaOps:
             if not sk_able:
                 raise CudaError("the split-K GEMM writes bf16 from row-major weights and has no arg-max / peer-wait epilogue")
             ks = 0 if sk is True else int(sk)
-            self._check(self.lib.blz_gemm_sk(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K,
-                                             _ptr(rs), _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]),
+            self._check(self.lib.blz_gemm_sk(kind, a, lda, w.data_ptr(), ldb, _ptr(out), ld_out, M, lin.N, lin.K,
+                                             rs, _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw),
                                              ks, act, limit, self._stream()), f"gemm_sk kind {kind}")
             return out
         if pair:
-            self._check(self.lib.blz_gemm_pair(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K, _ptr(rs),
-                                               _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]), int(f32), 0, 0, max_ctas, act, limit,
+            self._check(self.lib.blz_gemm_pair(kind, a, lda, w.data_ptr(), ldb, _ptr(out), ld_out, M, lin.N, lin.K, rs,
+                                               _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw), int(f32), 0, 0, max_ctas, act, limit,
                                                self._stream()), f"gemm_pair kind {kind}")
             return out
         if wide is None:
@@ -656,8 +658,8 @@ class CudaOps:
                     if tiles > self._wide_ctr.numel():
                         ks = 1
                     ws, ctr = self._wide_ws, self._wide_ctr
-            self._check(self.lib.blz_gemm_wide(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), out.stride(0), M, lin.N, lin.K,
-                                               _ptr(rs), _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]),
+            self._check(self.lib.blz_gemm_wide(kind, a, lda, w.data_ptr(), ldb, _ptr(out), out.stride(0), M, lin.N, lin.K,
+                                               rs, _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw),
                                                int(f32), int(swap), ks, _ptr(ws), self.WIDE_WS_BYTES if ws is not None else 0,
                                                _ptr(ctr), max_ctas, kt, act, limit, self._stream()), f"gemm_wide kind {kind}")
             return out
@@ -665,8 +667,8 @@ class CudaOps:
             rc = self.lib.blz_gemm_argmax_parts(_ptr(argmax_parts[0]), _ptr(argmax_parts[1]))
             if rc != 0:
                 raise CudaError(f"blz_gemm_argmax_parts failed: {rc}")
-        self._check(self.lib.blz_gemm_tc(kind, _ptr(a), lda, _ptr(w), ldb, _ptr(out), ld_out, M, lin.N, lin.K,
-                                         _ptr(rs), _ptr(pk["alpha"]), _ptr(pk["bias"]), _ptr(sfa), _ptr(pk["sf"]),
+        self._check(self.lib.blz_gemm_tc(kind, a, lda, w.data_ptr(), ldb, _ptr(out), ld_out, M, lin.N, lin.K,
+                                         rs, _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw),
                                          int(f32), bn, max_ctas, VP(0), 0, kt, act, limit, self._stream()), f"gemm kind {kind}")
         return out
 
@@ -675,12 +677,11 @@ class CudaOps:
         I = I2 // 2
         mode = self._qmode(quant_for)
         if mode == 0:
-            out = torch.empty(T, I, dtype=torch.bfloat16, device=self.device)
-            self._check(self.lib.blz_swiglu(_ptr(gu), _ptr(out), VP(0), VP(0), VP(0), T, I, 0, 0, self._stream()), "swiglu")
+            out = _rows(T, I, torch.bfloat16, self.device)
+            self._check(self.lib.blz_swiglu(_ptr(gu), _ptr(out), None, None, None, T, I, 0, 0, self._stream()), "swiglu")
             return out
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, I)
-        self._check(self.lib.blz_swiglu(_ptr(gu), VP(0), _ptr(qa.data), _ptr(qa.sf), _ptr(qa.row_scale), T, I, mode, 0,
-                                        self._stream()), "swiglu_q")
+        self._check(self.lib.blz_swiglu(_ptr(gu), None, *qa.addresses(), T, I, mode, 0, self._stream()), "swiglu_q")
         return qa
 
     def mul_sigmoid(self, x, gate):
@@ -720,6 +721,7 @@ class CudaOps:
         D = cfg.head_dim
         if kv.layout != "umma":
             raise CudaError("the CUDA attention path needs the FP8 'umma' KV layout (kv_dtype='fp8')")
+        pool = kv.kv[layer_idx]
         q = torch.empty(T, attn.heads, D, dtype=torch.bfloat16, device=self.device)
         gate = torch.empty(T, attn.heads, D, dtype=torch.bfloat16, device=self.device) if cfg.attn_output_gate else None
         # M-RoPE: three position streams [3, T]; frequency i reads stream 0 / 1 / 2 by the model's section sizes
@@ -731,11 +733,11 @@ class CudaOps:
                 m0, m1 = int(sec[0]), int(sec[0]) + int(sec[1])
             else:
                 m0 = m1 = cfg.rotary_dim // 2          # no sections: every frequency follows the first stream
-        self._check(self.lib.blz_attn_prep_runs(_ptr(qkv), _ptr(q), _ptr(gate), _ptr(kv.kv[layer_idx]), _ptr(pos),
+        self._check(self.lib.blz_attn_prep_runs(_ptr(qkv), _ptr(q), _ptr(gate), _ptr(pool), _ptr(pos),
                                                 _ptr(batch.slot_mapping), _ptr(model.inv_freq), _ptr(attn.q_norm), _ptr(attn.k_norm),
                                                 T, attn.heads, attn.kv_heads, D, cfg.rotary_dim, cfg.rms_norm_eps,
                                                 model.rope_scale, int(cfg.attn_output_gate), int(cfg.zero_centered_norm),
-                                                1.0, 1.0, kv.kv[layer_idx].stride(0), kv.kv[layer_idx].stride(1),
+                                                1.0, 1.0, pool.stride(0), pool.stride(1),
                                                 int(getattr(model, "kv_rotate", False)), pos_stride, m0, m1, int(batch.max_q_len), self._stream()),
                     "attn_prep")
         return q, gate
@@ -1414,19 +1416,18 @@ class CudaOps:
         features are whole tiles of 256, else tiles of 128 x 128."""
         kind = pk["kind"]
         if kind in (1, 2):
-            data, sfa, rs = a.data, a.sf, a.row_scale
-            lda = data.shape[1]
+            data, sfa, rs = a.addresses()
+            lda = a.row_bytes
         else:
-            data, sfa, rs = a, None, None
-            lda = a.shape[1] * 2
+            data, sfa, rs, lda = a.data_ptr(), None, None, a.shape[1] * 2
         w = pk["w"]
         if runs is not None and kind in (0, 1, 2) and pk["N"] % 256 == 0 and act in (0, 1):
-            self._check(self.lib.blz_gemm_pair_experts(kind, _ptr(data), lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
-                                                       M_pad // 128, pk["N"], pk["K"], n_exp, _ptr(rs), _ptr(pk["alpha"]), _ptr(sfa), _ptr(pk["sf"]),
+            self._check(self.lib.blz_gemm_pair_experts(kind, data, lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
+                                                       M_pad // 128, pk["N"], pk["K"], n_exp, rs, _ptr(pk["alpha"]), sfa, _ptr(pk["sf"]),
                                                        _ptr(runs[0]), runs[1], act, self._stream()), "grouped gemm")
             return out
-        self._check(self.lib.blz_gemm_tc(kind, _ptr(data), lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
-                                         M_pad, pk["N"], pk["K"], _ptr(rs), _ptr(pk["alpha"]), VP(0), _ptr(sfa), _ptr(pk["sf"]),
+        self._check(self.lib.blz_gemm_tc(kind, data, lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
+                                         M_pad, pk["N"], pk["K"], rs, _ptr(pk["alpha"]), VP(0), sfa, _ptr(pk["sf"]),
                                          0, 128, 0, _ptr(tile_expert), n_exp, 0, act, 0.0, self._stream()), "grouped gemm")
         return out
 
@@ -1464,14 +1465,13 @@ class CudaOps:
         max_tiles = (T * k + 127) // 128 + n_exp
         M_pad = max_tiles * 128
         dev = self.device
-        offsets = torch.empty(n_exp, dtype=torch.int32, device=dev)
-        fill = torch.empty(n_exp, dtype=torch.int32, device=dev)
-        tile_expert = torch.empty(max_tiles, dtype=torch.int32, device=dev)
-        tile_rows = torch.empty(max_tiles, dtype=torch.int32, device=dev)
-        row_map = torch.empty(T, k, dtype=torch.int32, device=dev)
         # rows per tile of the pair kernel by the rows that an expert gets on average: beyond them its weights are read again
         run = 128 if T * k <= 96 * n_exp else 256
-        runs = (torch.empty(T * k // run + n_exp + 1, 4, dtype=torch.int32, device=dev), run)
+        # the plan in one allocation, its parts on 16 bytes
+        n4, t4, n_runs = (n_exp + 3) // 4 * 4, (max_tiles + 3) // 4 * 4, T * k // run + n_exp + 1
+        run_list, offsets, fill, tile_expert, tile_rows, row_map = torch.empty(
+            4 * n_runs + 2 * n4 + 2 * t4 + T * k, dtype=torch.int32, device=dev).split((4 * n_runs, n4, n4, t4, t4, T * k))
+        runs, row_map = (run_list, run), row_map.view(T, k)
         self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(runs[0]), run, n_exp,
                                                max_tiles, self._stream()), "moe_plan")
         narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
@@ -1482,12 +1482,9 @@ class CudaOps:
             narrow = False
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)
         if mode:
-            proxy = Linear(gu["fmt"], gu["N"], gu["K"])
-            proxy.act_quant = True
-            xq = self.quantize_rows(x.contiguous(), proxy)
+            xq = self._quantize(x.contiguous(), mode)
             a = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, M_pad, H)
-            self._check(self.lib.blz_moe_scatter(mode, _ptr(xq.data), _ptr(xq.sf), _ptr(xq.row_scale), _ptr(a.data), _ptr(a.sf),
-                                                 _ptr(a.row_scale), _ptr(topk_id), _ptr(offsets), _ptr(fill), _ptr(row_map), T, H, k,
+            self._check(self.lib.blz_moe_scatter(mode, *xq.addresses(), *a.addresses(), _ptr(topk_id), _ptr(offsets), _ptr(fill), _ptr(row_map), T, H, k,
                                                  first, n_exp, VP(0), 0, self._stream()), "moe_scatter")
         else:
             a = torch.empty(M_pad, H, dtype=x.dtype, device=dev)
@@ -1548,14 +1545,13 @@ class CudaOps:
         """Expert GEMM over the padded row space with the features on the MMA lanes and only each tile's live rows on its columns."""
         kind = pk["kind"]
         if isinstance(a, QuantAct):
-            data, sfa, rs = a.data, a.sf, a.row_scale
-            lda = data.shape[1]
+            data, sfa, rs = a.addresses()
+            lda = a.row_bytes
         else:
-            data, sfa, rs = a, None, None
-            lda = a.shape[1] * 2
+            data, sfa, rs, lda = a.data_ptr(), None, None, a.shape[1] * 2
         w = pk["w"]
-        self._check(self.lib.blz_moe_gemm(kind, _ptr(data), lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
-                                          row_tiles, pk["N"], pk["K"], n_exp, _ptr(rs), _ptr(pk["alpha"]), _ptr(sfa), _ptr(pk["sf"]),
+        self._check(self.lib.blz_moe_gemm(kind, data, lda, _ptr(w), w.shape[1] * w.element_size(), _ptr(out), out.stride(0),
+                                          row_tiles, pk["N"], pk["K"], n_exp, rs, _ptr(pk["alpha"]), sfa, _ptr(pk["sf"]),
                                           _ptr(tile_expert), _ptr(tile_rows), act, self._stream()), f"moe_gemm kind {kind}")
 
     def _silu_mul_live(self, gu, quant_for, row_list, is_act: bool = False):
@@ -1567,12 +1563,12 @@ class CudaOps:
         if mode == 0:
             if is_act:
                 return gu
-            out = torch.empty(T, I, dtype=torch.bfloat16, device=self.device)
-            self._check(self.lib.blz_swiglu_live(_ptr(gu), _ptr(out), VP(0), VP(0), VP(0), n, I, 0, 0, _ptr(row_list), self._stream()),
+            out = _rows(T, I, torch.bfloat16, self.device)
+            self._check(self.lib.blz_swiglu_live(_ptr(gu), _ptr(out), None, None, None, n, I, 0, 0, _ptr(row_list), self._stream()),
                         "swiglu_live")
             return out
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, I)
-        self._check(self.lib.blz_swiglu_live(_ptr(gu), VP(0), _ptr(qa.data), _ptr(qa.sf), _ptr(qa.row_scale), n, I, mode, int(is_act),
+        self._check(self.lib.blz_swiglu_live(_ptr(gu), None, *qa.addresses(), n, I, mode, int(is_act),
                                              _ptr(row_list), self._stream()), "swiglu_live_q")
         return qa
 
