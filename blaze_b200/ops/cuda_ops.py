@@ -101,6 +101,8 @@ class CudaOps:
                                           VP, _c.c_longlong, VP, VP, _c.c_int, _c.c_int, _c.c_int, VP]
         lib.blz_quant_fp8_block.restype = _c.c_int
         lib.blz_quant_fp8_block.argtypes = [VP, _c.c_longlong, VP, VP, _c.c_longlong, _c.c_int, _c.c_int, VP]
+        lib.blz_swiglu_fp8_block.restype = _c.c_int
+        lib.blz_swiglu_fp8_block.argtypes = [VP, VP, VP, _c.c_longlong, _c.c_int, _c.c_int, VP]
         # FP8 checkpoints with 128x128 fp32 block scales: "exact" keeps the stored codes and scales and promotes every K block
         # in fp32 (blz_gemm_fp8_block); "mx" re-quantises the weight once to e4m3 with e8m0 scales per 32 elements and runs the
         # hardware block-scaled MMA (faster, but only exact when the stored scales are powers of two)
@@ -408,8 +410,7 @@ class CudaOps:
         """bf16 ``[T, K]`` -> (e4m3 codes ``[T, K]``, fp32 scales ``[K / 128, T4]``) with one scale per row and 128 columns."""
         T, K = x.shape
         ld = (T + 3) // 4 * 4
-        q = torch.empty(T, K, dtype=torch.uint8, device=self.device)
-        sc = torch.empty(K // 128, ld, dtype=torch.float32, device=self.device)
+        q, sc = _rows(T, K, torch.uint8, self.device), _rows(K // 128, ld, torch.float32, self.device)
         if x.stride(1) != 1:
             x = x.contiguous()
         self._check(self.lib.blz_quant_fp8_block(_ptr(x), x.stride(0), _ptr(q), _ptr(sc), ld, T, K, self._stream()), "quant_fp8_block")
@@ -677,6 +678,12 @@ class CudaOps:
         I = I2 // 2
         mode = self._qmode(quant_for)
         if mode == 0:
+            if quant_for is not None and quant_for.fmt == Format.FP8_BLOCK and self.pack(quant_for)["kind"] == 4 and gu.is_contiguous():
+                # the exact FP8 product quantises its input by groups of 128: here in the same pass
+                ld = (T + 3) // 4 * 4
+                q, sc = _rows(T, I, torch.uint8, self.device), _rows(I // 128, ld, torch.float32, self.device)
+                self._check(self.lib.blz_swiglu_fp8_block(_ptr(gu), _ptr(q), _ptr(sc), ld, T, I, self._stream()), "swiglu_fp8_block")
+                return QuantAct(Format.FP8_BLOCK, q, sc, None, T, I)
             out = _rows(T, I, torch.bfloat16, self.device)
             self._check(self.lib.blz_swiglu(_ptr(gu), _ptr(out), None, None, None, T, I, 0, 0, self._stream()), "swiglu")
             return out

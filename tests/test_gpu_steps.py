@@ -525,3 +525,30 @@ def test_fp8_block_product_on_cta_pairs(ops, M, N, K):      # noqa: F811
                 assert ops.take_status() == 0
                 # parts of K add in another order: up to 2^-24 of the terms' size per addition
                 assert torch.equal(out, want) if ks == 1 else _rel(out, want) < (1e-6 if dt == torch.float32 else 2e-3), (cn, ks)
+
+
+@pytest.mark.parametrize("T,K", [(1, 128), (7, 384), (8, 512), (9, 640), (65, 1152), (300, 25600)])
+def test_fp8_groups_with_and_without_the_activation(ops, T, K):      # noqa: F811
+    """Codes and scales are those of the definition bit for bit; gated rows give those of the activation rounded to bf16; rows that start
+    on 8 bytes only, an infinity and a NaN give the same codes as anywhere else."""
+    g = torch.Generator(device=DEV).manual_seed(13)
+    gu = torch.randn(T, 2 * K, generator=g, device=DEV).bfloat16()
+    # (no -0 among the gates: the activation kernel of rows beyond 24576 divides, which keeps the zero's sign, and silu() does not)
+    gu[0, :2] = torch.tensor([float("inf"), float("nan")], device=DEV)
+    gu[T // 2, 128:256] = 0
+    down = Linear.from_dense(torch.randn(128, K, generator=g, device=DEV), Format.FP8_BLOCK)
+    act = ops.silu_mul(gu)
+    wide = torch.zeros(T, K + 4, dtype=torch.bfloat16, device=DEV)
+    wide[:, 4:] = act
+    gated, (q, sc), (q8, sc8) = ops.silu_mul(gu, quant_for=down), ops.quantize_fp8_block(act), ops.quantize_fp8_block(wide[:, 4:])
+    torch.cuda.synchronize()
+    v = act.float().view(T, K // 128, 128)
+    most = torch.nan_to_num(v.abs(), nan=0.0, posinf=float("inf")).amax(-1)
+    want = (most / torch.full_like(most, 448.0)).clamp_min(1e-12)      # (a division by a number multiplies by its rounded inverse)
+    assert torch.equal(sc[:, :T].t(), want)
+    codes = (v / want.unsqueeze(-1)).view(T, K)
+    ok = codes.isfinite()
+    assert torch.equal(q.view(torch.float8_e4m3fn).float()[ok], codes.clamp(-448, 448).to(torch.float8_e4m3fn).float()[ok])
+    assert q.view(torch.float8_e4m3fn).float()[~ok].isnan().all()
+    for a, b in ((gated.data, gated.sf), (q8, sc8)):
+        assert torch.equal(a, q) and torch.equal(b[:, :T], sc[:, :T])
