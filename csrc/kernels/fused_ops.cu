@@ -351,19 +351,25 @@ __device__ __forceinline__ void quant_store16(const uint32_t (&w)[8], float bm, 
   }
 }
 
+// The squares are added up in the order of rmsnorm_reg_kernel with `sum_threads` threads of 8 elements per pass: another order moves the
+// root's last bit, and with it whole 4-bit codes, some in a few rows of thousands.  Where those threads take one pass, a thread here has the
+// elements of two neighbours of theirs, and 16 lanes add up what a warp would; else the rows go by way of shared memory
+// (8192 rows of 4096 in NVFP4 from cold caches: 53 us with 8 elements per thread, 51 so; within a step 45, where handing the first pass's sums
+// on to the threads of the second instead of the rows took 44).
 template <int QUANT, int CH>
 __global__ void __launch_bounds__(256) rmsnorm_row16_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                                               const __nv_bfloat16* __restrict__ w, uint8_t* __restrict__ q_out,
                                                               uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int H,
-                                                              float eps, int zero_centered, int sf_col_tiles, int zero_src) {
+                                                              float eps, int zero_centered, int sf_col_tiles, int zero_src, int sum_threads) {
   pdl_trigger();
   pdl_wait();
+  extern __shared__ __align__(16) uint4 row16[];
   __shared__ float red[32];
   const int t = blockIdx.x;
   __nv_bfloat16* xr = x + (size_t)t * H;
   __nv_bfloat16* rr = residual ? residual + (size_t)t * H : nullptr;
   uint32_t u[CH][8];
-  float ss = 0.f;
+  const bool one_pass = CH == 1 && H / 8 <= sum_threads;
   {
     uint32_t r[CH][8];
 #pragma unroll
@@ -387,11 +393,44 @@ __global__ void __launch_bounds__(256) rmsnorm_row16_kernel(__nv_bfloat16* __res
           reinterpret_cast<uint4*>(rr + i)[1] = make_uint4(u[c][4], u[c][5], u[c][6], u[c][7]);
         }
       }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { ss = fmaf(lo_f(u[c][j]), lo_f(u[c][j]), ss); ss = fmaf(hi_f(u[c][j]), hi_f(u[c][j]), ss); }
+      if (!one_pass && i < H) {
+        row16[i / 8] = make_uint4(u[c][0], u[c][1], u[c][2], u[c][3]);
+        row16[i / 8 + 1] = make_uint4(u[c][4], u[c][5], u[c][6], u[c][7]);
+      }
     }
   }
-  ss = block_reduce(ss, red, false);
+  float ss = 0.f;
+  if (one_pass) {
+    float p[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      p[j / 4] = fmaf(lo_f(u[0][j]), lo_f(u[0][j]), p[j / 4]);
+      p[j / 4] = fmaf(hi_f(u[0][j]), hi_f(u[0][j]), p[j / 4]);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      p[0] += __shfl_xor_sync(0xffffffffu, p[0], o);
+      p[1] += __shfl_xor_sync(0xffffffffu, p[1], o);
+    }
+    if ((threadIdx.x & 15) == 0) red[threadIdx.x >> 4] = p[0] + p[1];
+    __syncthreads();
+    for (int i = 0; i < (int)blockDim.x >> 4; ++i) ss += red[i];
+  } else {
+    __syncthreads();
+    for (int sw = threadIdx.x >> 5; sw < sum_threads >> 5; sw += blockDim.x >> 5) {
+      float part = 0.f;
+      for (int g = sw * 32 + (threadIdx.x & 31); g < H / 8; g += sum_threads) {
+        const uint4 v = row16[g];
+        const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { part = fmaf(lo_f(e[j]), lo_f(e[j]), part); part = fmaf(hi_f(e[j]), hi_f(e[j]), part); }
+      }
+      part = warp_sum(part);
+      if ((threadIdx.x & 31) == 0) red[sw] = part;
+    }
+    __syncthreads();
+    for (int i = 0; i < sum_threads >> 5; ++i) ss += red[i];
+  }
   const float rstd = rsqrtf(ss / H + eps);
   float bm[CH], amax = 0.f;
 #pragma unroll
@@ -1081,6 +1120,8 @@ static void configure_once() {
   cudaFuncSetAttribute(rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
   cudaFuncSetAttribute(rmsnorm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
   cudaFuncSetAttribute(rmsnorm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+  cudaFuncSetAttribute(rmsnorm_row16_kernel<1, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+  cudaFuncSetAttribute(rmsnorm_row16_kernel<2, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
   attr = true;
 }
 
@@ -1103,8 +1144,8 @@ static inline void reg_shape(int W, int T, int* threads, int* chunks) {
   }
 
 // The quantising row kernels with 16 elements per thread: rows of up to 6 chunks of 256 threads.  At any number of rows where rows are
-// normed or are activations already (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norm of 8192
-// x 4096 48 / 40, of 1 row 3.3 / 2.5), for gated rows from 512 on (825 rows of 12288 19.8 / 17.1, 256 rows 7.6 / 8.3: their
+// normed or are activations already (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norms, from
+// cold caches, of 825 rows of 4096 14.3 / 12.3, 3000 of 5120 34.8 / 28.7, 2000 of 12320 76 / 49), for gated rows from 512 on (825 rows of 12288 19.8 / 17.1, 256 rows 7.6 / 8.3: their
 // activation is the longer chain per thread there; the experts' short gated rows likewise 43.7 / 46.2).
 constexpr int ROW16_MOST = 6 * 256 * 16;
 static inline int row16_threads(int W, int chunks) { return (W / 16 + chunks * 32 - 1) / (chunks * 32) * 32; }
@@ -1134,9 +1175,10 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
   reg_shape(H, T, &rt, &ch);
   if (quant && H <= ROW16_MOST) {
     const int c16 = (H + 4095) / 4096;
+    const size_t sm16 = c16 == 1 && H / 8 <= rt ? 0 : sm;          // (see rmsnorm_row16_kernel)
 #define BLZ_RN(C)                                                                                                              \
-  if (quant == 1) launch_pdl(rmsnorm_row16_kernel<1, C>, dim3(T), dim3(row16_threads(H, C)), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src); \
-  else launch_pdl(rmsnorm_row16_kernel<2, C>, dim3(T), dim3(row16_threads(H, C)), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src)
+  if (quant == 1) launch_pdl(rmsnorm_row16_kernel<1, C>, dim3(T), dim3(row16_threads(H, C)), sm16, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src, rt); \
+  else launch_pdl(rmsnorm_row16_kernel<2, C>, dim3(T), dim3(row16_threads(H, C)), sm16, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src, rt)
     BLZ_CH_SWITCH(c16, BLZ_RN)
 #undef BLZ_RN
     return (int)cudaGetLastError();

@@ -552,3 +552,20 @@ def test_fp8_groups_with_and_without_the_activation(ops, T, K):      # noqa: F81
     assert q.view(torch.float8_e4m3fn).float()[~ok].isnan().all()
     for a, b in ((gated.data, gated.sf), (q8, sc8)):
         assert torch.equal(a, q) and torch.equal(b[:, :T], sc[:, :T])
+
+
+@pytest.mark.parametrize("mode", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("T,W", [(3, 32), (3, 2016), (1200, 2048), (1200, 2080), (1024, 4096), (1025, 4096), (1025, 2304), (1025, 3840), (40, 4128), (1025, 7168), (40, 12320), (3, 24576)])
+def test_quantised_norm_adds_squares_like_the_plain_one(ops, mode, T, W):      # noqa: F811
+    """One pass of the plain kernel's threads over a row, several, and both numbers of threads: the same row sums, so the same codes."""
+    g = torch.Generator(device=DEV).manual_seed(21)
+    lin = Linear(mode, 128, W)
+    lin.act_quant = True
+    x, r = (torch.randn(T, W, generator=g, device=DEV).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(W, generator=g, device=DEV)).bfloat16()
+    plain, _ = ops.norm(x.clone(), r.clone(), w, 1e-6)
+    got, want = ops.norm(x, r, w, 1e-6, quant_for=lin)[0], ops.quantize_rows(plain, lin)
+    per = 16 if mode == Format.NVFP4 else 32
+    assert torch.equal(got.data, want.data)
+    assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, T, W // per) for q in (got, want)))
+    assert mode != Format.NVFP4 or torch.equal(got.row_scale, want.row_scale)
