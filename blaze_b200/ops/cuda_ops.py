@@ -156,7 +156,7 @@ class CudaOps:
         self.NARROW_ROWS = int(os.environ.get("BLAZE_GEMM_NARROW_ROWS", "64"))
         self.NARROW_ALWAYS = os.environ.get("BLAZE_GEMM_NARROW_ALWAYS", "0") == "1"
         lib.blz_swiglu_live.argtypes = [VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, VP, VP]
-        # Experts that the pair kernel does not take (bf16, or features that are no multiple of 256): routed rows per expert up to this,
+        # Experts in bf16, or with features that are no multiple of 256 (others take pairs of CTAs at any number of rows): routed rows per expert up to this,
         # the expert GEMMs put the features on the tensor-core lanes and only the live rows on its columns (blz_moe_gemm), which streams
         # the weights; above it the 128-row tiles of the grouped GEMM are full enough (BLAZE_MOE_NARROW=0: never; 1 << 20: always, also
         # before the pair kernel).  MXFP8 weights of 2048 feature tiles and more up to 8/3 of it, a whole tile of rows: twice the
@@ -538,8 +538,8 @@ class CudaOps:
     def linear(self, lin: Linear, x, out_dtype=None, out: Optional[torch.Tensor] = None, bn: int = 0, max_ctas: int = 0,
                wide: Optional[bool] = None, ksplit: int = 0, swiglu: bool = False, argmax_parts=None, sk=None,
                glu_limit: Optional[float] = None, relu2: bool = False):
-        """``wide``: None = choose; False = the 128-column kernel (needed by the fused all-reduce epilogue); True = insist on
-        the wide-N kernel (raises when the shape is not covered).  ``sk``: None = choose; False = never; True or a K-slice
+        """``wide``: None = choose (pairs of CTAs where they can, see below); False = the 128-column kernel (needed by the fused
+        all-reduce epilogue); True = insist on the wide-N kernel (raises when the shape is not covered).  ``sk``: None = choose; False = never; True or a K-slice
         count 1..8 = the cluster split-K kernel (bf16 output, row-major weights).  ``swiglu`` with ``glu_limit``: the clamped
         gated activation instead of SwiGLU.  ``relu2``: squared ReLU of the result."""
         pk = self.pack(lin, swiglu=swiglu)

@@ -1,4 +1,4 @@
-// GEMM of many rows on CTA pairs:  C[tokens, features] = X[tokens, K] · W[features, K]^T.
+// GEMM on CTA pairs, for any number of rows, and experts' products:  C[tokens, features] = X[tokens, K] · W[features, K]^T.
 //
 // A pair (a cluster of two CTAs on neighbouring SMs) computes 256 features x up to 256 tokens with one tcgen05.mma.cta_group::2 per
 // K step: features are the MMA lanes (128 in each CTA), tokens its columns, half of their rows in either CTA's shared memory.  Per 128
@@ -13,14 +13,14 @@
 // Few tiles and a long K: a cluster of up to four pairs shares a tile's K, and the CTAs of one rank exchange their partial sums through
 // distributed shared memory (each owns some columns and adds the parts up in the pairs' order, so results do not depend on timing).
 //
-// Few tokens: tiles of 64 or 128 columns take less of a stage, so that up to ten stages are in flight, which is what a weight that is read
-// once needs (NVFP4 x 4096 x 4096, 64 rows 12.7 -> 9.1 us).  Experts (GROUPED): a tile is a run of one expert's routed rows.
+// Few tokens: tiles of 64 or 128 columns take less of a stage, so that more of a weight that is read once is in flight (NVFP4 x 4096 x
+// 4096, 64 rows 12.7 -> 9.1 us); where MMAs are short (64 columns, experts) a stage holds two K blocks, since its waits and commits cost
+// some 450 clocks.  Experts: a tile is a run of one expert's routed rows.
 //
 // 448 threads: warp 0 = TMA producer (one per CTA, its own half of the tile), warp 1 = MMA issuer (first CTA of the pair only), warps
 // 2-13 = epilogue.  Persistent, one pair per two SMs.  Barriers: `full` lives in the first CTA and counts both CTAs' bytes; `empty` and
-// `acc_full` are in both and raised by multicast commits; `acc_early`
-// and `acc_free` are in the first and count both CTAs' epilogue warps.  Every wait is bounded;
-// the hardware cluster barrier is used at the start and, by all threads, at the end.  No load is multicast.
+// `acc_full` are in both and raised by multicast commits; `acc_early` and `acc_free` are in the first and count both CTAs' epilogue
+// warps.  Every wait is bounded; the hardware cluster barrier is used at the start and, by all threads, at the end.  No load is multicast.
 //
 // Measured against one CTA per tile of 128 x 256 (gemm_wide.cu, gemm_tc.cu; back to back in a graph, inputs from memory): 8192 rows, NVFP4
 // x 4096 x 12288 177 -> 126 us (6.6 PFLOP/s), x 6144 x 4096 115 -> 75, x 24576 x 4096 with the gated activation 380 -> 306; bf16 x
@@ -632,8 +632,8 @@ BLZ_API int blz_gemm_pair(int kind, const void* X, long long ldx, const void* W,
 }
 
 // The routed rows of `experts` experts: X and C are in the padded row space of moe.cu (row_tiles x 128 rows), `heads` comes from
-// blz_moe_plan_runs with the same `run` (128 or 256 rows at most per tile), W holds the experts' weights one after the other, [experts * N, K].  N % 256 == 0; act 0, or 1 (rows of each
-// expert's W in [16 gate | 16 up] groups).
+// blz_moe_plan_runs with the same `run` (128 or 256 rows at most per tile), W holds the experts' weights one after the other,
+// [experts * N, K].  N % 256 == 0; act 0, or 1 (rows of each expert's W in [16 gate | 16 up] groups).
 BLZ_API int blz_gemm_pair_experts(int kind, const void* X, long long ldx, const void* W, long long ldw, void* C, long long ldc, int row_tiles,
                                   int N, int K, int experts, const float* row_scale, const float* alpha, const void* sfx, const void* sfw,
                                   const void* heads, int run, int act, cudaStream_t stream) {

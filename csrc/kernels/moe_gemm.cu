@@ -1,4 +1,5 @@
-// Grouped expert GEMM for decode-sized routing (a few rows per expert), features on the tensor-core lanes:
+// Grouped expert GEMM for decode-sized routing (a few rows per expert), features on the tensor-core lanes, for experts that the pairs of
+// gemm_pair.cu do not take (bf16 of few rows each, squared ReLU, features that are no multiple of 256):
 //     C[row, f] = (X[row, :] · W_e[f, :]) * row_scale[row] * alpha[e * N + f]      for the rows routed to expert e
 // The routed rows sit in a padded row space where every expert starts on a 128-row boundary (moe_plan / moe_scatter), so a
 // "row tile" (128 rows) belongs to one expert and holds `tile_rows[mt]` live rows, usually 8-32.  One CTA computes one
@@ -11,7 +12,7 @@
 // gate and up value of one feature sit 16 lanes apart in the same warp, one shuffle joins them and the [rows, 2I]
 // intermediate never reaches memory.
 //
-// The same kernel serves dense layers at small batch (at most 128 rows, e.g. single-user decoding or a verify step):
+// The same kernel serves dense layers of few rows that the pairs do not take (squared ReLU, fewer than 128 features):
 // tile_expert = null means one "expert" whose rows are the whole activation matrix.  Few rows mean few feature tiles and a
 // long K range per tile, so the K range can be split over a thread-block cluster of `ks` CTAs: each streams 1/ks of the
 // weights of its feature tile, and the fp32 partials (128 features x 32..128 rows, a few KB) meet in distributed shared
