@@ -1371,11 +1371,10 @@ class CudaOps:
             """``swiglu``: block-scaled rows in the order of the SwiGLU epilogue."""
             l0, E, dev = lins[0], len(lins), self.device
             swiglu = swiglu and l0.fmt in (Format.NVFP4, Format.MXFP8, Format.FP8_BLOCK) and l0.N % 32 == 0
-            order = self.swiglu_order(l0.N).to(dev) if swiglu else None
 
-            def rows(ts, dtype=None):        # every expert's rows one after the other, in that order
+            def rows(ts, dtype=None):        # every expert's rows one after the other, in that order (swiglu_order, as one strided copy)
                 t = torch.cat([t.to(dev) if dtype is None else t.to(dev, dtype) for t in ts])
-                return t if order is None else t.view(E, l0.N, -1)[:, order].reshape(t.shape)
+                return t.view(E, 2, l0.N // 32, 16, -1).transpose(1, 2).reshape(t.shape) if swiglu else t
 
             if l0.fmt in (Format.NVFP4, Format.MXFP8):
                 kind = 1 if l0.fmt == Format.NVFP4 else 2
