@@ -409,6 +409,8 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // predecessor still runs.  pdl_trigger() lets the successor of THIS kernel do so; pdl_wait() returns when the predecessor
 // has completed and its memory is visible — nothing it wrote may be read, and no global memory written, before that.
 // Both are no-ops for kernels launched the plain way.
+// A kernel with tensor memory triggers after its CTA holds it: a successor that becomes resident on the same SM waits for this kernel
+// to complete, so columns that it took first would never come back.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

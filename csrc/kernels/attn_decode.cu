@@ -127,7 +127,6 @@ __device__ __forceinline__ void load_some(const float* src, float (&v)[V]) {
 
 template <int RMAX>
 __global__ void __launch_bounds__(DecCfg<RMAX>::THREADS, (DecCfg<RMAX>::CTAS_PER_SM)) attn_decode_kernel(AttnParams p) {
-  pdl_trigger();
   using Cfg = DecCfg<RMAX>;
   constexpr int VW = RMAX % 4 == 0 ? 4 : 2;          // rows per access of shared memory
   constexpr int ST = Cfg::STAGES, D = Cfg::D, NB = Cfg::NB;
@@ -186,6 +185,7 @@ __global__ void __launch_bounds__(DecCfg<RMAX>::THREADS, (DecCfg<RMAX>::CTAS_PER
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   pdl_wait();          // the queries and this step's K/V rows come from the kernel before this one
 

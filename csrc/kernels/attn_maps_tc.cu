@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) maps_tc_kernel(MapsParams p, Ma
   float* s_tab = reinterpret_cast<float*>(s_item + 2);          // [group][tab_ld]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_trigger();
   pdl_wait();
   if (warp == 8) {
     // which sequence and row block this CTA has: the long sequences' blocks in order
@@ -103,6 +102,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) maps_tc_kernel(MapsParams p, Ma
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   const int b = s_item[0], q0 = s_item[1];
   const int g = blockIdx.y, bb = max(b, 0);

@@ -86,7 +86,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  pdl_trigger();        // this CTA holds its tensor memory: a dependent kernel that becomes resident cannot block it
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {

@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
                                                                               const __grid_constant__ CUtensorMap tmS, const FpParams p) {
   using Cfg = FpCfg<CN>;
   constexpr int STAGES = Cfg::STAGES, NBUF = Cfg::NBUF, SLOTS = Cfg::SLOTS;
-  pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);      // the same offset in every CTA of the cluster
   uint8_t* sA = base;
@@ -104,6 +103,7 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
   cluster_arrive();                         // the peers' barriers are initialised before anything signals them
   cluster_wait();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
 

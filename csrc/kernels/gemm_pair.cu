@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN, MODE>::THREADS, 1) gemm_pair
   using Cfg = PairCfg<KIND, CN, MODE>;
   constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, ATOMS = Cfg::SF_ATOMS, UB = Cfg::UB;
   constexpr bool GROUPED = MODE == kPairExperts, SPLIT = MODE == kPairSplit;
-  pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
   // both CTAs of a pair round the same way: dynamic shared memory starts at the same offset in each
   uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -167,6 +166,7 @@ __global__ void __launch_bounds__(PairCfg<KIND, CN, MODE>::THREADS, 1) gemm_pair
   cluster_arrive();                         // the peer's barriers are initialised before anything signals them
   cluster_wait();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   pdl_wait();
 

@@ -100,7 +100,6 @@ template <int KIND, int BN, bool OUT_F32>
 __global__ void __launch_bounds__(192, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmSA,
                const __grid_constant__ CUtensorMap tmSB, GemmParams p) {
-  pdl_trigger();
   using Cfg = GemmCfg<KIND, BN>;
   constexpr int BM = Cfg::BM, BK = Cfg::BK, STAGES = Cfg::STAGES, ACC = Cfg::ACC_BUFS;
   extern __shared__ uint8_t smem_raw[];
@@ -138,6 +137,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   if (threadIdx.x == 0) GT_STAMP(0);
 

@@ -83,7 +83,6 @@ template <int KIND, int BN, bool SWAP>
 __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                                                             const __grid_constant__ CUtensorMap tmSA, const __grid_constant__ CUtensorMap tmSB,
                                                             const WideParams p) {
-  pdl_trigger();
   using Cfg = WideCfg<KIND, BN>;
   constexpr int STAGES = Cfg::STAGES, BK = Cfg::BK, CPT = Cfg::CPT;
   extern __shared__ uint8_t smem_raw[];
@@ -124,6 +123,7 @@ __global__ void __launch_bounds__(320, 1) gemm_wide_kernel(const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   constexpr uint32_t SF_COL0 = BN;
   pdl_wait();

@@ -399,7 +399,6 @@ __global__ void __launch_bounds__(lr_threads(R), R <= 32 ? 2 : 1) latent_rows_ke
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, H = p.heads, D = p.D, ST = p.stages;
   const int b = blockIdx.y, rb = blockIdx.x / p.splits, split = blockIdx.x % p.splits;
-  pdl_trigger();
   pdl_wait();
   const int r0 = p.q_start[b], qlen = p.q_start[b + 1] - r0, rows = qlen * H;
   if (qlen <= 0 || qlen > p.max_tokens || rb * R >= rows) return;
@@ -442,6 +441,7 @@ __global__ void __launch_bounds__(lr_threads(R), R <= 32 ? 2 : 1) latent_rows_ke
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_trigger();        // after the allocation (sm100.cuh)
   const uint32_t tmem = *tmem_slot;
   if (warp == kLoader) {
     // -------------------------------------------------------------- page loader

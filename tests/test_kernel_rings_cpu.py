@@ -43,3 +43,25 @@ def test_few_rows_ctas_leave_after_their_copies_and_their_peers():
     order = [end.index(s) for s in ("__syncthreads();", "if (threadIdx.x == 0 && *abort_flag)", "mbar_wait(&full[", "mbar_wait(&sa_full[",
                                     "cluster_arrive();", "cluster_wait();", "tmem_dealloc(")]
     assert order == sorted(order)
+
+
+def _kernels():
+    """(name, body) of every kernel."""
+    folder = os.path.dirname(SRC)
+    for f in sorted(os.listdir(folder)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(folder, f)).read())
+        for part in re.split(r"__global__ ", text)[1:]:
+            body = part[:part.index("\n}\n") + 3]
+            yield f + ": " + re.search(r"(\w+)\s*\((?!\()(?:[^()]|\([^()]*\))*\)\s*\{", body[body.index("void"):]).group(1), body
+
+
+def test_dependents_may_start_when_tensor_memory_is_allocated():
+    """The successor of a kernel may become resident beside it and take tensor memory, which it holds until this kernel has completed: each
+    CTA has its own before it lets the successor start."""
+    seen = 0
+    for name, body in _kernels():
+        if "tmem_alloc" in body and "pdl_trigger" in body:
+            seen += 1
+            between = body[body.index("tmem_alloc"):body.index("pdl_trigger")] if body.index("tmem_alloc") < body.index("pdl_trigger") else ""
+            assert "__syncthreads();" in between, name
+    assert seen >= 8
