@@ -6,9 +6,9 @@
 // in turn) and their barriers: waits and commits per block cost as much as its products.
 //
 // Persistent, one pair per two SMs.  The token scales come by a tensor map into a ring of 8 slots in each CTA, with barriers of their own,
-// since they outlive the operands' stage: when a producer fills the slot of step i it has seen the MMAs of step i - STAGES complete, which
-// waited until the buffer of step i - STAGES - NBUF was handed back, and a warp hands a buffer back after it has read the scales of the step
-// before.  So STAGES + NBUF + 1 slots do.
+// since they outlive the operands' stage: `sa_full`, and `sa_empty`, on which every epilogue warp of the CTA arrives when it has read a slot.
+// (A buffer that is handed back says so too, but only of tensor memory, and to the MMA warp of the first CTA.)  A slot is filled STAGES
+// steps ahead of its products, which wait for the reading of a step NBUF before theirs, so with 8 slots that wait holds nothing up.
 //
 // Against one CTA per 128 x 128 tile, and one or a cluster of CTAs per 128 features up to 64 rows (us, inputs from memory): 64 rows x 10240 x
 // 5120 24.8 -> 17.2, x 5120 x 8192 23.9 -> 16.6, x 51200 x 5120 76 -> 58, x 5120 x 25600 47 -> 37; 128 rows of those 27 -> 19.5, 32 ->
@@ -51,8 +51,7 @@ struct FpCfg {
   static constexpr int EPI = CN / 8;                        // epilogue warps: one per lane quadrant and 32 columns
   static constexpr int THREADS = 64 + EPI * 32;
   static constexpr int SMEM = STAGES * STAGE_BYTES + SLOTS * CN * 8 + 1024 + 512;
-  static_assert(STAGES + NBUF + 1 <= SLOTS, "a scale slot is read before it is filled again");
-  static_assert((2 * STAGES + 2 * NBUF + SLOTS + 3) * 8 + 8 <= 512 && SMEM <= 227 * 1024, "shared memory");
+  static_assert((2 * STAGES + 2 * NBUF + 2 * SLOTS + 3) * 8 + 8 <= 512 && SMEM <= 227 * 1024, "shared memory");
 };
 
 template <int CN, bool SPLIT>
@@ -70,7 +69,8 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
   uint64_t* part_full = empty + STAGES;     // [NBUF] a block's products are complete
   uint64_t* part_empty = part_full + NBUF;  // [NBUF] both CTAs' epilogue warps have read them
   uint64_t* sa_full = part_empty + NBUF;    // [SLOTS]
-  uint64_t* drain = sa_full + SLOTS;
+  uint64_t* sa_empty = sa_full + SLOTS;     // [SLOTS] this CTA's epilogue warps have read a slot
+  uint64_t* drain = sa_empty + SLOTS;
   uint64_t* ring_free = drain + 1;          // every CTA of the split is done with its operands (its ring may be written)
   uint64_t* part_ready = ring_free + 1;     // and has handed out its sums
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(part_ready + 1);
@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < NBUF; ++i) { mbar_init(&part_full[i], 1); mbar_init(&part_empty[i], 2 * Cfg::EPI); }
-    for (int i = 0; i < SLOTS; ++i) mbar_init(&sa_full[i], 1);
+    for (int i = 0; i < SLOTS; ++i) { mbar_init(&sa_full[i], 1); mbar_init(&sa_empty[i], Cfg::EPI); }
     mbar_init(drain, 1);
     mbar_init(ring_free, ks);
     mbar_init(part_ready, ks);
@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
         tile_at(u, ft, t0);
         for (int kb = kb0; kb < kb1; ++kb, ++gb) {
           if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, p.status)) { ok = false; break; }
+          if (gb >= SLOTS && !mbar_wait(&sa_empty[gb % SLOTS], (gb / SLOTS - 1) & 1, abort_flag, p.status)) { ok = false; break; }
           const uint32_t bar = mapa_shared(smem_u32(&full[s]), lead);
           if (rank == 0) mbar_expect_tx(&full[s], 2u * Cfg::STAGE_BYTES);
           // (an odd number of blocks: the last one's neighbour lies beyond K and is filled with zeros)
@@ -229,6 +230,8 @@ __global__ void __launch_bounds__(FpCfg<CN>::THREADS, 1) gemm_fp8_pair_kernel(co
             fma_scaled_pair(acc[4 * j + 2], acc[4 * j + 3], r[4 * j + 2], r[4 * j + 3], s4.z, s4.w, w[h]);
           }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sa_empty[slot]);
       }
       const float bias = p.bias && feat_ok ? bf2f(p.bias[feat]) : 0.f;
       // finished sums of the columns [c, c + NC) of the tile

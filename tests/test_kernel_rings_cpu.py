@@ -65,3 +65,17 @@ def test_dependents_may_start_when_tensor_memory_is_allocated():
             between = body[body.index("tmem_alloc"):body.index("pdl_trigger")] if body.index("tmem_alloc") < body.index("pdl_trigger") else ""
             assert "__syncthreads();" in between, name
     assert seen >= 8
+
+
+def test_scales_of_a_pair_are_handed_back_by_the_warps_that_read_them():
+    """FP8 product on CTA pairs: a slot of the scales' ring is filled again when every epilogue warp of the same CTA has released it, behind
+    its last access.  (Handing back an accumulator orders tensor memory alone, and goes to the other CTA.)"""
+    text = open(os.path.join(os.path.dirname(SRC), "gemm_fp8_pair.cu")).read()
+    body = re.sub(r"//[^\n]*", "", text[text.index("gemm_fp8_pair_kernel("):])
+    assert "mbar_init(&sa_empty[i], Cfg::EPI)" in body
+    fill, read = body[body.index("if (warp == 0)"):body.index("else if (warp == 1)")], body[body.index("float acc[32];"):]
+    wait = fill.index("if (gb >= SLOTS && !mbar_wait(&sa_empty[gb % SLOTS], (gb / SLOTS - 1) & 1,")
+    assert wait < fill.index("mbar_expect_tx(") and wait < fill.index("tma_load_2d_pair(sSA")
+    after = read[read.index("= sa[j];"):]
+    assert after.index("__syncwarp();") < after.index("mbar_arrive(&sa_empty[slot]") < after.index("finish")
+    assert read.count("sa[j]") == 1
