@@ -594,6 +594,16 @@ class CudaOps:
             if rc != 0:
                 raise CudaError(f"blz_gemm_wait_flags failed: {rc}")
             x.wait = None
+        sk_able = not f32 and argmax_parts is None and pending is None and not kt
+        if self.tuning is not None and sk_able and act == 0 and wide is None and bn == 0 and sk is None and not max_ctas:
+            # a table measured on this device (tune.tune_linear): where a variant was faster than what the rules below pick
+            from ..tune import bucket
+            hit = self.tuning.get(f"gemm{kind}", lin.N, lin.K, bucket(M))
+            if hit is not None and hit["ms"] < hit.get("rule_ms", 0.0):
+                if hit["kernel"] == "tc":
+                    wide, bn, sk = False, hit["bn"], False
+                elif self._sk_ok and M <= self.SK_MAX_ROWS:
+                    sk = hit["ks"]
         pair = (wide is None and self._wide_ok and bn == 0 and kind in (0, 1, 2) and lin.N >= 128 and not kt and pending is None
                 and argmax_parts is None and max_ctas != 1 and not relu2 and (sk is None or sk is False)
                 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0)) and (not swiglu or lin.N % 32 == 0))
@@ -611,19 +621,12 @@ class CudaOps:
                                                  _ptr(pk["alpha"]), _ptr(bias), sfa, _ptr(sfw), 0, act, limit,
                                                  self._stream()), f"gemm_narrow kind {kind}")
             return out
-        sk_able = not f32 and argmax_parts is None and pending is None and not kt
         if sk is None:
             sk = False
             if self._sk_ok and sk_able and wide is None and bn == 0 and M <= self.SK_MAX_ROWS:
-                # Splitting K over a cluster pays where K is long and the tiles are few.  A tuning table measured on this device
-                # (tune.tune_linear) overrides the rule.
+                # splitting K over a cluster pays where K is long and the tiles are few
                 tiles = ((M + 127) // 128) * ((lin.N + 127) // 128)
                 sk = not pair and lin.K >= 8192 and tiles <= 2 * self._sm // 2
-                if self.tuning is not None:
-                    from ..tune import bucket
-                    hit = self.tuning.get(f"gemm{kind}", lin.N, lin.K, bucket(M))
-                    if hit is not None:
-                        sk = False if hit.get("kernel") != "sk" else (hit.get("ks") or True)
         if sk is not False and sk is not None:
             if not sk_able:
                 raise CudaError("the split-K GEMM writes bf16 from row-major weights and has no arg-max / peer-wait epilogue")

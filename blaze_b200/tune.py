@@ -2,8 +2,8 @@
 
 Reference: ``crates/blaze/src/tune.rs`` (row ``BUCKETS`` :13, candidates split x tiles :129, cache file
 ``~/.cache/blaze/tune-sm*.json`` :182, ``tune`` :243) and ``attn_tune.rs`` (attention split cache per GPU / rank).
-Here the tunables are the GEMM N-tile (128 / 256) and CTA cap per (kind, N, K, row bucket), and the kv-split count of
-the decode attention kernel per (batch bucket, context bucket).
+Here the tunables are the kernels that a linear layer could take instead of the one that ``CudaOps.linear`` picks by its rules, per
+(kind, N, K, row bucket): the table keeps the fastest of them beside the time of the rules' own pick, and is followed where it won.
 """
 from __future__ import annotations
 
@@ -78,8 +78,8 @@ class Tuning:
 
 
 def gemm_candidates(kind: int, N: int, K: int, rows: int):
-    """Kernel variants worth timing for one linear layer at ``rows`` rows: the one-CTA-per-tile kernel with 128- or
-    256-column tiles, and for decode-sized steps the cluster split-K kernel with its K-slice counts."""
+    """Kernel variants worth timing against the rules' own pick for one linear layer at ``rows`` rows: the one-CTA-per-tile kernel with
+    128- or 256-column tiles, and for decode-sized steps the cluster split-K kernel with its K-slice counts."""
     out = [{"kernel": "tc", "bn": 128}]
     if N % 256 == 0 and rows > 128:
         out.append({"kernel": "tc", "bn": 256})
@@ -92,7 +92,7 @@ def gemm_candidates(kind: int, N: int, K: int, rows: int):
 
 
 def tune_linear(ops, lin, rows: int, tuning: Tuning, iters: int = 5) -> Dict:
-    """Pick the N-tile for ``lin`` at ``rows`` rows on the current device."""
+    """The fastest variant for ``lin`` at ``rows`` rows on the current device (``ms``), and what the rules' own pick takes (``rule_ms``)."""
     import torch
     pk = ops.pack(lin)
     x = torch.randn(rows, lin.K, device=ops.device).bfloat16()
@@ -101,7 +101,9 @@ def tune_linear(ops, lin, rows: int, tuning: Tuning, iters: int = 5) -> Dict:
     out = torch.empty(rows, lin.N, dtype=torch.bfloat16, device=ops.device)
 
     def call(cfg):
-        if cfg["kernel"] == "sk":
+        if cfg["kernel"] == "rule":
+            ops.linear(lin, xin, out=out)
+        elif cfg["kernel"] == "sk":
             ops.linear(lin, xin, out=out, sk=cfg["ks"])
         else:
             ops.linear(lin, xin, out=out, bn=cfg["bn"], wide=False, sk=False)
@@ -121,12 +123,23 @@ def tune_linear(ops, lin, rows: int, tuning: Tuning, iters: int = 5) -> Dict:
         e1.record()
         torch.cuda.synchronize()
         return e0.elapsed_time(e1) / iters
-    return tuning.tune(f"gemm{pk['kind']}", (lin.N, lin.K, bucket(rows)), gemm_candidates(pk["kind"], lin.N, lin.K, rows), run)
+    kind, shape = f"gemm{pk['kind']}", (lin.N, lin.K, bucket(rows))
+    if "rule_ms" not in (tuning.get(kind, *shape) or {"rule_ms": 0}):
+        del tuning.table[tuning.key(kind, *shape)]        # from a table that did not know the rules' pick: time all of them anew
+    best = tuning.tune(kind, shape, gemm_candidates(pk["kind"], lin.N, lin.K, rows), run)
+    if "rule_ms" not in best:
+        table, ops.tuning = ops.tuning, None
+        try:
+            best["rule_ms"] = round(run({"kernel": "rule"}), 5)
+        finally:
+            ops.tuning = table
+        tuning.dirty = True
+    return best
 
 
 def tune_model(model, rows: Iterable[int] = (256,), tuning: Optional[Tuning] = None, save: bool = True) -> Tuning:
     """Time the kernel variants of every distinct linear shape of ``model`` at the given row counts and install the table
-    on its op set (``ops.tuning``), so that ``CudaOps.linear`` picks the measured winner per (format, N, K, row bucket).
+    on its op set (``ops.tuning``), so that ``CudaOps.linear`` takes the measured winner per (format, N, K, row bucket).
     The table is kept in the JSON cache of this device, so later runs only load it (reference: the start-up GEMV tuning of
     ``crates/blaze/src/model.rs:1568-1590`` and ``tune.rs:243``)."""
     ops = model.ops

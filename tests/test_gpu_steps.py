@@ -569,3 +569,26 @@ def test_quantised_norm_adds_squares_like_the_plain_one(ops, mode, T, W):      #
     assert torch.equal(got.data, want.data)
     assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, T, W // per) for q in (got, want)))
     assert mode != Format.NVFP4 or torch.equal(got.row_scale, want.row_scale)
+
+
+def test_a_tuned_route_is_taken_where_it_beat_the_rules(ops, tmp_path, monkeypatch):      # noqa: F811
+    """An entry of the tuning table counts where its kernel was faster than what the rules pick; one that was measured without the rules'
+    time does not count, and is measured anew."""
+    from blaze_b200 import tune
+    g = torch.Generator(device=DEV).manual_seed(41)
+    lin = Linear.from_dense(torch.randn(512, 8192, generator=g, device=DEV) * 0.02)
+    x = torch.randn(200, 8192, generator=g, device=DEV).bfloat16()
+    rule = ops.linear(lin, x)
+    by = {ks: ops.linear(lin, x, sk=ks) for ks in (1, 2, 3, 5, 7)}
+    ks = next(k for k in by if not torch.equal(by[k], rule))          # (parts of K add up in another order)
+    t = tune.Tuning(str(tmp_path / "t.json"))
+    monkeypatch.setattr(ops, "tuning", t)
+    for entry, want in (({"ms": 1.0, "rule_ms": 2.0}, by[ks]), ({"ms": 2.0, "rule_ms": 1.0}, rule), ({"ms": 1.0}, rule)):
+        t.table = {"gemm0:512x8192x256": {"kernel": "sk", "ks": ks, **entry}}
+        assert torch.equal(ops.linear(lin, x), want), entry
+    best = tune.tune_linear(ops, lin, 200, t, iters=3)
+    assert best["rule_ms"] > 0 and best == t.get("gemm0", 512, 8192, 256) and ops.tuning is t
+    t.table["gemm0:512x8192x256"] = {"kernel": "tc", "bn": 256, "ms": 1.0, "rule_ms": 2.0}
+    assert torch.equal(ops.linear(lin, x), ops.linear(lin, x, bn=256, wide=False, sk=False))
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
