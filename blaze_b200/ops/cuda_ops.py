@@ -1521,7 +1521,9 @@ class CudaOps:
                     else:
                         self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act=int(dst is g), runs=runs)
             return RoutedRows(y, row_map, weights, shared, gate)
-        act = bool(gu["swiglu"]) if experts.act != "relu2" else False      # the gated activation is in the product's epilogue
+        # The gated activation is in the product's epilogue, or, behind the narrow product, in the quantiser: its epilogue has half of a
+        # warp's lanes store (NVFP4, 64 experts of 1408 x 2048, 6 per token, 512 tokens: a layer 105 us in the epilogue, 87 so).
+        act = bool(gu["swiglu"]) and not narrow if experts.act != "relu2" else False
         g = torch.empty(M_pad, gu["N"] // 2 if act else gu["N"], dtype=x.dtype, device=dev)
         if experts.act == "relu2":
             y = torch.empty(M_pad, dn["N"], dtype=x.dtype, device=dev)
@@ -1547,7 +1549,7 @@ class CudaOps:
                 self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act, runs=runs)
         product(gu, a, g, int(act))
         # only the routed rows: the padded row space is up to (1 + experts * 128 / routed rows) times larger
-        product(dn, self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map, act), y)
+        product(dn, self._silu_mul_live(g, proxy_d if dn["kind"] in (1, 2) else None, row_map, 1 if act else 2 * bool(gu["swiglu"])), y)
         return RoutedRows(y, row_map, weights, shared, gate)
 
     def _moe_gemm(self, pk, a, row_tiles, tile_expert, tile_rows, n_exp, out, act: int = 0):
@@ -1563,21 +1565,22 @@ class CudaOps:
                                           row_tiles, pk["N"], pk["K"], n_exp, rs, _ptr(pk["alpha"]), sfa, _ptr(pk["sf"]),
                                           _ptr(tile_expert), _ptr(tile_rows), act, self._stream()), f"moe_gemm kind {kind}")
 
-    def _silu_mul_live(self, gu, quant_for, row_list, is_act: bool = False):
+    def _silu_mul_live(self, gu, quant_for, row_list, form: int = 0):
         """``silu_mul`` over the padded row space of the routed rows: only the rows named in ``row_list`` (-1 = none) are
-        touched, one CTA each.  ``is_act``: the rows are gated activations already, which are only quantised."""
-        T, I = gu.shape[0], gu.shape[1] if is_act else gu.shape[1] // 2
+        touched, one CTA each.  ``form`` 1: the rows are gated activations already, which are only quantised; 2: gate and up
+        values come in groups of 16 | 16."""
+        T, I = gu.shape[0], gu.shape[1] if form == 1 else gu.shape[1] // 2
         n = row_list.numel()
         mode = self._qmode(quant_for)
         if mode == 0:
-            if is_act:
+            if form == 1:
                 return gu
             out = _rows(T, I, torch.bfloat16, self.device)
-            self._check(self.lib.blz_swiglu_live(_ptr(gu), _ptr(out), None, None, None, n, I, 0, 0, _ptr(row_list), self._stream()),
+            self._check(self.lib.blz_swiglu_live(_ptr(gu), _ptr(out), None, None, None, n, I, 0, form, _ptr(row_list), self._stream()),
                         "swiglu_live")
             return out
         qa = self._alloc_qact(Format.NVFP4 if mode == 1 else Format.MXFP8, T, I)
-        self._check(self.lib.blz_swiglu_live(_ptr(gu), None, *qa.addresses(), n, I, mode, int(is_act),
+        self._check(self.lib.blz_swiglu_live(_ptr(gu), None, *qa.addresses(), n, I, mode, form,
                                              _ptr(row_list), self._stream()), "swiglu_live_q")
         return qa
 

@@ -156,10 +156,12 @@ __global__ void rmsnorm_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __r
 // ---------------------------------------------------------------------------------------------- SwiGLU (+quant)
 // gu [T, 2I] = [gate | up];  MODE 0: out bf16 [T, I];  MODE 1: NVFP4;  MODE 2: MXFP8.  Optional plain-row input
 // (gate_up == nullptr is invalid).  `src_is_act`: quantise `gu` itself ([T, I], no SwiGLU) — used for attention output.
+// `il` (here and in the kernels below): gate and up values in groups of 16 | 16, what a product of interleaved weights stores.
+__device__ __forceinline__ int gate_at(int i, int il) { return il ? 2 * i - (i & 15) : i; }
 template <int MODE>
 __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                               uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out, float* __restrict__ row_scale,
-                              int I, int src_is_act, int sf_col_tiles, const int* __restrict__ row_list) {
+                              int I, int src_is_act, int il, int sf_col_tiles, const int* __restrict__ row_list) {
   extern __shared__ __align__(16) uint8_t dyn[];
   __nv_bfloat16* row = reinterpret_cast<__nv_bfloat16*>(dyn);
   __shared__ float red[32];
@@ -167,13 +169,13 @@ __global__ void swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat1
   const int t = row_list ? row_list[blockIdx.x] : (int)blockIdx.x;
   if (t < 0) return;
   const __nv_bfloat16* g = gu + (size_t)t * (src_is_act ? I : 2 * I);
-  const __nv_bfloat16* u = g + I;
+  const __nv_bfloat16* u = g + (il ? 16 : I);
   float amax = 0.f;
   for (int i = threadIdx.x * 8; i < I; i += blockDim.x * 8) {
-    uint4 ug = *reinterpret_cast<const uint4*>(g + i);
+    uint4 ug = *reinterpret_cast<const uint4*>(g + gate_at(i, il));
     __nv_bfloat16* eg = reinterpret_cast<__nv_bfloat16*>(&ug);
     if (!src_is_act) {
-      uint4 uu = *reinterpret_cast<const uint4*>(u + i);
+      uint4 uu = *reinterpret_cast<const uint4*>(u + gate_at(i, il));
       const __nv_bfloat16* eu = reinterpret_cast<const __nv_bfloat16*>(&uu);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(256) rmsnorm_row16_kernel(__nv_bfloat16* __res
 // ACT: the source rows are activations already (no up half).
 template <int MODE, int CH, bool ACT>
 __global__ void __launch_bounds__(256) swiglu_row16_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ q_out,
-                                                             uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int I,
+                                                             uint8_t* __restrict__ sf_out, float* __restrict__ row_scale, int I, int il,
                                                              int sf_col_tiles, const int* __restrict__ row_list) {
   pdl_trigger();
   pdl_wait();
@@ -473,8 +475,8 @@ __global__ void __launch_bounds__(256) swiglu_row16_kernel(const __nv_bfloat16* 
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 16;
-    load16(a[c], src + i, i < I);
-    if constexpr (!ACT) load16(b[c], src + I + i, i < I);
+    load16(a[c], src + gate_at(i, il), i < I);
+    if constexpr (!ACT) load16(b[c], src + (il ? 16 : I) + gate_at(i, il), i < I);
   }
   float bm[CH], amax = 0.f;
 #pragma unroll
@@ -590,7 +592,7 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
 template <int MODE, int CH, bool ACT>
 __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                                            uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
-                                                           float* __restrict__ row_scale, int I, int sf_col_tiles,
+                                                           float* __restrict__ row_scale, int I, int il, int sf_col_tiles,
                                                            const int* __restrict__ row_list) {
   pdl_trigger();
   pdl_wait();
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
   const int t = row_list ? row_list[blockIdx.x] : (int)blockIdx.x;
   if (t < 0) return;
   const __nv_bfloat16* g = gu + (size_t)t * (ACT ? I : 2 * I);
-  const __nv_bfloat16* up = g + I;
+  const __nv_bfloat16* up = g + (il ? 16 : I);
   uint4 a[CH], b[ACT ? 1 : CH];
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
@@ -607,8 +609,8 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
     a[c] = make_uint4(0, 0, 0, 0);
     if constexpr (!ACT) b[c] = a[c];
     if (i < I) {
-      a[c] = *reinterpret_cast<const uint4*>(g + i);
-      if constexpr (!ACT) b[c] = *reinterpret_cast<const uint4*>(up + i);
+      a[c] = *reinterpret_cast<const uint4*>(g + gate_at(i, il));
+      if constexpr (!ACT) b[c] = *reinterpret_cast<const uint4*>(up + gate_at(i, il));
     }
   }
   float amax = 0.f;
@@ -648,7 +650,7 @@ __global__ void __launch_bounds__(512) swiglu_reg_kernel(const __nv_bfloat16* __
 template <int MODE>
 __global__ void __launch_bounds__(256) swiglu_rows_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                                             uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
-                                                            float* __restrict__ row_scale, int I, int src_is_act, int sf_col_tiles,
+                                                            float* __restrict__ row_scale, int I, int src_is_act, int il, int sf_col_tiles,
                                                             const int* __restrict__ row_list, int n_rows, int tpr) {
   pdl_trigger();
   pdl_wait();
@@ -663,8 +665,8 @@ __global__ void __launch_bounds__(256) swiglu_rows_kernel(const __nv_bfloat16* _
   uint4 a = make_uint4(0, 0, 0, 0), b = a;
   if (valid) {
     const __nv_bfloat16* g = gu + (size_t)t * (src_is_act ? I : 2 * I);
-    a = *reinterpret_cast<const uint4*>(g + i);
-    if (!src_is_act) b = *reinterpret_cast<const uint4*>(g + I + i);
+    a = *reinterpret_cast<const uint4*>(g + gate_at(i, il));
+    if (!src_is_act) b = *reinterpret_cast<const uint4*>(g + (il ? 16 : I) + gate_at(i, il));
   }
   __nv_bfloat16* eg = reinterpret_cast<__nv_bfloat16*>(&a);
   const __nv_bfloat16* eu = reinterpret_cast<const __nv_bfloat16*>(&b);
@@ -1198,7 +1200,7 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
   return (int)cudaGetLastError();
 }
 
-// mode as `quant` above; src_is_act = 1 quantises the [T, I] input as is (no SwiGLU).  blz_swiglu_live: T entries of row_list
+// mode as `quant` above; src_is_act = 1 quantises the [T, I] input as is (no SwiGLU), 2: gate and up values in groups of 16 | 16.  blz_swiglu_live: T entries of row_list
 // name the rows to process (-1 = skip): the live rows of the routed experts' padded row space.
 static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, float* row_scale, int T, int I,
                        int mode, int src_is_act, const int* row_list, cudaStream_t s);
@@ -1212,6 +1214,8 @@ BLZ_API int blz_swiglu_live(const void* gu, void* out, void* q_out, void* sf_out
 }
 static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, float* row_scale, int T, int I,
                        int mode, int src_is_act, const int* row_list, cudaStream_t s) {
+  const int il = src_is_act == 2;
+  if (il) src_is_act = 0;
   if (I % 32 || T < 0) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
   const int thr = norm_threads(I);
@@ -1230,9 +1234,9 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
     const int tpr = (I / 8 + 31) / 32 * 32, rows_per = tpr <= 128 ? 256 / tpr : 1;
     if (I <= 1024 && rows_per >= 2) {
       const dim3 grid((T + rows_per - 1) / rows_per), block(rows_per * tpr);
-      if (mode == 0) launch_pdl(swiglu_rows_kernel<0>, grid, block, 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, src_is_act, 0, row_list, T, tpr);
-      else if (mode == 1) launch_pdl(swiglu_rows_kernel<1>, grid, block, 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list, T, tpr);
-      else launch_pdl(swiglu_rows_kernel<2>, grid, block, 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list, T, tpr);
+      if (mode == 0) launch_pdl(swiglu_rows_kernel<0>, grid, block, 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, src_is_act, il, 0, row_list, T, tpr);
+      else if (mode == 1) launch_pdl(swiglu_rows_kernel<1>, grid, block, 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, il, ct, row_list, T, tpr);
+      else launch_pdl(swiglu_rows_kernel<2>, grid, block, 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, il, ct, row_list, T, tpr);
       return (int)cudaGetLastError();
     }
   }
@@ -1240,7 +1244,7 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   reg_shape(I, T, &rt, &ch);
   if (mode && I <= ROW16_MOST && (src_is_act || T >= 512)) {
     const int c16 = (I + 4095) / 4096;
-#define BLZ_SW2(Q, C, ACT) launch_pdl(swiglu_row16_kernel<Q, C, ACT>, dim3(T), dim3(row16_threads(I, C)), 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
+#define BLZ_SW2(Q, C, ACT) launch_pdl(swiglu_row16_kernel<Q, C, ACT>, dim3(T), dim3(row16_threads(I, C)), 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, il, ct, row_list)
 #define BLZ_SW(C) if (mode == 1) { if (src_is_act) BLZ_SW2(1, C, true); else BLZ_SW2(1, C, false); } else { if (src_is_act) BLZ_SW2(2, C, true); else BLZ_SW2(2, C, false); }
     BLZ_CH_SWITCH(c16, BLZ_SW)
 #undef BLZ_SW
@@ -1249,17 +1253,17 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   }
   if (ch && !(mode && src_is_act)) {
 #define BLZ_SW(C)                                                                                                              \
-  if (src_is_act) launch_pdl(swiglu_reg_kernel<0, C, true>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
-  else if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, 0, row_list); \
-  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list); \
-  else launch_pdl(swiglu_reg_kernel<2, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list)
+  if (src_is_act) launch_pdl(swiglu_reg_kernel<0, C, true>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, il, 0, row_list); \
+  else if (mode == 0) launch_pdl(swiglu_reg_kernel<0, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)out, (uint8_t*)nullptr, (uint8_t*)nullptr, (float*)nullptr, I, il, 0, row_list); \
+  else if (mode == 1) launch_pdl(swiglu_reg_kernel<1, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, il, ct, row_list); \
+  else launch_pdl(swiglu_reg_kernel<2, C, false>, dim3(T), dim3(rt), 0, s, (const bf16*)gu, (bf16*)nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, il, ct, row_list)
     BLZ_CH_SWITCH(ch, BLZ_SW)
 #undef BLZ_SW
     return (int)cudaGetLastError();
   }
-  if (mode == 0) swiglu_kernel<0><<<T, thr, 0, s>>>((const bf16*)gu, (bf16*)out, nullptr, nullptr, nullptr, I, src_is_act, 0, row_list);
-  else if (mode == 1) swiglu_kernel<1><<<T, thr, sm, s>>>((const bf16*)gu, nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list);
-  else swiglu_kernel<2><<<T, thr, sm, s>>>((const bf16*)gu, nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, ct, row_list);
+  if (mode == 0) swiglu_kernel<0><<<T, thr, 0, s>>>((const bf16*)gu, (bf16*)out, nullptr, nullptr, nullptr, I, src_is_act, il, 0, row_list);
+  else if (mode == 1) swiglu_kernel<1><<<T, thr, sm, s>>>((const bf16*)gu, nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, il, ct, row_list);
+  else swiglu_kernel<2><<<T, thr, sm, s>>>((const bf16*)gu, nullptr, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, src_is_act, il, ct, row_list);
   return (int)cudaGetLastError();
 }
 

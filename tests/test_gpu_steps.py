@@ -592,3 +592,35 @@ def test_a_tuned_route_is_taken_where_it_beat_the_rules(ops, tmp_path, monkeypat
     assert torch.equal(ops.linear(lin, x), ops.linear(lin, x, bn=256, wide=False, sk=False))
     torch.cuda.synchronize()
     assert ops.take_status() == 0
+
+
+@pytest.mark.parametrize("fmt", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("I", [32, 192, 704, 1056, 4128, 24608])
+def test_interleaved_gate_and_up_rows(ops, fmt, I):      # noqa: F811
+    """Gate and up values in groups of 16 | 16, as the narrow experts' product stores them, few rows and many: the codes and scales of the
+    same values side by side."""
+    g = torch.Generator(device=DEV).manual_seed(17)
+    lin = Linear(fmt, 128, I)
+    lin.act_quant = True
+    gu = torch.randn(600, 2 * I, generator=g, device=DEV).bfloat16()
+    mixed = gu.view(600, 2, I // 16, 16).transpose(1, 2).reshape(600, 2 * I)
+    per = 16 if fmt == Format.NVFP4 else 32
+    for n in (40, 600):
+        rows = torch.randperm(600, generator=torch.Generator().manual_seed(2))[:n].to(torch.int32).to(DEV)
+        a, b = ops._silu_mul_live(gu, lin, rows), ops._silu_mul_live(mixed, lin, rows, 2)
+        at = rows.long()
+        assert torch.equal(a.data[at], b.data[at]) and (fmt == Format.MXFP8 or torch.equal(a.row_scale[at], b.row_scale[at]))
+        assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, q.rows, I // per)[at] for q in (a, b)))
+        assert torch.equal(ops._silu_mul_live(gu, None, rows)[at], ops._silu_mul_live(mixed, None, rows, 2)[at])
+
+
+def test_narrow_experts_leave_the_activation_to_the_quantiser(ops, monkeypatch):      # noqa: F811
+    """Features that are no multiple of 256: the narrow product, whose epilogue is slow at it, stores gate and up sums."""
+    acts = []
+    real = ops._moe_gemm
+    monkeypatch.setattr(ops, "_moe_gemm", lambda *a, **k: (acts.append((list(a[7:]) + [k.get("act", 0)])[0]), real(*a, **k))[1])
+    x = torch.randn(40, 256, generator=torch.Generator(device=DEV).manual_seed(3), device=DEV).bfloat16()
+    ex = _experts(8, 256, 192, Format.NVFP4, 9)
+    w, ids = ops.router_topk(torch.randn(40, 8, device=DEV), 2, True, 0, 8)
+    out = ops.moe(x, w, ids, ex)
+    assert acts == [0, 0] and _rel(out, ref.moe_forward(x, w, ids, ex.forward_one, 8)) < 0.08
