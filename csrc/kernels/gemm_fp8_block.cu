@@ -504,6 +504,28 @@ static cudaError_t launch_fp8_rows(const FbParams& p, int ks, const void* A, lon
 // take the same four groups of eight neighbouring rows, so that the scales' 4-byte stores, ld_s apart within a warp, fill 32-byte sectors.
 // us, one warp per group with 4 elements a thread / now: 4096 rows of 25600 155 / 85, 825 rows 38 / 24, 64 rows 9.2 / 9.2; with the
 // gated activation (a kernel of its own before): 4096 rows 269 / 150, 825 rows 65 / 38, 64 rows 17.4 / 11.2, of 5120 13.3 / 9.2.
+// Plain rows of fewer than 3 x 2^18 elements are the warp's per group: so little work is bound by the longer chain of 16 divisions per
+// thread (back to back, 4 / 16 elements a thread: 1 row of 5120 1.93 / 2.26, 16 rows 2.04 / 2.46, 64 x 2048 2.09 / 2.58, 64 x 7168
+// 2.39 / 2.68, 128 x 5120 2.60 / 2.85; 150 x 5120 2.80 / 2.79, 64 x 12288 2.93 / 2.80).
+__global__ void __launch_bounds__(256)
+quant_fp8_few_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q, float* __restrict__ scales,
+                     long long ld_s, int T, int K) {
+  pdl_wait();
+  pdl_trigger();
+  const int groups = K / 128, lane = threadIdx.x & 31;
+  const int g = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+  if (g >= T * groups) return;
+  const int row = g / groups, kb = g % groups;
+  const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)row * ldx + kb * 128 + lane * 4);
+  const float v[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)};
+  const float m = warp_max(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+  const float scale = fmaxf(m / 448.f, 1e-12f);
+  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[0] / scale, v[1] / scale), __NV_SATFINITE, __NV_E4M3);
+  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[2] / scale, v[3] / scale), __NV_SATFINITE, __NV_E4M3);
+  *reinterpret_cast<uint32_t*>(q + (size_t)row * K + kb * 128 + lane * 4) = lo | hi << 16;
+  if (lane == 0) scales[(size_t)kb * ld_s + row] = scale;
+}
+
 template <bool GATED>
 __global__ void __launch_bounds__(256)
 quant_fp8_block_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q, float* __restrict__ scales,
@@ -557,22 +579,13 @@ quant_fp8_block_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8
 
 template <bool GATED>
 static cudaError_t launch_quant_fp8(const void* x, long long ldx, void* q, float* scales, long long ld_s, int T, int K, cudaStream_t stream) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((long long)((T + 7) / 8) * ((K + 511) / 512)));
-  cfg.blockDim = dim3(256);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  int n = 0;
-  if (pdl_enabled()) {
-    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = n;
+  const __nv_bfloat16* rows = reinterpret_cast<const __nv_bfloat16*>(x);
+  uint8_t* codes = reinterpret_cast<uint8_t*>(q);
+  if (!GATED && (long long)T * K < 3 << 18)
+    return launch_pdl(quant_fp8_few_kernel, dim3((unsigned)((T * (K / 128) + 7) / 8)), dim3(256), 0, stream, rows, ldx, codes, scales, ld_s, T, K);
   const int on16 = ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  return cudaLaunchKernelEx(&cfg, quant_fp8_block_kernel<GATED>, reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<uint8_t*>(q),
-                            scales, ld_s, T, K, on16);
+  return launch_pdl(quant_fp8_block_kernel<GATED>, dim3((unsigned)((long long)((T + 7) / 8) * ((K + 511) / 512))), dim3(256), 0, stream, rows, ldx,
+                    codes, scales, ld_s, T, K, on16);
 }
 
 }  // namespace blz

@@ -624,3 +624,17 @@ def test_narrow_experts_leave_the_activation_to_the_quantiser(ops, monkeypatch):
     w, ids = ops.router_topk(torch.randn(40, 8, device=DEV), 2, True, 0, 8)
     out = ops.moe(x, w, ids, ex)
     assert acts == [0, 0] and _rel(out, ref.moe_forward(x, w, ids, ex.forward_one, 8)) < 0.08
+
+
+@pytest.mark.parametrize("T,K", [(1535, 512), (191, 4096), (95, 8192), (6143, 128)])
+def test_fp8_groups_of_few_elements(ops, T, K):      # noqa: F811
+    """The last row counts whose groups are a warp's each, and one row more: the same codes and scales, also of rows that start on 8 bytes,
+    and of infinities and values that are not numbers."""
+    x = torch.randn(T + 1, K, generator=torch.Generator(device=DEV).manual_seed(14), device=DEV).bfloat16()
+    x[0, :3] = torch.tensor([float("inf"), float("nan"), -0.0], device=DEV)
+    x[T // 2, :128] = 0
+    wide = torch.zeros(T, K + 4, dtype=torch.bfloat16, device=DEV)
+    wide[:, 4:] = x[:T]
+    (qa, sa), (q, s), (q8, s8) = ops.quantize_fp8_block(x), ops.quantize_fp8_block(x[:T]), ops.quantize_fp8_block(wide[:, 4:])
+    assert T * K < 3 << 18 <= (T + 1) * K
+    assert torch.equal(q, qa[:T]) and torch.equal(s[:, :T], sa[:, :T]) and torch.equal(q8, q) and torch.equal(s8[:, :T], s[:, :T])
