@@ -1146,7 +1146,7 @@ static inline void reg_shape(int W, int T, int* threads, int* chunks) {
   }
 
 // The quantising row kernels with 16 elements per thread: rows of up to 6 chunks of 256 threads.  At any number of rows where rows are
-// normed or are activations already (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norms, from
+// normed or are activations already (but for those of 513 - 1024, see there) (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norms, from
 // cold caches, of 825 rows of 4096 14.3 / 12.3, 3000 of 5120 34.8 / 28.7, 2000 of 12320 76 / 49), for gated rows from 512 on (825 rows of 12288 19.8 / 17.1, 256 rows 7.6 / 8.3: their
 // activation is the longer chain per thread there; the experts' short gated rows likewise 43.7 / 46.2).
 constexpr int ROW16_MOST = 6 * 256 * 16;
@@ -1223,8 +1223,11 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   const int ct = mode == 1 ? (I + 63) / 64 : (I + 127) / 128;
   configure_once();
   {
+    // Two warps of 16 elements a thread lose to three or four of 8 while all rows are few (us, 8 / 16 elements a thread: NVFP4 4 rows of 768
+    // 2.40 / 2.76, 512 rows 2.44 / 2.90, 1024 rows 2.74 / 2.93, 4 rows of 1024 2.22 / 2.48, 150 rows 2.52 / 2.74; MXFP8 4 rows of 768
+    // 2.04 / 2.43; but 4096 rows of 1024 in NVFP4 6.25 / 4.20); one warp does not (4 rows of 512 2.30 / 2.39).
     const int tpr16 = (I / 16 + 31) / 32 * 32;
-    if (mode && src_is_act && I <= 1024) {
+    if (mode && src_is_act && I <= 1024 && (I <= 512 || (long long)T * I > 3 << 18)) {
       const int per = 256 / tpr16;
       const dim3 grid((T + per - 1) / per), block(per * tpr16);
       if (mode == 1) launch_pdl(quant_rows16_kernel<1>, grid, block, 0, s, (const bf16*)gu, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, I, ct, row_list, T, tpr16);

@@ -638,3 +638,19 @@ def test_fp8_groups_of_few_elements(ops, T, K):      # noqa: F811
     (qa, sa), (q, s), (q8, s8) = ops.quantize_fp8_block(x), ops.quantize_fp8_block(x[:T]), ops.quantize_fp8_block(wide[:, 4:])
     assert T * K < 3 << 18 <= (T + 1) * K
     assert torch.equal(q, qa[:T]) and torch.equal(s[:, :T], sa[:, :T]) and torch.equal(q8, q) and torch.equal(s8[:, :T], s[:, :T])
+
+
+@pytest.mark.parametrize("mode", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("T,W", [(1024, 768), (768, 1024), (1445, 544), (1536, 512)])
+def test_quantised_short_rows_of_few_elements(ops, mode, T, W):      # noqa: F811
+    """The last row counts with 8 elements per thread, one row more, and rows of one warp: the same codes and scales."""
+    lin = Linear(mode, 128, W)
+    lin.act_quant = True
+    x = torch.randn(T + 1, W, generator=torch.Generator(device=DEV).manual_seed(15), device=DEV).bfloat16()
+    x[0, :3] = torch.tensor([float("inf"), float("nan"), -0.0], device=DEV)
+    x[T // 2] = 0
+    assert T * W <= 3 << 18 < (T + 1) * W
+    few, many = ops.quantize_rows(x[:T], lin), ops.quantize_rows(x, lin)
+    per = 16 if mode == Format.NVFP4 else 32
+    assert torch.equal(few.data, many.data[:T]) and (mode == Format.MXFP8 or torch.equal(few.row_scale, many.row_scale[:T]))
+    assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, q.rows, W // per)[:T] for q in (few, many)))
