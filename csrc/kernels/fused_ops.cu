@@ -534,10 +534,12 @@ __global__ void __launch_bounds__(256) quant_rows16_kernel(const __nv_bfloat16* 
   quant_store16<MODE>(a, bm, valid, live ? t : 0, i, I, gs, q_out, sf_out, sf_col_tiles);
 }
 
-template <int CH>
+template <int QUANT, int CH>
 __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ residual,
                                                             const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out,
-                                                            int H, float eps, int zero_centered, int zero_src) {
+                                                            uint8_t* __restrict__ q_out, uint8_t* __restrict__ sf_out,
+                                                            float* __restrict__ row_scale, int H, float eps, int zero_centered,
+                                                            int sf_col_tiles, int zero_src) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[32];
@@ -573,6 +575,7 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
   }
   ss = block_reduce(ss, red, false);
   const float rstd = rsqrtf(ss / H + eps);
+  float amax = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (c * blockDim.x + threadIdx.x) * 8;
@@ -583,8 +586,21 @@ __global__ void __launch_bounds__(512) rmsnorm_reg_kernel(__nv_bfloat16* __restr
     for (int j = 0; j < 8; ++j) {
       const float wf = bf2f(ew[j]) + (zero_centered ? 1.f : 0.f);
       e[j] = __float2bfloat16(bf2f(e[j]) * rstd * wf);
+      if (QUANT) amax = fmaxf(amax, fabsf(bf2f(e[j])));
     }
-    if (i < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + i) = u[c];
+    if (QUANT == 0 && i < H) *reinterpret_cast<uint4*>(out + (size_t)t * H + i) = u[c];
+  }
+  if (QUANT == 0) return;
+  float g = 1.f;
+  if (QUANT == 1) {
+    amax = block_reduce(amax, red, true);
+    g = fmaxf(amax / (6.f * 448.f), 1e-30f);
+    if (threadIdx.x == 0) row_scale[t] = g;
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (c * blockDim.x + threadIdx.x) * 8;
+    quant_store8<QUANT>(u[c], i < H, t, i, H, g, q_out, sf_out, sf_col_tiles);
   }
 }
 
@@ -1146,7 +1162,7 @@ static inline void reg_shape(int W, int T, int* threads, int* chunks) {
   }
 
 // The quantising row kernels with 16 elements per thread: rows of up to 6 chunks of 256 threads.  At any number of rows where rows are
-// normed or are activations already (but for those of 513 - 1024, see there) (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norms, from
+// normed or are activations already (but for few long norms and few rows of 513 - 1024, see there) (us before / now: 8192 rows of 12288 activations, NVFP4, 77 / 46, 1 row 3.35 / 3.10; norms, from
 // cold caches, of 825 rows of 4096 14.3 / 12.3, 3000 of 5120 34.8 / 28.7, 2000 of 12320 76 / 49), for gated rows from 512 on (825 rows of 12288 19.8 / 17.1, 256 rows 7.6 / 8.3: their
 // activation is the longer chain per thread there; the experts' short gated rows likewise 43.7 / 46.2).
 constexpr int ROW16_MOST = 6 * 256 * 16;
@@ -1175,7 +1191,11 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
   const int ct = quant == 1 ? (H + 63) / 64 : (H + 127) / 128;
   int rt, ch;
   reg_shape(H, T, &rt, &ch);
-  if (quant && H <= ROW16_MOST) {
+  // Few long rows: the sums of rmsnorm_row16_kernel go by way of shared memory there, with two more barriers (us, 8 / 16 elements a
+  // thread: MXFP8 1 row of 5120 3.50 / 3.81, of 7168 3.50 / 4.00, 64 rows of 12288 4.51 / 5.12, 96 of 24576 7.42 / 8.01; NVFP4 16 rows of
+  // 4096 3.03 / 3.32, 1 of 12288 4.47 / 4.92; 150 rows of 5120 5.13 / 4.78, of 12288 6.84 / 6.42).  Few rows of two warps: see swiglu_impl.
+  const bool few = T <= 128 && (H >= 4096 || (H > 512 && H <= 1024));
+  if (quant && H <= ROW16_MOST && !few) {
     const int c16 = (H + 4095) / 4096;
     const size_t sm16 = c16 == 1 && H / 8 <= rt ? 0 : sm;          // (see rmsnorm_row16_kernel)
 #define BLZ_RN(C)                                                                                                              \
@@ -1185,10 +1205,12 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
 #undef BLZ_RN
     return (int)cudaGetLastError();
   }
-  if (!quant && ch) {
-#define BLZ_RN(C) launch_pdl(rmsnorm_reg_kernel<C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)out, H, eps, zero_centered, zero_src)
+  if (ch) {
+#define BLZ_RN2(Q, C) launch_pdl(rmsnorm_reg_kernel<Q, C>, dim3(T), dim3(rt), 0, s, (bf16*)x, (bf16*)residual, (const bf16*)w, (bf16*)out, (uint8_t*)q_out, (uint8_t*)sf_out, row_scale, H, eps, zero_centered, ct, zero_src)
+#define BLZ_RN(C) if (quant == 0) BLZ_RN2(0, C); else if (quant == 1) BLZ_RN2(1, C); else BLZ_RN2(2, C)
     BLZ_CH_SWITCH(ch, BLZ_RN)
 #undef BLZ_RN
+#undef BLZ_RN2
     return (int)cudaGetLastError();
   }
   if (quant == 0)

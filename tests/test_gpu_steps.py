@@ -654,3 +654,20 @@ def test_quantised_short_rows_of_few_elements(ops, mode, T, W):      # noqa: F81
     per = 16 if mode == Format.NVFP4 else 32
     assert torch.equal(few.data, many.data[:T]) and (mode == Format.MXFP8 or torch.equal(few.row_scale, many.row_scale[:T]))
     assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, q.rows, W // per)[:T] for q in (few, many)))
+
+
+@pytest.mark.parametrize("mode", [Format.NVFP4, Format.MXFP8])
+@pytest.mark.parametrize("W", [512, 544, 1024, 1056, 4064, 4096, 4128, 5120, 12320, 24576])
+def test_quantised_norm_of_few_rows(ops, mode, W):      # noqa: F811
+    """The most rows with 8 elements per thread, and one row more: the same residual, codes and scales."""
+    g = torch.Generator(device=DEV).manual_seed(16)
+    lin = Linear(mode, 128, W)
+    lin.act_quant = True
+    x, r = (torch.randn(129, W, generator=g, device=DEV).bfloat16() for _ in range(2))
+    x[0, 3], x[1, 5], r[2, 7] = float("inf"), float("nan"), float("-inf")
+    w, r1, r2 = (1 + 0.1 * torch.randn(W, generator=g, device=DEV)).bfloat16(), r.clone(), r[:128].clone()
+    many, few = ops.norm(x, r1, w, 1e-6, quant_for=lin)[0], ops.norm(x[:128].clone(), r2, w, 1e-6, quant_for=lin)[0]
+    per = 16 if mode == Format.NVFP4 else 32
+    assert torch.equal(r1[:128].view(torch.int16), r2.view(torch.int16)) and torch.equal(few.data, many.data[:128])
+    assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, q.rows, W // per)[:128] for q in (few, many)))
+    assert mode == Format.MXFP8 or torch.equal(few.row_scale.view(torch.int32), many.row_scale[:128].view(torch.int32))
