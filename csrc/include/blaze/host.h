@@ -26,15 +26,17 @@ inline cudaError_t encode_sf_tmap(CUtensorMap* out, const void* base, uint64_t r
   return encode_tmap(out, base, 4, 128, col_tiles, 512, 128, atoms, 0, row_tiles, col_tiles * 512, box_tiles);
 }
 
-// BLAZE_PDL=0 turns programmatic dependent launch off (every kernel then starts after its predecessor has finished).
-inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
+// Programmatic dependent launch by BLAZE_PDL: 0: every kernel starts after its predecessor has finished; unset: the products on CTA pairs
+// start before (pdl_pairs; see gemm_pair.cu); 1: so do all kernels of the pdl_trigger / pdl_wait protocol (pdl_enabled).
+inline int pdl_level() {
+  static const int level = [] {
     const char* e = getenv("BLAZE_PDL");
-    on = (e && e[0] == '1') ? 1 : 0;
-  }
-  return on != 0;
+    return !e || !e[0] ? 1 : e[0] == '1' ? 2 : 0;
+  }();
+  return level;
 }
+inline bool pdl_enabled() { return pdl_level() == 2; }
+inline bool pdl_pairs() { return pdl_level() >= 1; }
 
 // Launch a kernel that follows the pdl_trigger / pdl_wait protocol (sm100.cuh) so that its prologue — and, for the
 // GEMMs, the first weight tiles — overlap the tail of the kernel before it on the stream.

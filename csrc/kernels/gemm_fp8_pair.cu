@@ -332,7 +332,7 @@ static cudaError_t launch_fp8_pair(const CUtensorMap& tmW, const CUtensorMap& tm
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // the set-up beside the end of the kernel before (see gemm_pair.cu)
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl_pairs() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmS, p);
 }
 

@@ -507,7 +507,7 @@ static cudaError_t launch_pair(const CUtensorMap& tmW, const CUtensorMap& tmX, c
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = pdl_pairs() ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, tmSW, tmSX, p);
 }
 

@@ -1,6 +1,7 @@
 """Order of a kernel's ring buffers, from the waits in its source: a slot is read before it is filled again."""
 import os
 import re
+import subprocess
 
 SRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "csrc", "kernels", "gemm_fp8_block.cu")
 
@@ -79,3 +80,22 @@ def test_scales_of_a_pair_are_handed_back_by_the_warps_that_read_them():
     after = read[read.index("= sa[j];"):]
     assert after.index("__syncwarp();") < after.index("mbar_arrive(&sa_empty[slot]") < after.index("finish")
     assert read.count("sa[j]") == 1
+
+
+def test_programmatic_launch_has_one_switch(tmp_path):
+    """BLAZE_PDL: unset, the products on CTA pairs alone start before their predecessor has finished; 0, nothing does; 1, all may.  Every
+    launch with the attribute asks."""
+    prog = tmp_path / "level.cpp"
+    prog.write_text('#include "blaze/host.h"\n#include <stdio.h>\nint main() { printf("%d %d", blz::pdl_pairs(), blz::pdl_enabled()); }\n')
+    root = os.path.dirname(os.path.dirname(os.path.dirname(SRC)))
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I" + os.path.join(root, "csrc", "include"), "-I" + cuda, str(prog), "-o", str(tmp_path / "level")], check=True)
+    env = {k: v for k, v in os.environ.items() if k != "BLAZE_PDL"}
+    got = [subprocess.run([str(tmp_path / "level")], env={**env, **e}, capture_output=True, text=True).stdout for e in ({}, {"BLAZE_PDL": "0"}, {"BLAZE_PDL": "1"})]
+    assert got == ["1 0", "0 0", "1 1"]
+    folder = os.path.dirname(SRC)
+    for f in sorted(os.listdir(folder)):
+        text = open(os.path.join(folder, f)).read()
+        for at in re.finditer("cudaLaunchAttributeProgrammaticStreamSerialization", text):
+            near = text[max(0, at.start() - 600):at.start() + 1500]
+            assert "pdl_enabled()" in near or "pdl_pairs()" in near, f
