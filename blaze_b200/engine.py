@@ -487,7 +487,7 @@ class Engine:
     def _expert_limits(self) -> Set[int]:
         if self._limits is None:
             ops, moe = self.model.ops, [L.mlp for L in self.model.layers if getattr(L.mlp, "experts", None) is not None]
-            self._limits = {ops.moe_narrow_tokens(M.experts, M.top_k) for M in moe}
+            self._limits = set().union(*(ops.expert_limits(M.experts, M.top_k) for M in moe))
         return self._limits
 
     def _key_splits(self, n: int) -> int:

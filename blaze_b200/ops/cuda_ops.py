@@ -1451,11 +1451,30 @@ class CudaOps:
         return out
 
     def moe_narrow_tokens(self, experts, k: int) -> int:
-        """The most tokens of a step whose routed rows (``k`` per token) take the narrow expert kernel."""
+        """The most tokens of a step whose routed rows (``k`` per token) take the narrow expert kernel, where it is taken at all."""
         gu, rows = self.pack_experts(experts)["gate_up"], self.MOE_NARROW_ROWS
         if gu["kind"] == 2 and experts.count * gu["N"] >= 2048 * 128:
             rows = rows * 8 // 3
         return rows * experts.count // k
+
+    def _expert_form(self, experts, k: int, T: int) -> Tuple[bool, int]:
+        """How the routed experts of a step of ``T`` tokens are computed: whether by the narrow kernel, and the rows per tile on pairs of
+        CTAs, by the rows that an expert gets on average, since beyond them its weights are read again (0: no product takes pairs)."""
+        pk = self.pack_experts(experts)
+        gu, dn = pk["gate_up"], pk["down"]
+        narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
+        # The pair kernel beats the narrow one for block-scaled experts at any number of rows (us, both products of a layer, narrow / tiles
+        # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 102 / 145 / 94, 4096 278 / 264 / 147; MXFP8, 512
+        # experts of 1024 x 2048, 1 token 43 / 51 / 29, 256 313 / 575 / 307, 1024 322 / 580 / 313, 4096 428 / 580 / 352)
+        if gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2" and self.MOE_NARROW_ROWS < 1 << 20:
+            narrow = False
+        pairs = not narrow and experts.act != "relu2" and gu["kind"] in (0, 1, 2) and (gu["N"] % 256 == 0 or dn["N"] % 256 == 0)
+        return narrow, 0 if not pairs else 128 if T * k <= 96 * experts.count else 256
+
+    def expert_limits(self, experts, k: int) -> set:
+        """The most tokens of a step before its experts are computed in another form (:meth:`_expert_form`)."""
+        at = {self.moe_narrow_tokens(experts, k), 96 * experts.count // k}
+        return {T for T in at if self._expert_form(experts, k, T) != self._expert_form(experts, k, T + 1)}
 
     def moe_rows(self, x, topk_w, topk_id, experts, shared=None, gate=None) -> RoutedRows:
         """The routed experts' outputs as rows (:meth:`branch_norm` and :meth:`branch_step` sum them up, with ``shared`` added, there times
@@ -1474,8 +1493,8 @@ class CudaOps:
         max_tiles = (T * k + 127) // 128 + n_exp
         M_pad = max_tiles * 128
         dev = self.device
-        # rows per tile of the pair kernel by the rows that an expert gets on average: beyond them its weights are read again
-        run = 128 if T * k <= 96 * n_exp else 256
+        narrow, run = self._expert_form(experts, k, T)
+        run = run or 256
         # the plan in one allocation, its parts on 16 bytes
         n4, t4, n_runs = (n_exp + 3) // 4 * 4, (max_tiles + 3) // 4 * 4, T * k // run + n_exp + 1
         run_list, offsets, fill, tile_expert, tile_rows, row_map = torch.empty(
@@ -1483,12 +1502,6 @@ class CudaOps:
         runs, row_map = (run_list, run), row_map.view(T, k)
         self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(runs[0]), run, n_exp,
                                                max_tiles, self._stream()), "moe_plan")
-        narrow = T <= self.moe_narrow_tokens(experts, k) and gu["kind"] in (0, 1, 2) and gu["N"] % 128 == 0 and dn["N"] % 128 == 0
-        # The pair kernel beats the narrow one for block-scaled experts at any number of rows (us, both products of a layer, narrow / tiles
-        # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 102 / 145 / 94, 4096 278 / 264 / 147; MXFP8, 512
-        # experts of 1024 x 2048, 1 token 43 / 51 / 29, 256 313 / 575 / 307, 1024 322 / 580 / 313, 4096 428 / 580 / 352)
-        if gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2" and self.MOE_NARROW_ROWS < 1 << 20:
-            narrow = False
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)
         if mode:
             xq = self._quantize(x.contiguous(), mode)

@@ -671,3 +671,16 @@ def test_quantised_norm_of_few_rows(ops, mode, W):      # noqa: F811
     assert torch.equal(r1[:128].view(torch.int16), r2.view(torch.int16)) and torch.equal(few.data, many.data[:128])
     assert torch.equal(*(quant.unswizzle_sf_128x4(q.sf, q.rows, W // per)[:128] for q in (few, many)))
     assert mode == Format.MXFP8 or torch.equal(few.row_scale.view(torch.int32), many.row_scale[:128].view(torch.int32))
+
+
+@pytest.mark.parametrize("kind,E,N,D,k,want", [
+    (1, 128, 1536, 2048, 8, {1536}), (2, 512, 1024, 2048, 10, {4915}), (1, 64, 1408, 2048, 6, {512, 1024}), (0, 128, 1536, 2048, 8, {768, 1536}),
+    (1, 64, 1280, 1920, 6, {512, 1024}), (1, 64, 1408, 1920, 6, {512})])
+def test_where_experts_change_their_form(ops, kind, E, N, D, k, want):      # noqa: F811
+    """A step's experts are computed in one form up to each limit and in another beyond: pairs' rows per tile, and the narrow kernel where
+    it is taken."""
+    ex = _A()
+    ex.count, ex.act, ex.cuda_pack = E, "swiglu", {"gate_up": {"kind": kind, "N": N}, "down": {"kind": kind, "N": D}}
+    assert ops.expert_limits(ex, k) == want
+    forms = [ops._expert_form(ex, k, T) for T in range(1, 6000)]
+    assert {T for T in range(1, 5999) if forms[T - 1] != forms[T]} == want
