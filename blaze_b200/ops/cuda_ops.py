@@ -114,6 +114,12 @@ class CudaOps:
         self._sk_ok = os.environ.get("BLAZE_GEMM_SK", "1") != "0"
         self.SK_MAX_ROWS = 512
         self.tuning = None         # optional tune.Tuning: per-shape kernel choices measured on this device
+        # pairs of CTAs, unless BLAZE_GEMM_PAIR=0 or the context has no room for one
+        self._pair_ok = False
+        if hasattr(self.lib, "blz_pair_room"):
+            lib.blz_pair_room.restype, lib.blz_pair_room.argtypes = _c.c_int, [_c.c_int]
+            with torch.cuda.device(self.device):
+                self._pair_ok = self.lib.blz_pair_room(2) > 0
         lib.blz_gemm_pair.restype = _c.c_int
         lib.blz_gemm_pair.argtypes = [_c.c_int, VP, _c.c_longlong, VP, _c.c_longlong, VP, _c.c_longlong, _c.c_int, _c.c_int, _c.c_int,
                                       VP, VP, VP, VP, VP, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_int, _c.c_float, VP]
@@ -604,7 +610,7 @@ class CudaOps:
                     wide, bn, sk = False, hit["bn"], False
                 elif self._sk_ok and M <= self.SK_MAX_ROWS:
                     sk = hit["ks"]
-        pair = (wide is None and self._wide_ok and bn == 0 and kind in (0, 1, 2) and lin.N >= 128 and not kt and pending is None
+        pair = (wide is None and self._pair_ok and bn == 0 and kind in (0, 1, 2) and lin.N >= 128 and not kt and pending is None
                 and argmax_parts is None and max_ctas != 1 and not relu2 and (sk is None or sk is False)
                 and (f32 or (lin.N % 2 == 0 and ld_out % 2 == 0 and out.data_ptr() % 4 == 0)) and (not swiglu or lin.N % 32 == 0))
         # Pairs of CTAs stream a weight fastest (us of a call, NVFP4, one CTA per tile or K over a cluster / pairs, 1, 64, 256, 8192 rows:
@@ -1466,9 +1472,10 @@ class CudaOps:
         # The pair kernel beats the narrow one for block-scaled experts at any number of rows (us, both products of a layer, narrow / tiles
         # of 128 / pairs: NVFP4, 128 experts of 1536 x 2048, 1 token 41 / 39 / 24, 256 102 / 145 / 94, 4096 278 / 264 / 147; MXFP8, 512
         # experts of 1024 x 2048, 1 token 43 / 51 / 29, 256 313 / 575 / 307, 1024 322 / 580 / 313, 4096 428 / 580 / 352)
-        if gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2" and self.MOE_NARROW_ROWS < 1 << 20:
+        if (self._pair_ok and gu["kind"] in (1, 2) and gu["N"] % 256 == 0 and dn["N"] % 256 == 0 and experts.act != "relu2"
+                and self.MOE_NARROW_ROWS < 1 << 20):
             narrow = False
-        pairs = not narrow and experts.act != "relu2" and gu["kind"] in (0, 1, 2) and (gu["N"] % 256 == 0 or dn["N"] % 256 == 0)
+        pairs = self._pair_ok and not narrow and experts.act != "relu2" and gu["kind"] in (0, 1, 2) and (gu["N"] % 256 == 0 or dn["N"] % 256 == 0)
         return narrow, 0 if not pairs else 128 if T * k <= 96 * experts.count else 256
 
     def expert_limits(self, experts, k: int) -> set:
@@ -1494,13 +1501,13 @@ class CudaOps:
         M_pad = max_tiles * 128
         dev = self.device
         narrow, run = self._expert_form(experts, k, T)
-        run = run or 256
+        pairs, run = run > 0, run or 256
         # the plan in one allocation, its parts on 16 bytes
         n4, t4, n_runs = (n_exp + 3) // 4 * 4, (max_tiles + 3) // 4 * 4, T * k // run + n_exp + 1
         run_list, offsets, fill, tile_expert, tile_rows, row_map = torch.empty(
             4 * n_runs + 2 * n4 + 2 * t4 + T * k, dtype=torch.int32, device=dev).split((4 * n_runs, n4, n4, t4, t4, T * k))
-        runs, row_map = (run_list, run), row_map.view(T, k)
-        self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(runs[0]), run, n_exp,
+        runs, row_map = (run_list, run) if pairs else None, row_map.view(T, k)
+        self._check(self.lib.blz_moe_plan_runs(_ptr(counts), _ptr(offsets), _ptr(fill), _ptr(tile_expert), _ptr(tile_rows), _ptr(run_list), run, n_exp,
                                                max_tiles, self._stream()), "moe_plan")
         mode = 1 if (gu["fmt"] == Format.NVFP4 and gu["act_quant"]) else (2 if gu["kind"] == 2 else 0)
         if mode:

@@ -36,6 +36,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "blaze/glu.cuh"
 #include "blaze/host.h"
 #include "blaze/sm100.cuh"
@@ -535,8 +537,12 @@ static PairParams pair_params(int kind, int N, int K, void* C, long long ldc, co
 }
 
 // Clusters of `ctas` CTAs that run at the same time on the current device (whole within a GPC each; one CTA fits an SM, whatever the kind).
+// 0 for all with BLAZE_GEMM_PAIR=0: products then take the kernels of single CTAs, as in a context without room for a pair.  The number is
+// that of the first context that asks on a device.
 int pair_cluster_room(int ctas) {
-  static int cache[64][9] = {{0}};
+  static std::atomic<int> cache[64][9];
+  static const bool off = [] { const char* e = getenv("BLAZE_GEMM_PAIR"); return e && e[0] == '0'; }();
+  if (off) return 0;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || ctas < 2 || ctas > 8) return 0;
@@ -588,6 +594,9 @@ static void pair_shape(int kind, int M, int N, int K, int* cn, int* ks) {
 }
 
 }  // namespace blz
+
+// How many clusters of `ctas` CTAs (2 - 8) run at once on the current device; for 2: whether products can take pairs at all.
+BLZ_API int blz_pair_room(int ctas) { return blz::pair_cluster_room(ctas); }
 
 // C[M, N] = X[M, K] · W[N, K]^T with the operand conventions of blz_gemm_tc (ldx / ldw in BYTES, ldc in elements).  kind: 0 bf16,
 // 1 NVFP4, 2 MXFP8.  N even, or a multiple of 32 with act (bf16 out, [M, N/2]).  cn: tokens per tile, 64 / 128 / 192 / 256, and

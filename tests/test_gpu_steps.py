@@ -684,3 +684,57 @@ def test_where_experts_change_their_form(ops, kind, E, N, D, k, want):      # no
     assert ops.expert_limits(ex, k) == want
     forms = [ops._expert_form(ex, k, T) for T in range(1, 6000)]
     assert {T for T in range(1, 5999) if forms[T - 1] != forms[T]} == want
+
+
+_PAIRS_OFF = """
+import sys
+import torch
+from blaze_b200.linear import Linear
+from blaze_b200.ops.cuda_ops import CudaOps
+from blaze_b200.quant import Format
+from test_gpu_kernels import _experts
+off = sys.argv[2] == "off"
+ops = CudaOps("cuda:0")
+assert ops._pair_ok == (ops.lib.blz_pair_room(2) > 0) == (not off)
+g = torch.Generator(device="cuda:0").manual_seed(51)
+rand = lambda *s: torch.randn(*s, generator=g, device="cuda:0")      # noqa: E731
+out, launches = {}, ops.launches
+for f in (Format.DENSE, Format.NVFP4, Format.MXFP8, Format.FP8_BLOCK):
+    lin = Linear.from_dense(rand(768, 1024) * 0.05, f)
+    for M in (1, 64, 300):
+        out[f"{f} {M}"] = ops.linear(lin, rand(M, 1024).bfloat16())
+    gu = Linear.from_dense(rand(512, 1024) * 0.05, f)
+    out[f"{f} glu"] = ops.linear_swiglu(gu, rand(100, 1024).bfloat16())
+for f in (Format.DENSE, Format.NVFP4, Format.MXFP8):
+    for T in (5, 700):
+        ex = _experts(8, 256, 256, f, 9)
+        w, ids = ops.router_topk(rand(T, 8), 2, True, 0, 8)
+        out[f"experts {f} {T}"] = ops.moe(rand(T, 256).bfloat16(), w, ids, ex)
+torch.cuda.synchronize()
+assert ops.take_status() == 0
+torch.save(out, sys.argv[1])
+"""
+
+
+def test_products_without_pairs_of_ctas(tmp_path):
+    """BLAZE_GEMM_PAIR=0, or a context without room for a pair: every product, FP8 and experts too, takes the kernels of single CTAs."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    for name, env in (("on", {}), ("off", {"BLAZE_GEMM_PAIR": "0"})):
+        path = os.pathsep.join([os.path.dirname(here), here])
+        subprocess.run([sys.executable, "-c", _PAIRS_OFF, str(tmp_path / name), name], env={**os.environ, "PYTHONPATH": path, **env}, check=True, timeout=300)
+    on, off = (torch.load(tmp_path / n) for n in ("on", "off"))
+    for k, v in on.items():
+        assert _rel(off[k], v) < 2e-3, k           # (K in other parts; a sum may round to the neighbouring bf16)
+
+
+def test_fp8_rows_without_pairs_of_ctas(tmp_path):
+    """The FP8 product of few rows with K over a cluster is what calls take where no pair fits."""
+    import os
+    import subprocess
+    import sys
+    run = [sys.executable, "-m", "pytest", "-q", "-x", os.path.abspath(__file__), "-k", "test_fp8_block_product_of_few_rows"]
+    got = subprocess.run(run, env={**os.environ, "BLAZE_GEMM_PAIR": "0"}, capture_output=True, text=True, timeout=300)
+    assert got.returncode == 0 and " passed" in got.stdout, got.stdout[-2000:]
