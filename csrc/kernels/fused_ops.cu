@@ -1130,17 +1130,19 @@ __global__ void argmax_parts_kernel(const float* __restrict__ val, const int* __
 using namespace blz;
 typedef __nv_bfloat16 bf16;
 
-static void configure_once() {
-  static bool attr = false;
-  if (attr) return;
-  cudaFuncSetAttribute(swiglu_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(swiglu_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(rmsnorm_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(rmsnorm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(rmsnorm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(rmsnorm_row16_kernel<1, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  cudaFuncSetAttribute(rmsnorm_row16_kernel<2, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-  attr = true;
+// Rows of more than 40 KB (beyond 20480 elements) in shared memory, on any device of the process.
+static cudaError_t allow_smem(size_t bytes) {
+  if (bytes <= 40 * 1024) return cudaSuccess;
+  static PerDeviceOnce once[7];
+  constexpr int MOST = 100 * 1024;
+  cudaError_t e = once[0].smem_limit(swiglu_kernel<1>, MOST);
+  if (e == cudaSuccess) e = once[1].smem_limit(swiglu_kernel<2>, MOST);
+  if (e == cudaSuccess) e = once[2].smem_limit(rmsnorm_kernel<0>, MOST);
+  if (e == cudaSuccess) e = once[3].smem_limit(rmsnorm_kernel<1>, MOST);
+  if (e == cudaSuccess) e = once[4].smem_limit(rmsnorm_kernel<2>, MOST);
+  if (e == cudaSuccess) e = once[5].smem_limit(rmsnorm_row16_kernel<1, 6>, MOST);
+  if (e == cudaSuccess) e = once[6].smem_limit(rmsnorm_row16_kernel<2, 6>, MOST);
+  return e;
 }
 
 // threads and chunks per thread of the register-resident row kernels; chunks == 0: width not covered
@@ -1185,9 +1187,9 @@ BLZ_API int blz_rmsnorm(void* x, void* residual, const void* w, void* out, void*
                         float* row_scale, int T, int H, float eps, int zero_centered, int quant, int zero_src, cudaStream_t s) {
   if (H % 32 || T < 0) return (int)cudaErrorInvalidValue;
   if (T == 0) return 0;
-  configure_once();
   const int thr = norm_threads(H);
   const size_t sm = (size_t)H * 2;
+  if (cudaError_t e = allow_smem(sm)) return (int)e;
   const int ct = quant == 1 ? (H + 63) / 64 : (H + 127) / 128;
   int rt, ch;
   reg_shape(H, T, &rt, &ch);
@@ -1242,8 +1244,8 @@ static int swiglu_impl(const void* gu, void* out, void* q_out, void* sf_out, flo
   if (T == 0) return 0;
   const int thr = norm_threads(I);
   const size_t sm = (size_t)I * 2;
+  if (cudaError_t e = allow_smem(sm)) return (int)e;
   const int ct = mode == 1 ? (I + 63) / 64 : (I + 127) / 128;
-  configure_once();
   {
     // Two warps of 16 elements a thread lose to three or four of 8 while all rows are few (us, 8 / 16 elements a thread: NVFP4 4 rows of 768
     // 2.40 / 2.76, 512 rows 2.44 / 2.90, 1024 rows 2.74 / 2.93, 4 rows of 1024 2.22 / 2.48, 150 rows 2.52 / 2.74; MXFP8 4 rows of 768

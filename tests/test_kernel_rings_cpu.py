@@ -99,3 +99,13 @@ def test_programmatic_launch_has_one_switch(tmp_path):
         for at in re.finditer("cudaLaunchAttributeProgrammaticStreamSerialization", text):
             near = text[max(0, at.start() - 600):at.start() + 1500]
             assert "pdl_enabled()" in near or "pdl_pairs()" in near, f
+
+
+def test_kernel_attributes_are_set_for_every_device():
+    """A limit of shared memory that is set for the process's first device only does not hold on its second."""
+    folder = os.path.dirname(SRC)
+    host = open(os.path.join(os.path.dirname(folder), "include", "blaze", "host.h")).read()
+    once = host[host.index("struct PerDeviceOnce"):]
+    assert host.count("cudaFuncSetAttribute(") == 1 and once.index("done[dev]") < once.index("cudaFuncSetAttribute(") < once.index("\n};")
+    for f in sorted(os.listdir(folder)):
+        assert "cudaFuncSetAttribute(" not in open(os.path.join(folder, f)).read(), f
