@@ -647,7 +647,7 @@ class CudaOps:
                                                self._stream()), f"gemm_pair kind {kind}")
             return out
         if wide is None:
-            # what the pairs do not take (tile-major weights, one CTA at most): 256-feature tiles for block-scaled kinds, the swapped
+            # what the pairs do not take (tile-major weights, one CTA at most, no room for a pair): 256-feature tiles for block-scaled kinds, the swapped
             # orientation for a very wide bf16 head, which fetches each weight once
             wide = self._wide_ok and bn == 0 and ((M <= 256 and kind == 0 and lin.N >= 32768 and not swiglu)
                                                   or (kind in (1, 2) and lin.N % 256 == 0 and M > 256))

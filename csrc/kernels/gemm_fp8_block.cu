@@ -15,7 +15,8 @@
 // warp per scheduler the tensor pipe sat at 32 % and the FMA pipe at 19 %).  Every wait is a bounded mbarrier wait that
 // reports through the status word.  No TMA load is cluster-multicast.
 //
-// Both kernels here are what calls take that gemm_fp8_pair.cu does not (see blz_gemm_fp8_block).
+// Both products here are what calls take that gemm_fp8_pair.cu does not (see blz_gemm_fp8_block): this one where the token scales are off 16
+// bytes, and where no pair fits the context or pairs are off (BLAZE_GEMM_PAIR=0), the one of few rows below among them.
 //
 // Reference counterpart: the FP8 block-scale linear of kernels/src/cuda/fp8_linear.cu (fp8_block_* kernels: dequantise to
 // bf16 and run a bf16 GEMM, or 1x128-quantised activations with per-block fp32 rescale on mma.sync), routed from

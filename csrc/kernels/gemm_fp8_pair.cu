@@ -13,7 +13,9 @@
 // Against one CTA per 128 x 128 tile, and one or a cluster of CTAs per 128 features up to 64 rows (us, inputs from memory): 64 rows x 10240 x
 // 5120 24.8 -> 17.2, x 5120 x 8192 23.9 -> 16.6, x 51200 x 5120 76 -> 58, x 5120 x 25600 47 -> 37; 128 rows of those 27 -> 19.5, 32 ->
 // 19.6, 78 -> 61, 88 -> 43; 1000 rows 89 -> 71, 80 -> 65, 357 -> 298, 252 -> 190; 4096 rows 292 -> 244, 223 -> 188, 1345 -> 1330,
-// 775 -> 629.  (With one block per stage 1000 rows x 51200 x 5120 took 380; loads of the next partials ahead of the sums spill.)
+// 775 -> 629.  (With one block per stage 1000 rows x 51200 x 5120 took 380.  The forms of 128 tokens, 18 warps, have 96 registers a thread
+// and spill 20 and, split, 44 bytes; loads of the next partials ahead of the sums spill more.)  A slot that is released with the next
+// step's buffer instead of a barrier of its own holds the producer up: 64 rows x 10240 x 5120 15.3 -> 16.3, 16 x 5120 x 25600 30.7 -> 35.6.
 //
 // Few tiles: K is split over the pairs of a cluster, which exchange their sums through distributed shared memory as in gemm_pair.cu.
 // Every wait is bounded; no load is multicast.

@@ -96,7 +96,8 @@ struct PairCfg {
   static_assert(SF_COLS <= 64, "the accumulators may share two chunks of 32 columns at most");
 };
 
-// (x * s) * a + b of two neighbours at once, each rounded as by fmaf(x * s, a, b)
+// (x * s) * a + b of two neighbours at once, each rounded as by fmaf(x * s, a, b): token scale first, as in gemm_tc.cu; the narrow kernel
+// of moe_gemm.cu multiplies by the feature's first, which may round the other way
 __device__ __forceinline__ void scale_pair(uint32_t x0, uint32_t x1, float s0, float s1, float a, float b, float& y0, float& y1) {
   asm("{\n\t.reg .b64 x, s, a, b;\n\t"
       "mov.b64 x, {%2, %3};\n\tmov.b64 s, {%4, %5};\n\tmov.b64 a, {%6, %6};\n\tmov.b64 b, {%7, %7};\n\t"

@@ -2,8 +2,8 @@
 //     C[M,N] = (A[M,K] · B[N,K]^T) * row_scale[m] * alpha[n] (+ bias[n]),  bf16 output
 // for the same four operand kinds as gemm_tc.cu (0 bf16, 1 NVFP4, 2 MXFP8, 3 FP8).
 //
-// Taken where a tuning table or the caller asks for it, and in place of gemm_tc.cu where gemm_pair.cu is not taken (FP8 weights with one
-// scale per feature): K long and tiles few.  At decode sizes (M <= 256 rows) a GEMM has only a few dozen 128x128 output tiles, so a kernel with
+// Taken where the caller asks for it or a tuning table says that it beat what the rules pick, and in place of gemm_tc.cu where gemm_pair.cu is
+// not taken (FP8 weights with one scale per feature; contexts without room for a pair): K long and tiles few.  At decode sizes (M <= 256 rows) a GEMM has only a few dozen 128x128 output tiles, so a kernel with
 // one CTA per tile leaves a third of the 148 SMs idle and each busy SM pulls its tile's whole K range through its own
 // L2 port (measured ~90 GB/s per SM): the time follows bytes per SM, not bytes per GPU.  Here every output tile is
 // computed by a cluster of `ks` CTAs, each streaming 1/ks of the K range into its own TMEM accumulator; the partial

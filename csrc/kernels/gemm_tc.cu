@@ -7,8 +7,8 @@
 //
 // One persistent CTA per SM, 192 threads: warp 0 = TMA producer, warp 1 = MMA issuer (one elected lane,
 // owns the TMEM allocation), warps 2-5 = epilogue (one TMEM lane quadrant each).  Operands are staged in
-// 128B-swizzled shared memory by TMA tensor loads (never multicast); scale factors arrive by 1-D bulk
-// copies in the 128x4 tiled layout and are moved to tensor memory with tcgen05.cp; accumulators live in
+// 128B-swizzled shared memory by TMA tensor loads (never multicast); scale factors arrive by tensor maps of
+// their 128x4 tiles (host.h) and are moved to tensor memory with tcgen05.cp; accumulators live in
 // TMEM, double-buffered so the epilogue of tile i overlaps the main loop of tile i+1.
 //
 // Covers what the reference spreads over kernels/src/cuda/nvfp4_gemm.cu (w4a4_kernel :114, sm_120a-only

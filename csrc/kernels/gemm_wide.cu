@@ -1,5 +1,5 @@
-// Wide-N GEMM on tcgen05 by single CTAs, for what gemm_pair.cu does not take (tile-major weights, one CTA at most, or a caller that
-// insists): one 128-row operand tile against up to 256 rows of the other operand per MMA, so that each
+// Wide-N GEMM on tcgen05 by single CTAs, for what gemm_pair.cu does not take (tile-major weights, one CTA at most, contexts without room
+// for a pair, or a caller that insists): one 128-row operand tile against up to 256 rows of the other operand per MMA, so that each
 // instruction reads 1.5 shared-memory bytes per accumulator column instead of 2 — the 4-bit kinds are otherwise bound by
 // shared-memory reads, not by the tensor pipe — and each scale-factor copy is amortised over twice the math.
 //

@@ -10,9 +10,10 @@
 //
 // Epilogue variants: plain bf16 rows, or (act = 1) SwiGLU on a weight whose rows are interleaved [16 gate | 16 up]: the
 // gate and up value of one feature sit 16 lanes apart in the same warp, one shuffle joins them and the [rows, 2I]
-// intermediate never reaches memory.
+// intermediate never reaches memory.  (Half of a warp's lanes store then, and all work on the activation: block-scaled experts, whose
+// activations are quantised in a pass of their own anyway, store gate and up sums instead and leave the activation to that pass.)
 //
-// The same kernel serves dense layers of few rows that the pairs do not take (squared ReLU, fewer than 128 features):
+// The same kernel serves dense layers of few rows that the pairs do not take (squared ReLU; all where no pair fits the context):
 // tile_expert = null means one "expert" whose rows are the whole activation matrix.  Few rows mean few feature tiles and a
 // long K range per tile, so the K range can be split over a thread-block cluster of `ks` CTAs: each streams 1/ks of the
 // weights of its feature tile, and the fp32 partials (128 features x 32..128 rows, a few KB) meet in distributed shared
