@@ -475,7 +475,8 @@ class Engine:
         that fill a step up are computed and routed like the others, and what such a step replaces was not padded, only launched one
         by one: with powers of two alone 65 sequences would compute 128 rows, and five take up to a fifth more experts' weights.  The
         kernels choose their forms at multiples of 64 rows and, for experts, at the row limits below; up to 1024 rows no bucket holds
-        such a limit inside, so a step's form does not depend on its padding either.  Per step, us, launched one by one / replayed in these buckets / in powers of two, contexts of 300 - 600:
+        such a limit inside, so a step's form does not depend on its padding either.  (The quantisers change theirs anywhere, to the same
+        bits.)  Per step, us, launched one by one / replayed in these buckets / in powers of two, contexts of 300 - 600:
         12 layers of the 8B shape, NVFP4: 5 sequences 1968 / 1276 / 1322, 65: 2306 / 1579 / 1606, 257: 3700 / 2740 / 3056; in bf16 65:
         2475 / 2247 / 2278, 257: 4030 / 3713 / 4358; 6 layers with 128 experts, NVFP4: 5: 1704 / 878 / 911, 129: 2543 / 1294 / 1480, 257:
         3412 / 1717 / 1968."""
