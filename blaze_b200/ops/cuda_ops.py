@@ -1559,7 +1559,7 @@ class CudaOps:
                 else:
                     self._grouped_gemm(w, src, M_pad, tile_expert, n_exp, dst, act=3 if dst is g else 0)
             return RoutedRows(y, row_map, weights, shared, gate)
-        proxy_d = Linear(dn["fmt"], dn["N"], dn["K"])
+        proxy_d = Linear(Format.MXFP8 if dn["kind"] == 2 else dn["fmt"], dn["N"], dn["K"])      # (FP8 blocks are packed as MXFP8)
         proxy_d.act_quant = dn["act_quant"]
         y = torch.empty(M_pad, dn["N"], dtype=torch.bfloat16, device=dev)
         def product(w, src, dst, act=0):

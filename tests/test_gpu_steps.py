@@ -738,3 +738,17 @@ def test_fp8_rows_without_pairs_of_ctas(tmp_path):
     run = [sys.executable, "-m", "pytest", "-q", "-x", os.path.abspath(__file__), "-k", "test_fp8_block_product_of_few_rows"]
     got = subprocess.run(run, env={**os.environ, "BLAZE_GEMM_PAIR": "0"}, capture_output=True, text=True, timeout=300)
     assert got.returncode == 0 and " passed" in got.stdout, got.stdout[-2000:]
+
+
+@pytest.mark.parametrize("T,I", [(5, 256), (300, 256), (40, 192)])
+def test_experts_stored_in_fp8_blocks(ops, T, I):      # noqa: F811
+    """Experts with 128 x 128 block scales, which are packed as MXFP8, by the pairs and by the narrow product: the stored weights' result,
+    within what both formats' 3-bit mantissas leave (2^-4 at most per weight and per activation)."""
+    ex = _experts(8, 256, I, Format.FP8_BLOCK, 9)
+    g = torch.Generator(device=DEV).manual_seed(18)
+    x = torch.randn(T, 256, generator=g, device=DEV).bfloat16()
+    w, ids = ops.router_topk(torch.randn(T, 8, generator=g, device=DEV), 2, True, 0, 8)
+    out = ops.moe(x, w, ids, ex)
+    torch.cuda.synchronize()
+    assert ops.take_status() == 0
+    assert _rel(out, ref.moe_forward(x, w, ids, ex.forward_one, 8)) < 0.08
